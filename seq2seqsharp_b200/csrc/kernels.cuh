@@ -378,6 +378,9 @@ struct LatentArgs {
 };
 int latent_pick_splits(DeviceState* st, const LatentShape& a, int B, int S, int T);
 bool latent_expanded(int dtype, const LatentShape& a, int q_stride, int S);
+// the expanded form's attention on tcgen05 (attn_prefill_tc.cu): bf16, rows of whole 64-column boxes
+bool latent_prefill_tc_shape(int dtype, const LatentShape& a);
+int launch_latent_prefill_tc(int device, const LatentArgs& a, cudaStream_t s);
 int launch_latent_attention(int device, DeviceState* st, int dtype, const LatentArgs& a, cudaStream_t s);
 // ---- grouped-query attention with a window, a distance bias, a sink and gated heads (ops_grouped.cu) ------------------------
 struct GroupedShape {
@@ -444,6 +447,9 @@ int launch_matrix_memory(int device, DeviceState* st, int dtype, const MemoryArg
 int init_tc_attrs(int device);
 int tc_take_error();
 int64_t linear_workspace_bytes(int M, int K, int N);
+// causal prompt attention of fp16 rows, head size 64 / 128, 1 / 2 / 4 / 8 query heads per KV head (attn_prefill_tc.cu)
+int launch_attn_prefill_tc(int device, void* out, const void* q, int64_t q_rs, const void* cK, const void* cV, int B, int S, int H, int Hkv, int hd, int T0,
+                           int Tmax, float scale, cudaStream_t s);
 int launch_attention(int device, DeviceState* st, int dtype, void* out, const void* q, int64_t q_rs, const void* cK,
                      const void* cV, int B, int S, int H, int Hkv, int hd, int T0, const int* dT0, int Tmax, int splits_hint,
                      void* ws, int64_t ws_bytes, cudaStream_t s);

@@ -1008,6 +1008,8 @@ int launch_latent_attention(int device, DeviceState* st, int dtype, const Latent
     ep.y = a.kv;
     ep.act = TSB200_ACT_NONE;
     TSB_TRY(launch_linear(device, st, dtype, rows, a.ukv_packed, a.B * T, sh.row, kvw, ep, a.lin_ws, a.lin_ws_bytes, s, true));
+    if (latent_prefill_tc_shape(dtype, sh) && (((uintptr_t)a.q | (uintptr_t)a.kv | (uintptr_t)a.cache) % 16) == 0 && a.seq_stride % 8 == 0)
+      return launch_latent_prefill_tc(device, a, s);
     const int qk = (sh.dim + sh.rot + 15) / 16 * 16, vn = latent_vn(sh.vdim);
     const size_t smem = latent_prefill_smem(qk, vn);
     const dim3 grid((a.S + kLpRows - 1) / kLpRows, sh.H, a.B);
