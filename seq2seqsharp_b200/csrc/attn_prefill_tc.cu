@@ -37,6 +37,7 @@ struct PaArgs {
   int k_boxes;                               // 64-column boxes of a key that mapK holds; the others come from mapR
   int kx, vx, vx0, rx;                       // column of a head's keys / values: head * kx, vx0 + head * vx; of the shared key part: rx
   int z_seq, z_head;                         // outermost coordinate of mapK / mapV: b * z_seq + head * z_head
+  const int* starts;                         // packed rows: first row of every sequence (B + 1), or NULL: S rows each
   int vec_out;                               // out is 16-byte aligned
   int* error;
 };
@@ -164,12 +165,14 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
   // the longest key ranges start first, over all sequences and heads
   const int kvh = (int)(blockIdx.x % a.heads), b = (int)((blockIdx.x / a.heads) % a.B);
   const int q0 = (a.tiles - 1 - (int)(blockIdx.x / a.heads / a.B)) * 2 * a.QT;
+  const int row0 = a.starts ? a.starts[b] : b * a.S, S = a.starts ? a.starts[b + 1] - row0 : a.S;
+  if (q0 >= S) return;   // a shorter sequence
   // key tiles of the two row tiles: up to the last query that exists; the second may have no query at all
   int n_of[2];
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int first = q0 + t * a.QT, last = min(a.S, first + a.QT) - 1;
-    n_of[t] = first < a.S ? (a.T0 + last + kPaKeys) / kPaKeys : 0;
+    const int first = q0 + t * a.QT, last = min(S, first + a.QT) - 1;
+    n_of[t] = first < S ? (a.T0 + last + kPaKeys) / kPaKeys : 0;
   }
   const int n_tiles = max(n_of[0], n_of[1]);
 
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
       for (int t = 0; t < 2; ++t) {
         if (n_of[t] == 0) continue;
         tc_mbar_expect_tx(&q_full[t], QB * kPaBox);
-        for (int i = 0; i < QB; ++i) pa_load_4d(sQ + (t * QB + i) * kPaBox, &mapQ, 64 * i, kvh * a.G, q0 + t * a.QT, b, &q_full[t]);
+        for (int i = 0; i < QB; ++i) pa_load_4d(sQ + (t * QB + i) * kPaBox, &mapQ, 64 * i, kvh * a.G, (a.starts ? row0 : 0) + q0 + t * a.QT, a.starts ? 0 : b, &q_full[t]);
       }
       const int z = b * a.z_seq + kvh * a.z_head;
       int ks = 0, vs = 0;   // tiles asked for so far
@@ -293,7 +296,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
     pa_more_registers<kPaSoftmaxRegs>();
     const int t = w >> 2, row = tid & 127, n = t ? n_of[1] : n_of[0];
     const int pos = q0 + t * a.QT + row / a.G, head = kvh * a.G + row % a.G;
-    const bool live = pos < a.S;
+    const bool live = pos < S;
     const int lim = live ? a.T0 + pos + 1 : 0x7fffffff;                            // keys [0, lim) are visible (a row without a query: zeros, never stored)
     const int warp_lim = a.T0 + q0 + t * a.QT + (row & ~31) / a.G + 1;             // the smallest of the warp
     const uint32_t lanes = (uint32_t)((w & 3) * 32) << 16;
@@ -367,7 +370,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
     if (n > 0 && ok && __all_sync(0xffffffffu, pa_wait(&o_full[t], 0, err))) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inv = l > 0.0f ? 1.0f / l : 0.0f;
-      H* out = reinterpret_cast<H*>(a.out) + (((int64_t)b * a.S + pos) * a.H + head) * (VB * 64);
+      H* out = reinterpret_cast<H*>(a.out) + (((int64_t)row0 + pos) * a.H + head) * (VB * 64);
 #pragma unroll 1
       for (int q = 0; q < VB * 2; ++q) {
         uint32_t o[32];
@@ -442,13 +445,14 @@ static int pa_launch(int device, const CUtensorMap& q, const CUtensorMap& k, con
 }
 
 int launch_attn_prefill_tc(int device, void* out, const void* q, int64_t q_rs, const void* cK, const void* cV, int B, int S, int H, int Hkv, int hd, int T0,
-                           int Tmax, float scale, cudaStream_t s) {
+                           int Tmax, float scale, const PackedRows* pack, cudaStream_t s) {
   PaArgs a{};
+  a.starts = pack ? pack->starts : nullptr;
   a.out = out; a.B = B; a.S = S; a.T0 = T0; a.H = H; a.heads = Hkv; a.G = H / Hkv; a.QT = kPaRows / a.G;
   a.c = scale * 1.44269504088896340736f;
   a.k_boxes = hd / 64; a.z_seq = Hkv; a.z_head = 1;
   CUtensorMap mq, mk, mv;
-  TSB_TRY(pa_map_q(&mq, TSB200_F16, q, hd, H, S, B, q_rs, a.G));
+  TSB_TRY(pa_map_q(&mq, TSB200_F16, q, hd, H, pack ? pack->rows : S, pack ? 1 : B, q_rs, a.G));
   TSB_TRY(pa_map_rows(&mk, TSB200_F16, cK, hd, T0 + S, B * Hkv, hd, (int64_t)Tmax * hd));
   TSB_TRY(pa_map_rows(&mv, TSB200_F16, cV, hd, T0 + S, B * Hkv, hd, (int64_t)Tmax * hd));
   if (hd == 64) return pa_launch<__half, 1, 1, 4, 4>(device, mq, mk, mk, mv, a, s);

@@ -44,15 +44,15 @@ int chk_take_engine() { return 0; }
 template <typename T>
 __global__ void embed_kernel(float* x, const T* E, const T* PE, const int* ids,
                              int rows, int S, int d, int V, float sf, int pe_mode, int pe_rows, int T0_arg,
-                             const int* dT0) {
+                             const int* dT0, const int2* where) {
   pdl_trigger();
   pdl_wait();
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     int id = ids[r];
     TSB_DEV_CHECK(engine, id >= 0 && id < V, 0x101, (void)0)          // token id outside the vocabulary (the row is embedded as id 0)
     if (id < 0 || id >= V) id = 0;
-    const int s = r % S;
-    const int T0 = state_len(dT0, r / S, T0_arg);
+    const int s = where ? where[r].y : r % S;
+    const int T0 = state_len(dT0, where ? where[r].x : r / S, T0_arg);
     int pos = (pe_mode == 1) ? s : T0 + s;  // pe_mode 1: the reference peeks APE rows [0, S) (PositionEmbedding.cs:30-33)
     TSB_DEV_CHECK(engine, pe_mode == 0 || pos < pe_rows, 0x102, (void)0)   // position beyond the position table (clamped)
     if (pos >= pe_rows) pos = pe_rows - 1;
@@ -66,9 +66,15 @@ __global__ void embed_kernel(float* x, const T* E, const T* PE, const int* ids,
   }
 }
 
-// last prompt row of every sequence; `lens` (device, or NULL): prompts of different lengths padded to S columns
-__global__ void gather_last_kernel(float* xl, const float* x, int B, int S, int d, const int* lens) {
+// last prompt row of every sequence; `lens` (device, or NULL): prompts of different lengths padded to S columns;
+// `starts` (device, or NULL): prompts of different lengths one after the other
+__global__ void gather_last_kernel(float* xl, const float* x, int B, int S, int d, const int* lens, const int* starts) {
   for (int b = blockIdx.x; b < B; b += gridDim.x) {
+    if (starts) {
+      const int64_t row = starts[b + 1] - 1;
+      for (int i = threadIdx.x; i < d; i += blockDim.x) xl[(int64_t)b * d + i] = x[row * d + i];
+      continue;
+    }
     int last = lens ? lens[b] - 1 : S - 1;
     last = last < 0 ? 0 : (last >= S ? S - 1 : last);
     for (int i = threadIdx.x; i < d; i += blockDim.x) xl[(int64_t)b * d + i] = x[((int64_t)b * S + last) * d + i];
@@ -235,6 +241,7 @@ struct Gpt {
   bool force_per_seq = false;  // keep the per-sequence state in use even while the sequences agree (TSB200_GptSetPerSequenceState)
   int stop_fin = 0;            // per-sequence stop rule in the captured step (ragged decode with stop_on_eos)
   int seq0 = 0;                // first sequence the per-sequence buffers address (a single-slot prompt run), else 0
+  PackedRows pack;                    // rows > 0 during a prefill whose prompts of different lengths lie one after the other
   const int* gather_lens = nullptr;   // device prompt lengths of a padded prefill (NULL: every prompt fills its S columns)
   bool probs_valid = false;
   // graph
@@ -913,7 +920,9 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
   NvtxRange nvtx_(S == 1 ? "tsb200.forward.step" : "tsb200.forward.prompt");
   PdlScope pdl_scope(g->pdl && S == 1);
   const TSB200GptConfig& c = g->c;
-  const int dev = c.device, dt = c.dtype, d = c.d, rows = B * S;
+  const int dev = c.device, dt = c.dtype, d = c.d;
+  const PackedRows* pack = g->pack.rows > 0 ? &g->pack : nullptr;
+  const int rows = pack ? pack->rows : B * S;
   const int* dT = use_state ? g->state : nullptr;
   const int Hd = c.H * c.hd, KVd = c.Hkv * c.hd;
   const int pe_mode = (c.pe_type == 1) ? (c.ape_decode_pos0 ? 1 : 2) : 0;
@@ -923,9 +932,9 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     const int gsz = rows < g->st->sm_count * 8 ? rows : g->st->sm_count * 8;
     const int* ids = (S == 1 && use_state) ? g->ids_cur : g->ids_in;
     if (dt == TSB200_F32)
-      TSB_CUDA(launch_k(embed_kernel<float>, dim3(gsz), dim3(256), 0, g->s, g->x, (const float*)g->E, (const float*)g->PE, ids, rows, S, d, c.V, sf, pe_mode, g->pe_rows, T0, dT));
+      TSB_CUDA(launch_k(embed_kernel<float>, dim3(gsz), dim3(256), 0, g->s, g->x, (const float*)g->E, (const float*)g->PE, ids, rows, S, d, c.V, sf, pe_mode, g->pe_rows, T0, dT, pack ? pack->where : nullptr));
     else
-      TSB_CUDA(launch_k(embed_kernel<__half>, dim3(gsz), dim3(256), 0, g->s, g->x, (const __half*)g->E, (const __half*)g->PE, ids, rows, S, d, c.V, sf, pe_mode, g->pe_rows, T0, dT));
+      TSB_CUDA(launch_k(embed_kernel<__half>, dim3(gsz), dim3(256), 0, g->s, g->x, (const __half*)g->E, (const __half*)g->PE, ids, rows, S, d, c.V, sf, pe_mode, g->pe_rows, T0, dT, pack ? pack->where : nullptr));
     count_launch(dev);
     prof_end(g, KC_EMBED);
     TSB_TRY(check_launch("embed"));
@@ -985,9 +994,9 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     }
     if (!appended) {
       TSB_TRY(engine_linear(g, rows, nullptr, g->x, L.n1_g, L.n1_b, g->h, L.wqkv, d, g->Nqkv, make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0)));
-      PROF(KC_ROPE_APPEND, launch_rope_append(dev, g->st, dt, qp, kp, vp, g->Nqkv, g->Nqkv, L.cK, L.cV, B, S, c.H, c.Hkv, c.hd, T0, dT, c.max_tokens, c.pe_type == 2, (double)c.rope_base, g->rope_tab, g->s));
+      PROF(KC_ROPE_APPEND, launch_rope_append(dev, g->st, dt, qp, kp, vp, g->Nqkv, g->Nqkv, L.cK, L.cV, B, S, c.H, c.Hkv, c.hd, T0, dT, c.max_tokens, c.pe_type == 2, (double)c.rope_base, g->rope_tab, g->s, pack));
     }
-    PROF(KC_ATTENTION, launch_attention(dev, g->st, dt, g->attn, qp, g->Nqkv, L.cK, L.cV, B, S, c.H, c.Hkv, c.hd, T0, dT, c.max_tokens, splits, g->attn_ws, g->attn_ws_bytes, g->s));
+    PROF(KC_ATTENTION, launch_attention(dev, g->st, dt, g->attn, qp, g->Nqkv, L.cK, L.cV, B, S, c.H, c.Hkv, c.hd, T0, dT, c.max_tokens, splits, g->attn_ws, g->attn_ws_bytes, g->s, pack));
     TSB_TRY(row_parallel_linear(g, rows, g->attn, L.wo, Hd, L.bo));
     if (c.cross_attn) {
       // x += W0 (softmax(Q K^T / sqrt(hd)) V) + b0 with Q from the normed stream, K / V the encoder rows prepared by
@@ -1018,7 +1027,7 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     return engine_linear(g, g->n_want, nullptr, g->want_x, g->nf_g, g->nf_b, g->want_h, g->head_w, d, c.V, make_ep(g->head_b, nullptr, nullptr, g->want_logits, TSB200_ACT_NONE, 0));
   }
   if (S > 1) {
-    gather_last_kernel<<<B, 256, 0, g->s>>>(g->xl, g->x, B, S, d, g->gather_lens);
+    gather_last_kernel<<<B, 256, 0, g->s>>>(g->xl, g->x, B, S, d, g->gather_lens, pack ? pack->starts : nullptr);
     count_launch(dev);
     TSB_TRY(check_launch("gather_last"));
     xlast = g->xl;
@@ -1806,6 +1815,34 @@ int TSB200_GptReset(void* h) {
 
 }  // extern "C"
 
+// Prompts of different lengths one after the other: [ids | (sequence, position) of every row | first row of every sequence, and the
+// end].  The list of rows goes on with the positions between a prompt's end and the end of its last tile of 128 keys (at most S):
+// the append clears the values there, because the attention multiplies whole tiles and a hidden key's weight of zero does not
+// hide a NaN that was left in the cache.  n_rows stays 0 when no row is saved.
+static void pack_prompts(const int32_t* ids, int B, int S, const int32_t* plen, std::vector<int>& out, int& n_rows, size_t& where_at, size_t& starts_at) {
+  int64_t total = 0;
+  for (int b = 0; b < B; ++b) total += plen[b];
+  if (total == (int64_t)B * S) return;
+  n_rows = (int)total;
+  for (int b = 0; b < B; ++b) out.insert(out.end(), ids + (size_t)b * S, ids + (size_t)b * S + plen[b]);
+  out.resize((out.size() + 1) / 2 * 2);
+  where_at = out.size();
+  for (int tail = 0; tail < 2; ++tail)
+    for (int b = 0; b < B; ++b) {
+      const int end = tail ? std::min(S, (plen[b] + 127) / 128 * 128) : plen[b];
+      for (int s = tail ? plen[b] : 0; s < end; ++s) {
+        out.push_back(b);
+        out.push_back(s);
+      }
+    }
+  starts_at = out.size();
+  int at = 0;
+  for (int b = 0; b <= B; ++b) {
+    out.push_back(at);
+    if (b < B) at += plen[b];
+  }
+}
+
 // Runs S prompt tokens per sequence through the stack on top of T0 = g->T cached positions (0: a fresh prompt;
 // > 0: the suffix of a prompt whose first T0 tokens are already cached), samples the next id.
 // `plen` (prefill only, or NULL): the prompts' own lengths; shorter prompts are padded to S columns (the pad ids are
@@ -1829,12 +1866,22 @@ static int run_prompt(Gpt* g, const int32_t* ids, int B, int S, const TSB200Deco
     for (int b = 0; b < B; ++b) TSB_CHECK(plen[b] >= 1 && plen[b] <= S, "gpt_prefill: prompt length %d of sequence %d is outside [1, %d]", plen[b], b, S);
   }
   TSB_TRY(ensure_act(g, (int64_t)B * S));
+  // prompts of different lengths: where the attention can find a sequence's rows by their start, the pad rows are left out
+  std::vector<int> packed;
+  size_t where_at = 0, starts_at = 0;
+  int n_rows = 0;
+  if (plen && !g->ly && attention_takes_packed(c.dtype, g->c.H, g->c.Hkv, c.hd, S)) pack_prompts(ids, B, S, plen, packed, n_rows, where_at, starts_at);
   void* ids_dev = nullptr;
-  TSB_CUDA(cudaMalloc(&ids_dev, (size_t)B * S * 4));
+  TSB_CUDA(cudaMalloc(&ids_dev, (size_t)B * S * 4 + packed.size() * 4 + 16));
   g->ids_in = (int*)ids_dev;
+  int* packed_dev = (int*)((char*)ids_dev + ((size_t)B * S * 4 + 15) / 16 * 16);
   int ok = 1;
   do {
     if (cudaMemcpyAsync(ids_dev, ids, (size_t)B * S * 4, cudaMemcpyHostToDevice, g->s) != cudaSuccess) { ok = 0; set_last_error("gpt_prefill: id upload failed"); break; }
+    if (n_rows > 0) {
+      if (cudaMemcpyAsync(packed_dev, packed.data(), packed.size() * 4, cudaMemcpyHostToDevice, g->s) != cudaSuccess) { ok = 0; set_last_error("gpt_prefill: id upload failed"); break; }
+      g->ids_in = packed_dev;
+    }
     // history = the prompt (the reference passes the whole sequence as decodedSequence: Decoder.cs:761)
     //  an extension overwrites the pending id at position T0: the caller's tokens are the text from there on
     if (cudaMemcpy2DAsync(g->hist + T0, (size_t)c.max_tokens * 4, ids_dev, (size_t)S * 4, (size_t)S * 4, B, cudaMemcpyDeviceToDevice, g->s) != cudaSuccess) { ok = 0; set_last_error("gpt_prefill: history copy failed"); break; }
@@ -1856,8 +1903,15 @@ static int run_prompt(Gpt* g, const int32_t* ids, int B, int S, const TSB200Deco
     const long long l0 = g->st->launches;
     cudaEventRecord(g->ev0, g->s);
     g->gather_lens = plen ? g->state + kStateLens : nullptr;
+    if (n_rows > 0) {
+      g->pack.rows = n_rows;
+      g->pack.listed = (int)((starts_at - where_at) / 2);
+      g->pack.where = (const int2*)(packed_dev + where_at);
+      g->pack.starts = packed_dev + starts_at;
+    }
     ok = enqueue_forward(g, B, S, T0, false, 1);
     g->gather_lens = nullptr;
+    g->pack = PackedRows{};
     if (!ok) break;
     g->T = T0 + S;
     if (plen) refresh_ragged(g);   // T = the longest prompt

@@ -743,9 +743,9 @@ static int enqueue_layered(Gpt* g, int B, int S, int T0, bool use_state, int T_p
     prof_begin(g, KC_EMBED);
     const int gsz = rows < g->st->sm_count * 8 ? rows : g->st->sm_count * 8;
     if (dt == TSB200_F32)
-      TSB_CUDA(launch_k(embed_kernel<float>, dim3(gsz), dim3(256), 0, g->s, g->x, (const float*)g->E, (const float*)nullptr, ids, rows, S, d, g->c.V, ly->c.embed_scale, 0, 0, T0, dT));
+      TSB_CUDA(launch_k(embed_kernel<float>, dim3(gsz), dim3(256), 0, g->s, g->x, (const float*)g->E, (const float*)nullptr, ids, rows, S, d, g->c.V, ly->c.embed_scale, 0, 0, T0, dT, (const int2*)nullptr));
     else
-      TSB_CUDA(launch_k(embed_kernel<__nv_bfloat16>, dim3(gsz), dim3(256), 0, g->s, g->x, (const __nv_bfloat16*)g->E, (const __nv_bfloat16*)nullptr, ids, rows, S, d, g->c.V, ly->c.embed_scale, 0, 0, T0, dT));
+      TSB_CUDA(launch_k(embed_kernel<__nv_bfloat16>, dim3(gsz), dim3(256), 0, g->s, g->x, (const __nv_bfloat16*)g->E, (const __nv_bfloat16*)nullptr, ids, rows, S, d, g->c.V, ly->c.embed_scale, 0, 0, T0, dT, (const int2*)nullptr));
     count_launch(dev);
     TSB_TRY(check_launch("embed"));
     TSB_TRY(launch_table_route(dev, (const RouteLayer*)rt.layers.p, ly->n_route, ly->max_experts, ids, rows, g->c.V, rt.block, g->s));

@@ -447,18 +447,27 @@ int launch_matrix_memory(int device, DeviceState* st, int dtype, const MemoryArg
 int init_tc_attrs(int device);
 int tc_take_error();
 int64_t linear_workspace_bytes(int M, int K, int N);
+// Prompts of different lengths one after the other (no pad rows): `rows` of them; where[r] = (sequence, position) of row r, for
+// `listed` rows: those from `rows` on are positions whose values the append clears; starts[b]: first row of sequence b, starts[B] = rows.
+struct PackedRows {
+  int rows = 0, listed = 0;
+  const int2* where = nullptr;
+  const int* starts = nullptr;
+};
+// whether launch_attention reads packed rows for prompts of up to S tokens
+bool attention_takes_packed(int dtype, int H, int Hkv, int hd, int S);
 // causal prompt attention of fp16 rows, head size 64 / 128, 1 / 2 / 4 / 8 query heads per KV head (attn_prefill_tc.cu)
 int launch_attn_prefill_tc(int device, void* out, const void* q, int64_t q_rs, const void* cK, const void* cV, int B, int S, int H, int Hkv, int hd, int T0,
-                           int Tmax, float scale, cudaStream_t s);
+                           int Tmax, float scale, const PackedRows* pack, cudaStream_t s);
 int launch_attention(int device, DeviceState* st, int dtype, void* out, const void* q, int64_t q_rs, const void* cK,
                      const void* cV, int B, int S, int H, int Hkv, int hd, int T0, const int* dT0, int Tmax, int splits_hint,
-                     void* ws, int64_t ws_bytes, cudaStream_t s);
+                     void* ws, int64_t ws_bytes, cudaStream_t s, const PackedRows* pack = nullptr);
 int64_t attn_workspace_bytes(int B, int H, int hd, int T);
 int attn_pick_splits(DeviceState* st, int dtype, int B, int H, int Hkv, int hd, int T);
 int launch_rope_table(int device, DeviceState* st, float2* tab, int Tmax, int hd, double base, cudaStream_t s);
 int launch_rope_append(int device, DeviceState* st, int dtype, void* q, const void* k, const void* v, int64_t q_rs,
                        int64_t kv_rs, void* cK, void* cV, int B, int S, int H, int Hkv, int hd, int T0, const int* dT0,
-                       int Tmax, int use_rope, double base, const float2* tab, cudaStream_t s);
+                       int Tmax, int use_rope, double base, const float2* tab, cudaStream_t s, const PackedRows* pack = nullptr);
 int launch_softmax_argmax(int device, DeviceState* st, int* out_ids, float* probs, const float* logits, int B, int V,
                           float temperature, int use_temp, const int* blocked_dev, int n_blocked, cudaStream_t s);
 int launch_beam_topk(int device, DeviceState* st, int* out_ids, float* out_p, float* out_logp, float* probs, int rows, int V, int K,

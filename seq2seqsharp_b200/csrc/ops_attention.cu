@@ -54,57 +54,60 @@ __global__ void rope_table_kernel(float2* __restrict__ tab, int Tmax, int hd, do
   }
 }
 
-// q [B,S,H,hd] rotated in place; k rotated and stored with v into the cache at positions T0 + s.
-// One thread per pair.  tab may be NULL (then cos/sin are evaluated here).
-template <typename T>
+// q [rows,H,hd] rotated in place; k rotated and stored with v into the cache at positions T0 + s.  A thread takes V elements
+// (16 bytes, or one pair where a pointer or a size is not a multiple of that), a CTA one row at a time.
+// `where`: packed rows (kernels.cuh); from row `rows` on, up to `listed`, the position's value is cleared.
+// tab may be NULL (then cos/sin are evaluated here).
+// What bounds it: bytes (16384 rows of 48 heads of 64: 200 MB; 154 us with one pair per thread and 64-bit index arithmetic).
+template <typename T, int V>
 __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
-                                   int64_t kv_rs, T* cK, T* cV, int B, int S, int H, int Hkv, int hd,
+                                   int64_t kv_rs, T* cK, T* cV, int rows, int listed, const int2* where, int S, int H, int Hkv, int hd,
                                    int T0_arg, const int* dT0, int Tmax, int use_rope, double base,
                                    const float2* tab) {
   pdl_trigger();
   pdl_wait();
-  const int hp = hd / 2;
-  const int64_t per_row = (int64_t)(H + 2 * Hkv) * hp;
-  const int64_t n = (int64_t)B * S * per_row;
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t row = p / per_row;  // b*S + s
-    int rem = (int)(p % per_row);
-    const int b = (int)(row / S), s = (int)(row % S);
+  struct __align__(V > 2 ? 16 : sizeof(T)) Piece { T e[V]; };
+  const int pieces = hd / V, per_row = (H + 2 * Hkv) * pieces;
+  for (int row = blockIdx.x; row < listed; row += gridDim.x) {
+    const int b = where ? where[row].x : row / S, s = where ? where[row].y : row % S;
     const int T0 = state_len(dT0, b, T0_arg);  // the engine keeps the cache lengths on the device so one CUDA graph serves every step
     const int pos = T0 + s;
     TSB_DEV_CHECK(attention, pos >= 0 && pos < Tmax, 0x201, (void)0)   // append position outside the cache (row skipped)
     if (pos >= Tmax) continue;  // capacity is checked on the host; never write past the cache
-    const int head = rem / hp, i = rem % hp;
-    float c = 1.0f, sn = 0.0f;
-    if (use_rope && head < H + Hkv) {
-      if (tab) {
-        const float2 cs = tab[(int64_t)pos * hp + i];
-        c = cs.x;
-        sn = cs.y;
+    const bool clear = row >= rows;
+    for (int it = threadIdx.x + (clear ? (H + Hkv) * pieces : 0); it < per_row; it += blockDim.x) {
+      const int head = it / pieces, i = (it % pieces) * V;
+      Piece x;
+      if (clear) {
+#pragma unroll
+        for (int e = 0; e < V; ++e) x.e[e] = from_f<T>(0.0f);
       } else {
-        rope_cs(i, hd, pos, base, c, sn);
+        const T* src = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
+                                : (head < H + Hkv ? k + (int64_t)row * kv_rs + (int64_t)(head - H) * hd : v + (int64_t)row * kv_rs + (int64_t)(head - H - Hkv) * hd);
+        if constexpr (V > 2) x = *reinterpret_cast<const Piece*>(src + i);
+        else x.e[0] = src[i], x.e[1] = src[i + 1];
       }
-    }
-    if (head < H) {
-      T* qp = q + row * q_rs + (int64_t)head * hd + 2 * i;
-      const float a = to_f<T>(qp[0]), bb = to_f<T>(qp[1]);
-      if (use_rope) {
-        qp[0] = from_f<T>(a * c - bb * sn);
-        qp[1] = from_f<T>(bb * c + a * sn);
+      if (use_rope && head < H + Hkv) {
+#pragma unroll
+        for (int e = 0; e < V; e += 2) {
+          float c, sn;
+          if (tab) {
+            const float2 cs = tab[(int64_t)pos * (hd / 2) + (i + e) / 2];
+            c = cs.x;
+            sn = cs.y;
+          } else {
+            rope_cs((i + e) / 2, hd, pos, base, c, sn);
+          }
+          const float x0 = to_f<T>(x.e[e]), x1 = to_f<T>(x.e[e + 1]);
+          x.e[e] = from_f<T>(x0 * c - x1 * sn);
+          x.e[e + 1] = from_f<T>(x1 * c + x0 * sn);
+        }
       }
-    } else if (head < H + Hkv) {
-      const int g = head - H;
-      const T* kp = k + row * kv_rs + (int64_t)g * hd + 2 * i;
-      const float a = to_f<T>(kp[0]), bb = to_f<T>(kp[1]);
-      T* dst = cK + (((int64_t)b * Hkv + g) * Tmax + pos) * hd + 2 * i;
-      dst[0] = from_f<T>(use_rope ? a * c - bb * sn : a);
-      dst[1] = from_f<T>(use_rope ? bb * c + a * sn : bb);
-    } else {
-      const int g = head - H - Hkv;
-      const T* vp = v + row * kv_rs + (int64_t)g * hd + 2 * i;
-      T* dst = cV + (((int64_t)b * Hkv + g) * Tmax + pos) * hd + 2 * i;
-      dst[0] = vp[0];
-      dst[1] = vp[1];
+      if (head < H && !use_rope) continue;
+      T* dst = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
+                        : (head < H + Hkv ? cK : cV) + (((int64_t)b * Hkv + (head < H + Hkv ? head - H : head - H - Hkv)) * Tmax + pos) * hd;
+      if constexpr (V > 2) *reinterpret_cast<Piece*>(dst + i) = x;
+      else dst[i] = x.e[0], dst[i + 1] = x.e[1];
     }
   }
 }
@@ -652,6 +655,17 @@ static bool mma_decode_shape(int dtype, int H, int Hkv, int hd) {
   return dtype == TSB200_F16 && (hd == 64 || hd == 128) && (group == 1 || group == 2 || group == 4 || group == 8);
 }
 
+// fp16, head size 64 / 128, up to 8 query heads per KV head: scores and P V on the tensor cores
+static bool attn_mma_enabled() {
+  static int on = -1;
+  if (on < 0) {
+    const char* e = getenv("TSB200_ATTN_MMA");  // "0": keep the shuffle/FMA kernels (A/B measurements)
+    on = (e && e[0] == '0') ? 0 : 1;
+  }
+  return on != 0;
+}
+bool attention_takes_packed(int dtype, int H, int Hkv, int hd, int S) { return attn_mma_enabled() && S >= 16 && mma_decode_shape(dtype, H, Hkv, hd); }
+
 int64_t attn_workspace_bytes(int B, int H, int hd, int T) {
   (void)T;
   return (int64_t)B * H * 64 * (hd + 2) * sizeof(float);
@@ -660,7 +674,7 @@ int64_t attn_workspace_bytes(int B, int H, int hd, int T) {
 template <typename T>
 static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_t q_rs, const T* cK, const T* cV, int B, int S,
                          int H, int Hkv, int hd, int T0, const int* dT0, int Tmax, int splits_hint, float* ws, int64_t ws_bytes,
-                         cudaStream_t s) {
+                         cudaStream_t s, const PackedRows* pack) {
   constexpr int EPL = Vec16<T>::N;
   const int lpt = hd / EPL;
   TSB_CHECK(hd % EPL == 0 && lpt >= 1 && lpt <= 32 && (lpt & (lpt - 1)) == 0,
@@ -692,15 +706,10 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
     const char* e = getenv("TSB200_ATTN_STAGED");  // "0": register-only kernel for every case (A/B measurements)
     staged = (e && e[0] == '0') ? 0 : 1;
   }
-  // fp16, head_dim 64 / 128, up to 8 query heads per KV head: scores and P V on the warp-level tensor cores
-  static int use_mma = -1;
-  if (use_mma < 0) {
-    const char* e = getenv("TSB200_ATTN_MMA");  // "0": keep the shuffle/FMA kernels (A/B measurements)
-    use_mma = (e && e[0] == '0') ? 0 : 1;
-  }
+  const bool use_mma = attn_mma_enabled();
   if constexpr (sizeof(T) == 2) {
-    if (use_mma && S >= 16 && mma_shape && !dT0) {   // a prompt: its length is known on the host
-      return launch_attn_prefill_tc(device, out, q, q_rs, cK, cV, B, S, H, Hkv, hd, T0, Tmax, scale, s);
+    if (use_mma && S >= 16 && mma_shape && !dT0) {
+      return launch_attn_prefill_tc(device, out, q, q_rs, cK, cV, B, S, H, Hkv, hd, T0, Tmax, scale, pack, s);
     }
     // at every grid size (7B-class model, sequences of 530 tokens: faster than the shuffle / FMA kernels from 16 CTAs on)
     if (use_mma && staged && S == 1 && (hd == 64 || hd == 128) && group <= 8 && ygroups == Hkv) {
@@ -788,14 +797,15 @@ int attn_pick_splits(DeviceState* st, int dtype, int B, int H, int Hkv, int hd, 
 
 int launch_attention(int device, DeviceState* st, int dtype, void* out, const void* q, int64_t q_rs, const void* cK,
                      const void* cV, int B, int S, int H, int Hkv, int hd, int T0, const int* dT0, int Tmax, int splits_hint,
-                     void* ws, int64_t ws_bytes, cudaStream_t s) {
+                     void* ws, int64_t ws_bytes, cudaStream_t s, const PackedRows* pack) {
   if (B == 0 || S == 0) return 1;
+  TSB_CHECK(!pack || (!dT0 && attention_takes_packed(dtype, H, Hkv, hd, S)), "attention: packed rows are not served for this shape");
   if (dtype == TSB200_F32)
     return launch_attn_t<float>(device, st, (float*)out, (const float*)q, q_rs, (const float*)cK, (const float*)cV, B, S, H, Hkv,
-                                hd, T0, dT0, Tmax, splits_hint, (float*)ws, ws_bytes, s);
+                                hd, T0, dT0, Tmax, splits_hint, (float*)ws, ws_bytes, s, pack);
   if (dtype == TSB200_F16)
     return launch_attn_t<__half>(device, st, (__half*)out, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, B, S, H,
-                                 Hkv, hd, T0, dT0, Tmax, splits_hint, (float*)ws, ws_bytes, s);
+                                 Hkv, hd, T0, dT0, Tmax, splits_hint, (float*)ws, ws_bytes, s, pack);
   TSB_FAIL("attention: unsupported dtype %d", dtype);
 }
 
@@ -807,23 +817,40 @@ int launch_rope_table(int device, DeviceState* st, float2* tab, int Tmax, int hd
   return check_launch("rope_table");
 }
 
+template <typename T, int V>
+static int launch_rope_append_t(int device, DeviceState* st, T* q, const T* k, const T* v, int64_t q_rs, int64_t kv_rs, T* cK, T* cV, int B, int S, int H,
+                                int Hkv, int hd, int T0, const int* dT0, int Tmax, int use_rope, double base, const float2* tab, const PackedRows* pack,
+                                cudaStream_t s) {
+  const int rows = pack ? pack->rows : B * S, listed = pack ? pack->listed : rows;
+  const int64_t per_row = (int64_t)(H + 2 * Hkv) * (hd / V);
+  const int threads = per_row <= 512 ? (int)(per_row + 31) / 32 * 32 : 256;
+  const int grid = listed < st->sm_count * 16 ? listed : st->sm_count * 16;
+  TSB_CUDA(launch_k(rope_append_kernel<T, V>, dim3(grid), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, listed, pack ? pack->where : (const int2*)nullptr,
+                    S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
+  return 1;
+}
+
 int launch_rope_append(int device, DeviceState* st, int dtype, void* q, const void* k, const void* v, int64_t q_rs,
                        int64_t kv_rs, void* cK, void* cV, int B, int S, int H, int Hkv, int hd, int T0, const int* dT0,
-                       int Tmax, int use_rope, double base, const float2* tab, cudaStream_t s) {
+                       int Tmax, int use_rope, double base, const float2* tab, cudaStream_t s, const PackedRows* pack) {
   if (B == 0 || S == 0) return 1;
   TSB_CHECK(hd % 2 == 0, "rope_append: head_dim must be even");
   TSB_CHECK(dT0 || (T0 >= 0 && T0 + S <= Tmax), "rope_append: cache capacity exceeded (%d + %d > %d)", T0, S, Tmax);
-  const int64_t n = (int64_t)B * S * (H + 2 * Hkv) * (hd / 2);
-  int64_t g = (n + 255) / 256;
-  if (g > (int64_t)st->sm_count * 16) g = (int64_t)st->sm_count * 16;
-  if (dtype == TSB200_F32)
-    TSB_CUDA(launch_k(rope_append_kernel<float>, dim3((int)g), dim3(256), 0, s, (float*)q, (const float*)k, (const float*)v, q_rs, kv_rs,
-                      (float*)cK, (float*)cV, B, S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
-  else if (dtype == TSB200_F16)
-    TSB_CUDA(launch_k(rope_append_kernel<__half>, dim3((int)g), dim3(256), 0, s, (__half*)q, (const __half*)k, (const __half*)v, q_rs,
-                      kv_rs, (__half*)cK, (__half*)cV, B, S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
-  else
-    TSB_FAIL("rope_append: unsupported dtype %d", dtype);
+  TSB_CHECK((int64_t)B * S <= 0x7fffffff, "rope_append: too many rows");
+  TSB_CHECK(dtype == TSB200_F32 || dtype == TSB200_F16, "rope_append: unsupported dtype %d", dtype);
+  const int V = 16 / (int)dtype_size(dtype);
+  const bool wide = hd % V == 0 && q_rs % V == 0 && kv_rs % V == 0 && (((uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cK | (uintptr_t)cV) % 16) == 0;
+#define TSB_ROPE(T, W)                                                                                                                        \
+  TSB_TRY((launch_rope_append_t<T, W>(device, st, (T*)q, (const T*)k, (const T*)v, q_rs, kv_rs, (T*)cK, (T*)cV, B, S, H, Hkv, hd, T0, dT0, Tmax, \
+                                      use_rope, base, tab, pack, s)))
+  if (dtype == TSB200_F32) {
+    if (wide) TSB_ROPE(float, 4);
+    else TSB_ROPE(float, 2);
+  } else {
+    if (wide) TSB_ROPE(__half, 8);
+    else TSB_ROPE(__half, 2);
+  }
+#undef TSB_ROPE
   count_launch(device);
   return check_launch("rope_append");
 }

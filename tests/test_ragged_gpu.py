@@ -203,3 +203,36 @@ def test_ragged_errors(cuda):
     with pytest.raises(RuntimeError, match="OOM"):
         g.SlotExtend(0, list(range(1, 40)), opts)
     g.close()
+
+
+def test_prompts_of_different_lengths_without_pad_rows(cuda):
+    """Prompts long enough for the tensor-core attention lie one after the other: every sequence's logits are those of the prompt run
+    alone, on an engine whose cache still holds NaN from an earlier use of it."""
+    cfg = GPTConfig(name="gqa_rope_fp16", L=2, d=256, H=4, Hkv=1, hd=64, F=512, V=1009, norm=Nm.RMSNorm, act=A.SwiGLU, pe=P.RoPE, attn=M.GQA, dtype="float16")
+    w = synthetic_weights(cfg, 5, std=0.05)
+    lens = [200, 17, 128, 129, 1]
+    full = prompt_ids(8, len(lens), max(lens), cfg.V)
+    prompts = [list(map(int, full[b, :n])) for b, n in enumerate(lens)]
+    opts = _opts(DS.GreedySearch, 260)
+    gpt = GPT(cfg, max_batch=len(lens), max_tokens=260)
+    bad = {k: v.copy() for k, v in w.items()}
+    for k in bad:
+        if ".SelfAttn_" in k and k.endswith((".K", ".V")):
+            bad[k][...] = np.nan
+    gpt.LoadWeights(bad)
+    gpt.Prefill(prompt_ids(9, len(lens), 255, cfg.V), opts)
+    gpt.Reset()
+    gpt.LoadWeights(w)
+    gpt.PrefillRagged(prompts, opts)
+    logits = gpt.Logits()[0].copy()
+    np.testing.assert_array_equal(gpt.CacheLengths(), lens)
+    fed = np.arange(len(lens), dtype=np.int32) + 11
+    gpt.StepHost(fed, opts)
+    later = gpt.Logits()[0].copy()
+    for b, p in enumerate(prompts):
+        one = GPT(cfg, max_batch=1, max_tokens=260)
+        one.LoadWeights(w)
+        one.Prefill(np.asarray([p], dtype=np.int32), opts)
+        assert rel_err(logits[b:b + 1], one.Logits()[0]) < tol_for(cfg)
+        one.StepHost(fed[b:b + 1], opts)
+        assert rel_err(later[b:b + 1], one.Logits()[0]) < tol_for(cfg)
