@@ -58,6 +58,75 @@ __global__ void __launch_bounds__(1024) norm_kernel(TH* __restrict__ h, TX* __re
   }
 }
 
+// The fused form with the row in registers: NV pieces of four columns per thread, one read and one write of memory per element, no
+// shared-memory row.  What bounds it: bytes for many rows (16384 rows of 2048: 119 us with scalar accesses and the row in shared memory),
+// latency for a few (one piece per thread: every load of the row is in flight at once).
+template <typename TH, int NV>
+__global__ void __launch_bounds__(1024) norm_wide_kernel(TH* h, float* x, const TH* delta, const TH* gamma, const TH* beta, int norm_type, float eps, int rows, int cols) {
+  __shared__ float red[32];
+  struct __align__(4 * sizeof(TH)) Four { TH e[4]; };
+  pdl_trigger();
+  const int n4 = cols / 4;
+  pdl_wait();
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    float4* xr = reinterpret_cast<float4*>(x + (int64_t)r * cols);
+    float4 v[NV];
+    float s = 0.0f;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      v[k] = i < n4 ? xr[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    if (delta) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const int i = threadIdx.x + k * blockDim.x;
+        if (i >= n4) continue;
+        const Four t = reinterpret_cast<const Four*>(delta + (int64_t)r * cols)[i];
+        v[k].x += to_f<TH>(t.e[0]);
+        v[k].y += to_f<TH>(t.e[1]);
+        v[k].z += to_f<TH>(t.e[2]);
+        v[k].w += to_f<TH>(t.e[3]);
+        xr[i] = v[k];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) s += norm_type == 0 ? (v[k].x + v[k].y) + (v[k].z + v[k].w) : (v[k].x * v[k].x + v[k].y * v[k].y) + (v[k].z * v[k].z + v[k].w * v[k].w);
+    s = block_sum(s, red);
+    float mean = 0.0f, div;
+    if (norm_type == 0) {
+      mean = s / cols;
+      float sq = 0.0f;
+#pragma unroll
+      for (int k = 0; k < NV; ++k) {
+        const float a = v[k].x - mean, b = v[k].y - mean, c = v[k].z - mean, d = v[k].w - mean;
+        if (threadIdx.x + k * blockDim.x < n4) sq += (a * a + b * b) + (c * c + d * d);
+      }
+      sq = block_sum(sq, red);
+      div = sqrtf(eps + sq / cols);
+    } else {
+      div = sqrtf(s / (float)cols + eps);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const int i = threadIdx.x + k * blockDim.x;
+      if (i >= n4) continue;
+      const Four g = reinterpret_cast<const Four*>(gamma)[i];
+      float y[4] = {to_f<TH>(g.e[0]) * ((v[k].x - mean) / div), to_f<TH>(g.e[1]) * ((v[k].y - mean) / div), to_f<TH>(g.e[2]) * ((v[k].z - mean) / div),
+                    to_f<TH>(g.e[3]) * ((v[k].w - mean) / div)};
+      if (beta) {
+        const Four t = reinterpret_cast<const Four*>(beta)[i];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[e] += to_f<TH>(t.e[e]);
+      }
+      Four o;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) o.e[e] = from_f<TH>(y[e]);
+      reinterpret_cast<Four*>(h + (int64_t)r * cols)[i] = o;
+    }
+  }
+}
+
 static inline int norm_threads(int cols) {
   int t = 128;
   while (t < 1024 && t * 4 < cols) t <<= 1;
@@ -105,18 +174,36 @@ static int norm_entry(int device, const TSB200Tensor* result, const TSB200Tensor
   TSB_FAIL("norm: unsupported dtype %d", src->dtype);
 }
 
+template <typename TH>
+static int launch_norm_residual_t(DeviceState* st, TH* h, float* x, const TH* delta, const TH* gamma, const TH* beta, int norm_type, float eps, int M, int d,
+                                  cudaStream_t s) {
+  const int g = M < st->sm_count * 8 ? M : st->sm_count * 8;
+  // four columns at a time where every row starts on a boundary of 4 elements; up to four pieces of a row per thread
+  const uintptr_t al = (uintptr_t)h | (uintptr_t)delta | (uintptr_t)gamma | (uintptr_t)beta;
+  if (d % 4 == 0 && d <= 16384 && ((uintptr_t)x % 16) == 0 && al % (4 * sizeof(TH)) == 0) {
+    // a few rows: the whole row at once; many: 256 threads, so that several rows share an SM
+    const int n4 = d / 4, at_least = M <= 2 * st->sm_count ? 1024 : 256;
+    const int nv = n4 <= at_least ? 1 : (n4 <= 2 * at_least ? 2 : 4);
+    int th = ((n4 + nv - 1) / nv + 31) / 32 * 32;
+    if (th <= 1024) {
+      auto k = nv == 1 ? norm_wide_kernel<TH, 1> : (nv == 2 ? norm_wide_kernel<TH, 2> : norm_wide_kernel<TH, 4>);
+      TSB_CUDA(launch_k(k, dim3(g), dim3(th), 0, s, h, x, delta, gamma, beta, norm_type, eps, M, d));
+      return 1;
+    }
+  }
+  TSB_CUDA(launch_k(norm_kernel<float, TH, true>, dim3(g), dim3(norm_threads(d)), d * sizeof(float), s, h, x, delta, gamma, beta, norm_type, eps, M, d, (int64_t)d,
+                    (int64_t)d));
+  return 1;
+}
+
 // Internal launcher shared with the engine.
 int launch_norm_residual(int device, DeviceState* st, int dtype, void* h, float* x, const void* delta, const void* gamma,
                          const void* beta, int norm_type, float eps, int M, int d, cudaStream_t s) {
   if (M == 0) return 1;
-  const int g = M < st->sm_count * 8 ? M : st->sm_count * 8;
-  const int th = norm_threads(d);
   if (dtype == TSB200_F32)
-    TSB_CUDA(launch_k(norm_kernel<float, float, true>, dim3(g), dim3(th), d * sizeof(float), s, (float*)h, x, (const float*)delta,
-                      (const float*)gamma, (const float*)beta, norm_type, eps, M, d, (int64_t)d, (int64_t)d));
+    TSB_TRY(launch_norm_residual_t<float>(st, (float*)h, x, (const float*)delta, (const float*)gamma, (const float*)beta, norm_type, eps, M, d, s));
   else
-    TSB_CUDA(launch_k(norm_kernel<float, __half, true>, dim3(g), dim3(th), d * sizeof(float), s, (__half*)h, x, (const __half*)delta,
-                      (const __half*)gamma, (const __half*)beta, norm_type, eps, M, d, (int64_t)d, (int64_t)d));
+    TSB_TRY(launch_norm_residual_t<__half>(st, (__half*)h, x, (const __half*)delta, (const __half*)gamma, (const __half*)beta, norm_type, eps, M, d, s));
   count_launch(device);
   return check_launch("norm_residual");
 }

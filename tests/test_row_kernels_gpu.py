@@ -1,0 +1,56 @@
+"""Norms of whole rows in registers, rotation and append by 16-byte pieces, at the edges of the rules that choose them."""
+import numpy as np
+import pytest
+import torch
+
+from seq2seqsharp_b200 import _native as N
+from tests.test_fused_gpu import dev, host, stream
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.float16, 4e-3)])   # 4e-3: two roundings to fp16 of values up to 8
+@pytest.mark.parametrize("norm_type", [0, 1])
+@pytest.mark.parametrize("M,d", [(1, 768), (3, 4096), (300, 2048), (700, 4096), (2, 4100), (301, 1028), (5, 12288), (4, 130), (2, 33)])
+def test_norm_of_rows(cuda, oracle, dtype, tol, norm_type, M, d):
+    rng = np.random.default_rng(M + d)
+    x = dev((rng.standard_normal((M, d)) * 1.7 + 0.2).astype(np.float32))
+    delta = dev((rng.standard_normal((M, d)) * 0.3).astype(np.float32), dtype)
+    g, b = dev((1 + 0.1 * rng.standard_normal(d)).astype(np.float32), dtype), dev((0.1 * rng.standard_normal(d)).astype(np.float32), dtype)
+    for dl, beta in ((None, b), (delta, None)):
+        rows = x.clone()
+        h = torch.empty(M, d, device="cuda", dtype=dtype)
+        torch.cuda.synchronize()
+        N.call("TSB200_NormResidual", 0, N.F16 if dtype == torch.float16 else N.F32, h.data_ptr(), rows.data_ptr(), dl.data_ptr() if dl is not None else None, g.data_ptr(),
+               beta.data_ptr() if beta is not None else None, norm_type, 1e-6, M, d, stream())
+        want = host(x) + (host(dl) if dl is not None else 0.0)
+        np.testing.assert_allclose(host(rows), want, atol=1e-6)
+        bh = host(beta) if beta is not None else None
+        ref = oracle.layernorm(want, host(g), bh if bh is not None else np.zeros(d, np.float32), 1e-6) if norm_type == 0 else oracle.rmsnorm(want, host(g), bh, 1e-6)
+        np.testing.assert_allclose(host(h), ref, atol=tol * max(1.0, float(np.abs(ref).max()) / 4))
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 2e-5), (torch.float16, 4e-3)])   # 4e-3: rounding to fp16 of values up to 5
+@pytest.mark.parametrize("hd,shift", [(64, 0), (64, 2), (6, 0), (8, 0), (12, 0)])      # 16-byte pieces; an odd boundary or head size: pairs
+def test_rotation_and_append(cuda, dtype, tol, hd, shift):
+    B, S, H, Hkv, T0, Tmax = 2, 5, 4, 2, 3, 11
+    Nq, dt = (H + 2 * Hkv) * hd, N.F16 if dtype == torch.float16 else N.F32
+    rng = np.random.default_rng(hd + shift)
+    qkv0 = rng.standard_normal((B, S, Nq)).astype(np.float32)
+    raw = torch.zeros(B * S * Nq + shift, device="cuda", dtype=dtype)
+    raw[shift:] = dev(qkv0.reshape(-1), dtype)
+    qkv = raw[shift:].reshape(B, S, Nq)
+    before = host(qkv).astype(np.float64)
+    cK, cV = (torch.zeros(B, Hkv, Tmax, hd, device="cuda", dtype=dtype) for _ in range(2))
+    es = qkv.element_size()
+    torch.cuda.synchronize()
+    N.call("TSB200_RopeAppend", 0, dt, qkv.data_ptr(), qkv.data_ptr() + H * hd * es, qkv.data_ptr() + (H + Hkv) * hd * es, Nq, Nq, cK.data_ptr(), cV.data_ptr(), B, S, H,
+           Hkv, hd, T0, Tmax, 1, 10000.0, stream())
+    x = before.reshape(B, S, H + 2 * Hkv, hd)
+    angle = (T0 + np.arange(S))[:, None] * 10000.0 ** (-2.0 * np.arange(hd // 2) / hd)
+    c, s = np.cos(angle)[None, :, None], np.sin(angle)[None, :, None]
+    turned = np.stack((x[..., 0::2] * c - x[..., 1::2] * s, x[..., 1::2] * c + x[..., 0::2] * s), -1).reshape(x.shape)
+    np.testing.assert_allclose(host(qkv).reshape(x.shape)[:, :, :H], turned[:, :, :H], atol=tol)
+    np.testing.assert_allclose(host(cK)[:, :, T0:T0 + S], turned[:, :, H:H + Hkv].transpose(0, 2, 1, 3), atol=tol)
+    np.testing.assert_array_equal(host(cV)[:, :, T0:T0 + S], x[:, :, H + Hkv:].transpose(0, 2, 1, 3).astype(np.float32))
+    assert not host(cK)[:, :, T0 + S:].any() and not host(cV)[:, :, :T0].any()
