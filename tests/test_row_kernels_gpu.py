@@ -1,9 +1,11 @@
-"""Norms of whole rows in registers, rotation and append by 16-byte pieces, at the edges of the rules that choose them."""
+"""Norms of whole rows in registers, rotation and append by 16-byte pieces, softmax on a cluster and the head of a nucleus, at the edges of
+the rules that choose them."""
 import numpy as np
 import pytest
 import torch
 
 from seq2seqsharp_b200 import _native as N
+from seq2seqsharp_b200.ops import Ops
 from tests.test_fused_gpu import dev, host, stream
 
 pytestmark = pytest.mark.gpu
@@ -54,3 +56,47 @@ def test_rotation_and_append(cuda, dtype, tol, hd, shift):
     np.testing.assert_allclose(host(cK)[:, :, T0:T0 + S], turned[:, :, H:H + Hkv].transpose(0, 2, 1, 3), atol=tol)
     np.testing.assert_array_equal(host(cV)[:, :, T0:T0 + S], x[:, :, H + Hkv:].transpose(0, 2, 1, 3).astype(np.float32))
     assert not host(cK)[:, :, T0 + S:].any() and not host(cV)[:, :, :T0].any()
+
+
+@pytest.mark.parametrize("B,V", [(1, 4095), (1, 4096), (3, 4099), (2, 32769), (74, 32000), (75, 32000), (1, 65537), (1, 131072), (1, 131073)])
+def test_softmax_and_first_maximum(cuda, oracle, B, V):
+    rng = np.random.default_rng(V)
+    z = (rng.standard_normal((B, V)) * 2).astype(np.float32)
+    z[0, [7, V // 2, V - 1]] = z[0].max() + 1.0     # three equal maxima, in different parts of the row: the lowest index
+    if B > 1:
+        z[-1, 3:V // 3] = -np.inf
+    blocked = dev(np.array([0, V - 1], dtype=np.int32))
+    for t in (1.0, 0.7):
+        ids, probs = torch.empty(B, dtype=torch.int32, device="cuda"), torch.empty(B, V, device="cuda")
+        zd = dev(z)
+        torch.cuda.synchronize()
+        N.call("TSB200_SoftmaxArgmax", 0, ids.data_ptr(), probs.data_ptr(), zd.data_ptr(), B, V, t, blocked.data_ptr(), 2, stream())
+        zt = (z / np.float32(t)).astype(np.float64)
+        e = np.exp(zt - zt.max(1, keepdims=True))
+        p = e / e.sum(1, keepdims=True)
+        p[:, [0, V - 1]] -= 1.0
+        # an exponent of up to 30 is rounded to 2^-24 of itself, the exponential to a few units in the last place
+        np.testing.assert_allclose(host(probs), p, atol=1e-7, rtol=5e-6)
+        np.testing.assert_array_equal(ids.cpu().numpy(), oracle.argmax(host(probs)))
+        assert ids[0].item() == 7
+
+
+@pytest.mark.parametrize("rows", [2, 40])      # a cluster per row; one CTA per row
+@pytest.mark.parametrize("n", [1, 2, 5, 900, 1025, 2047, 2048, 2049, 3000])
+def test_nuclei_around_the_selection_limit(cuda, oracle, rows, n):
+    """n equal or nearly equal weights hold 0.96 of the mass: the nucleus of 0.9 is inside them, with ties in the order of their indexes."""
+    V = 32000
+    rng = np.random.default_rng(n)
+    p = np.full((rows, V), 0.04 / (V - n), dtype=np.float32)
+    for r in range(rows):
+        at = rng.permutation(V)[:n]
+        p[r, at] = (0.96 / n) * (1.0 if r % 2 else 1.0 + 0.3 * rng.random(n))
+    u = rng.random(rows).astype(np.float32)
+    for top in (0.5, 0.9, 0.9595, 2.0):
+        out = Ops.TopPSample(torch.from_numpy(p).cuda(), top, 0.0, None, torch.from_numpy(u))
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy(), oracle.topp(p, top, 0.0, None, u))
+    big = p * np.float32(4.0)      # weights that add up to more than the selection's units hold
+    out = Ops.TopPSample(torch.from_numpy(big).cuda(), 2.2, 0.0, None, torch.from_numpy(u))
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(out.cpu().numpy(), oracle.topp(big, 2.2, 0.0, None, u))
