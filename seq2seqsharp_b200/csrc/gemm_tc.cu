@@ -68,11 +68,17 @@ __device__ __forceinline__ void tc_finish(const TcArgs& a, int row, int col0, co
   }
 }
 
-// The same epilogue for a full chunk of 32 columns when every pointer is 16-byte aligned and N is a multiple of 32
-// (TcArgs::vec_ok): 16-byte loads of bias and residual, 16-byte stores, i.e. whole 32-byte sectors instead of one
-// 2-byte store per element (scalar stores made the epilogue longer than the mainloop of a 128 x 256 x 4096 tile).
-template <typename H>
-__device__ __forceinline__ void tc_finish_fast(const TcArgs& a, int row, int col0, const float* v) {
+// The same epilogue for 32 rows x 32 columns of a warp (lane = row, v = its columns) when every pointer is 16-byte aligned and N is a
+// multiple of 32 (TcArgs::vec_ok).  The finished values cross the warp's corner of shared memory, so that gate, residual and output are
+// read and written as whole 32-byte sectors of few rows per instruction (a lane writing its own row touches 32 lines with every
+// instruction).  The activation is chosen outside of the loop over the columns: with the choice inside, the 32 copies of every
+// activation's code were fetched afresh for each chunk by every SM, and the epilogue took 13 us of a 128 x 256 tile.
+constexpr int kStagePitch = 36;                             // floats; 32 columns, conflict-free float4 rows
+constexpr int kStageBytes = 4 * 32 * kStagePitch * 4;       // the four epilogue warps' corners
+template <typename H, int ACT, bool GLU>
+__device__ __forceinline__ void tc_finish_as(const TcArgs& a, int row0, int n_live, int col0, const float* v, float* stage) {
+  constexpr int kOut = GLU ? 16 : 32, kPitch = GLU ? 20 : kStagePitch, kLanes = kOut / 4;   // kLanes lanes per row
+  const int lane = threadIdx.x & 31;
   float b[32];
   if (a.ep.bias) {
     const uint4* bp = reinterpret_cast<const uint4*>(reinterpret_cast<const H*>(a.ep.bias) + col0);
@@ -91,64 +97,70 @@ __device__ __forceinline__ void tc_finish_fast(const TcArgs& a, int row, int col
 #pragma unroll
     for (int j = 0; j < 32; ++j) b[j] = 0.0f;
   }
-  float x[32];
-  int n_out;
-  size_t o;
-  if (!a.ep.glu) {
+  float x[kOut];
 #pragma unroll
-    for (int j = 0; j < 32; ++j) x[j] = ep_act(v[j] + b[j], a.ep.act);
-    n_out = 32;
-    o = (size_t)row * a.N + col0;
-  } else {
-#pragma unroll
-    for (int j = 0; j < 16; ++j) x[j] = ep_glu(v[2 * j] + b[2 * j], v[2 * j + 1] + b[2 * j + 1], a.ep);
-    n_out = 16;
-    o = (size_t)row * (a.N / 2) + (col0 >> 1);
-  }
-  if (a.ep.gate) {
-    const uint4* gp = reinterpret_cast<const uint4*>(reinterpret_cast<const H*>(a.ep.gate) + o);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q * 8 < n_out) {
-        const uint4 t = gp[q];
-        const uint32_t h[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 f = Pair16<H>::get(h[i]);
-          x[q * 8 + 2 * i] *= f.x;
-          x[q * 8 + 2 * i + 1] *= f.y;
-        }
-      }
+  for (int j = 0; j < kOut; ++j) {
+    if constexpr (GLU) {
+      Epilogue ep;
+      ep.act = ACT; ep.glu_limit = a.ep.glu_limit; ep.glu_slope = a.ep.glu_slope; ep.glu_shift = a.ep.glu_shift;
+      x[j] = ep_glu(v[2 * j] + b[2 * j], v[2 * j + 1] + b[2 * j + 1], ep);
+    } else {
+      x[j] = ep_act(v[j] + b[j], ACT);
     }
   }
-  if (a.ep.residual) {
-    const float4* rp = reinterpret_cast<const float4*>(a.ep.residual + o);
+  float4* mine = reinterpret_cast<float4*>(stage + lane * kPitch);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (q * 4 < n_out) {
-        const float4 t = rp[q];
-        x[q * 4] += t.x; x[q * 4 + 1] += t.y; x[q * 4 + 2] += t.z; x[q * 4 + 3] += t.w;
+  for (int q = 0; q < kLanes; ++q) mine[q] = make_float4(x[4 * q], x[4 * q + 1], x[4 * q + 2], x[4 * q + 3]);
+  __syncwarp();
+  const int Nout = GLU ? a.N / 2 : a.N, r = lane / kLanes, c = (lane % kLanes) * 4;
+#pragma unroll
+  for (int it = 0; it < kLanes; ++it) {
+    const int rr = it * (32 / kLanes) + r;
+    if (rr < n_live) {
+      float4 t = *reinterpret_cast<const float4*>(stage + rr * kPitch + c);
+      const size_t o = (size_t)(row0 + rr) * Nout + (GLU ? col0 >> 1 : col0) + c;
+      if (a.ep.gate) {
+        const uint2 g = *reinterpret_cast<const uint2*>(reinterpret_cast<const H*>(a.ep.gate) + o);
+        const float2 g0 = Pair16<H>::get(g.x), g1 = Pair16<H>::get(g.y);
+        t.x *= g0.x; t.y *= g0.y; t.z *= g1.x; t.w *= g1.y;
       }
+      if (a.ep.residual) {
+        const float4 s = *reinterpret_cast<const float4*>(a.ep.residual + o);
+        t.x += s.x; t.y += s.y; t.z += s.z; t.w += s.w;
+      }
+      if (a.ep.y32) *reinterpret_cast<float4*>(a.ep.y32 + o) = t;
+      else *reinterpret_cast<uint2*>(reinterpret_cast<H*>(a.ep.y) + o) = make_uint2(Pair16<H>::put(t.x, t.y), Pair16<H>::put(t.z, t.w));
     }
   }
-  if (a.ep.y32) {
-    float4* yp = reinterpret_cast<float4*>(a.ep.y32 + o);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (q * 4 < n_out) yp[q] = make_float4(x[q * 4], x[q * 4 + 1], x[q * 4 + 2], x[q * 4 + 3]);
-  } else {
-    uint4* yp = reinterpret_cast<uint4*>(reinterpret_cast<H*>(a.ep.y) + o);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (q * 8 < n_out) {
-        uint4 t;
-        t.x = Pair16<H>::put(x[q * 8], x[q * 8 + 1]);
-        t.y = Pair16<H>::put(x[q * 8 + 2], x[q * 8 + 3]);
-        t.z = Pair16<H>::put(x[q * 8 + 4], x[q * 8 + 5]);
-        t.w = Pair16<H>::put(x[q * 8 + 6], x[q * 8 + 7]);
-        yp[q] = t;
-      }
+  __syncwarp();   // the corner is free again
+}
+// all lanes of the warp; rows row0 .. row0 + n_live - 1 exist
+template <typename H>
+__device__ __forceinline__ void tc_finish_rows(const TcArgs& a, int row0, int n_live, int col0, const float* v, float* stage) {
+  if (!a.vec_ok || col0 + 32 > a.N) {
+    if ((int)(threadIdx.x & 31) < n_live) tc_finish<H>(a, row0 + (int)(threadIdx.x & 31), col0, v);
+    return;
+  }
+  if (a.ep.glu) {
+    switch (a.ep.act) {
+      case TSB200_ACT_SILU:
+      case TSB200_ACT_SWIGLU: return tc_finish_as<H, TSB200_ACT_SWIGLU, true>(a, row0, n_live, col0, v, stage);
+      case TSB200_ACT_CLAMP_GLU: return tc_finish_as<H, TSB200_ACT_CLAMP_GLU, true>(a, row0, n_live, col0, v, stage);
+      case TSB200_ACT_RELU: return tc_finish_as<H, TSB200_ACT_RELU, true>(a, row0, n_live, col0, v, stage);
+      case TSB200_ACT_LEAKYRELU: return tc_finish_as<H, TSB200_ACT_LEAKYRELU, true>(a, row0, n_live, col0, v, stage);
+      case TSB200_ACT_GELU: return tc_finish_as<H, TSB200_ACT_GELU, true>(a, row0, n_live, col0, v, stage);
+      case TSB200_ACT_SIGMOID: return tc_finish_as<H, TSB200_ACT_SIGMOID, true>(a, row0, n_live, col0, v, stage);
+      default: return tc_finish_as<H, TSB200_ACT_NONE, true>(a, row0, n_live, col0, v, stage);
     }
+  }
+  switch (a.ep.act) {
+    case TSB200_ACT_RELU: return tc_finish_as<H, TSB200_ACT_RELU, false>(a, row0, n_live, col0, v, stage);
+    case TSB200_ACT_SILU:
+    case TSB200_ACT_SWIGLU: return tc_finish_as<H, TSB200_ACT_SILU, false>(a, row0, n_live, col0, v, stage);
+    case TSB200_ACT_LEAKYRELU: return tc_finish_as<H, TSB200_ACT_LEAKYRELU, false>(a, row0, n_live, col0, v, stage);
+    case TSB200_ACT_GELU: return tc_finish_as<H, TSB200_ACT_GELU, false>(a, row0, n_live, col0, v, stage);
+    case TSB200_ACT_SIGMOID: return tc_finish_as<H, TSB200_ACT_SIGMOID, false>(a, row0, n_live, col0, v, stage);
+    default: return tc_finish_as<H, TSB200_ACT_NONE, false>(a, row0, n_live, col0, v, stage);
   }
 }
 
@@ -244,19 +256,19 @@ __global__ void __launch_bounds__(kTcThreads, 2) gemm_tc_kernel(const __grid_con
     const int row = m_tile * kBM + q * 32 + lane;
     const int n0 = n_tile * kBN;
     const bool live = ok && row < a.M;
+    const int n_live = __all_sync(0xffffffffu, ok) ? min(32, a.M - (m_tile * kBM + q * 32)) : 0;
+    float* stage = reinterpret_cast<float*>(sA) + q * 32 * kStagePitch;   // every product has read its operands
     const size_t Npad = (size_t)gridDim.x * kBN;
 #pragma unroll 1
     for (int c = 0; c < kBN; c += 32) {
       uint32_t v[32];
       tmem_ld32(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c, v);
-      if (!live) continue;
       if (a.ksplit == 1) {
         float f[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-        if (a.vec_ok && n0 + c + 32 <= a.N) tc_finish_fast<H>(a, row, n0 + c, f);
-        else tc_finish<H>(a, row, n0 + c, f);
-      } else {
+        tc_finish_rows<H>(a, row - lane, n_live, n0 + c, f, stage);
+      } else if (live) {
         // raw partial sums of this K slice; the last CTA of the tile adds the slices in a fixed order
         float4* dst = reinterpret_cast<float4*>(a.partials + ((size_t)blockIdx.z * a.M + row) * Npad + n0 + c);
 #pragma unroll
@@ -275,7 +287,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) gemm_tc_kernel(const __grid_con
         if (s_last) a.counters[tile] = 0u;
       }
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (s_last && live) {
+      if (s_last) {
         __threadfence();
 #pragma unroll 1
         for (int c = 0; c < kBN; c += 32) {
@@ -283,7 +295,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) gemm_tc_kernel(const __grid_con
 #pragma unroll
           for (int j = 0; j < 32; ++j) f[j] = 0.0f;
           // two K slices in flight per round trip, added in slice order (bitwise reproducible)
-          int z = 0;
+          int z = live ? 0 : a.ksplit;
           for (; z + 1 < a.ksplit; z += 2) {
             const float4* s0 = reinterpret_cast<const float4*>(a.partials + ((size_t)z * a.M + row) * Npad + n0 + c);
             const float4* s1 = reinterpret_cast<const float4*>(a.partials + ((size_t)(z + 1) * a.M + row) * Npad + n0 + c);
@@ -307,8 +319,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) gemm_tc_kernel(const __grid_con
               f[4 * j] += t.x; f[4 * j + 1] += t.y; f[4 * j + 2] += t.z; f[4 * j + 3] += t.w;
             }
           }
-          if (a.vec_ok && n0 + c + 32 <= a.N) tc_finish_fast<H>(a, row, n0 + c, f);
-          else tc_finish<H>(a, row, n0 + c, f);
+          tc_finish_rows<H>(a, row - lane, n_live, n0 + c, f, stage);
         }
       }
     }
@@ -462,6 +473,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_persistent_kernel(const
   } else if (w >= 4) {
     // ---------------- epilogue: warp (w - 4) owns TMEM lanes 32*(w-4) .. +31 = rows of the tile
     const int q = w - 4;
+    float* stage = reinterpret_cast<float*>(smem + kP_Stages * (kP_ABytes + kP_BBytes) + 256) + q * 32 * kStagePitch;
     int n_done = 0;
     for (int t = blockIdx.x; t < n_total; t += gridDim.x, ++n_done) {
       const TcTile tl = tc_tile_of(t, m_tiles, n_tiles);
@@ -474,22 +486,20 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_persistent_kernel(const
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       int row = tl.m_tile * kBM + q * 32 + lane;
       const int n0 = tl.n_tile * kP_BN;
-      bool live = row < a.M;
+      int n_live = min(32, a.M - (row - lane));
       if constexpr (GROUPED) {
         const RowBlock rb = g.table[tl.m_tile];
         row = rb.row0 + q * 32 + lane;
-        live = q * 32 + lane < rb.rows && row < a.M;
+        n_live = min(32, min(rb.rows - q * 32, a.M - (rb.row0 + q * 32)));
       }
 #pragma unroll 1
       for (int c = 0; c < kP_BN; c += 32) {
         uint32_t v[32];
         tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kP_BN + c), v);
-        if (!live) continue;
         float f[32];
 #pragma unroll
         for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-        if (a.vec_ok && n0 + c + 32 <= a.N) tc_finish_fast<H>(a, row, n0 + c, f);
-        else tc_finish<H>(a, row, n0 + c, f);
+        tc_finish_rows<H>(a, row - lane, n_live, n0 + c, f, stage);
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
@@ -529,7 +539,7 @@ EncodeTiledFn get_encode() {
 int init_tc_attrs(int device) {
   static bool done[kMaxDevices] = {};
   if (done[device]) return 1;
-  const int one = kTcStages * (kABytes + kBBytes) + 1024 + 256, pers = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256;
+  const int one = kTcStages * (kABytes + kBBytes) + 1024 + 256, pers = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256 + kStageBytes;
   const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
   TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__half>, dyn, one));
   TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__nv_bfloat16>, dyn, one));
@@ -605,7 +615,7 @@ int launch_gemm_tc_grouped(int device, DeviceState* st, int dtype, const void* x
   a.M = rows; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.ksplit = 1;
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
   a.vec_ok = tc_vec_ok(N, ep);
-  const size_t smem_p = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256;
+  const size_t smem_p = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256 + kStageBytes;
   gemm_tc_persistent_kernel<__nv_bfloat16, true><<<st->sm_count, kTcThreads, smem_p, s>>>(mapA, a, 0, (N + kP_BN - 1) / kP_BN, groups);
   count_launch(device);
   return check_launch("gemm_tc_grouped");
@@ -645,7 +655,7 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
     if (pers && tiles >= st->sm_count) {
       a.ksplit = 1;
       int g = st->sm_count;
-      const size_t smem_p = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256;
+      const size_t smem_p = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256 + kStageBytes;
       if (dtype == TSB200_BF16) gemm_tc_persistent_kernel<__nv_bfloat16, false><<<g, kTcThreads, smem_p, s>>>(mapA, a, m_tiles, n_tiles, RowGroups{});
       else gemm_tc_persistent_kernel<__half, false><<<g, kTcThreads, smem_p, s>>>(mapA, a, m_tiles, n_tiles, RowGroups{});
       count_launch(device);
