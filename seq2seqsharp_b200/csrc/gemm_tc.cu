@@ -25,7 +25,11 @@
 namespace tsb {
 
 constexpr int kBM = 128, kBN = 128, kBK = 64;
-constexpr int kTcStages = 3;   // 3 x 32 KB: two CTAs per SM, so one CTA's epilogue overlaps the other's mainloop
+// Stages of 32 KB.  Three: two CTAs per SM, so one CTA's epilogue overlaps the other's mainloop.  Six: one CTA per SM, taken when there are
+// no more CTAs than SMs: what bounds such a launch is the way of the operands (about 1 us from HBM), and with three stages in
+// flight a step of 64 k took 0.35 us where its products take 0.14.
+constexpr int kTcStages = 3, kTcDeepStages = 6;
+constexpr int tc_smem(int stages) { return stages * (kBM + kBN) * kBK * 2 + 1024 + 256; }
 constexpr int kTcThreads = 256;
 constexpr int kABytes = kBM * kBK * 2;  // 16 KB
 constexpr int kBBytes = kBN * kBK * 2;  // 16 KB
@@ -164,8 +168,8 @@ __device__ __forceinline__ void tc_finish_rows(const TcArgs& a, int row0, int n_
   }
 }
 
-template <typename H>
-__global__ void __launch_bounds__(kTcThreads, 2) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, TcArgs a) {
+template <typename H, int kTcStages>
+__global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, TcArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   // carve: [stages][A 16K][B 16K] (1024-byte aligned for the 128B swizzle atoms), then barriers
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -539,10 +543,12 @@ EncodeTiledFn get_encode() {
 int init_tc_attrs(int device) {
   static bool done[kMaxDevices] = {};
   if (done[device]) return 1;
-  const int one = kTcStages * (kABytes + kBBytes) + 1024 + 256, pers = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256 + kStageBytes;
+  const int pers = kP_Stages * (kP_ABytes + kP_BBytes) + 1024 + 256 + kStageBytes;
   const auto dyn = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__half>, dyn, one));
-  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__nv_bfloat16>, dyn, one));
+  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__half, kTcStages>, dyn, tc_smem(kTcStages)));
+  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__nv_bfloat16, kTcStages>, dyn, tc_smem(kTcStages)));
+  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__half, kTcDeepStages>, dyn, tc_smem(kTcDeepStages)));
+  TSB_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<__nv_bfloat16, kTcDeepStages>, dyn, tc_smem(kTcDeepStages)));
   TSB_CUDA(cudaFuncSetAttribute(gemm_tc_persistent_kernel<__half, false>, dyn, pers));
   TSB_CUDA(cudaFuncSetAttribute(gemm_tc_persistent_kernel<__nv_bfloat16, false>, dyn, pers));
   TSB_CUDA(cudaFuncSetAttribute(gemm_tc_persistent_kernel<__nv_bfloat16, true>, dyn, pers));
@@ -691,9 +697,10 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
       }
     }
   }
-  const size_t smem = kTcStages * (kABytes + kBBytes) + 1024 + 256;
-  if (dtype == TSB200_BF16) gemm_tc_kernel<__nv_bfloat16><<<grid, kTcThreads, smem, s>>>(mapA, a);
-  else gemm_tc_kernel<__half><<<grid, kTcThreads, smem, s>>>(mapA, a);
+  const bool deep = (int64_t)grid.x * grid.y * grid.z <= st->sm_count;
+  auto k = dtype == TSB200_BF16 ? (deep ? gemm_tc_kernel<__nv_bfloat16, kTcDeepStages> : gemm_tc_kernel<__nv_bfloat16, kTcStages>)
+                                : (deep ? gemm_tc_kernel<__half, kTcDeepStages> : gemm_tc_kernel<__half, kTcStages>);
+  k<<<grid, kTcThreads, tc_smem(deep ? kTcDeepStages : kTcStages), s>>>(mapA, a);
   count_launch(device);
   return check_launch("gemm_tc");
 }
