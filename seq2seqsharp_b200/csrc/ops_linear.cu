@@ -266,6 +266,151 @@ __global__ void __launch_bounds__(256) gemm_generic_kernel(GemmArgs g, Epilogue 
   }
 }
 
+// ---- fp32 linears of more than 16 rows on packed weights -----------------------------------------------------------------
+// CUDA cores (no tensor-core type keeps fp32).  A CTA takes 16 TM rows x 64 columns (half a packed tile) of a range of K tiles; the ranges
+// of an output tile are the CTAs of a cluster, whose sums meet through distributed shared memory in rank order.  A thread holds
+// TM x 4 sums and reads four k of its rows and columns with 16-byte loads (16 TM products for TM + 4 loads); four stages by cp.async.
+// What bounds it: for a prompt's few rows the way of the operands, hence the split of K until the tiles cover the SMs.  32 rows,
+// 512 -> 2048 and 2048 -> 512: 202 us on average with one CTA per 64 x 64 tile, scalar loads and no copy in flight.
+constexpr int kF32Stages = 4, kF32PitchA = 36;
+template <int TM>
+constexpr int f32_stage_floats() { return 16 * TM * kF32PitchA + 32 * 64; }
+
+__device__ __forceinline__ void f32_cp16(void* dst, const void* src, bool live) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
+}
+
+template <int TM>
+__global__ void __launch_bounds__(256) gemm_f32_kernel(const float* x, const float* Wp, int M, int N, int K, int KB, int ks, Epilogue ep) {
+  extern __shared__ __align__(16) float f32_smem[];
+  constexpr int BM = 16 * TM, kStage = f32_stage_floats<TM>();
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int rank = (int)(blockIdx.x % ks), n_tile = (int)(blockIdx.x / ks), m0 = blockIdx.y * BM;
+  const int kb0 = KB * rank / ks, kb1 = KB * (rank + 1) / ks;
+  const float* w = Wp + ((int64_t)(n_tile >> 1) * KB) * 4096 + (n_tile & 1) * 64;   // packed tile: [32 k][128 columns]
+  auto load = [&](int kb) {
+    if (kb < kb1) {
+      float* st = f32_smem + ((kb - kb0) % kF32Stages) * kStage;
+#pragma unroll
+      for (int i = tid; i < BM * 8; i += 256) {
+        const int m = i >> 3, c = (i & 7) * 4, k = kb * 32 + c;
+        const bool live = m0 + m < M && k < K;
+        f32_cp16(st + m * kF32PitchA + c, x + (live ? (int64_t)(m0 + m) * K + k : 0), live);
+      }
+#pragma unroll
+      for (int i = tid; i < 512; i += 256) f32_cp16(st + BM * kF32PitchA + i * 4, w + (int64_t)kb * 4096 + (i >> 4) * 128 + (i & 15) * 4, true);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  float acc[TM][4];
+#pragma unroll
+  for (int i = 0; i < TM; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+  for (int i = 0; i < kF32Stages - 1; ++i) load(kb0 + i);
+  for (int kb = kb0; kb < kb1; ++kb) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kF32Stages - 2) : "memory");
+    __syncthreads();
+    load(kb + kF32Stages - 1);
+    const float* A = f32_smem + ((kb - kb0) % kF32Stages) * kStage;
+    const float* B = A + BM * kF32PitchA;
+#pragma unroll
+    for (int k = 0; k < 32; k += 4) {
+      float4 a[TM], b[4];
+#pragma unroll
+      for (int i = 0; i < TM; ++i) a[i] = *reinterpret_cast<const float4*>(A + (ty * TM + i) * kF32PitchA + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) b[q] = *reinterpret_cast<const float4*>(B + (k + q) * 64 + tx * 4);
+#pragma unroll
+      for (int i = 0; i < TM; ++i) {
+        const float av[4] = {a[i].x, a[i].y, a[i].z, a[i].w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc[i][0] = fmaf(av[q], b[q].x, acc[i][0]);
+          acc[i][1] = fmaf(av[q], b[q].y, acc[i][1]);
+          acc[i][2] = fmaf(av[q], b[q].z, acc[i][2]);
+          acc[i][3] = fmaf(av[q], b[q].w, acc[i][3]);
+        }
+      }
+    }
+  }
+  __syncthreads();   // the stages are read
+  float4* mine = reinterpret_cast<float4*>(f32_smem);   // [BM][16] groups of four columns
+#pragma unroll
+  for (int i = 0; i < TM; ++i) mine[(ty * TM + i) * 16 + tx] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  if (ks > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  } else {
+    __syncthreads();
+  }
+  // this CTA finishes rows rank * BM / ks ..
+  const float* bias = reinterpret_cast<const float*>(ep.bias);
+  const int rows = BM / ks, No = ep.glu ? N / 2 : N;
+  for (int i = tid; i < rows * 16; i += 256) {
+    const int at = rank * rows * 16 + i, m = m0 + (at >> 4), c = n_tile * 64 + (at & 15) * 4;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int r = 0; r < ks; ++r) {
+      float4 t;
+      if (ks == 1) {
+        t = mine[at];
+      } else {
+        uint32_t ra;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"((uint32_t)__cvta_generic_to_shared(mine + at)), "r"(r));
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(t.x), "=f"(t.y), "=f"(t.z), "=f"(t.w) : "r"(ra) : "memory");
+      }
+      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+    }
+    if (m >= M) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c + j < N && bias) v[j] += bias[c + j];
+    if (!ep.glu) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < N) ep_store<float>(ep, (size_t)m * N + c + j, ep_act(v[j], ep.act));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j += 2)
+        if (c + j + 1 < N) ep_store<float>(ep, (size_t)m * No + ((c + j) >> 1), ep_glu(v[j], v[j + 1], ep));
+    }
+  }
+  if (ks > 1) {   // the others have read this CTA's sums
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+}
+
+template <int TM>
+static int launch_gemm_f32(int device, DeviceState* st, const float* x, const float* Wp, int M, int K, int N, const Epilogue& ep, cudaStream_t s) {
+  constexpr int smem = kF32Stages * f32_stage_floats<TM>() * 4;
+  static bool done[kMaxDevices] = {};
+  if (!done[device]) {
+    TSB_CUDA(cudaFuncSetAttribute(gemm_f32_kernel<TM>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    done[device] = true;
+  }
+  const int KB = (K + 31) / 32, n_tiles = (N + 63) / 64, m_tiles = (M + 16 * TM - 1) / (16 * TM);
+  // K ranges while the tiles do not cover the SMs, at least four tiles of 32 k each
+  int ks = 1;
+  while (ks < 8 && (int64_t)n_tiles * m_tiles * ks * 2 <= st->sm_count + st->sm_count / 2 && KB / (ks * 2) >= 4) ks *= 2;
+  TSB_CHECK(m_tiles <= 65535, "linear: too many rows (%d)", M);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(n_tiles * ks, m_tiles);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, gemm_f32_kernel<TM>, x, Wp, M, N, K, KB, ks, ep));
+  count_launch(device);
+  return check_launch("gemm_f32");
+}
+
 // ------------------------------------------------------------------------------------------------ host side
 struct GemvPlan {
   int ctiles, ksplit, kchunk;
@@ -396,6 +541,11 @@ int launch_linear(int device, DeviceState* st, int dtype, const void* x, const v
 #undef TSB_GEMV
     }
     return 1;
+  }
+  // rows of whole 16-byte pieces; 64 rows per tile once there are enough tiles to cover the SMs with them
+  if (packed && dtype == TSB200_F32 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && (int64_t)M <= 65535 * 32) {
+    if ((int64_t)((M + 63) / 64) * ((N + 63) / 64) >= st->sm_count) return launch_gemm_f32<4>(device, st, (const float*)x, (const float*)W, M, K, N, ep, s);
+    return launch_gemm_f32<2>(device, st, (const float*)x, (const float*)W, M, K, N, ep, s);
   }
   GemmArgs g{};
   g.A = x; g.B = W; g.src = nullptr; g.C = nullptr;

@@ -1,4 +1,5 @@
-"""Linears at the edges of the rules that choose their kernels: deep and shallow rings of the tensor-core kernel and its epilogues."""
+"""Linears at the edges of the rules that choose their kernels: fp32 rows beyond 16 (clusters over K), deep and shallow rings of the
+tensor-core kernel and its epilogues."""
 import numpy as np
 import pytest
 import torch
@@ -7,6 +8,22 @@ from seq2seqsharp_b200 import _native as N
 from tests.test_fused_gpu import dev, host, linear_packed
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,K,Nn", [(17, 4, 8), (32, 512, 2048), (33, 2048, 512), (64, 100, 130), (65, 96, 64), (200, 132, 1001), (1000, 512, 1536), (40, 36, 5), (20, 131, 72)])
+def test_fp32_rows(cuda, oracle, M, K, Nn):
+    rng = np.random.default_rng(M + K + Nn)
+    x, W = dev(rng.standard_normal((M, K)).astype(np.float32)), dev((rng.standard_normal((K, Nn)) * 0.05).astype(np.float32))
+    b, res = dev((rng.standard_normal((1, Nn)) * 0.1).astype(np.float32)), dev(rng.standard_normal((M, Nn)).astype(np.float32))
+    ref = host(x).astype(np.float64) @ host(W).astype(np.float64) + host(b)
+    tol = K * 2.0 ** -23 * float(np.abs(host(x)).max() * np.abs(host(W)).max()) + 1e-6     # every one of K roundings at its largest
+    got = host(linear_packed(x, W, b, N.ACT_NONE))
+    np.testing.assert_allclose(got, ref, atol=tol)
+    np.testing.assert_array_equal(host(linear_packed(x, W, b, N.ACT_NONE)), got)
+    np.testing.assert_allclose(host(linear_packed(x, W, b, N.ACT_NONE, residual=res, want_f32=True)), ref + host(res), atol=tol)
+    np.testing.assert_allclose(host(linear_packed(x, W, b, N.ACT_RELU)), np.maximum(ref, 0), atol=tol)
+    if Nn % 2 == 0:
+        np.testing.assert_allclose(host(linear_packed(x, W, b, N.ACT_GLU_NOACT)), ref[:, 0::2] * ref[:, 1::2], atol=2 * tol * max(1.0, np.abs(ref).max()))
 
 
 @pytest.mark.parametrize("M,K,Nn", [(129, 32, 128), (129, 96, 160), (256, 1056, 2048), (257, 256, 1009), (1300, 128, 1920), (1301, 128, 2048), (70, 4096, 512), (2000, 2080, 2592)])
