@@ -736,17 +736,6 @@ static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid
       return r;
     }
   }
-  if (ng && dt == TSB200_F16 && rows <= 8 && g->fuse_step) {
-    // up to eight rows: the tensor-core streaming kernel norms the rows itself (no norm launch)
-    prof_begin(g, KC_LINEAR);
-    const int r = launch_gemm_stream_mma_norm(dev, g->st, x_resid, ng, c.norm_type == 0 ? nb : nullptr, c.norm_type, c.eps, Wp, rows, K, N, ep,
-                                              g->err_flag, g->pdl, g->lin_ws, g->lin_ws_bytes, g->s);
-    if (r != 2) {
-      g->lin_syms_used = true;
-      prof_end(g, KC_LINEAR);
-      return r;
-    }
-  }
   if (ng) {
     PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, h_tmp, const_cast<float*>(x_resid), nullptr, ng, c.norm_type == 0 ? nb : nullptr,
                                        c.norm_type, c.eps, rows, K, g->s));
@@ -976,21 +965,25 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     void* kp = (char*)g->qkv + (int64_t)Hd * g->es;
     void* vp = (char*)g->qkv + (int64_t)(Hd + KVd) * g->es;
     bool appended = false;
-    if (S == 1 && dt == TSB200_F16 && rows <= 8 && g->fuse_step) {
-      // one new position per sequence, up to eight sequences: norm, q | k | v projection, RoPE and the cache append in one launch
+    if (S == 1 && dt == TSB200_F16 && rows <= 64 && g->fuse_step) {
+      // one new position per sequence: RoPE and the cache append in the epilogue of the q | k | v projection
       RopeFuse rf{};
       rf.cK = L.cK; rf.cV = L.cV; rf.Hd = Hd; rf.KVd = KVd; rf.hd = c.hd; rf.Tmax = c.max_tokens;
       rf.use_rope = c.pe_type == 2 ? 1 : 0; rf.T0 = T0; rf.state = dT; rf.tab = g->rope_tab;
+      PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, g->h, g->x, nullptr, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, rows, d, g->s));
       prof_begin(g, KC_LINEAR);
-      const int r = launch_gemm_stream_mma_norm(dev, g->st, g->x, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, L.wqkv, rows, d,
-                                                g->Nqkv, make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0), g->err_flag, g->pdl, g->lin_ws,
-                                                g->lin_ws_bytes, g->s, &rf);
+      const Epilogue ep = make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0);
+      const int r = launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
       if (r == 0) return 0;
-      if (r == 1) {
-        g->lin_syms_used = true;
+      g->lin_syms_used = true;
+      if (r == 2) {
+        TSB_TRY(launch_linear(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->lin_ws, g->lin_ws_bytes, g->s, true));
         prof_end(g, KC_LINEAR);
-        appended = true;
+        PROF(KC_ROPE_APPEND, launch_rope_append(dev, g->st, dt, qp, kp, vp, g->Nqkv, g->Nqkv, L.cK, L.cV, B, S, c.H, c.Hkv, c.hd, T0, dT, c.max_tokens, c.pe_type == 2, (double)c.rope_base, g->rope_tab, g->s));
+      } else {
+        prof_end(g, KC_LINEAR);
       }
+      appended = true;
     }
     if (!appended) {
       TSB_TRY(engine_linear(g, rows, nullptr, g->x, L.n1_g, L.n1_b, g->h, L.wqkv, d, g->Nqkv, make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0)));
@@ -1071,7 +1064,6 @@ static int check_err_flag(Gpt* g, const int* pre = nullptr) {
   if (g->lin_syms_used) {
     e |= tc_take_error();
     e |= gs_take_error();
-    e |= stc_take_error();
     g->lin_syms_used = false;
   }
   if (g->tp > 1) e |= comm_peer_take_error();

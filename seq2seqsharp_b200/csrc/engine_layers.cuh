@@ -415,7 +415,6 @@ static int ensure_sandwich(Gpt* g, int B, int S, int T) {
   auto lin = [&](int64_t K, int64_t N) {
     for (int64_t m : {(int64_t)1, std::min<int64_t>(rows, 64)}) {
       ws = std::max(ws, linear_workspace_bytes((int)m, (int)K, (int)N));
-      if (is_16bit(dt)) ws = std::max(ws, gemm_stream_sections_workspace_bytes((int)m, (int)K, (int)N, g->st->sm_count));
     }
   };
   lin(d, ly->c.V);
@@ -467,7 +466,6 @@ static int ensure_layered(Gpt* g, int B, int S, int T, bool step) {
   auto lin = [&](int64_t K, int64_t N) {
     for (int64_t m : {(int64_t)1, std::min<int64_t>(rows, 64)}) {
       ws = std::max(ws, linear_workspace_bytes((int)m, (int)K, (int)N));
-      if (is_16bit(dt)) ws = std::max(ws, gemm_stream_mma_workspace_bytes((int)m, (int)K, (int)N, g->st->sm_count));
     }
   };
   lin(d, ly->c.V);
@@ -480,10 +478,7 @@ static int ensure_layered(Gpt* g, int B, int S, int T, bool step) {
     } else {
       nkv = std::max(nkv, (int64_t)B * T * L.sh.H * (L.sh.dim + L.sh.vdim));
       if (B > 1) ncomp = std::max(ncomp, (int64_t)B * T * L.sh.row);
-      for (int64_t m : {(int64_t)16, (int64_t)64})
-        ws = std::max(ws, gemm_stream_mma_workspace_bytes((int)m, L.sh.row, L.sh.H * (L.sh.dim + L.sh.vdim), g->st->sm_count));
     }
-    if (is_16bit(dt)) ws = std::max(ws, gemm_stream_sections_workspace_bytes((int)std::min<int64_t>(rows, 64), (int)d, (int)(2 * d + L.Nq + L.Nkv), g->st->sm_count));
     lin(d, d);
     lin(d, L.Nq + L.Nkv);
     lin(L.sh.H * L.sh.vdim, d);
@@ -605,7 +600,7 @@ static int gated_layers(Gpt* g, LayerPass& ps) {
       if (rows <= 64 && ff) {
         const LinearSection sec[3] = {{d, e1, 0}, {d, e2, 1}, {Nqkv, e3, 2}};
         prof_begin(g, KC_LINEAR);
-        r = launch_gemm_stream_sections(dev, g->st, dt, h1, L.fused, rows, d, sec, 3, pdl, ws, wsb, g->s);
+        r = launch_gemm_cluster_sections(dev, g->st, dt, h1, L.fused, rows, d, sec, 3, pdl, g->s);
         if (r == 0) return 0;
         if (r == 1) prof_end(g, KC_LINEAR);
       }
@@ -695,7 +690,7 @@ static int sandwich_layers(Gpt* g, LayerPass& ps) {
       const Epilogue eg = make_ep(L.gates_b, nullptr, nullptr, (float*)ly->gates.p, TSB200_ACT_NONE, 0);
       const LinearSection sec[2] = {{L.Nq, eq, 0}, {2 * L.ms.H, eg, 0}};
       prof_begin(g, KC_LINEAR);
-      const int r = launch_gemm_stream_sections(dev, g->st, dt, h, L.fused, rows, d, sec, 2, g->pdl, ws, wsb, g->s);
+      const int r = launch_gemm_cluster_sections(dev, g->st, dt, h, L.fused, rows, d, sec, 2, g->pdl, g->s);
       if (r == 0) return 0;
       if (r == 1) prof_end(g, KC_LINEAR);
       if (r == 2) {

@@ -1,20 +1,17 @@
-// Linear layer for decode batches of 5..64 rows on packed fp16 or bf16 weights: y[M,N] = epilogue(x[M,K] * W[K,N]).
-//
-// At these row counts the product is still bound by streaming the weights once (HBM), but there are too many rows
-// for FMA pipes and too few output tiles for a tile-per-CTA tensor-core GEMM (its split-K variants spend most of their
-// time in pipeline fill, drain and partial-sum hand-over).  So this kernel keeps the structure of the streaming GEMV:
+// Stream-K products on packed 16-bit weights with mma.sync consumers: the row blocks of a mixture of experts (at most 16 rows each, weights
+// of one expert per block), and the linear of up to 8 fp16 rows that norms its rows itself (TSB200_LinearPacked).
 //   * persistent CTAs, one per SM, each owning a contiguous, evenly sized range of the packed 16 KB weight tiles
 //     (stream-K over column-tile-major order);
 //   * a producer lane feeds a shared-memory ring: per stage one linear bulk copy of a weight tile (stored as its
-//     128-byte-swizzled shared-memory image) and one TMA tensor copy of the matching activation tile [rows][32 k]
-//     (64-byte swizzle, rows beyond M zero-filled);
+//     128-byte-swizzled shared-memory image) and, without the norm, one TMA tensor copy of the matching activation tile
+//     [rows][32 k] (64-byte swizzle, rows beyond the block zero-filled or unread);
 //   * eight consumer warps, 32 columns each: ldmatrix.trans of the weight fragments, ldmatrix of the activation
-//     fragments, mma.sync m16n8k16 with fp32 accumulators for up to 8 row blocks;
+//     fragments, mma.sync m16n8k16 with fp32 accumulators;
 //   * at the end of a CTA's share of a column tile the accumulators go to a scratch slot; the CTA that delivers the
 //     last share adds the slots in fixed order (bitwise reproducible) and applies bias / activation / gate / residual.
 // Every mbarrier wait is bounded; on timeout the error word is raised and the CTA drains and returns.
-//
-// Replaces cublasGemmEx + bias / activation kernels for decode batches (TensorSharp.CUDA/MatrixMul/CudaMatrixMulMM.cs:305-362).
+// The plain linears of a decode step run in gemm_cluster_tc.cu: there the sums meet without a last arriver, whose slots, bias and stores
+// took 6 to 7 us of every launch here.
 #include <cuda.h>
 
 #include <cstdlib>
@@ -30,21 +27,13 @@ constexpr int kGsStageBytes = kTileBytes + kGsXBytes;
 // Raised by a kernel whose bounded wait ran out; read and cleared by gs_take_error().
 __device__ int g_gs_error;
 
-// what a launch computes: one linear / several linears of equal K on stacked row blocks / the blocks of a row-grouped product
-constexpr int kGsPlain = 0, kGsSections = 1, kGsGrouped = 2;
-constexpr int kGsMaxSections = 4;
-struct GsSection {
-  int ct_end;   // first column tile after the section
-  int N;
-  int x_block;  // stacked row block it reads
-  Epilogue ep;
-};
+// what a launch computes: one linear whose rows are normed here / the blocks of a row-grouped product
+constexpr int kGsPlain = 0, kGsGrouped = 1;
 
 struct GsArgs {
   const unsigned char* Wp;
   int M, K, N, KB, CT;
   int stages, max_contrib;
-  int prefetch;             // 1: the first ring-full of weight tiles is requested before the wait on the previous kernel
   // KQ > 0 instantiations: the rows come from the fp32 residual stream and are normed here (no activation tiles by TMA)
   const float* xres;        // [M][K]
   const void* gamma;
@@ -57,8 +46,6 @@ struct GsArgs {
   unsigned int* counters;   // [CT], zero on entry, self-resetting
   int* error_flag;
   Epilogue ep;
-  int n_sec;                // kGsSections
-  GsSection sec[kGsMaxSections];
   RowGroups groups;         // kGsGrouped: CT counts the column tiles of ONE matrix
 };
 
@@ -88,7 +75,6 @@ __device__ __forceinline__ void gs_consumers_sync() { asm volatile("bar.sync 1, 
 // rows are read from the fp32 residual stream, normed by the consumer warps (LayerNorm / RMSNorm, the arithmetic of
 // norm_kernel) and kept in shared memory as fp16 for the whole kernel - the norm launch in front of the linear disappears and
 // a stage is the weight tile alone.
-// MODE kGsSections: column tile ct belongs to section i (the first with ct < ct_end), which reads activation rows x_block * M ..;
 // MODE kGsGrouped: "column tiles" run over (row block, column tile of its matrix) pairs; how many there are is read from the device.
 template <typename H, int NB, int KQ = 0, int MODE = kGsPlain>  // row blocks of 8: M <= 8 * NB
 __global__ void __launch_bounds__(kStreamThreads, 1) gemm_stream_mma_kernel(const __grid_constant__ CUtensorMap mapX, GsArgs a) {
@@ -140,11 +126,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_stream_mma_kernel(cons
   };
   auto tile_row = [&](int vct) {
     if constexpr (MODE == kGsGrouped) return a.groups.table[vct / a.CT].row0;
-    if constexpr (MODE == kGsSections) {
-      int i = 0;
-      while (i < a.n_sec - 1 && vct >= a.sec[i].ct_end) ++i;
-      return a.sec[i].x_block * a.M;
-    }
     return 0;
   };
 
@@ -158,7 +139,7 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_stream_mma_kernel(cons
       // The weights do not depend on the previous kernel: the first ring-full of tiles is requested before the wait on it,
       // so the stream starts while that kernel's last CTAs still reduce and store (and while a norm kernel in between runs).
       constexpr unsigned TX = NORM ? kTileBytes : kTileBytes + NB * 8 * 64;
-      const int n_pre = MODE != kGsGrouped && (a.prefetch || NORM) ? min(S, u_end - u_begin) : 0;
+      const int n_pre = NORM ? min(S, u_end - u_begin) : 0;
       for (int i = 0; i < n_pre; ++i) {
         mbar_expect_tx(&full[i], TX);
         bulk_g2s(smem + (size_t)i * STAGE, src + (size_t)i * kTileBytes, kTileBytes, &full[i]);
@@ -398,12 +379,8 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_stream_mma_kernel(cons
     gs_consumers_sync();
     if (*(volatile int*)&s_last) {
       const float* all = a.partials + ((size_t)cur_ct * max_contrib * MS) * NT;
-      int si = 0;
-      if constexpr (MODE == kGsSections)
-        while (si < a.n_sec - 1 && cur_ct >= a.sec[si].ct_end) ++si;
-      const Epilogue& ep = MODE == kGsSections ? a.sec[si].ep : a.ep;
-      const int N = MODE == kGsSections ? a.sec[si].N : a.N;
-      const int lct = MODE == kGsSections ? (si ? cur_ct - a.sec[si - 1].ct_end : cur_ct) : (MODE == kGsGrouped ? cur_ct % a.CT : cur_ct);
+      const Epilogue& ep = a.ep;
+      const int N = a.N, lct = MODE == kGsGrouped ? cur_ct % a.CT : cur_ct;
       const H* bias = reinterpret_cast<const H*>(ep.bias);
       const int No = ep.glu ? N / 2 : N;
       // work items: (row, group of 4 columns); per item up to eight slots are read at once and added in slot order
@@ -479,218 +456,6 @@ __global__ void __launch_bounds__(kStreamThreads, 1) gemm_stream_mma_kernel(cons
   }
 }
 
-// ---- column-chunk variant for 17..64 rows ------------------------------------------------------------------------------
-// With many rows the stream-K hand-over is expensive: every CTA leaves M x 256 floats per shared column tile and the
-// last arriver adds up to ten such slots alone.  Here a CTA owns ONE 64-column box of the packed tiles (4 KB per k tile,
-// contiguous) over a K range, so a box has few contributors (ksplit, usually 1..4) and a partial is M x 64 floats.
-// Stage = two k tiles of the box (2 x 4 KB bulk copies) + the activation tile [rows][64 k] (TMA tensor copy, 128-byte
-// swizzle).  Four consumer warps own 16 columns each; three CTAs fit on an SM, so one CTA's prologue and epilogue
-// overlap the others' streaming.
-constexpr int kGcThreads = 160;            // 4 consumer warps + producer warp
-constexpr int kGcStages = 4;
-constexpr int kGcStageBytes = 8192 + 8192; // W: 2 k tiles x 4 KB; x: 64 rows x 128 B
-
-struct GcArgs {
-  const unsigned char* Wp;
-  int M, K, N, KB, CT;
-  int ksplit, k2_per;        // K ranges per box; stages (pairs of k tiles) per range
-  int prefetch;              // 1: the first ring-full of weight tiles is requested before the wait on the previous kernel
-  float* partials;           // [boxes][ksplit][M][64]
-  unsigned int* counters;    // [boxes], zero on entry, self-resetting
-  int* error_flag;
-  Epilogue ep;
-  int n_sec;                 // kGsSections
-  GsSection sec[kGsMaxSections];
-};
-
-template <typename H, int NB, int MODE>
-__global__ void __launch_bounds__(kGcThreads, 3) gemm_chunk_mma_kernel(const __grid_constant__ CUtensorMap mapX, GcArgs a) {
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + kGcStages * kGcStageBytes);
-  uint64_t* empty = full + kGcStages;
-  float* red = reinterpret_cast<float*>(smem);  // [M][64] after the main loop (the stages are free then)
-  __shared__ int s_err, s_last;
-
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int M = a.M, KB = a.KB;
-  const int box = blockIdx.x / a.ksplit, ks = blockIdx.x % a.ksplit;   // the K ranges of a box run side by side
-  const int ct = box >> 2, j = box & 3;
-  int si = 0;
-  if constexpr (MODE == kGsSections)
-    while (si < a.n_sec - 1 && ct >= a.sec[si].ct_end) ++si;
-  const int xrow = MODE == kGsSections ? a.sec[si].x_block * M : 0;
-  const int k2_total = (KB + 1) / 2;
-  const int k2_beg = ks * a.k2_per, k2_end = min(k2_total, k2_beg + a.k2_per);
-  const int n_st = max(k2_end - k2_beg, 0);
-
-  if (tid == 0) {
-    for (int i = 0; i < kGcStages; ++i) {
-      mbar_init(&full[i], 1);
-      mbar_init(&empty[i], 4);
-    }
-    s_err = 0;
-    s_last = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  grid_dep_launch();
-  if (!(w == 4 && lane == 0)) grid_dep_wait();  // scratch slots, counters and residual rows belong to earlier kernels too
-
-  if (w == 4) {
-    if (lane == 0) {
-      const unsigned char* wsrc = a.Wp + ((size_t)ct * KB) * kTileBytes + (size_t)j * 4096;
-      auto put_w = [&](int i) {
-        const int s = i % kGcStages;
-        const int kb0 = (k2_beg + i) * 2;
-        const bool two = kb0 + 1 < KB;
-        unsigned char* dst = smem + (size_t)s * kGcStageBytes;
-        mbar_expect_tx(&full[s], (two ? 8192 : 4096) + NB * 8 * 128);
-        bulk_g2s(dst, wsrc + (size_t)kb0 * kTileBytes, 4096, &full[s]);
-        if (two) bulk_g2s(dst + 4096, wsrc + (size_t)(kb0 + 1) * kTileBytes, 4096, &full[s]);
-      };
-      // the weights do not depend on the previous kernel: the first ring-full is requested before the wait on it
-      const int n_pre = a.prefetch ? min(kGcStages, n_st) : 0;
-      for (int i = 0; i < n_pre; ++i) put_w(i);
-      grid_dep_wait();  // the activation rows come from the previous kernel
-      int done = 0;
-      for (int i = 0; i < n_st; ++i) {
-        const int s = i % kGcStages, r = i / kGcStages;
-        if (i >= kGcStages && !mbar_wait(&empty[s], (unsigned)((r - 1) & 1))) {
-          s_err = 1;
-          break;
-        }
-        if (i >= n_pre) put_w(i);
-        gs_tma_load_2d(smem + (size_t)s * kGcStageBytes + 8192, &mapX, (k2_beg + i) * 2 * kKT, xrow, &full[s]);  // x = kb0 * 32 halves: a 64-byte multiple
-        done = i + 1;
-      }
-      if (*(volatile int*)&s_err) {
-        // stages requested ahead get their activation tile too, so that every copy into this CTA has landed on return
-        for (int i = done; i < n_pre; ++i) gs_tma_load_2d(smem + (size_t)(i % kGcStages) * kGcStageBytes + 8192, &mapX, 0, 0, &full[i % kGcStages]);
-        if (done < n_pre) done = n_pre;
-        const int first = done > kGcStages ? done - kGcStages : 0;
-        for (int i = first; i < done; ++i) mbar_wait(&full[i % kGcStages], (unsigned)((i / kGcStages) & 1), 1u << 16);
-        g_gs_error = 1;
-        if (a.error_flag) *a.error_flag = 1;
-      }
-    }
-  } else {
-    // ---------------- consumer warps: warp w owns columns [w*16, w*16+16) of the box
-    const int g8 = lane >> 2, t4 = lane & 3;
-    const int lrow = (lane & 7) + ((lane >> 4) << 3);
-    const int lunit = (lane >> 3) & 1;
-    const int xr = lane & 7, xc = lane >> 3;
-    float d[NB][4];
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) d[nb][e] = 0.0f;
-    bool dead = false;
-    for (int i = 0; i < n_st; ++i) {
-      const int s = i % kGcStages, r = i / kGcStages;
-      if (*(volatile int*)&s_err) dead = true;
-      if (!mbar_wait(&full[s], (unsigned)(r & 1), dead ? 4096u : kSpinLimit)) {
-        s_err = 1;
-        dead = true;
-      }
-      const uint32_t wbase = smem_u32(smem + (size_t)s * kGcStageBytes);
-      const uint32_t xbase = wbase + 8192;
-      const int kk_end = ((k2_beg + i) * 2 + 1 < KB) ? 4 : 2;  // a missing second k tile was not copied
-#pragma unroll
-      for (int h2 = 0; h2 < 2; ++h2) {            // the two k tiles of the stage
-        if (h2 * 2 >= kk_end) break;
-        // activation fragments of this k tile: rows of 128 B, 16-byte chunks XOR-ed with row & 7
-        uint32_t bf[NB][4];
-#pragma unroll
-        for (int nb = 0; nb < NB; ++nb) {
-          const int n = nb * 8 + xr;
-          const int c = h2 * 4 + xc;
-          gs_ldmatrix_x4(xbase + n * 128 + ((c ^ (n & 7)) << 4), bf[nb][0], bf[nb][1], bf[nb][2], bf[nb][3]);
-        }
-#pragma unroll
-        for (int kk = 0; kk < 2; ++kk) {
-          const int k = kk * 16 + lrow;
-          const int unit = w * 2 + lunit;
-          uint32_t a0, a1, a2, a3;
-          gs_ldmatrix_x4_trans(wbase + h2 * 4096 + k * 128 + ((unit ^ (k & 7)) << 4), a0, a1, a2, a3);
-#pragma unroll
-          for (int nb = 0; nb < NB; ++nb) mma_16816<H>(d[nb], a0, a1, a2, a3, bf[nb][2 * kk], bf[nb][2 * kk + 1]);
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&empty[s]);
-    }
-    // ---- accumulators -> red[row][64] (the stages are free: every copy has been consumed)
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-#pragma unroll
-    for (int nb = 0; nb < NB; ++nb)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int row = nb * 8 + 2 * t4 + (e & 1);
-        if (row < M) red[row * 64 + w * 16 + g8 + (e >> 1) * 8] = d[nb][e];
-      }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    bool finish = a.ksplit == 1;
-    if (a.ksplit > 1) {
-      float* mine = a.partials + ((size_t)blockIdx.x * M) * 64;   // [box][ks] = blockIdx.x
-      for (int idx = tid; idx < M * 16; idx += 128) reinterpret_cast<float4*>(mine)[idx] = reinterpret_cast<const float4*>(red)[idx];
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (tid == 0) {
-        const unsigned int prev = gs_atom_add_acq_rel(&a.counters[box], 1u);
-        const int last = (prev == (unsigned int)(a.ksplit - 1));
-        if (last) a.counters[box] = 0u;
-        s_last = last;
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (*(volatile int*)&s_last) {
-        const float4* all = reinterpret_cast<const float4*>(a.partials + ((size_t)box * a.ksplit * M) * 64);
-        for (int idx = tid; idx < M * 16; idx += 128) {
-          float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-          for (int z = 0; z < a.ksplit; ++z) {
-            const float4 t = __ldcg(all + (size_t)z * M * 16 + idx);
-            acc.x += t.x; acc.y += t.y; acc.z += t.z; acc.w += t.w;
-          }
-          reinterpret_cast<float4*>(red)[idx] = acc;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        finish = true;
-      }
-    }
-    if (finish) {
-      const Epilogue& ep = MODE == kGsSections ? a.sec[si].ep : a.ep;
-      const int N = MODE == kGsSections ? a.sec[si].N : a.N;
-      const int lct = MODE == kGsSections && si ? ct - a.sec[si - 1].ct_end : ct;
-      const H* bias = reinterpret_cast<const H*>(ep.bias);
-      const int No = ep.glu ? N / 2 : N;
-      for (int idx = tid; idx < M * 16; idx += 128) {
-        const int row = idx >> 4, c = lct * 256 + j * 64 + (idx & 15) * 4;
-        const float4 t = reinterpret_cast<const float4*>(red)[idx];
-        const float v[4] = {t.x, t.y, t.z, t.w};
-        if (!ep.glu) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (c + e < N) {
-              ep_store<H>(ep, (size_t)row * N + c + e, ep_act(v[e] + (bias ? to_f<H>(bias[c + e]) : 0.0f), ep.act));
-            }
-          }
-        } else {
-#pragma unroll
-          for (int e = 0; e < 4; e += 2) {
-            if (c + e + 1 < N) {
-              const float av = v[e] + (bias ? to_f<H>(bias[c + e]) : 0.0f), gv = v[e + 1] + (bias ? to_f<H>(bias[c + e + 1]) : 0.0f);
-              ep_store<H>(ep, (size_t)row * No + ((c + e) >> 1), ep_glu(av, gv, ep));
-            }
-          }
-        }
-      }
-    }
-    if (tid == 0 && *(volatile int*)&s_err) {
-      g_gs_error = 1;
-      if (a.error_flag) *a.error_flag = 1;
-    }
-  }
-}
-
 // ---- host side ---------------------------------------------------------------------------------------------------------
 typedef CUresult (*GsEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                     const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
@@ -756,163 +521,7 @@ int64_t gemm_stream_mma_workspace_bytes(int M, int K, int N, int sm_count) {
   if (g > KB * CT) g = KB * CT;
   const long long per = (KB * CT) / (g > 0 ? g : 1);
   const long long mc = KB / (per > 0 ? per : 1) + 2;
-  const long long chunk = (long long)((N + 63) / 64) * 8 * M * 64 * 4;  // column-chunk variant: up to 8 K ranges per box
-  const long long stream = CT * mc * M * 256 * 4;
-  return kWsCounterBytes + (chunk > stream ? chunk : stream) + 256;
-}
-
-static int gs_prefetch_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("TSB200_GEMM_PREFETCH");  // "0": weights are requested only after the previous kernel has ended (A/B measurements)
-    on = (e && e[0] == '0') ? 0 : 1;
-  }
-  return on;
-}
-
-template <typename H, int NB, int MODE = kGsPlain>
-static int gc_launch(int device, const CUtensorMap& mapX, const GcArgs& a, int grid, bool pdl, cudaStream_t s) {
-  static bool attr_done[kMaxDevices] = {};
-  const size_t smem = kGcStages * kGcStageBytes + 1024 + 128;
-  if (!attr_done[device]) {
-    TSB_CUDA(cudaFuncSetAttribute(gemm_chunk_mma_kernel<H, NB, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done[device] = true;
-  }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(kGcThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = (pdl && pdl_enabled()) ? 1 : 0;
-  TSB_CUDA(cudaLaunchKernelEx(&cfg, gemm_chunk_mma_kernel<H, NB, MODE>, mapX, a));
-  count_launch(device);
-  return 1;
-}
-
-static int gc_map_x(CUtensorMap* map, int dtype, const void* x, int rows, int K, int NB) {
-  GsEncodeTiledFn enc = gs_get_encode();
-  if (!enc) return 2;
-  const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)(NB * 8)};
-  const cuuint32_t el[2] = {1, 1};
-  const CUresult r = enc(map, gs_map_type(dtype), 2, const_cast<void*>(x), dims, strides, box, el, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TSB_CHECK(r == CUDA_SUCCESS, "gemm_chunk: cuTensorMapEncodeTiled failed with %d", (int)r);
-  return 1;
-}
-// K ranges per box and scratch; 1 ok, 2 the scratch does not suffice
-static int gc_plan(GcArgs* a, DeviceState* st, int boxes, void* ws, int64_t ws_bytes) {
-  const int k2_total = (a->KB + 1) / 2;
-  // about two CTAs per SM in flight (three fit); a K range is at least 8 stages long
-  int ks = (2 * st->sm_count + boxes - 1) / boxes;
-  if (ks > k2_total / 8) ks = k2_total / 8;
-  if (ks < 1) ks = 1;
-  if (ks > 8) ks = 8;
-  a->k2_per = (k2_total + ks - 1) / ks;
-  ks = (k2_total + a->k2_per - 1) / a->k2_per;     // no empty range
-  a->ksplit = ks;
-  a->prefetch = gs_prefetch_enabled();
-  const int64_t need = kWsCounterBytes + (int64_t)boxes * ks * a->M * 64 * 4;
-  if (ks > 1 && (!ws || ws_bytes < need || (int64_t)boxes * 4 > kWsCounterBytes - 256)) return 2;
-  a->counters = reinterpret_cast<unsigned int*>(ws);
-  a->partials = ws ? reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + kWsCounterBytes) : nullptr;
-  return 1;
-}
-
-// Column-chunk variant (17..64 rows).  1 ok, 0 error, 2 not handled.
-static int launch_gemm_chunk_mma(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep,
-                                 int* error_flag, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s) {
-  const int NB = M <= 32 ? 4 : 8;
-  GcArgs a{};
-  a.Wp = reinterpret_cast<const unsigned char*>(Wp);
-  a.M = M; a.K = K; a.N = N;
-  a.KB = (K + kKT - 1) / kKT;
-  a.CT = (N + 255) / 256;
-  const int boxes = (N + 63) / 64;                 // boxes that hold real columns (the last column tile may have fewer than 4)
-  if (gc_plan(&a, st, boxes, ws, ws_bytes) != 1) return 2;
-  a.error_flag = error_flag;
-  a.ep = ep;
-  CUtensorMap mapX;
-  const int r = gc_map_x(&mapX, dtype, x, M, K, NB);
-  if (r != 1) return r;
-  const int grid = boxes * a.ksplit;
-  if (dtype == TSB200_BF16) return NB == 4 ? gc_launch<__nv_bfloat16, 4>(device, mapX, a, grid, pdl, s) : gc_launch<__nv_bfloat16, 8>(device, mapX, a, grid, pdl, s);
-  return NB == 4 ? gc_launch<__half, 4>(device, mapX, a, grid, pdl, s) : gc_launch<__half, 8>(device, mapX, a, grid, pdl, s);
-}
-
-// 1 ok, 0 error, 2 shape not handled (caller falls back).
-int launch_gemm_stream_mma(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep,
-                           int* error_flag, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s) {
-  {
-    static int enabled = -1;
-    if (enabled < 0) {
-      const char* e = getenv("TSB200_GEMM_STREAM");  // "0": decode batches go to the tile-per-CTA tensor-core GEMM (A/B measurements)
-      enabled = (e && e[0] == '0') ? 0 : 1;
-    }
-    if (!enabled) return 2;
-  }
-  if (M < 1 || M > 64 || K % 8 != 0 || ((uintptr_t)x % 16) != 0 || ((uintptr_t)Wp % 16) != 0) return 2;
-  if (M > 16) {
-    static int chunk = -1;
-    if (chunk < 0) {
-      const char* e = getenv("TSB200_GEMM_CHUNK");  // "0": stream-K hand-over for every row count (A/B measurements)
-      chunk = (e && e[0] == '0') ? 0 : 1;
-    }
-    if (chunk) {
-      const int r = launch_gemm_chunk_mma(device, st, dtype, x, Wp, M, K, N, ep, error_flag, pdl, ws, ws_bytes, s);
-      if (r != 2) return r;
-    }
-  }
-  GsEncodeTiledFn enc = gs_get_encode();
-  if (!enc) return 2;
-  const int NB = M <= 8 ? 1 : (M <= 16 ? 2 : (M <= 32 ? 4 : 8));
-  GsArgs a{};
-  a.Wp = reinterpret_cast<const unsigned char*>(Wp);
-  a.M = M; a.K = K; a.N = N;
-  a.KB = (K + kKT - 1) / kKT;
-  a.CT = (N + 255) / 256;
-  const long long U = (long long)a.KB * a.CT;
-  long long g = st->sm_count;
-  if (g > U) g = U;
-  a.max_contrib = (int)(a.KB / (U / g)) + 2;
-  const size_t fixed = 32 * sizeof(uint64_t) + 1024 + 128;
-  int stages = (int)((225 * 1024 - fixed) / kGsStageBytes);
-  if (stages > 16) stages = 16;
-  a.stages = stages;
-  a.prefetch = gs_prefetch_enabled();
-  const int64_t need = kWsCounterBytes + (int64_t)a.CT * a.max_contrib * M * 256 * 4;
-  if (!ws || ws_bytes < need) return 2;
-  a.counters = reinterpret_cast<unsigned int*>(ws);
-  a.partials = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + kWsCounterBytes);
-  a.error_flag = error_flag;
-  a.ep = ep;
-  CUtensorMap mapX;
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {32, (cuuint32_t)(NB * 8)};
-    const cuuint32_t el[2] = {1, 1};
-    const CUresult r = enc(&mapX, gs_map_type(dtype), 2, const_cast<void*>(x), dims, strides, box, el,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    TSB_CHECK(r == CUDA_SUCCESS, "gemm_stream: cuTensorMapEncodeTiled failed with %d", (int)r);
-  }
-  const size_t smem = fixed + (size_t)stages * kGsStageBytes;
-  if (dtype == TSB200_BF16) {
-    if (NB > 2) return 2;   // the column-chunk variant serves more rows of this type
-    return NB == 1 ? gs_launch<__nv_bfloat16, 1>(device, mapX, a, (int)g, smem, pdl, s) : gs_launch<__nv_bfloat16, 2>(device, mapX, a, (int)g, smem, pdl, s);
-  }
-  switch (NB) {
-    case 1: return gs_launch<__half, 1>(device, mapX, a, (int)g, smem, pdl, s);
-    case 2: return gs_launch<__half, 2>(device, mapX, a, (int)g, smem, pdl, s);
-    case 4: return gs_launch<__half, 4>(device, mapX, a, (int)g, smem, pdl, s);
-    default: return gs_launch<__half, 8>(device, mapX, a, (int)g, smem, pdl, s);
-  }
+  return kWsCounterBytes + CT * mc * M * 256 * 4 + 256;
 }
 
 // activation tiles [NB * 8 rows][32 k] of a row-major [rows, K] matrix
@@ -936,70 +545,6 @@ static size_t gs_ring(GsArgs* a) {   // stages and shared memory of a launch wit
   return fixed + (size_t)stages * kGsStageBytes;
 }
 
-int64_t gemm_stream_sections_workspace_bytes(int M, int K, int total_N, int sm_count) {
-  return gemm_stream_mma_workspace_bytes(M, K, total_N + 256 * kGsMaxSections, sm_count);
-}
-
-int launch_gemm_stream_sections(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, const LinearSection* sec,
-                                int n_sec, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s) {
-  if (dtype != TSB200_BF16 || M < 1 || M > 64 || n_sec < 1 || n_sec > kGsMaxSections || K % 8 != 0 || ((uintptr_t)x % 16) != 0 ||
-      ((uintptr_t)Wp % 16) != 0)
-    return 2;
-  int x_blocks = 1;
-  for (int i = 0; i < n_sec; ++i) x_blocks = sec[i].x_block + 1 > x_blocks ? sec[i].x_block + 1 : x_blocks;
-  if (M > 16) {   // the column-chunk kernel; every section starts on a column tile, so its boxes are whole tiles but for the last section's
-    GcArgs c{};
-    c.Wp = reinterpret_cast<const unsigned char*>(Wp);
-    c.M = M; c.K = K;
-    c.KB = (K + kKT - 1) / kKT;
-    c.n_sec = n_sec;
-    for (int i = 0; i < n_sec; ++i) {
-      c.CT += (sec[i].N + 255) / 256;
-      c.sec[i].ct_end = c.CT;
-      c.sec[i].N = sec[i].N;
-      c.sec[i].ep = sec[i].ep;
-      c.sec[i].x_block = sec[i].x_block;
-    }
-    const int last = (sec[n_sec - 1].N + 255) / 256, boxes = (c.CT - last) * 4 + (sec[n_sec - 1].N + 63) / 64;
-    if (gc_plan(&c, st, boxes, ws, ws_bytes) != 1) return 2;
-    const int nb = M <= 32 ? 4 : 8;
-    CUtensorMap map;
-    const int r = gc_map_x(&map, dtype, x, x_blocks * M, K, nb);
-    if (r != 1) return r;
-    return nb == 4 ? gc_launch<__nv_bfloat16, 4, kGsSections>(device, map, c, boxes * c.ksplit, pdl, s)
-                   : gc_launch<__nv_bfloat16, 8, kGsSections>(device, map, c, boxes * c.ksplit, pdl, s);
-  }
-  const int NB = M <= 8 ? 1 : 2;
-  GsArgs a{};
-  a.Wp = reinterpret_cast<const unsigned char*>(Wp);
-  a.M = M; a.K = K;
-  a.KB = (K + kKT - 1) / kKT;
-  a.n_sec = n_sec;
-  for (int i = 0; i < n_sec; ++i) {
-    a.CT += (sec[i].N + 255) / 256;
-    a.sec[i].ct_end = a.CT;
-    a.sec[i].N = sec[i].N;
-    a.sec[i].ep = sec[i].ep;
-    a.sec[i].x_block = sec[i].x_block;
-  }
-  const long long U = (long long)a.KB * a.CT;
-  long long g = st->sm_count;
-  if (g > U) g = U;
-  a.max_contrib = (int)(a.KB / (U / g)) + 2;
-  a.prefetch = gs_prefetch_enabled();
-  const int64_t need = kWsCounterBytes + (int64_t)a.CT * a.max_contrib * M * 256 * 4;
-  if (!ws || ws_bytes < need || (int64_t)a.CT * 4 > kWsCounterBytes - 256) return 2;
-  a.counters = reinterpret_cast<unsigned int*>(ws);
-  a.partials = reinterpret_cast<float*>(reinterpret_cast<char*>(ws) + kWsCounterBytes);
-  CUtensorMap mapX;
-  const int r = gs_map_x(&mapX, dtype, x, x_blocks * M, K, NB);
-  if (r != 1) return r;
-  const size_t smem = gs_ring(&a);
-  return NB == 1 ? gs_launch<__nv_bfloat16, 1, 0, kGsSections>(device, mapX, a, (int)g, smem, pdl, s)
-                 : gs_launch<__nv_bfloat16, 2, 0, kGsSections>(device, mapX, a, (int)g, smem, pdl, s);
-}
-
-// slots: every (block, column tile) has KB / per + 2 of them, per = units per CTA >= 1, and units / per <= 2 CTAs
 int64_t gemm_stream_grouped_workspace_bytes(int block_rows, int N, int max_blocks, int sm_count) {
   const int64_t vct = (int64_t)((N + 255) / 256) * max_blocks;
   return kWsCounterBytes + (2 * (int64_t)sm_count + 3 * vct) * block_rows * 256 * 4 + 256;
@@ -1061,7 +606,6 @@ int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, c
   if (stages > 16) stages = 16;
   if (stages < 4) return 2;
   a.stages = stages;
-  a.prefetch = 1;
   a.xres = x32;
   a.gamma = gamma;
   a.beta = beta;

@@ -241,20 +241,13 @@ struct LinearSection {
   Epilogue ep;
   int x_block;             // which of the stacked row blocks of x the section reads
 };
-int launch_gemm_stream_sections(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, const LinearSection* sec,
-                                int n_sec, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s);
-int64_t gemm_stream_sections_workspace_bytes(int M, int K, int total_N, int sm_count);
+int launch_gemm_cluster_sections(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, const LinearSection* sec, int n_sec, bool pdl,
+                                 cudaStream_t s);
 int64_t gemm_tc_workspace_bytes(int M, int N, int sm_count);
-// stream-K mma.sync GEMM for decode batches of up to 64 rows on packed fp16 weights (gemm_stream_mma.cu)
 // mixture-of-experts feed-forward (ops_moe.cu): x32 += sum over the token's experts of score * W2_e act(W1_e h)
 int launch_moe_ffn(int device, DeviceState* st, int dtype, float* x32, const void* h, const void* router_w, const void* router_b,
                    const void* W1, const void* W2, void* hidden, int* picks, float* scores, int rows, int d, int E, int k, int act,
                    cudaStream_t s);
-// tcgen05 streaming GEMM for 17..64 rows (gemm_stream_tc.cu): the weights are the 128-row operand, the activation rows N
-int launch_gemm_stream_tc(int device, DeviceState* st, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep,
-                          int* error_flag, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s);
-int64_t gemm_stream_tc_workspace_bytes(int M, int K, int N, int sm_count);
-int stc_take_error();
 // The packed q | k | v projection of a decode step (one new position per sequence) with RoPE and the cache append done by
 // the linear's epilogue: q columns are rotated and go to the output rows, k columns are rotated and go to the K cache row of
 // the sequence's position, v columns go to the V cache row - the arithmetic of rope_append_kernel (the value is rounded to the
@@ -271,8 +264,9 @@ struct RopeFuse {
 int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, const void* gamma, const void* beta, int norm_type, float eps,
                                 const void* Wp, int M, int K, int N, const Epilogue& ep, int* error_flag, bool pdl, void* ws, int64_t ws_bytes,
                                 cudaStream_t s, const RopeFuse* rope = nullptr);
-int launch_gemm_stream_mma(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep,
-                           int* error_flag, bool pdl, void* ws, int64_t ws_bytes, cudaStream_t s);
+// 1..64 rows of a 16-bit type, the K ranges of 128 columns on the CTAs of a cluster (gemm_cluster_tc.cu); 1 ok, 0 error, 2 not handled
+int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
+                           const RopeFuse* rope = nullptr);
 int64_t gemm_stream_mma_workspace_bytes(int M, int K, int N, int sm_count);
 int gs_take_error();
 // ---- blocks of layered engines (ops_blocks.cu) ---------------------------------------------------------------------------

@@ -67,6 +67,10 @@ __global__ void __launch_bounds__(1024) norm_wide_kernel(TH* h, float* x, const 
   struct __align__(4 * sizeof(TH)) Four { TH e[4]; };
   pdl_trigger();
   const int n4 = cols / 4;
+  Four g[NV];   // the gains do not depend on the kernel before
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (threadIdx.x + k * blockDim.x < n4) g[k] = reinterpret_cast<const Four*>(gamma)[threadIdx.x + k * blockDim.x];
   pdl_wait();
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     float4* xr = reinterpret_cast<float4*>(x + (int64_t)r * cols);
@@ -111,9 +115,8 @@ __global__ void __launch_bounds__(1024) norm_wide_kernel(TH* h, float* x, const 
     for (int k = 0; k < NV; ++k) {
       const int i = threadIdx.x + k * blockDim.x;
       if (i >= n4) continue;
-      const Four g = reinterpret_cast<const Four*>(gamma)[i];
-      float y[4] = {to_f<TH>(g.e[0]) * ((v[k].x - mean) / div), to_f<TH>(g.e[1]) * ((v[k].y - mean) / div), to_f<TH>(g.e[2]) * ((v[k].z - mean) / div),
-                    to_f<TH>(g.e[3]) * ((v[k].w - mean) / div)};
+      float y[4] = {to_f<TH>(g[k].e[0]) * ((v[k].x - mean) / div), to_f<TH>(g[k].e[1]) * ((v[k].y - mean) / div), to_f<TH>(g[k].e[2]) * ((v[k].z - mean) / div),
+                    to_f<TH>(g[k].e[3]) * ((v[k].w - mean) / div)};
       if (beta) {
         const Four t = reinterpret_cast<const Four*>(beta)[i];
 #pragma unroll

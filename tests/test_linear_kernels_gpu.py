@@ -1,5 +1,5 @@
-"""Linears at the edges of the rules that choose their kernels: fp32 rows beyond 16 (clusters over K), deep and shallow rings of the
-tensor-core kernel and its epilogues."""
+"""Linears at the edges of the rules that choose their kernels: fp32 rows beyond 16 (clusters over K), deep and shallow rings of the tensor-core
+kernel, narrow widths with the norm inside."""
 import numpy as np
 import pytest
 import torch
@@ -44,3 +44,26 @@ def test_tensor_core_epilogues(cuda, oracle, M, K, Nn):
         a, g = ref[:, 0::2], ref[:, 1::2]
         np.testing.assert_allclose(host(linear_packed(x, W, b, N.ACT_GLU_NOACT, dtype=torch.float16)), a * g, atol=tol * scale)
         np.testing.assert_allclose(host(linear_packed(x, W, b, N.ACT_SWIGLU, dtype=torch.float16)), oracle.act(a.astype(np.float32), 1) * g, atol=tol * scale)
+
+
+@pytest.mark.parametrize("d,H,B,norm", [(64, 1, 8, "LayerNorm"), (320, 5, 3, "RMSNorm"), (768, 12, 8, "LayerNorm"), (992, 31, 7, "RMSNorm"), (1056, 33, 8, "LayerNorm"),
+                                        (2080, 65, 4, "RMSNorm")])
+def test_norm_inside_the_step_at_any_width(cuda, monkeypatch, d, H, B, norm):
+    """The captured step with the norm inside its linears against the same step with a launch for every norm."""
+    from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, GPT, GPTConfig, MultiHeadAttentionTypeEnums, NormEnums, PositionEmbeddingEnums, synthetic_weights)
+    cfg = GPTConfig(L=2, d=d, H=H, hd=d // H, F=256, V=515, norm=getattr(NormEnums, norm), act=ActivateFuncEnums.GELU, pe=PositionEmbeddingEnums.RoPE,
+                    attn=MultiHeadAttentionTypeEnums.MHA, dtype="float16")
+    w = synthetic_weights(cfg, 7, std=0.05, bias_std=0.02)
+    prompt = np.random.default_rng(d).integers(1, cfg.V, size=(B, 9)).astype(np.int32)
+    opts = DecodingOptions(MaxTgtSentLength=20)
+    logits = []
+    for fused in ("1", "0"):
+        monkeypatch.setenv("TSB200_FUSED_STEP", fused)
+        gpt = GPT(cfg, max_batch=B, max_tokens=24)
+        gpt.LoadWeights(w)
+        gpt.Prefill(prompt, opts)
+        for i in range(3):
+            gpt.StepHost(np.arange(B, dtype=np.int32) + 3 + i, opts)
+        logits.append(gpt.Logits()[0].copy())
+    # the linears' sums are the same up to their order; a normed value next to a rounding boundary moves by 2^-11
+    assert np.abs(logits[0] - logits[1]).max() <= 4 * 2.0 ** -11 * np.abs(logits[1]).max()
