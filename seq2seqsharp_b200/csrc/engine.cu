@@ -688,21 +688,66 @@ static std::vector<CachePart> cache_parts(Gpt* g) {
   }
   return v;
 }
+// Rows of several cache parts <-> the compact buffer, one launch for up to kCopyParts of them.  A CTA copies 32 KB of one row with eight
+// 16-byte loads per thread in flight.  What bounds it: bytes, read and written once (the strided copies of the runtime move 67 MB
+// parts of 16384-token sequences in 69 us, 1.9 TB/s each way).
+constexpr int kCopyParts = 64, kCopyThreads = 256, kCopyUnits = kCopyThreads * 8;
+struct CopyPart {
+  unsigned char *cache, *compact;
+  int64_t pitch;      // bytes from a row of the cache to the next; the compact rows follow each other
+  int64_t units;      // 16-byte units of a row
+  int rows, chunks;   // chunks of kCopyUnits per row
+};
+struct CopyBatch {
+  CopyPart part[kCopyParts];
+};
+__global__ void __launch_bounds__(kCopyThreads) copy_parts_kernel(const __grid_constant__ CopyBatch b, int save) {
+  const CopyPart& p = b.part[blockIdx.y];
+  const int row = blockIdx.x / p.chunks;
+  if (row >= p.rows) return;
+  const int64_t u0 = (int64_t)(blockIdx.x % p.chunks) * kCopyUnits + threadIdx.x;
+  uint4* cache = reinterpret_cast<uint4*>(p.cache + row * p.pitch);
+  uint4* compact = reinterpret_cast<uint4*>(p.compact) + row * p.units;
+  const uint4* src = save ? cache : compact;
+  uint4* dst = save ? compact : cache;
+  uint4 v[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (u0 + i * kCopyThreads < p.units) v[i] = src[u0 + i * kCopyThreads];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (u0 + i * kCopyThreads < p.units) dst[u0 + i * kCopyThreads] = v[i];
+}
+
 // n_seq sequences from `slot` on <-> a compact buffer ([part][sequence][used bytes])
 static int copy_parts(Gpt* g, unsigned char* compact, int slot, int n_seq, int T, bool save) {
+  CopyBatch batch;
+  int n = 0;
+  unsigned blocks = 0;
+  auto flush = [&]() -> int {
+    if (n == 0) return 1;
+    copy_parts_kernel<<<dim3(blocks, n), kCopyThreads, 0, g->s>>>(batch, save ? 1 : 0);
+    count_launch(g->c.device);
+    n = 0;
+    blocks = 0;
+    return check_launch("copy_parts");
+  };
   for (const CachePart& p : cache_parts(g)) {
     unsigned char* at = (unsigned char*)*p.base + (size_t)slot * p.seq_bytes(g);
-    if (p.row_bytes) {
-      const size_t row = (size_t)T * p.row_bytes, pitch = (size_t)g->c.max_tokens * p.row_bytes, rows = (size_t)n_seq * p.heads;
+    const size_t row = p.row_bytes ? (size_t)T * p.row_bytes : (size_t)p.state_bytes, pitch = p.row_bytes ? (size_t)g->c.max_tokens * p.row_bytes : p.state_bytes;
+    const size_t rows = (size_t)n_seq * (p.row_bytes ? p.heads : 1);
+    const uint64_t chunks = (row / 16 + kCopyUnits - 1) / kCopyUnits;
+    if ((((uintptr_t)at | (uintptr_t)compact | row | pitch) % 16) == 0 && row > 0 && chunks * rows <= 0x7fffffff) {
+      batch.part[n++] = CopyPart{at, compact, (int64_t)pitch, (int64_t)(row / 16), (int)rows, (int)chunks};
+      blocks = std::max(blocks, (unsigned)(chunks * rows));
+      if (n == kCopyParts) TSB_TRY(flush());
+    } else if (row > 0) {   // rows that are not whole 16-byte units
       if (save) TSB_CUDA(cudaMemcpy2DAsync(compact, row, at, pitch, row, rows, cudaMemcpyDeviceToDevice, g->s));
       else TSB_CUDA(cudaMemcpy2DAsync(at, pitch, compact, row, row, rows, cudaMemcpyDeviceToDevice, g->s));
-    } else {
-      const size_t bytes = (size_t)n_seq * p.state_bytes;
-      TSB_CUDA(cudaMemcpyAsync(save ? compact : at, save ? at : compact, bytes, cudaMemcpyDeviceToDevice, g->s));
     }
     compact += (size_t)n_seq * p.used_bytes(T);
   }
-  return 1;
+  return flush();
 }
 static size_t parts_bytes(Gpt* g, int T) {   // of one sequence of T tokens
   size_t n = 0;
