@@ -273,14 +273,11 @@ struct Gpt {
   bool use_stack = true;
   bool fuse_step = true;       // per-operation path, up to eight rows: norm (and RoPE + cache append) inside the linear's launch
                                // (TSB200_FUSED_STEP=0: separate norm / RoPE-append launches, e.g. for a checker engine)
-  // Measured crossover on the 7B-class model (ms per step, persistent kernel against one launch per operation with the
-  // mma.sync linears): 1 sequence 3.41 / 3.95, 2 sequences 3.79 / 3.92, 3 sequences 4.23 / 3.91, 4 sequences 4.62 / 3.96 --
-  // the persistent kernel's dependency chain grows with every row, the per-operation path is flat up to 8 sequences.
-  // Tensor-parallel engines keep the persistent kernel (the exchange lives there).
-  int stack_cap = -1;          // largest batch the persistent kernels are used for on one GPU (TSB200_STACK_MAXB); -1: fp16 none
-                               // (one launch per operation on the tensor-core linears is faster at every batch), fp32 two
-  int gemv_rows = -1;          // largest row count of the FMA streaming GEMV in the per-operation path (TSB200_GEMV_MAXROWS);
-                               // -1: fp16 none (the tensor-core streaming kernel is faster from one row on), fp32 four
+  // One GPU: one launch per operation at every batch (linears on clusters; 7B-class fp16, one sequence: 2.69 ms per step against 3.20 with the
+  // stream-K persistent kernel and 3.10 with the owner-partitioned one; tiny fp32 model: 0.18 ms against 0.30).
+  // Tensor-parallel engines keep the persistent kernels (the exchange lives there).
+  int stack_cap = -1;          // largest batch the persistent kernels are used for on one GPU (TSB200_STACK_MAXB); -1: none
+  int gemv_rows = -1;          // largest row count of the FMA streaming GEMV in the per-operation path (TSB200_GEMV_MAXROWS); -1: none
   std::vector<StackOp> stack_host;
   StackOp* stack_dev = nullptr;
   int stack_B = 0;
@@ -771,7 +768,7 @@ static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid
                          const void* Wp, int K, int N, const Epilogue& ep) {
   const TSB200GptConfig& c = g->c;
   const int dev = c.device, dt = c.dtype;
-  if (rows <= (g->gemv_rows >= 0 ? g->gemv_rows : (dt == TSB200_F16 ? 0 : 4))) {
+  if (rows <= g->gemv_rows) {
     prof_begin(g, KC_LINEAR);
     const int r = launch_gemv_stream(dev, g->st, dt, Wp, ng ? (const void*)x_resid : x_T, ng ? (c.norm_type == 0 ? 2 : 1) : 0, ng,
                                      c.norm_type == 0 ? nb : nullptr, c.eps, rows, K, N, ep, g->err_flag, g->pdl, g->lin_ws,
@@ -832,7 +829,7 @@ static int ensure_stack(Gpt* g, int B) {
   g->own_B = 0;
   if (g->ly) return 1;                        // layered models run one launch per operation
   g->stack_max_B = (c.dtype == TSB200_F16) ? 8 : 4;  // fp16: tensor-core consumers take up to 8 rows
-  const int cap = g->stack_cap >= 0 ? g->stack_cap : (c.dtype == TSB200_F16 ? 0 : 2);
+  const int cap = g->stack_cap >= 0 ? g->stack_cap : 0;
   if (g->tp == 1 && cap < g->stack_max_B) g->stack_max_B = cap;
   g->own_B = 0;
   if (!g->use_stack || g->ragged) return 1;   // sequences of different lengths: one launch per operation
@@ -1010,7 +1007,7 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     void* kp = (char*)g->qkv + (int64_t)Hd * g->es;
     void* vp = (char*)g->qkv + (int64_t)(Hd + KVd) * g->es;
     bool appended = false;
-    if (S == 1 && dt == TSB200_F16 && rows <= 64 && g->fuse_step) {
+    if (S == 1 && rows <= (dt == TSB200_F16 ? 64 : 8) && g->fuse_step && rows > g->gemv_rows) {
       // one new position per sequence: RoPE and the cache append in the epilogue of the q | k | v projection
       RopeFuse rf{};
       rf.cK = L.cK; rf.cV = L.cV; rf.Hd = Hd; rf.KVd = KVd; rf.hd = c.hd; rf.Tmax = c.max_tokens;
@@ -1018,7 +1015,8 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
       PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, g->h, g->x, nullptr, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, rows, d, g->s));
       prof_begin(g, KC_LINEAR);
       const Epilogue ep = make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0);
-      const int r = launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
+      const int r = dt == TSB200_F16 ? launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf)
+                                     : launch_gemv_cluster_f32(dev, g->st, (const float*)g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
       if (r == 0) return 0;
       g->lin_syms_used = true;
       if (r == 2) {

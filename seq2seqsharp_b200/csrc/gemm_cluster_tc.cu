@@ -11,6 +11,7 @@
 // shared memory, so that the next launch's CTAs are resident, have their barriers, TMEM and first weight tiles (at these sizes often
 // their whole share) before the current launch ends.  Only the activation tiles wait for it.
 // warp 0: copies; warp 1: TMEM and products; warps 2-5: accumulators out of TMEM; all warps: sums and epilogue.
+#include "cluster_sums.cuh"
 #include "stream_common.cuh"
 #include "tc_common.cuh"
 
@@ -35,15 +36,6 @@ struct LcArgs {
   RopeFuse rope;
 };
 
-__device__ __forceinline__ void lc_push(float* local, uint32_t cta, float v) {
-  uint32_t ra;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(s_u32(local)), "r"(cta));
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(ra), "f"(v) : "memory");
-}
-__device__ __forceinline__ void lc_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 template <int NR>
 __device__ __forceinline__ void lc_tmem_ld(uint32_t taddr, uint32_t* r) {
   if constexpr (NR == 16) {
@@ -80,7 +72,7 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   int si = 0;
   while (si < a.n_sec - 1 && (group >> 1) >= a.sec[si].ct_end) ++si;
   const Epilogue& ep = a.sec[si].ep;
-  const int N = a.sec[si].N, No = ep.glu ? N / 2 : N, xrow = a.sec[si].x_block * M;
+  const int N = a.sec[si].N, xrow = a.sec[si].x_block * M;
   const int col0 = (group - (si ? a.sec[si - 1].ct_end * 2 : 0)) * 128;   // of the section
   const int KP = (KB + 1) / 2, p0 = KP * rank / ks, n_it = KP * (rank + 1) / ks - p0;   // pairs of k tiles
 
@@ -115,7 +107,7 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   if (tid == 0)
     for (int i = 0; i < n_pre; ++i) weights(i);
   __syncwarp();
-  if (ks > 1) lc_cluster_sync();   // the other CTAs exist before anything is pushed to them
+  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
 
   if (tid == 0) {
@@ -159,19 +151,9 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   __syncwarp();
 
   const int per = M * 32 / ks;   // groups of four columns this CTA finishes
-  const H* bias = reinterpret_cast<const H*>(ep.bias);
   // what the first group of this thread needs besides its sums is on its way while the products run
-  float bias0[4] = {0.0f, 0.0f, 0.0f, 0.0f}, res0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  {
-    const int item = rank * per + tid, c = col0 + (item & 31) * 4;
-    if (tid < per) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        if (bias && c + e < N) bias0[e] = to_f<H>(bias[c + e]);
-        if (ep.residual && !ep.glu && c + e < N) res0[e] = ep.residual[(size_t)(item >> 5) * N + c + e];
-      }
-    }
-  }
+  float bias[4], res[4];
+  if (tid < per) cl_addends<H>(ep, N, (rank * per + tid) >> 5, col0 + ((rank * per + tid) & 31) * 4, bias, res);
   if (w >= 2) {
     // ---------------- sums out of TMEM: warp w reads lanes 32 (w % 4) .. = columns of the group
     const bool ok = __all_sync(0xffffffffu, tc_mbar_wait(acc, 0));
@@ -188,72 +170,26 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
         if (row < M) {
           const int item = row * 32 + (col >> 2), owner = item / per;
           float* at = red + ((size_t)(rank * per + item - owner * per) * 4 + (col & 3));
-          if (ks > 1) lc_push(at, (uint32_t)owner, __uint_as_float(v[r]));
+          if (ks > 1) cl_push(at, (uint32_t)owner, __uint_as_float(v[r]));
           else *at = __uint_as_float(v[r]);
         }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   }
-  if (ks > 1) lc_cluster_sync();
+  if (ks > 1) cl_sync();
   else __syncthreads();
 
   // ---------------- epilogue
   for (int i = tid; i < per; i += kLcThreads) {
     const int item = rank * per + i, row = item >> 5, c = col0 + (item & 31) * 4;
-    const bool first = i == tid;
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int r = 0; r < ks; ++r) {
       const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + i) * 4);
       v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
     }
-    if (a.rope_on) {
-      // four columns = two rotation pairs of one head (the head size and the section boundaries are multiples of four)
-      if (c + 3 < N) {
-        const RopeFuse& rf = a.rope;
-        const int pos = state_len(rf.state, row, rf.T0);
-        const int sec = c < rf.Hd ? 0 : (c < rf.Hd + rf.KVd ? 1 : 2);
-        const int cc = c - (sec == 0 ? 0 : (sec == 1 ? rf.Hd : rf.Hd + rf.KVd));
-        const int head = cc / rf.hd, e0 = cc % rf.hd;
-        float t[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) t[e] = to_f<H>(from_f<H>(v[e] + (first ? bias0[e] : (bias ? to_f<H>(bias[c + e]) : 0.0f))));
-        if (rf.use_rope && sec < 2 && pos < rf.Tmax) {
-          const float2 cs0 = rf.tab[(int64_t)pos * (rf.hd / 2) + e0 / 2], cs1 = rf.tab[(int64_t)pos * (rf.hd / 2) + e0 / 2 + 1];
-          const float a0 = t[0], b0 = t[1], a1 = t[2], b1 = t[3];
-          t[0] = a0 * cs0.x - b0 * cs0.y; t[1] = b0 * cs0.x + a0 * cs0.y;
-          t[2] = a1 * cs1.x - b1 * cs1.y; t[3] = b1 * cs1.x + a1 * cs1.y;
-        }
-        const uint2 out = make_uint2(Pair16<H>::put(t[0], t[1]), Pair16<H>::put(t[2], t[3]));
-        if (sec == 0) {
-          *reinterpret_cast<uint2*>(reinterpret_cast<H*>(ep.y) + (size_t)row * N + c) = out;
-        } else if (pos < rf.Tmax) {   // capacity is checked on the host; never write past the cache
-          H* dst = reinterpret_cast<H*>(sec == 1 ? rf.cK : rf.cV) + (((int64_t)row * (rf.KVd / rf.hd) + head) * rf.Tmax + pos) * rf.hd + e0;
-          *reinterpret_cast<uint2*>(dst) = out;
-        }
-      }
-      continue;
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] += first ? bias0[e] : (bias && c + e < N ? to_f<H>(bias[c + e]) : 0.0f);
-    if (ep.glu) {
-      if (c + 1 < N) ep_store<H>(ep, (size_t)row * No + (c >> 1), ep_glu(v[0], v[1], ep));
-      if (c + 3 < N) ep_store<H>(ep, (size_t)row * No + (c >> 1) + 1, ep_glu(v[2], v[3], ep));
-      continue;
-    }
-    if (ep.act != TSB200_ACT_NONE) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = ep_act(v[e], ep.act);
-    }
-    const size_t o = (size_t)row * N + c;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      if (c + e >= N) continue;
-      if (ep.gate) v[e] *= to_f<H>(reinterpret_cast<const H*>(ep.gate)[o + e]);
-      if (ep.residual) v[e] += first ? res0[e] : ep.residual[o + e];
-      if (ep.y32) ep.y32[o + e] = v[e];
-      else reinterpret_cast<H*>(ep.y)[o + e] = from_f<H>(v[e]);
-    }
+    if (i != tid) cl_addends<H>(ep, N, row, c, bias, res);
+    cl_finish4<H>(ep, N, row, c, v, bias, res, a.rope_on, a.rope);
   }
   __syncthreads();
   if (w == 1) {
@@ -333,11 +269,7 @@ int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x
   a.M = M; a.n_sec = 1;
   a.sec[0].ct_end = (N + 255) / 256; a.sec[0].N = N; a.sec[0].ep = ep;
   if (rope) {
-    // q | k | v columns with whole heads of a multiple of four elements, 16-bit output rows, no activation / gate / residual
-    if (rope->hd % 4 != 0 || rope->Hd % rope->hd != 0 || rope->KVd % rope->hd != 0 || rope->Hd + 2 * rope->KVd != N || N % 4 != 0 || !ep.y ||
-        ep.y32 || ep.residual || ep.gate || ep.glu || ep.act != TSB200_ACT_NONE || (rope->use_rope && !rope->tab) || ((uintptr_t)ep.y % 8) != 0 ||
-        ((uintptr_t)rope->cK % 8) != 0 || ((uintptr_t)rope->cV % 8) != 0)
-      return 2;
+    if (!cl_rope_fits(*rope, ep, N, 2)) return 2;
     a.rope_on = 1;
     a.rope = *rope;
   }

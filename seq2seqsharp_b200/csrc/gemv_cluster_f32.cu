@@ -1,0 +1,198 @@
+// fp32 linear of 1..8 rows on packed weights: y[M,N] = epilogue(x[M,K] * W[K,N]), the K ranges of 128 columns on the CTAs of a cluster.
+//
+// The fp32 counterpart of gemm_cluster_tc.cu (no tensor-core type keeps fp32): a CTA streams its 16 KB tiles ([32 k][128 columns]) through a
+// ring of bulk copies, eight warps take four k of a tile each (a lane four columns of every row), the warps' sums meet in shared memory, the
+// cluster's through distributed shared memory in rank order.  Two CTAs fit an SM; the weights are asked for before the launch in front
+// has ended.  What bounds a small model's step is the chain of its launches (512-wide, six layers, one sequence, a
+// 128-token request: 42.7 ms with the persistent stream-K kernel, 24.7 with this one).
+#include "cluster_sums.cuh"
+#include "stream_common.cuh"
+
+namespace tsb {
+
+constexpr int kFcThreads = 288, kFcStages = 5;
+
+struct FcArgs {
+  const float* x;
+  const unsigned char* Wp;
+  int M, N, K, KB, ks;
+  int* error;
+  Epilogue ep;
+  int rope_on;
+  RopeFuse rope;
+};
+// dynamic shared memory: ring | sums of the cluster [M * 32 groups][4] | rows of x over the CTA's range
+static size_t fc_smem(int RM, int tiles) { return (size_t)kFcStages * kTileBytes + (size_t)RM * 512 + (size_t)RM * tiles * 128; }
+
+template <int RM>
+__global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) {
+  extern __shared__ __align__(1024) unsigned char fc_raw[];
+  __shared__ uint64_t full[kFcStages], empty[kFcStages];
+  __shared__ int s_err;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int ks = a.ks, M = a.M, rank = (int)(blockIdx.x % ks), group = (int)(blockIdx.x / ks);
+  const int t0 = a.KB * rank / ks, n_it = a.KB * (rank + 1) / ks - t0;
+  float* red = reinterpret_cast<float*>(fc_raw + kFcStages * kTileBytes);
+  float* xs = red + RM * 128;   // [RM][n_it * 32]
+  if (tid == 0) {
+    for (int i = 0; i < kFcStages; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 8);
+    }
+    s_err = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  pdl_trigger();
+  const unsigned char* src = a.Wp + ((size_t)group * a.KB + t0) * kTileBytes;
+  const int n_pre = min(kFcStages, n_it);
+  if (tid == 256)
+    for (int i = 0; i < n_pre; ++i) {
+      mbar_expect_tx(&full[i], kTileBytes);
+      bulk_g2s(fc_raw + i * kTileBytes, src + (size_t)i * kTileBytes, kTileBytes, &full[i]);
+    }
+  __syncwarp();
+  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
+  pdl_wait();
+  float bias[4], res[4];
+  const int per = M * 32 / ks;   // groups of four columns this CTA finishes
+  if (w == 8) {
+    if (lane == 0) {
+      for (int i = n_pre; i < n_it; ++i) {
+        const int s = i % kFcStages;
+        if (!mbar_wait(&empty[s], (unsigned)((i / kFcStages - 1) & 1))) {
+          s_err = 1;
+          for (int j = i - kFcStages; j < i; ++j) mbar_wait(&full[j % kFcStages], (unsigned)((j / kFcStages) & 1));   // copies in flight land first
+          break;
+        }
+        mbar_expect_tx(&full[s], kTileBytes);
+        bulk_g2s(fc_raw + s * kTileBytes, src + (size_t)i * kTileBytes, kTileBytes, &full[s]);
+      }
+    }
+    __syncwarp();
+  } else {
+    if (tid < per) cl_addends<float>(a.ep, a.N, (rank * per + tid) >> 5, group * 128 + ((rank * per + tid) & 31) * 4, bias, res);
+    const int kc = n_it * 32;
+    for (int i = tid; i < RM * kc; i += 256) {
+      const int m = i / kc, k = t0 * 32 + i % kc;
+      xs[i] = m < M && k < a.K ? a.x[(size_t)m * a.K + k] : 0.0f;
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    float4 acc[RM];
+#pragma unroll
+    for (int m = 0; m < RM; ++m) acc[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int i = 0; i < n_it; ++i) {
+      const int s = i % kFcStages;
+      if (!mbar_wait(&full[s], (unsigned)((i / kFcStages) & 1))) s_err = 1;
+      const float4* t = reinterpret_cast<const float4*>(fc_raw + s * kTileBytes) + w * 4 * 32 + lane;
+      float4 wv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) wv[q] = t[q * 32];
+#pragma unroll
+      for (int m = 0; m < RM; ++m) {
+        const float4 xv = *reinterpret_cast<const float4*>(xs + m * kc + i * 32 + w * 4);
+        const float xq[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          acc[m].x = fmaf(xq[q], wv[q].x, acc[m].x);
+          acc[m].y = fmaf(xq[q], wv[q].y, acc[m].y);
+          acc[m].z = fmaf(xq[q], wv[q].z, acc[m].z);
+          acc[m].w = fmaf(xq[q], wv[q].w, acc[m].w);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    asm volatile("bar.sync 1, 256;" ::: "memory");   // every tile is read: the ring holds the warps' sums now
+    float4* part = reinterpret_cast<float4*>(fc_raw);   // [warp][row][32 groups]
+#pragma unroll
+    for (int m = 0; m < RM; ++m) part[(w * RM + m) * 32 + lane] = acc[m];
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    for (int i = tid; i < M * 32; i += 256) {
+      float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 p = part[(q * RM + (i >> 5)) * 32 + (i & 31)];
+        v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
+      }
+      const int owner = i / per;
+      float* at = red + (size_t)(rank * per + i - owner * per) * 4;
+      if (ks > 1) {
+        cl_push(at, (uint32_t)owner, v.x);
+        cl_push(at + 1, (uint32_t)owner, v.y);
+        cl_push(at + 2, (uint32_t)owner, v.z);
+        cl_push(at + 3, (uint32_t)owner, v.w);
+      } else {
+        *reinterpret_cast<float4*>(at) = v;
+      }
+    }
+    __syncwarp();
+  }
+  if (ks > 1) cl_sync();
+  else __syncthreads();
+  for (int i = tid; i < per && tid < 256; i += 256) {
+    const int item = rank * per + i, row = item >> 5, c = group * 128 + (item & 31) * 4;
+    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int r = 0; r < ks; ++r) {
+      const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + i) * 4);
+      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+    }
+    cl_finish4<float>(a.ep, a.N, row, c, v, bias, res, a.rope_on, a.rope);   // per <= 256: the addends are this group's
+  }
+  if (tid == 0 && s_err && a.error) *a.error = 1;
+}
+
+template <int RM>
+static int fc_launch(int device, const FcArgs& a, int groups, size_t smem, bool pdl, cudaStream_t s) {
+  static bool done[kMaxDevices] = {};
+  if (!done[device]) {
+    TSB_CUDA(cudaFuncSetAttribute(gemv_cluster_f32_kernel<RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+    done[device] = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(groups * a.ks);
+  cfg.blockDim = dim3(kFcThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = a.ks;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = (pdl && pdl_enabled()) ? 2 : 1;
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, gemv_cluster_f32_kernel<RM>, a));
+  count_launch(device);
+  return check_launch("gemv_cluster_f32");
+}
+
+// 1 ok, 0 error, 2 shape not handled (the caller takes another kernel)
+int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
+                            const RopeFuse* rope) {
+  if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
+  FcArgs a{};
+  a.x = x; a.Wp = reinterpret_cast<const unsigned char*>(Wp);
+  a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep;
+  if (rope) {
+    if (!cl_rope_fits(*rope, ep, N, 4)) return 2;
+    a.rope_on = 1;
+    a.rope = *rope;
+  }
+  const int groups = (N + 127) / 128, RM = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
+  // K ranges while all CTAs are resident at once (two per SM), of at least two tiles of 32 k
+  a.ks = 1;
+  while (a.ks < 8 && (int64_t)groups * a.ks * 2 <= 2 * st->sm_count && a.KB / (a.ks * 2) >= 2) a.ks *= 2;
+  const size_t smem = fc_smem(RM, (a.KB + a.ks - 1) / a.ks);
+  if (smem > 220 * 1024) return 2;   // rows too long for the shared memory
+  a.error = tc_error_word(device);
+  switch (RM) {
+    case 1: return fc_launch<1>(device, a, groups, smem, pdl, s);
+    case 2: return fc_launch<2>(device, a, groups, smem, pdl, s);
+    case 4: return fc_launch<4>(device, a, groups, smem, pdl, s);
+    default: return fc_launch<8>(device, a, groups, smem, pdl, s);
+  }
+}
+
+}  // namespace tsb

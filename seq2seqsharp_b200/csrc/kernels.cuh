@@ -267,6 +267,9 @@ int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, c
 // 1..64 rows of a 16-bit type, the K ranges of 128 columns on the CTAs of a cluster (gemm_cluster_tc.cu); 1 ok, 0 error, 2 not handled
 int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
                            const RopeFuse* rope = nullptr);
+// 1..8 fp32 rows in the same manner on the CUDA cores (gemv_cluster_f32.cu)
+int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
+                            const RopeFuse* rope = nullptr);
 int64_t gemm_stream_mma_workspace_bytes(int M, int K, int N, int sm_count);
 int gs_take_error();
 // ---- blocks of layered engines (ops_blocks.cu) ---------------------------------------------------------------------------
@@ -440,6 +443,7 @@ int64_t memory_scratch_bytes(int dtype, const MemoryShape& a, int B, int S);
 int launch_matrix_memory(int device, DeviceState* st, int dtype, const MemoryArgs& a, cudaStream_t s);
 int init_tc_attrs(int device);
 int tc_take_error();
+int* tc_error_word(int device);   // device address of the word that tc_take_error() reads
 int64_t linear_workspace_bytes(int M, int K, int N);
 // Prompts of different lengths one after the other (no pad rows): `rows` of them; where[r] = (sequence, position) of row r, for
 // `listed` rows: those from `rows` on are positions whose values the append clears; starts[b]: first row of sequence b, starts[B] = rows.
