@@ -10,6 +10,7 @@
 // float, angle = theta_i * position in float, cos/sin evaluated in double and rounded to float.
 #include <cstdlib>
 
+#include "cluster_sums.cuh"
 #include "kernels.cuh"
 
 namespace tsb {
@@ -146,14 +147,74 @@ template <> struct Vec16<float> {
 
 constexpr int kAttnThreads = 128;
 
+// End of a split: the states [nstates][G][hd + 2] (maximum, sum, accumulator) of a CTA become one, and the splits of a (row, KV head) meet.
+// box == NULL: one split writes the output, several leave records for attn_combine_kernel.  box: the splits are the CTAs of a cluster; a
+// thread pushes its merged element to the CTA that finishes it (elements in runs of 32, round robin), one cluster barrier, and the
+// records are combined in split order - no launch for the merge and no scratch (7B-class, one sequence of 530 tokens: 2.64 -> 2.55 ms per step).
+constexpr int kAttnMaxCluster = 8;
+__host__ __device__ inline int attn_box_items(int items, int splits) { return ((items + 31) / 32 + splits - 1) / splits * 32; }   // of one owner
+template <typename T>
+__device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm, int nstates, int G, int hd, int row, int H, int h0, int splits, int split, float* box) {
+  const int rec = hd + 2, items = G * hd, per = attn_box_items(items, splits);
+  for (int idx = threadIdx.x; idx < items; idx += kAttnThreads) {
+    const int g = idx / hd, e = idx % hd;
+    float mx = -INFINITY;
+    for (int i = 0; i < nstates; ++i) mx = fmaxf(mx, sm[((int64_t)i * G + g) * rec]);
+    float L = 0.0f, A = 0.0f;
+    for (int i = 0; i < nstates; ++i) {
+      const float* r = sm + ((int64_t)i * G + g) * rec;
+      const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
+      L += r[1] * c;
+      A += r[2 + e] * c;
+    }
+    const int h = h0 + g;
+    if (splits == 1) {
+      out[((int64_t)row * H + h) * hd + e] = from_f<T>(L > 0.0f ? A / L : 0.0f);
+    } else if (box) {
+      const int run = idx >> 5, owner = run % splits;
+      float* at = box + ((size_t)split * per + run / splits * 32 + (idx & 31)) * 3;
+      cl_push(at, (uint32_t)owner, mx);
+      cl_push(at + 1, (uint32_t)owner, L);
+      cl_push(at + 2, (uint32_t)owner, A);
+    } else {
+      float* pr = part + (((int64_t)row * H + h) * splits + split) * rec;
+      if (e == 0) {
+        pr[0] = mx;
+        pr[1] = L;
+      }
+      pr[2 + e] = A;
+    }
+  }
+  if (splits == 1 || !box) return;
+  __syncwarp();
+  cl_sync();
+  for (int i = threadIdx.x; i < per; i += kAttnThreads) {
+    const int idx = ((i >> 5) * splits + split) * 32 + (i & 31);
+    if (idx >= items) continue;
+    float mx = -INFINITY;
+    for (int q = 0; q < splits; ++q) mx = fmaxf(mx, box[((size_t)q * per + i) * 3]);
+    float L = 0.0f, A = 0.0f;
+    for (int q = 0; q < splits; ++q) {
+      const float* r = box + ((size_t)q * per + i) * 3;
+      const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
+      L += r[1] * c;
+      A += r[2] * c;
+    }
+    out[((int64_t)row * H + h0 + idx / hd) * hd + idx % hd] = from_f<T>(L > 0.0f ? A / L : 0.0f);
+  }
+}
+
 template <typename T, int G>
 __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
                                                             const T* q, int64_t q_rs,
                                                             const T* cK, const T* cV, int S, int H,
                                                             int Hkv, int hd, int T0_arg, const int* dT0, int Tmax,
-                                                            int splits, float scale) {
+                                                            int splits, float scale, int box_at) {
   constexpr int EPL = Vec16<T>::N;
+  extern __shared__ float sm[];  // [nstates][G][hd + 2]
+  float* box = box_at ? sm + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
+  if (box) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z / S, T0_arg);
   const int lpt = hd / EPL;              // lanes per token (power of two, <= 32)
@@ -224,7 +285,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
     }
   }
   // merge the nwarps*tpw lane-group states through shared memory
-  extern __shared__ float sm[];  // [nstates][G][hd + 2]
   const int nstates = nwarps * tpw;
   const int st = w * tpw + sub;
   const int rec = hd + 2;
@@ -239,29 +299,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
     for (int e = 0; e < EPL; ++e) r[2 + li * EPL + e] = acc[g][e];
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < G * hd; idx += kAttnThreads) {
-    const int g = idx / hd, e = idx % hd;
-    float mx = -INFINITY;
-    for (int i = 0; i < nstates; ++i) mx = fmaxf(mx, sm[((int64_t)i * G + g) * rec]);
-    float L = 0.0f, A = 0.0f;
-    for (int i = 0; i < nstates; ++i) {
-      const float* r = sm + ((int64_t)i * G + g) * rec;
-      const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
-      L += r[1] * c;
-      A += r[2 + e] * c;
-    }
-    const int h = h0 + g;
-    if (splits == 1) {
-      out[((int64_t)row * H + h) * hd + e] = from_f<T>(L > 0.0f ? A / L : 0.0f);
-    } else {
-      float* pr = part + (((int64_t)row * H + h) * splits + split) * rec;
-      if (e == 0) {
-        pr[0] = mx;
-        pr[1] = L;
-      }
-      pr[2 + e] = A;
-    }
-  }
+  attn_finish<T>(out, part, sm, nstates, G, hd, row, H, h0, splits, split, box);
 }
 
 // Decode variant (one query position per sequence) with the cached K/V rows staged through shared memory by
@@ -445,13 +483,15 @@ __device__ __forceinline__ void at_mma(float* d, uint32_t a0, uint32_t a1, uint3
 template <int HD>
 __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, float* part, const __half* q, int64_t q_rs,
                                                                 const __half* cK, const __half* cV, int H, int Hkv, int T0_arg,
-                                                                const int* dT0, int Tmax, int splits, float scale) {
+                                                                const int* dT0, int Tmax, int splits, float scale, int box_at) {
   constexpr int RB = HD * 2;            // bytes per row
   constexpr int CPR = RB / 16;          // 16-byte chunks per row
   constexpr int KS = HD / 16;           // k steps of Q K^T
   constexpr int NBO = HD / 8;           // n blocks of O
   extern __shared__ __align__(128) unsigned char attn_smem[];
+  float* box = box_at ? reinterpret_cast<float*>(attn_smem) + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
+  if (box) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z, T0_arg);
   TSB_DEV_CHECK(attention, T0 >= 0 && T0 < Tmax, 0x202, (void)0)   // cache length beyond the capacity (keys are clamped to Tmax below)
@@ -590,29 +630,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
   }
   __syncthreads();
   const int nstates = kAttnThreads / 32;
-  for (int idx = threadIdx.x; idx < G * HD; idx += kAttnThreads) {
-    const int g = idx / HD, e = idx % HD;
-    float mx = -INFINITY;
-    for (int i = 0; i < nstates; ++i) mx = fmaxf(mx, sm[((int64_t)i * G + g) * rec]);
-    float L = 0.0f, A = 0.0f;
-    for (int i = 0; i < nstates; ++i) {
-      const float* r = sm + ((int64_t)i * G + g) * rec;
-      const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
-      L += r[1] * c;
-      A += r[2 + e] * c;
-    }
-    const int h = h0 + g;
-    if (splits == 1) {
-      out[((int64_t)row * H + h) * HD + e] = __float2half_rn(L > 0.0f ? A / L : 0.0f);
-    } else {
-      float* pr = part + (((int64_t)row * H + h) * splits + split) * rec;
-      if (e == 0) {
-        pr[0] = mx;
-        pr[1] = L;
-      }
-      pr[2 + e] = A;
-    }
-  }
+  attn_finish<__half>(out, part, sm, nstates, G, HD, row, H, h0, splits, split, box);
 }
 
 template <typename T>
@@ -633,6 +651,26 @@ __global__ void attn_combine_kernel(T* out, const float* part, int hd, int split
     }
     out[rh * hd + e] = from_f<T>(L > 0.0f ? A / L : 0.0f);
   }
+}
+
+// a launch whose grid rows of `cluster` CTAs are clusters
+template <typename... KArgs, typename... Args>
+static cudaError_t launch_clusters(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, int cluster, cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
 
 static int pick_splits(DeviceState* st, int B, int Hkv_groups, int T, int min_keys = 32) {
@@ -695,6 +733,10 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
     const int64_t need = (int64_t)B * S * H * splits * (hd + 2) * sizeof(float);
     if (!ws || ws_bytes < need) splits = 1;
   }
+  // up to eight splits: the CTAs of a cluster.  (Capping more at eight loses: four sequences of 16384 tokens, ten splits and a combine launch
+  // 19.9 ms for 16 steps, eight in a cluster 21.3.)
+  const bool as_cluster = S == 1 && splits > 1 && splits <= kAttnMaxCluster;
+  const size_t box_bytes = as_cluster ? (size_t)splits * attn_box_items(G * hd, splits) * 12 : 0;
   const int tpw = 32 / lpt;
   const size_t smem = (size_t)(kAttnThreads / 32) * tpw * G * (hd + 2) * sizeof(float);
   TSB_CHECK(smem <= 48 * 1024, "attention: shared memory need %zu exceeds 48 KB", smem);
@@ -717,19 +759,20 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
       dim3 g3(splits, Hkv, B);
       static bool attr_done[kMaxDevices] = {};
       if (!attr_done[device]) {
-        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
-        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
         attr_done[device] = true;
       }
-      if (hd == 64)
-        TSB_CUDA(launch_k(attn_mma_kernel<64>, g3, dim3(kAttnThreads), sm3, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK,
-                          (const __half*)cV, H, Hkv, T0, dT0, Tmax, splits, scale));
+      auto k = hd == 64 ? attn_mma_kernel<64> : attn_mma_kernel<128>;
+      if (as_cluster)
+        TSB_CUDA(launch_clusters(k, g3, dim3(kAttnThreads), sm3 + box_bytes, splits, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, H,
+                                 Hkv, T0, dT0, Tmax, splits, scale, (int)(sm3 / 4)));
       else
-        TSB_CUDA(launch_k(attn_mma_kernel<128>, g3, dim3(kAttnThreads), sm3, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK,
-                          (const __half*)cV, H, Hkv, T0, dT0, Tmax, splits, scale));
+        TSB_CUDA(launch_k(k, g3, dim3(kAttnThreads), sm3, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, H, Hkv, T0, dT0, Tmax,
+                          splits, scale, 0));
       count_launch(device);
       TSB_TRY(check_launch("attention_mma"));
-      if (splits > 1) {
+      if (splits > 1 && !as_cluster) {
         TSB_CUDA(launch_k(attn_combine_kernel<T>, dim3(B * S * H), dim3(hd < 128 ? 64 : 128), 0, s, out, (const float*)ws, hd, splits));
         count_launch(device);
         TSB_TRY(check_launch("attention_combine"));
@@ -768,7 +811,15 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
       return 1;
     }
   }
-#define TSB_ATTN(GG) TSB_CUDA(launch_k(attn_kernel<T, GG>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, Tmax, splits, scale))
+  const bool in_cluster = as_cluster && smem + box_bytes <= 48 * 1024;
+#define TSB_ATTN(GG)                                                                                                                                        \
+  do {                                                                                                                                                      \
+    if (in_cluster)                                                                                                                                         \
+      TSB_CUDA(launch_clusters(attn_kernel<T, GG>, grid, dim3(kAttnThreads), smem + box_bytes, splits, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
+                               Tmax, splits, scale, (int)(smem / 4)));                                                                                      \
+    else                                                                                                                                                    \
+      TSB_CUDA(launch_k(attn_kernel<T, GG>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, Tmax, splits, scale, 0));  \
+  } while (0)
   switch (G) {
     case 8: TSB_ATTN(8); break;
     case 4: TSB_ATTN(4); break;
@@ -778,7 +829,7 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
 #undef TSB_ATTN
   count_launch(device);
   TSB_TRY(check_launch("attention"));
-  if (splits > 1) {
+  if (splits > 1 && !in_cluster) {
     TSB_CUDA(launch_k(attn_combine_kernel<T>, dim3(B * S * H), dim3(hd < 128 ? 64 : 128), 0, s, out, (const float*)ws, hd, splits));
     count_launch(device);
     TSB_TRY(check_launch("attention_combine"));
