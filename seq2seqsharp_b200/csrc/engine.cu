@@ -762,8 +762,8 @@ static std::vector<size_t> parts_layout(Gpt* g) {   // two engines with the same
 }
 
 // One linear layer of the engine on packed weights.  With `ng` the input is the fp32 residual stream and the layer's
-// LayerNorm / RMSNorm comes first: fused into the streaming GEMV as a prologue for decode-sized row counts, a
-// separate launch (into g->h) otherwise.
+// LayerNorm / RMSNorm comes first, as a launch of its own into g->h (inside the FMA streaming GEMV where
+// TSB200_GEMV_MAXROWS asks for that kernel).
 static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid, const void* ng, const void* nb, void* h_tmp,
                          const void* Wp, int K, int N, const Epilogue& ep) {
   const TSB200GptConfig& c = g->c;
@@ -784,8 +784,12 @@ static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid
     x_T = h_tmp;
   }
   g->lin_syms_used = true;   // these kernels report a wait that ran out through their own error symbols
-  PROF(KC_LINEAR, launch_linear(dev, g->st, dt, x_T, Wp, rows, K, N, ep, g->lin_ws, g->lin_ws_bytes, g->s, true));
-  return 1;
+  prof_begin(g, KC_LINEAR);
+  int r = 2;
+  if (dt == TSB200_F32 && rows <= 8) r = launch_gemv_cluster_f32(dev, g->st, (const float*)x_T, Wp, rows, K, N, ep, g->pdl, g->s);
+  if (r == 2) r = launch_linear(dev, g->st, dt, x_T, Wp, rows, K, N, ep, g->lin_ws, g->lin_ws_bytes, g->s, true);
+  if (r == 1) prof_end(g, KC_LINEAR);
+  return r == 1;
 }
 
 // x += in[rows,K] * Wp[K,d] + bias: the out-projection of attention and the FFN down-projection.  Under tensor

@@ -503,10 +503,6 @@ int launch_linear(int device, DeviceState* st, int dtype, const void* x, const v
     const int r = launch_gemm_cluster_tc(device, st, dtype, x, W, M, K, N, ep, true, s);
     if (r != 2) return r;
   }
-  if (packed && dtype == TSB200_F32 && M <= 8) {
-    const int r = launch_gemv_cluster_f32(device, st, (const float*)x, W, M, K, N, ep, true, s);
-    if (r != 2) return r;
-  }
   if (packed && is_16bit(dtype) && M > 16) {
     const int r = launch_gemm_tc(device, st, dtype, x, W, M, K, N, ep, nullptr, ws, ws_bytes, s);
     if (r != 2) return r;
