@@ -498,7 +498,7 @@ void set_gemv_trace(long long* p) { g_gemv_trace = p; }
 int launch_gemv_stream(int device, DeviceState* st, int dtype, const void* Wp, const void* x, int xmode, const void* gamma,
                        const void* beta, float eps, int M, int K, int N, const Epilogue& ep, int* error_flag, bool pdl, void* ws,
                        int64_t ws_bytes, cudaStream_t s) {
-  if (M < 1 || M > 4) return 2;
+  if (M < 1 || M > 4 || ((uintptr_t)Wp % 16) != 0) return 2;   // tiles arrive by bulk copies
   if (xmode != 0 && K > 12288) return 2;  // the norm prologue keeps a row in registers
   StreamArgs a{};
   a.Wp = Wp; a.x = x; a.gamma = gamma; a.beta = beta; a.xmode = xmode; a.eps = eps; a.K = K; a.N = N;

@@ -536,7 +536,7 @@ int launch_linear(int device, DeviceState* st, int dtype, const void* x, const v
     return 1;
   }
   // rows of whole 16-byte pieces; 64 rows per tile once there are enough tiles to cover the SMs with them
-  if (packed && dtype == TSB200_F32 && K % 4 == 0 && ((uintptr_t)x % 16) == 0 && (int64_t)M <= 65535 * 32) {
+  if (packed && dtype == TSB200_F32 && K % 4 == 0 && (((uintptr_t)x | (uintptr_t)W) % 16) == 0 && (int64_t)M <= 65535 * 32) {
     if ((int64_t)((M + 63) / 64) * ((N + 63) / 64) >= st->sm_count) return launch_gemm_f32<4>(device, st, (const float*)x, (const float*)W, M, K, N, ep, s);
     return launch_gemm_f32<2>(device, st, (const float*)x, (const float*)W, M, K, N, ep, s);
   }
