@@ -1,0 +1,43 @@
+"""Calls at both sides of a rule that chooses a kernel: the smaller one must not cost clearly more than its neighbour.  Times are the smallest
+of several replays of a captured row of calls, both sides in turn; the limits leave room for noise, not for the wrong kernel."""
+import pytest
+import torch
+
+from seq2seqsharp_b200 import _native as N
+
+pytestmark = pytest.mark.gpu
+
+
+def times(*calls, n=10):
+    """us per call of each of `calls` (functions of a stream)."""
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graphs, best = [], [1e9] * len(calls)
+    with torch.cuda.stream(s):
+        for f in calls:
+            f(s.cuda_stream)
+            s.synchronize()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=s):
+                for _ in range(n):
+                    f(torch.cuda.current_stream().cuda_stream)
+            graphs.append(g)
+        for _ in range(8):
+            for i, g in enumerate(graphs):
+                a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+                a.record(s)
+                g.replay()
+                b.record(s)
+                s.synchronize()
+                best[i] = min(best[i], a.elapsed_time(b) * 1000.0 / n)
+    return best
+
+
+def test_append_of_one_row_without_a_table(cuda):
+    def call(H, Hkv, hd):
+        q, k = torch.randn(1, 1, (H + 2 * Hkv) * hd, device="cuda", dtype=torch.float16), torch.zeros(1, Hkv, 2, hd, device="cuda", dtype=torch.float16)
+        v = torch.zeros_like(k)
+        at = [q.data_ptr() + i * hd * 2 for i in (0, H, H + Hkv)]
+        return lambda st: N.call("TSB200_RopeAppend", 0, N.F16, *at, q.shape[2], q.shape[2], k.data_ptr(), v.data_ptr(), 1, 1, H, Hkv, hd, 1, 2, 1, 10000.0, st)
+    wide, narrow = times(call(32, 8, 128), call(4, 2, 8))
+    assert wide < 2.0 * narrow, (wide, narrow)      # one CTA for the row and four pairs per thread: 4.3
