@@ -8,6 +8,7 @@
 // RoPE follows TensorSharp/TensorApplyCPU.cs:1148-1178 (same math as TensorSharp.CUDA/DeviceCode/
 // AdvFuncKernels.cs:1245-1279 without fast-math): interleaved pairs (2i, 2i+1), theta_i = base^(-2i/hd) rounded to
 // float, angle = theta_i * position in float, cos/sin evaluated in double and rounded to float.
+#include <algorithm>
 #include <cstdlib>
 
 #include "cluster_sums.cuh"
@@ -151,14 +152,15 @@ template <> struct Vec16<float> {
 constexpr int kAttnThreads = 128;
 
 // End of a split: the states [nstates][G][hd + 2] (maximum, sum, accumulator) of a CTA become one, and the splits of a (row, KV head) meet.
-// box == NULL: one split writes the output, several leave records for attn_combine_kernel.  box: the splits are the CTAs of a cluster; a
+// Without BOX one split writes the output and several leave records for attn_combine_kernel.  With BOX the splits are the CTAs of a cluster; a
 // thread pushes its merged element to the CTA that finishes it (elements in runs of 32, round robin), one cluster barrier, and the
 // records are combined in split order - no launch for the merge and no scratch (7B-class, one sequence of 530 tokens: 2.64 -> 2.55 ms per step).
+// Kernels of their own: the cluster's code costs a launch that does not use it up to 0.5 us (one split of 200 keys: 3.9 against 4.4 us).
 constexpr int kAttnMaxCluster = 8;
 __host__ __device__ inline int attn_box_items(int items, int splits) { return ((items + 31) / 32 + splits - 1) / splits * 32; }   // of one owner
-template <typename T>
+template <typename T, bool BOX>
 __device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm, int nstates, int G, int hd, int row, int H, int h0, int splits, int split, float* box) {
-  const int rec = hd + 2, items = G * hd, per = attn_box_items(items, splits);
+  const int rec = hd + 2, items = G * hd, per = BOX ? attn_box_items(items, splits) : 0;
   for (int idx = threadIdx.x; idx < items; idx += kAttnThreads) {
     const int g = idx / hd, e = idx % hd;
     float mx = -INFINITY;
@@ -171,14 +173,14 @@ __device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm
       A += r[2 + e] * c;
     }
     const int h = h0 + g;
-    if (splits == 1) {
-      out[((int64_t)row * H + h) * hd + e] = from_f<T>(L > 0.0f ? A / L : 0.0f);
-    } else if (box) {
+    if constexpr (BOX) {
       const int run = idx >> 5, owner = run % splits;
       float* at = box + ((size_t)split * per + run / splits * 32 + (idx & 31)) * 3;
       cl_push(at, (uint32_t)owner, mx);
       cl_push(at + 1, (uint32_t)owner, L);
       cl_push(at + 2, (uint32_t)owner, A);
+    } else if (splits == 1) {
+      out[((int64_t)row * H + h) * hd + e] = from_f<T>(L > 0.0f ? A / L : 0.0f);
     } else {
       float* pr = part + (((int64_t)row * H + h) * splits + split) * rec;
       if (e == 0) {
@@ -188,26 +190,27 @@ __device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm
       pr[2 + e] = A;
     }
   }
-  if (splits == 1 || !box) return;
-  __syncwarp();
-  cl_sync();
-  for (int i = threadIdx.x; i < per; i += kAttnThreads) {
-    const int idx = ((i >> 5) * splits + split) * 32 + (i & 31);
-    if (idx >= items) continue;
-    float mx = -INFINITY;
-    for (int q = 0; q < splits; ++q) mx = fmaxf(mx, box[((size_t)q * per + i) * 3]);
-    float L = 0.0f, A = 0.0f;
-    for (int q = 0; q < splits; ++q) {
-      const float* r = box + ((size_t)q * per + i) * 3;
-      const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
-      L += r[1] * c;
-      A += r[2] * c;
+  if constexpr (BOX) {
+    __syncwarp();
+    cl_sync();
+    for (int i = threadIdx.x; i < per; i += kAttnThreads) {
+      const int idx = ((i >> 5) * splits + split) * 32 + (i & 31);
+      if (idx >= items) continue;
+      float mx = -INFINITY;
+      for (int q = 0; q < splits; ++q) mx = fmaxf(mx, box[((size_t)q * per + i) * 3]);
+      float L = 0.0f, A = 0.0f;
+      for (int q = 0; q < splits; ++q) {
+        const float* r = box + ((size_t)q * per + i) * 3;
+        const float c = (r[0] == -INFINITY) ? 0.0f : __expf(r[0] - mx);
+        L += r[1] * c;
+        A += r[2] * c;
+      }
+      out[((int64_t)row * H + h0 + idx / hd) * hd + idx % hd] = from_f<T>(L > 0.0f ? A / L : 0.0f);
     }
-    out[((int64_t)row * H + h0 + idx / hd) * hd + idx % hd] = from_f<T>(L > 0.0f ? A / L : 0.0f);
   }
 }
 
-template <typename T, int G>
+template <typename T, int G, bool BOX>
 __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
                                                             const T* q, int64_t q_rs,
                                                             const T* cK, const T* cV, int S, int H,
@@ -215,9 +218,9 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
                                                             int splits, float scale, int box_at) {
   constexpr int EPL = Vec16<T>::N;
   extern __shared__ float sm[];  // [nstates][G][hd + 2]
-  float* box = box_at ? sm + box_at : nullptr;   // splits as a cluster
+  float* box = BOX ? sm + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
-  if (box) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z / S, T0_arg);
   const int lpt = hd / EPL;              // lanes per token (power of two, <= 32)
@@ -302,7 +305,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
     for (int e = 0; e < EPL; ++e) r[2 + li * EPL + e] = acc[g][e];
   }
   __syncthreads();
-  attn_finish<T>(out, part, sm, nstates, G, hd, row, H, h0, splits, split, box);
+  attn_finish<T, BOX>(out, part, sm, nstates, G, hd, row, H, h0, splits, split, box);
 }
 
 // Decode variant (one query position per sequence) with the cached K/V rows staged through shared memory by
@@ -483,7 +486,7 @@ __device__ __forceinline__ void at_mma(float* d, uint32_t a0, uint32_t a1, uint3
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int HD>
+template <int HD, bool BOX>
 __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, float* part, const __half* q, int64_t q_rs,
                                                                 const __half* cK, const __half* cV, int H, int Hkv, int T0_arg,
                                                                 const int* dT0, int Tmax, int splits, float scale, int box_at) {
@@ -492,9 +495,9 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
   constexpr int KS = HD / 16;           // k steps of Q K^T
   constexpr int NBO = HD / 8;           // n blocks of O
   extern __shared__ __align__(128) unsigned char attn_smem[];
-  float* box = box_at ? reinterpret_cast<float*>(attn_smem) + box_at : nullptr;   // splits as a cluster
+  float* box = BOX ? reinterpret_cast<float*>(attn_smem) + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
-  if (box) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z, T0_arg);
   TSB_DEV_CHECK(attention, T0 >= 0 && T0 < Tmax, 0x202, (void)0)   // cache length beyond the capacity (keys are clamped to Tmax below)
@@ -633,7 +636,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
   }
   __syncthreads();
   const int nstates = kAttnThreads / 32;
-  attn_finish<__half>(out, part, sm, nstates, G, HD, row, H, h0, splits, split, box);
+  attn_finish<__half, BOX>(out, part, sm, nstates, G, HD, row, H, h0, splits, split, box);
 }
 
 template <typename T>
@@ -736,10 +739,15 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
     const int64_t need = (int64_t)B * S * H * splits * (hd + 2) * sizeof(float);
     if (!ws || ws_bytes < need) splits = 1;
   }
-  // up to eight splits: the CTAs of a cluster.  (Capping more at eight loses: four sequences of 16384 tokens, ten splits and a combine launch
-  // 19.9 ms for 16 steps, eight in a cluster 21.3.)
-  const bool as_cluster = S == 1 && splits > 1 && splits <= kAttnMaxCluster;
-  const size_t box_bytes = as_cluster ? (size_t)splits * attn_box_items(G * hd, splits) * 12 : 0;
+  // Up to eight splits: the CTAs of a cluster.  (Capping more at eight loses: four sequences of 16384 tokens, ten splits and a combine launch
+  // 19.9 ms for 16 steps, eight in a cluster 21.3.)  Only while every cluster is resident at once: CTAs that start together leave holes in the
+  // waves that follow (8 KV heads of 128, four query heads each, two CTAs per SM: 16 sequences of 530 tokens, 384 CTAs, 12.4 us as single
+  // CTAs and a combine launch, 15.7 as clusters; 8 of 530, 192 CTAs, 8.9 and 8.1).
+  const bool may_cluster = S == 1 && splits > 1 && splits <= kAttnMaxCluster;
+  const size_t box_bytes = may_cluster ? (size_t)splits * attn_box_items(G * hd, splits) * 12 : 0;
+  auto resident = [&](size_t smem, int at_most) {   // 228 KB of an SM, 1 KB of them reserved per CTA
+    return (int64_t)B * ygroups * splits <= (int64_t)std::min((int)(228 * 1024 / (smem + 1024)), at_most) * st->sm_count;
+  };
   const int tpw = 32 / lpt;
   const size_t smem = (size_t)(kAttnThreads / 32) * tpw * G * (hd + 2) * sizeof(float);
   TSB_CHECK(smem <= 48 * 1024, "attention: shared memory need %zu exceeds 48 KB", smem);
@@ -762,17 +770,19 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
       dim3 g3(splits, Hkv, B);
       static bool attr_done[kMaxDevices] = {};
       if (!attr_done[device]) {
-        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
-        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<128, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<64, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
+        TSB_CUDA(cudaFuncSetAttribute(attn_mma_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 116 * 1024));
         attr_done[device] = true;
       }
-      auto k = hd == 64 ? attn_mma_kernel<64> : attn_mma_kernel<128>;
+      const bool as_cluster = may_cluster && resident(sm3 + box_bytes, 4);
       if (as_cluster)
-        TSB_CUDA(launch_clusters(k, g3, dim3(kAttnThreads), sm3 + box_bytes, splits, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, H,
+        TSB_CUDA(launch_clusters(hd == 64 ? attn_mma_kernel<64, true> : attn_mma_kernel<128, true>, g3, dim3(kAttnThreads), sm3 + box_bytes, splits, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, H,
                                  Hkv, T0, dT0, Tmax, splits, scale, (int)(sm3 / 4)));
       else
-        TSB_CUDA(launch_k(k, g3, dim3(kAttnThreads), sm3, s, (__half*)out, ws, (const __half*)q, q_rs, (const __half*)cK, (const __half*)cV, H, Hkv, T0, dT0, Tmax,
-                          splits, scale, 0));
+        TSB_CUDA(launch_k(hd == 64 ? attn_mma_kernel<64, false> : attn_mma_kernel<128, false>, g3, dim3(kAttnThreads), sm3, s, (__half*)out, ws, (const __half*)q, q_rs,
+                          (const __half*)cK, (const __half*)cV, H, Hkv, T0, dT0, Tmax, splits, scale, 0));
       count_launch(device);
       TSB_TRY(check_launch("attention_mma"));
       if (splits > 1 && !as_cluster) {
@@ -814,14 +824,14 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
       return 1;
     }
   }
-  const bool in_cluster = as_cluster && smem + box_bytes <= 48 * 1024;
+  const bool in_cluster = may_cluster && smem + box_bytes <= 48 * 1024 && resident(smem + box_bytes, 2);   // two: registers of the widest group
 #define TSB_ATTN(GG)                                                                                                                                        \
   do {                                                                                                                                                      \
     if (in_cluster)                                                                                                                                         \
-      TSB_CUDA(launch_clusters(attn_kernel<T, GG>, grid, dim3(kAttnThreads), smem + box_bytes, splits, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
+      TSB_CUDA(launch_clusters(attn_kernel<T, GG, true>, grid, dim3(kAttnThreads), smem + box_bytes, splits, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
                                Tmax, splits, scale, (int)(smem / 4)));                                                                                      \
     else                                                                                                                                                    \
-      TSB_CUDA(launch_k(attn_kernel<T, GG>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, Tmax, splits, scale, 0));  \
+      TSB_CUDA(launch_k(attn_kernel<T, GG, false>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, Tmax, splits, scale, 0));  \
   } while (0)
   switch (G) {
     case 8: TSB_ATTN(8); break;

@@ -41,3 +41,23 @@ def test_append_of_one_row_without_a_table(cuda):
         return lambda st: N.call("TSB200_RopeAppend", 0, N.F16, *at, q.shape[2], q.shape[2], k.data_ptr(), v.data_ptr(), 1, 1, H, Hkv, hd, 1, 2, 1, 10000.0, st)
     wide, narrow = times(call(32, 8, 128), call(4, 2, 8))
     assert wide < 2.0 * narrow, (wide, narrow)      # one CTA for the row and four pairs per thread: 4.3
+
+
+@pytest.mark.parametrize("B,launches", [(8, 1), (16, 2)])
+def test_splits_are_a_cluster_only_while_all_are_resident(cuda, B, launches):
+    """8 KV heads of 128, 530 keys: three splits.  192 CTAs fit at two per SM; 384 do not, and run as single CTAs before a launch that merges."""
+    H, Hkv, hd, T = 32, 8, 128, 530
+    k, v = (torch.randn(B, Hkv, T, hd, device="cuda", dtype=torch.float16) for _ in range(2))
+    q = torch.randn(B, H * hd, device="cuda", dtype=torch.float16)
+    o, ws = torch.empty_like(q), torch.empty(N.lib().TSB200_FlashDecodeWorkspaceBytes(B, H, hd, T), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    n = [N.C.c_int64(), N.C.c_int64()]
+    N.call("TSB200_LaunchCount", 0, N.C.byref(n[0]))
+    N.call("TSB200_FlashDecode", 0, N.F16, o.data_ptr(), q.data_ptr(), H * hd, k.data_ptr(), v.data_ptr(), B, H, Hkv, hd, T, T, ws.data_ptr(), ws.numel(), None)
+    N.call("TSB200_LaunchCount", 0, N.C.byref(n[1]))
+    assert n[1].value - n[0].value == launches
+    N.call("TSB200_Synchronize", 0, None)
+    g = H // Hkv
+    z = torch.einsum("bhgd,bhtd->bhgt", q.double().reshape(B, Hkv, g, hd), k.double()) * hd ** -0.5
+    ref = torch.einsum("bhgt,bhtd->bhgd", z.softmax(-1), v.double()).reshape(B, H * hd)
+    assert (o.double() - ref).abs().max().item() <= 2.0 ** -10     # outputs of N(0, 1/23): weights and outputs rounded to fp16
