@@ -33,6 +33,19 @@ def times(*calls, n=10):
     return best
 
 
+def prompt_attention(B, S, H, Hkv, hd):
+    q = torch.randn(B, S, (H + 2 * Hkv) * hd, device="cuda", dtype=torch.float16)
+    k, v = (torch.randn(B, Hkv, S, hd, device="cuda", dtype=torch.float16) for _ in range(2))
+    o = torch.empty(B, S, H * hd, device="cuda", dtype=torch.float16)
+    return lambda st: N.call("TSB200_PrefillAttention", 0, N.F16, o.data_ptr(), q.data_ptr(), q.shape[2], k.data_ptr(), v.data_ptr(), B, S, H, Hkv, hd, 0, S, st)
+
+
+@pytest.mark.parametrize("B,H,Hkv,hd", [(64, 12, 12, 64), (64, 32, 8, 64), (64, 32, 32, 128), (64, 32, 8, 128)])
+def test_short_prompts_cost_less_than_long_ones(cuda, B, H, Hkv, hd):
+    short, long_ = times(prompt_attention(B, 16, H, Hkv, hd), prompt_attention(B, 128, H, Hkv, hd))
+    assert short < 0.3 * long_, (short, long_)      # an eighth of the tokens; with whole tiles of 256 rows 0.33 to 0.87 of the time
+
+
 def test_append_of_one_row_without_a_table(cuda):
     def call(H, Hkv, hd):
         q, k = torch.randn(1, 1, (H + 2 * Hkv) * hd, device="cuda", dtype=torch.float16), torch.zeros(1, Hkv, 2, hd, device="cuda", dtype=torch.float16)

@@ -38,3 +38,25 @@ def test_against_float64(cuda, hd, H, Hkv, S, T0):
         torch.cuda.synchronize()
         np.testing.assert_allclose(out.reshape(B, S, H, hd).double().cpu().numpy(), ref.cpu().numpy(), atol=TOL)
         assert raw[:shift].abs().sum() == 0 and raw[shift + B * S * H * hd:].abs().sum() == 0
+
+
+@pytest.mark.parametrize("hd,H,Hkv,S,T0", [(64, 4, 4, 16, 48), (64, 4, 4, 16, 49), (64, 8, 1, 64, 64), (64, 8, 2, 65, 64), (64, 12, 12, 128, 0), (128, 8, 2, 64, 0), (128, 8, 2, 100, 28),
+                                            (128, 8, 4, 65, 0), (128, 8, 8, 64, 0), (128, 8, 8, 65, 0), (128, 8, 1, 129, 0)])
+def test_at_the_limits_of_short_prompts(cuda, hd, H, Hkv, S, T0):
+    """Keys and heads at both sides of the rule that chooses between mma.sync and tcgen05."""
+    test_against_float64(cuda, hd, H, Hkv, S, T0)
+
+
+@pytest.mark.parametrize("B", [37, 75])      # 16 rows on top of 60 keys, 8 KV heads: within and beyond two waves of whole SMs
+def test_many_short_prompts_on_a_cache(cuda, B):
+    H, Hkv, hd, S, T0 = 8, 8, 64, 16, 130
+    q = torch.randn(B, S, H * hd, device="cuda").half()
+    k, v = (torch.randn(B, Hkv, T0 + S, hd, device="cuda").half() for _ in range(2))
+    o = torch.empty_like(q)
+    torch.cuda.synchronize()
+    N.call("TSB200_PrefillAttention", 0, N.F16, o.data_ptr(), q.data_ptr(), H * hd, k.data_ptr(), v.data_ptr(), B, S, H, Hkv, hd, T0, T0 + S, None)
+    N.call("TSB200_Synchronize", 0, None)
+    z = q.reshape(B, S, H, hd).transpose(1, 2).double() @ k.double().transpose(2, 3) * hd ** -0.5
+    seen = torch.arange(T0 + S, device="cuda")[None] <= T0 + torch.arange(S, device="cuda")[:, None]
+    ref = (z.masked_fill(~seen, float("-inf")).softmax(-1) @ v.double()).transpose(1, 2).reshape(B, S, H * hd)
+    assert (o.double() - ref).abs().max().item() <= TOL
