@@ -678,10 +678,11 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
     // Only with a single row tile: from two row tiles on (M > 128) the tiles of a weight column block already share its
     // columns through L2 and the K slices' partial sums cost more than the idle SMs (512 x 4096 x 4096: 59.7 us with two
     // slices, 39.9 us without; 256 x 4096 x 6144: 79.8 against 41.4 us).
-    if (tiles < st->sm_count && grid.y == 1 && k_total >= 8 && ws) {
-      // about 1.5 CTAs per SM (two fit); every extra K slice costs the last arriver another partial to add
-      int ks = (int)((3 * st->sm_count / 2 + tiles - 1) / tiles);
-      if (ks > k_total / 4) ks = k_total / 4;
+    // And only for long K: a slice saves its part of 0.37 us per 64 k of a tile alone, and costs the last arriver 2 to 4 us to add.  100 rows
+    // with slices / without: 4096 x 4096 67.0 / 27.1 us, 2048 x 3072 32.1 / 17.4, 8192 x 2048 33.4 / 47.  No more slices than SMs, which
+    // keeps the deep rings (100 x 11008 x 4096: six slices of three stages 76.9, four of six stages 36.6).
+    if (grid.y == 1 && k_total >= 96 && ws) {
+      int ks = (int)(st->sm_count / tiles);
       if (ks > 6) ks = 6;
       if (ks > 1) {
         const int k_per = (k_total + ks - 1) / ks;

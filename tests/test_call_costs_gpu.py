@@ -74,3 +74,23 @@ def test_splits_are_a_cluster_only_while_all_are_resident(cuda, B, launches):
     z = torch.einsum("bhgd,bhtd->bhgt", q.double().reshape(B, Hkv, g, hd), k.double()) * hd ** -0.5
     ref = torch.einsum("bhgt,bhtd->bhgd", z.softmax(-1), v.double()).reshape(B, H * hd)
     assert (o.double() - ref).abs().max().item() <= 2.0 ** -10     # outputs of N(0, 1/23): weights and outputs rounded to fp16
+
+
+def linear(M, K, n, dtype):
+    code = N.F16 if dtype == torch.float16 else N.F32
+    W = (torch.randn(K, n, device="cuda") * 0.05).to(dtype)
+    Wp = torch.empty(N.lib().TSB200_PackedWeightBytes(code, K, n), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    N.call("TSB200_PackWeight", 0, code, Wp.data_ptr(), W.data_ptr(), code, K, n, None)
+    N.call("TSB200_Synchronize", 0, None)
+    x, y = torch.randn(M, K, device="cuda").to(dtype), torch.empty(M, n, device="cuda", dtype=dtype)
+    ws = torch.empty(N.lib().TSB200_LinearPackedWorkspaceBytes(code, M, K, n), dtype=torch.uint8, device="cuda")
+    keep = (Wp, x, y, ws)
+    return lambda st, keep=keep: N.call("TSB200_LinearPacked", 0, code, y.data_ptr(), None, x.data_ptr(), None, None, None, -1, 0.0, Wp.data_ptr(), None, None, M, K, n, -1,
+                                        ws.data_ptr(), ws.numel(), st)
+
+
+@pytest.mark.parametrize("K,n", [(4096, 4096), (2048, 3072)])
+def test_linear_of_one_row_tile_against_two(cuda, K, n):
+    one, two = times(linear(100, K, n, torch.float16), linear(160, K, n, torch.float16))
+    assert one < 1.3 * two, (one, two)          # with K slices for the single row tile 1.7 to 2.3
