@@ -28,19 +28,37 @@ inline bool cl_rope_fits(const RopeFuse& r, const Epilogue& ep, int N, size_t el
          ep.act == TSB200_ACT_NONE && (!r.use_rope || r.tab) && al % (4 * elem) == 0;
 }
 
-// bias and residual of four columns (zeros where there are none), for cl_finish4
+// whether four columns of every row lie on a boundary of theirs, in all that an epilogue reads and writes
+inline bool cl_whole_pieces(const Epilogue& ep, int N, size_t elem) {
+  return N % 4 == 0 && ((uintptr_t)ep.y | (uintptr_t)ep.bias | (uintptr_t)ep.gate) % (4 * elem) == 0 && ((uintptr_t)ep.y32 | (uintptr_t)ep.residual) % 16 == 0;
+}
+
+// bias of four columns (zeros where there is none), for cl_finish4
 template <typename H>
-__device__ __forceinline__ void cl_addends(const Epilogue& ep, int N, int row, int c, float* bias, float* res) {
+__device__ __forceinline__ void cl_bias(const Epilogue& ep, int N, int c, float* bias) {
   const H* b = reinterpret_cast<const H*>(ep.bias);
 #pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    bias[e] = b && c + e < N ? to_f<H>(b[c + e]) : 0.0f;
-    res[e] = ep.residual && !ep.glu && c + e < N ? ep.residual[(size_t)row * N + c + e] : 0.0f;
+  for (int e = 0; e < 4; ++e) bias[e] = b && c + e < N ? to_f<H>(b[c + e]) : 0.0f;
+}
+// residual of four columns of a row (zeros where there is none)
+__device__ __forceinline__ void cl_residual(const Epilogue& ep, int N, int row, int c, bool pieces, float* res) {
+  res[0] = res[1] = res[2] = res[3] = 0.0f;
+  if (!ep.residual || ep.glu) return;
+  const float* r = ep.residual + (size_t)row * N + c;
+  if (pieces) {
+    if (c < N) {
+      const float4 t = *reinterpret_cast<const float4*>(r);
+      res[0] = t.x; res[1] = t.y; res[2] = t.z; res[3] = t.w;
+    }
+    return;
   }
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    if (c + e < N) res[e] = r[e];
 }
 // the finished sums v of columns c .. c + 3 of a row: bias first, then rotation and cache append, gate product, or activation / gate / residual
 template <typename H>
-__device__ __forceinline__ void cl_finish4(const Epilogue& ep, int N, int row, int c, float* v, const float* bias, const float* res, int rope_on, const RopeFuse& rf) {
+__device__ __forceinline__ void cl_finish4(const Epilogue& ep, int N, int row, int c, bool pieces, float* v, const float* bias, const float* res, int rope_on, const RopeFuse& rf) {
 #pragma unroll
   for (int e = 0; e < 4; ++e) v[e] += bias[e];
   if (rope_on) {
@@ -66,6 +84,14 @@ __device__ __forceinline__ void cl_finish4(const Epilogue& ep, int N, int row, i
   }
   if (ep.glu) {
     const int No = N / 2;
+    if (pieces && !ep.gate && !ep.residual && !ep.y32) {
+      if (c >= N) return;
+      const float y0 = ep_glu(v[0], v[1], ep), y1 = ep_glu(v[2], v[3], ep);
+      H* dst = reinterpret_cast<H*>(ep.y) + (size_t)row * No + (c >> 1);
+      if constexpr (sizeof(H) == 4) *reinterpret_cast<float2*>(dst) = make_float2(y0, y1);
+      else *reinterpret_cast<uint32_t*>(dst) = Pair16<H>::put(y0, y1);
+      return;
+    }
     if (c + 1 < N) ep_store<H>(ep, (size_t)row * No + (c >> 1), ep_glu(v[0], v[1], ep));
     if (c + 3 < N) ep_store<H>(ep, (size_t)row * No + (c >> 1) + 1, ep_glu(v[2], v[3], ep));
     return;
@@ -75,6 +101,20 @@ __device__ __forceinline__ void cl_finish4(const Epilogue& ep, int N, int row, i
     for (int e = 0; e < 4; ++e) v[e] = ep_act(v[e], ep.act);
   }
   const size_t o = (size_t)row * N + c;
+  if (pieces) {
+    if (c >= N) return;
+    if (ep.gate) {
+      struct __align__(4 * sizeof(H)) Four { H e[4]; };
+      const Four g = *reinterpret_cast<const Four*>(reinterpret_cast<const H*>(ep.gate) + o);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[e] *= to_f<H>(g.e[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] += res[e];
+    if (ep.y32) cl_store4<float>(ep.y32 + o, v);
+    else cl_store4<H>(reinterpret_cast<H*>(ep.y) + o, v);
+    return;
+  }
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     if (c + e >= N) continue;

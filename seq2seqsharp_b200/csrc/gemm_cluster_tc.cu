@@ -4,7 +4,7 @@
 // The WEIGHTS are the 128-row operand of tcgen05.mma (A, read in place from the packed tiles, MN-major, 128-byte swizzle), the activation
 // rows its N dimension (B: [16 / 32 / 64 rows][64 k], K-major, one TMA tensor copy per stage, rows beyond M zero-filled).  A CTA owns
 // 128 columns over a range of K; the 1, 2, 4 or 8 CTAs of a cluster share the columns.  When its products are done a CTA pushes every
-// sum into the shared memory of the CTA that finishes it (each finishes 1 / ks of the rows x columns), one cluster barrier, and the sums
+// sum into the shared memory of the CTA that finishes it (each finishes 1 / ks of the columns), one cluster barrier, and the sums
 // are added in rank order (bitwise reproducible): no scratch in global memory, no counters, no last arriver that reads the others' slots.
 //
 // What bounds a decode step's linears is the chain from one launch to the next, not their bytes: a CTA takes at most half of an SM's
@@ -24,6 +24,7 @@ struct LcSection {
   int ct_end;   // first column tile (256 columns) after the section
   int N;
   int x_block;  // stacked row block it reads
+  int pieces;   // four columns at a time in the epilogue
   Epilogue ep;
 };
 struct LcArgs {
@@ -150,16 +151,26 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   }
   __syncwarp();
 
-  const int per = M * 32 / ks;   // groups of four columns this CTA finishes
-  // what the first group of this thread needs besides its sums is on its way while the products run
+  // This CTA finishes 128 / ks of the columns, in groups of four, of every row.  The CTA that finishes a column is the same for all rows, and a
+  // thread's groups, kLcThreads apart, have the same columns: no index arithmetic per row.  (Rows x columns shared out as one range cost a
+  // division per pushed sum; as straight-line code of 40 KB that was the launch's longest part, 0.15 us per row: 64 rows of 64 -> 64 19.5 us,
+  // now 10.7; of 4096 -> 22016 53.0, now 42.0.)  Bias and the first group's residual are on their way while the products run.
+  const int gsh = 5 - (31 - __clz(ks)), per = M << gsh;   // log2 of a row's groups here; groups of this CTA
+  const int c = col0 + ((rank << gsh) + (tid & ((1 << gsh) - 1))) * 4;
+  const bool pieces = a.sec[si].pieces != 0;
   float bias[4], res[4];
-  if (tid < per) cl_addends<H>(ep, N, (rank * per + tid) >> 5, col0 + ((rank * per + tid) & 31) * 4, bias, res);
+  cl_bias<H>(ep, N, c, bias);
+  if (tid < per) cl_residual(ep, N, tid >> gsh, c, pieces, res);
   if (w >= 2) {
     // ---------------- sums out of TMEM: warp w reads lanes 32 (w % 4) .. = columns of the group
     const bool ok = __all_sync(0xffffffffu, tc_mbar_wait(acc, 0));
     if (!ok) s_err = 1;
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int col = (w & 3) * 32 + lane;
+    const int col = (w & 3) * 32 + lane, owner = col >> (gsh + 2);
+    float* at = red + ((size_t)rank * per + ((col >> 2) & ((1 << gsh) - 1))) * 4 + (col & 3);   // [source rank][row][group][4]
+    const uint32_t local = s_u32(at), step = 16u << gsh;
+    uint32_t remote = local;
+    if (ks > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(owner));
 #pragma unroll
     for (int h = 0; h < (NR + 31) / 32; ++h) {
       uint32_t v[NR < 32 ? NR : 32];
@@ -168,10 +179,8 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
       for (int r = 0; r < (NR < 32 ? NR : 32); ++r) {
         const int row = h * 32 + r;
         if (row < M) {
-          const int item = row * 32 + (col >> 2), owner = item / per;
-          float* at = red + ((size_t)(rank * per + item - owner * per) * 4 + (col & 3));
-          if (ks > 1) cl_push(at, (uint32_t)owner, __uint_as_float(v[r]));
-          else *at = __uint_as_float(v[r]);
+          if (ks > 1) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(remote + row * step), "r"(v[r]) : "memory");
+          else asm volatile("st.shared.b32 [%0], %1;" ::"r"(local + row * step), "r"(v[r]) : "memory");
         }
       }
     }
@@ -181,15 +190,18 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   else __syncthreads();
 
   // ---------------- epilogue
+#pragma unroll 1
   for (int i = tid; i < per; i += kLcThreads) {
-    const int item = rank * per + i, row = item >> 5, c = col0 + (item & 31) * 4;
+    float next[4];
+    if (i + kLcThreads < per) cl_residual(ep, N, (i + kLcThreads) >> gsh, c, pieces, next);
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int r = 0; r < ks; ++r) {
       const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + i) * 4);
       v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
     }
-    if (i != tid) cl_addends<H>(ep, N, row, c, bias, res);
-    cl_finish4<H>(ep, N, row, c, v, bias, res, a.rope_on, a.rope);
+    cl_finish4<H>(ep, N, i >> gsh, c, pieces, v, bias, res, a.rope_on, a.rope);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) res[e] = next[e];
   }
   __syncthreads();
   if (w == 1) {
@@ -200,9 +212,12 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
 }
 
 template <typename H, int NR>
-static int lc_launch(int device, const CUtensorMap& map, LcArgs a, int groups, bool pdl, cudaStream_t s) {
+static int lc_launch(int device, const CUtensorMap& map, LcArgs a, int groups, int sms, bool pdl, cudaStream_t s) {
   constexpr int kStage = 16384 + NR * 128;
-  a.stages = (112 * 1024 - 1024 - 256 - NR * 512) / kStage;   // two CTAs per SM
+  // two CTAs per SM; three where that makes one wave of what would be a full and a nearly empty one (two to three groups per SM; 32 rows of
+  // 768 -> 50257: 26.4 -> 17.6 us; the rings of more rows than 32 do not fit three times)
+  const int per_sm = NR <= 32 && groups > 2 * sms && groups <= 3 * sms ? 75 : 112;
+  a.stages = (per_sm * 1024 - 1024 - 256 - NR * 512) / kStage;
   const int smem = a.stages * kStage + NR * 512 + 256 + 1024;
   static bool done[kMaxDevices] = {};
   if (!done[device]) {
@@ -250,8 +265,8 @@ static int lc_run(int device, DeviceState* st, int dtype, const void* x, int row
                          el, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   TSB_CHECK(r == CUDA_SUCCESS, "gemm_cluster_tc: cuTensorMapEncodeTiled failed with %d", (int)r);
 #define TSB_LC(H)                                                     \
-  (NR == 16 ? lc_launch<H, 16>(device, map, a, groups, pdl, s)        \
-            : (NR == 32 ? lc_launch<H, 32>(device, map, a, groups, pdl, s) : lc_launch<H, 64>(device, map, a, groups, pdl, s)))
+  (NR == 16 ? lc_launch<H, 16>(device, map, a, groups, st->sm_count, pdl, s)        \
+            : (NR == 32 ? lc_launch<H, 32>(device, map, a, groups, st->sm_count, pdl, s) : lc_launch<H, 64>(device, map, a, groups, st->sm_count, pdl, s)))
   return dtype == TSB200_BF16 ? TSB_LC(__nv_bfloat16) : TSB_LC(__half);
 #undef TSB_LC
 }
@@ -267,7 +282,7 @@ int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x
   LcArgs a{};
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
   a.M = M; a.n_sec = 1;
-  a.sec[0].ct_end = (N + 255) / 256; a.sec[0].N = N; a.sec[0].ep = ep;
+  a.sec[0].ct_end = (N + 255) / 256; a.sec[0].N = N; a.sec[0].ep = ep; a.sec[0].pieces = cl_whole_pieces(ep, N, 2);
   if (rope) {
     if (!cl_rope_fits(*rope, ep, N, 2)) return 2;
     a.rope_on = 1;
@@ -287,6 +302,7 @@ int launch_gemm_cluster_sections(int device, DeviceState* st, int dtype, const v
   for (int i = 0; i < n_sec; ++i) {
     ct += (sec[i].N + 255) / 256;
     a.sec[i].ct_end = ct; a.sec[i].N = sec[i].N; a.sec[i].ep = sec[i].ep; a.sec[i].x_block = sec[i].x_block;
+    a.sec[i].pieces = cl_whole_pieces(sec[i].ep, sec[i].N, 2);
     if (sec[i].x_block + 1 > blocks) blocks = sec[i].x_block + 1;
   }
   const int last = sec[n_sec - 1].N;   // an odd half of the last column tile is left out

@@ -18,6 +18,7 @@ struct FcArgs {
   int M, N, K, KB, ks;
   int* error;
   Epilogue ep;
+  int pieces;  // four columns at a time in the epilogue
   int rope_on;
   RopeFuse rope;
 };
@@ -55,7 +56,8 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   float bias[4], res[4];
-  const int per = M * 32 / ks;   // groups of four columns this CTA finishes
+  const int per = M * 32 / ks;   // groups of four columns this CTA finishes: at most 256, one per thread
+  const int c = group * 128 + ((rank * per + tid) & 31) * 4;
   if (w == 8) {
     if (lane == 0) {
       for (int i = n_pre; i < n_it; ++i) {
@@ -71,7 +73,10 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     }
     __syncwarp();
   } else {
-    if (tid < per) cl_addends<float>(a.ep, a.N, (rank * per + tid) >> 5, group * 128 + ((rank * per + tid) & 31) * 4, bias, res);
+    if (tid < per) {
+      cl_bias<float>(a.ep, a.N, c, bias);
+      cl_residual(a.ep, a.N, (rank * per + tid) >> 5, c, a.pieces != 0, res);
+    }
     const int kc = n_it * 32;
     for (int i = tid; i < RM * kc; i += 256) {
       const int m = i / kc, k = t0 * 32 + i % kc;
@@ -130,14 +135,13 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   }
   if (ks > 1) cl_sync();
   else __syncthreads();
-  for (int i = tid; i < per && tid < 256; i += 256) {
-    const int item = rank * per + i, row = item >> 5, c = group * 128 + (item & 31) * 4;
+  if (tid < per) {
     float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     for (int r = 0; r < ks; ++r) {
-      const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + i) * 4);
+      const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + tid) * 4);
       v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
     }
-    cl_finish4<float>(a.ep, a.N, row, c, v, bias, res, a.rope_on, a.rope);   // per <= 256: the addends are this group's
+    cl_finish4<float>(a.ep, a.N, (rank * per + tid) >> 5, c, a.pieces != 0, v, bias, res, a.rope_on, a.rope);
   }
   if (tid == 0 && s_err && a.error) *a.error = 1;
 }
@@ -174,7 +178,7 @@ int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const v
   if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
   FcArgs a{};
   a.x = x; a.Wp = reinterpret_cast<const unsigned char*>(Wp);
-  a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep;
+  a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.pieces = cl_whole_pieces(ep, N, 4);
   if (rope) {
     if (!cl_rope_fits(*rope, ep, N, 4)) return 2;
     a.rope_on = 1;

@@ -90,6 +90,11 @@ def linear(M, K, n, dtype):
                                         ws.data_ptr(), ws.numel(), st)
 
 
+def test_linear_of_64_short_rows(cuda):
+    many, few = times(linear(64, 64, 64, torch.float16), linear(5, 64, 64, torch.float16))
+    assert many < 2.0 * few, (many, few)        # one group of four columns after the other, each with its own loads: 3.1
+
+
 @pytest.mark.parametrize("K,n", [(4096, 4096), (2048, 3072)])
 def test_linear_of_one_row_tile_against_two(cuda, K, n):
     one, two = times(linear(100, K, n, torch.float16), linear(160, K, n, torch.float16))

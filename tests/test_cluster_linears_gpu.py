@@ -52,6 +52,13 @@ def check(M, K, n, dtype, shifts):
             np.testing.assert_allclose(host(linear(x, W, b, N.ACT_GLU_NOACT, shift=s)), ref[:, 0::2] * ref[:, 1::2], atol=2 * tol * big + half * big * big)
 
 
+# 8 k: one step of one rank; 264 and 4104: a last pair with one tile; 1024 columns and fewer: eight ranks; 20000: one
+@pytest.mark.parametrize("M,K,n", [(5, 8, 5), (8, 264, 130), (16, 4104, 1024), (17, 72, 516), (31, 1024, 127), (33, 512, 128), (48, 4096, 260), (64, 64, 64), (64, 136, 20000),
+                                   (64, 2048, 2050), (63, 11008, 384)])
+def test_fp16_rows(cuda, M, K, n):
+    check(M, K, n, torch.float16, (0, 1))
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("M", [1, 3, 8, 20, 70])
 def test_weights_off_a_16_byte_boundary(cuda, dtype, M):
