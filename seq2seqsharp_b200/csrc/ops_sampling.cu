@@ -142,8 +142,9 @@ __global__ void __launch_bounds__(1024) softmax_argmax_kernel(int* out_ids, floa
 }
 
 // The same on a cluster of eight CTAs per row: a CTA keeps its eighth of the row in registers (NV values per thread: one read of the
-// logits, one exponential per value instead of two), maxima, sums and winners meet through distributed shared memory, summed in rank
-// order.  What bounds it: latency (one CTA per row: three passes over 128 KB at the rate of one SM, 24 us at V = 32000, 40 us at 50257).
+// logits, one exponential per value instead of two), maxima, sums and winners meet through distributed shared memory, the eight sums
+// added in a fixed tree.  What bounds it: latency (one CTA per row: three passes over 128 KB at the rate of one SM).  One row of V = 32000:
+// 22 -> 6.2 us, 50257: 34 -> 8.0, 131072: 105 -> 18.4; softmax_ctas_per_sm() says when it is taken.
 constexpr int kSmCluster = 8, kSmThreads = 512, kSmMaxV = kSmCluster * kSmThreads * 32;
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -1064,13 +1065,23 @@ int init_topp_attrs(int device) {
   return 1;
 }
 
+// How many CTAs per SM a cluster of eight per row may ask for before one CTA of 1024 threads per row is faster.  That one takes 5.2 us at
+// V = 4096, 7.6 at 8000, 22 at 32000, 56 at 70000 and 105 at 131072, for any number of rows up to the SMs'; the clusters 5.3 to 6.1 us
+// for a row of V up to 8000 (three barriers and the reductions between them) and more with every CTA that an SM holds:
+//   V = 8000: 37 rows 7.4 us, 64 rows 13.1;  32000: 74 rows 16.1;  50257: 26.2;  131072: 106
+//   V = 70000, where 32 values per thread leave two CTAs per SM and almost half of them stay empty: 37 rows 39.6 us, 64 rows 64.7
+// Rows beyond a cluster's registers take the passes over memory.
+static int softmax_ctas_per_sm(int V) {
+  if (V < 6144) return 0;
+  if (V < 8000) return 1;
+  if (V < 20000) return 2;
+  return V > kSmMaxV / 2 && V <= kSmMaxV / 4 * 3 ? 2 : 4;
+}
+
 int launch_softmax_argmax(int device, DeviceState* st, int* out_ids, float* probs, const float* logits, int B, int V,
                           float temperature, int use_temp, const int* blocked_dev, int n_blocked, cudaStream_t s) {
   if (B == 0) return 1;
-  // eight CTAs per row while they all fit the GPU at once (four of 512 threads per SM; V = 32000: 6.4 us instead of 24); more rows than that
-  // fill the SMs with one CTA each.  Short rows are not worth the cluster barriers, longer ones than a cluster's registers hold take
-  // the passes over memory.
-  if (V >= 4096 && V <= kSmMaxV && (int64_t)B * kSmCluster <= 4LL * (st ? st->sm_count : 148)) {
+  if (V <= kSmMaxV && (int64_t)B * kSmCluster <= (int64_t)softmax_ctas_per_sm(V) * (st ? st->sm_count : 148)) {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(B * kSmCluster);
     cfg.blockDim = dim3(kSmThreads);

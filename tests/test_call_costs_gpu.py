@@ -46,6 +46,15 @@ def test_short_prompts_cost_less_than_long_ones(cuda, B, H, Hkv, hd):
     assert short < 0.3 * long_, (short, long_)      # an eighth of the tokens; with whole tiles of 256 rows 0.33 to 0.87 of the time
 
 
+@pytest.mark.parametrize("V", [4096, 8000])
+def test_softmax_of_many_short_rows(cuda, V):
+    def call(B):
+        z, p, ids = torch.randn(B, V, device="cuda"), torch.empty(B, V, device="cuda"), torch.empty(B, dtype=torch.int32, device="cuda")
+        return lambda st: N.call("TSB200_SoftmaxArgmax", 0, ids.data_ptr(), p.data_ptr(), z.data_ptr(), B, V, 1.0, None, 0, st)
+    fewer, more = times(call(74), call(75))
+    assert fewer < 1.3 * more, (fewer, more)        # eight CTAs for each of 74 rows: 1.8 to 2.5
+
+
 def test_append_of_one_row_without_a_table(cuda):
     def call(H, Hkv, hd):
         q, k = torch.randn(1, 1, (H + 2 * Hkv) * hd, device="cuda", dtype=torch.float16), torch.zeros(1, Hkv, 2, hd, device="cuda", dtype=torch.float16)

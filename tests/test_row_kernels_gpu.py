@@ -100,3 +100,9 @@ def test_nuclei_around_the_selection_limit(cuda, oracle, rows, n):
     out = Ops.TopPSample(torch.from_numpy(big).cuda(), 2.2, 0.0, None, torch.from_numpy(u))
     torch.cuda.synchronize()
     np.testing.assert_array_equal(out.cpu().numpy(), oracle.topp(big, 2.2, 0.0, None, u))
+
+
+@pytest.mark.parametrize("B,V", [(1, 6143), (18, 6144), (19, 6144), (18, 7999), (37, 8000), (38, 8000), (38, 19999), (74, 20000), (74, 65536), (37, 65537), (38, 98304), (74, 98305)])
+def test_softmax_at_the_limits_of_the_clusters(cuda, oracle, B, V):
+    """Rows and widths at both sides of the rule that gives a row eight CTAs or one."""
+    test_softmax_and_first_maximum(cuda, oracle, B, V)
