@@ -296,7 +296,7 @@ struct ToppSmem {
   int2 warp_pair[32];
   uint32_t tot[256];    // cluster sort: this CTA's count per digit (read by the other CTAs of the cluster)
   uint32_t base[256];   // cluster sort: global offset of this CTA's first key of a digit, minus its local offset
-  uint32_t share;       // selection: sum of this CTA's weights (float bits)
+  uint32_t share[2];    // selection: sum of this CTA's weights and of the squares (float bits)
   uint32_t cut;         // selection: lowest bin taken
   uint32_t n_sel;       // selection: entries taken so far (CTA 0's counts for the cluster)
 };
@@ -603,13 +603,16 @@ __device__ void exact_prefix(const uint32_t* keys, float* accs, int n_valid, flo
 
 // ---- the head of the order without sorting the rest -------------------------------------------------------------------
 // Only the entries up to the one whose running sum reaches topP matter.  The weights are added up by the top 11 bits of
-// their keys (eight bins per octave, 2^-30 units rounded down), the bins are walked from the largest until they hold more
+// their keys (eight bins per octave from 2^-30 to 4, in 2^-30 units rounded down), the bins are walked from the largest until they hold more
 // than topP + 2^-11, and only their entries are sorted, when there are at most kSelMax.  The 2^-11 covers what the fp32
 // running sum over kSelMax entries of at most 3 can fall short by (2^11 * 2^-24 * 3 < 2^-11): the running sum then reaches
 // topP inside the selection, and entries outside are never looked at, so that the answer is the full sort's.  Otherwise
-// (flat rows, topP close to 1, sums above 3) nothing has been changed and the caller sorts everything.
-// Rows whose nucleus is a handful of ids: 8 rows of V = 50257 on clusters 100 -> 37 us, one row of 32000 75 -> 19 us.
-constexpr int kSelBins = 2048, kSelMax = 2048;
+// (flat rows, topP close to 1, sums above 3) nothing has been changed and the caller sorts everything.  Such a row pays for the look, so it
+// leaves as soon as the sum of the squares, or the number of entries that the taken bins hold at least, says so; every lane has its own
+// copy of the bins, because the keys of a flat row meet in two or three of them.  Flat rows (V = 50257, one CTA per row: 486 us to sort, 521
+// with 2048 shared bins and no early way out, 487 now; one row of 32000 on a cluster 162, 172, 162), equal weights (260, 300, 262).
+// Rows whose nucleus is a handful of ids: 8 rows of V = 50257 on clusters 105 -> 27 us, one row of 32000 72 -> 18 us.
+constexpr int kSelBins = 256, kSelLow = (127 - 30) << 3, kSelMax = 2048, kSelUnroll = 4;   // kSelLow: key >> 20 of 2^-30
 
 __device__ __forceinline__ uint32_t add_dsmem_u32(uint32_t* local_ptr, uint32_t cta, uint32_t v) {
   uint32_t a = (uint32_t)__cvta_generic_to_shared(local_ptr), ra, old;
@@ -619,72 +622,115 @@ __device__ __forceinline__ uint32_t add_dsmem_u32(uint32_t* local_ptr, uint32_t 
 }
 
 // keys [s_beg, s_end) are this CTA's; CL CTAs share the row.  True on all CTAs or on none; then CTA 0 finds the selection in
-// sorted order in keys / idx [0, sm.n_sel) (idx: any scratch; tk / ti: scratch for the unsorted selection).
+// sorted order in keys / idx [0, sm.n_sel) (idx: any scratch; tk / ti: scratch for the unsorted selection).  sq: this thread's part of the
+// sum of the squares, before any penalty.  kSelMax entries add up to at most sqrt(kSelMax * that sum): below topP there is no selection.
+// Without a cluster, and for long rows, a flat row leaves here before its bins are counted; for the others the exchange would cost
+// a peaked row more than it saves a flat one, and the sum travels with the weights' own.
 template <int CL>
-__device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_t* ti, int s_beg, int s_end, float topP, ToppSmem& sm, int crank) {
+__device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_t* ti, int s_beg, int s_end, int V, float topP, float sq, ToppSmem& sm, int crank) {
+  if (!(topP < 2.5f)) return false;   // beyond what the units can count; NaN
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  uint32_t* bins = &sm.hist[0][0];
-  for (int i = tid; i < kSelBins; i += kTopPThreads) bins[i] = 0u;
+  uint32_t* mine = &sm.hist[0][0] + lane;   // [bin][lane]
+  sq = warp_sum(sq);
+  if (lane == 0) sm.chunk[w] = sq;
+  for (int i = tid; i < kSelBins * 32; i += kTopPThreads) (&sm.hist[0][0])[i] = 0u;
   if (tid == 0) {
     sm.cut = 0xffffffffu;
     sm.n_sel = 0u;
   }
   __syncthreads();
+  sq = warp_sum(sm.chunk[lane]);   // 32 warps
+  if (tid == 0) sm.share[1] = __float_as_uint(sq);
+  const float least = topP * topP * (0.999f / kSelMax);
+  if (CL == 1 || V >= 65536) {
+    if constexpr (CL > 1) {
+      cluster_sync_all();
+      sq = 0.0f;
+#pragma unroll
+      for (int c = 0; c < CL; ++c) sq += __uint_as_float(ld_dsmem_u32(&sm.share[1], (uint32_t)c));
+    }
+    if (sq < least) return false;
+  }
   float sum = 0.0f;
-  for (int j = s_beg + tid; j < s_end; j += kTopPThreads) {
-    const uint32_t k = keys[j];
-    if (k) {
-      const float v = __uint_as_float(k);
+  for (int base = s_beg; base < s_end; base += kTopPThreads * kSelUnroll) {
+    uint32_t k[kSelUnroll];
+#pragma unroll
+    for (int q = 0; q < kSelUnroll; ++q) {
+      const int j = base + q * kTopPThreads + tid;
+      k[q] = j < s_end ? keys[j] : 0u;
+    }
+#pragma unroll
+    for (int q = 0; q < kSelUnroll; ++q) {
+      const float v = __uint_as_float(k[q]);
       sum += v;
-      atomicAdd(&bins[k >> 20], __float2uint_rz(fminf(v, 1.0f) * 1073741824.0f));
+      const uint32_t units = __float2uint_rz(fminf(v, 1.0f) * 1073741824.0f);
+      if (units) atomicAdd(mine + min((k[q] >> 20) - kSelLow, kSelBins - 1u) * 32, units);
     }
   }
-  sum = block_sum(sum, reinterpret_cast<float*>(sm.warp_tot));
-  if (tid == 0) sm.share = __float_as_uint(sum);
+  sum = warp_sum(sum);
+  if (lane == 0) sm.chunk[32 + w] = sum;
+  __syncthreads();
+  sum = warp_sum(sm.chunk[32 + lane]);
+  {
+    // the lanes' copies together, four threads per bin
+    const uint32_t* b = &sm.hist[0][0] + (tid >> 2) * 32 + (tid & 3) * 8;
+    uint32_t t = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) t += b[(q + (tid >> 2)) & 7];
+    t += __shfl_xor_sync(0xffffffffu, t, 1);
+    t += __shfl_xor_sync(0xffffffffu, t, 2);
+    if ((tid & 3) == 0) sm.tot[tid >> 2] = t;
+  }
+  if (tid == 0) sm.share[0] = __float_as_uint(sum);
   if constexpr (CL > 1) {
     cluster_sync_all();
-    sum = 0.0f;
+    sum = sq = 0.0f;
 #pragma unroll
-    for (int c = 0; c < CL; ++c) sum += __uint_as_float(ld_dsmem_u32(&sm.share, (uint32_t)c));
+    for (int c = 0; c < CL; ++c) {
+      sum += __uint_as_float(ld_dsmem_u32(&sm.share[0], (uint32_t)c));
+      sq += __uint_as_float(ld_dsmem_u32(&sm.share[1], (uint32_t)c));
+    }
   } else {
     __syncthreads();
   }
-  const bool usable = sum < 3.0f && topP < 2.5f;   // false for NaN too
-  if (usable) {
-    // inclusive sums over the bins from the largest key down; a thread takes two neighbours
-    const int hi = kSelBins - 1 - 2 * tid;
-    uint32_t a0 = 0, a1 = 0;
+  if (!(sum < 3.0f) || sq < least) return false;   // sums that are NaN too; the same answer on all CTAs, and nothing is read from them any more
+  uint32_t units = 0;
+  const int bin = kSelBins - 1 - tid;   // the first 256 threads take a bin each, from the largest key down
+  if (tid < kSelBins) {
+    // inclusive sums over the bins
     if constexpr (CL > 1) {
 #pragma unroll
-      for (int c = 0; c < CL; ++c) {
-        a0 += ld_dsmem_u32(&bins[hi], (uint32_t)c);
-        a1 += ld_dsmem_u32(&bins[hi - 1], (uint32_t)c);
-      }
+      for (int c = 0; c < CL; ++c) units += ld_dsmem_u32(&sm.tot[bin], (uint32_t)c);
     } else {
-      a0 = bins[hi];
-      a1 = bins[hi - 1];
+      units = sm.tot[bin];
     }
-    uint32_t incl = a0 + a1;
+  }
+  uint32_t incl = units;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    __syncthreads();   // block_sum's use of warp_tot is over
-    if (lane == 31) sm.warp_tot[w] = incl;
-    __syncthreads();
-    uint32_t before = incl - a0 - a1;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  if (lane == 31) sm.warp_tot[w] = incl;
+  __syncthreads();
+  if (tid < kSelBins) {
+    uint32_t before = incl - units;
     for (int i = 0; i < w; ++i) before += sm.warp_tot[i];
     const uint32_t target = __float2uint_rz((fmaxf(topP, 0.0f) + 0.00048828125f) * 1073741824.0f);
-    if (before < target && before + a0 >= target) sm.cut = (uint32_t)hi;
-    else if (before + a0 < target && before + a0 + a1 >= target) sm.cut = (uint32_t)(hi - 1);
+    if (before < target && before + units >= target) sm.cut = (uint32_t)bin;
   }
   __syncthreads();
-  const uint32_t cut = sm.cut;
-  if (cut == 0xffffffffu) {
+  uint32_t cut = sm.cut;
+  bool fits = cut != 0xffffffffu;
+  if (fits) {   // the entries that the taken bins hold at least: each is smaller than its bin's upper end
+    const float n = units && (uint32_t)bin >= cut ? (float)units / (1073741824.0f * __uint_as_float((uint32_t)(bin + kSelLow + 1) << 20)) : 0.0f;
+    fits = block_sum(n, reinterpret_cast<float*>(sm.warp_tot)) <= (float)kSelMax;
+  }
+  if (!fits) {
     if constexpr (CL > 1) cluster_sync_all();   // the others have read this CTA's bins
     return false;
   }
+  cut += kSelLow;
   for (int base = s_beg; base < s_end; base += kTopPThreads) {
     const int j = base + tid;
     const uint32_t k = j < s_end ? keys[j] : 0u;
@@ -761,8 +807,10 @@ __global__ void __launch_bounds__(kTopPThreads) topp_kernel(int* out, const floa
   const int len = (history && history_len) ? history_len[r] : 0;
 
   // 1. keys (+ repeat penalty on the last occurrence of each id in the history)
+  float sq = 0.0f;
   for (int j = threadIdx.x; j < V; j += blockDim.x) {
     const float w = p[j];
+    sq += fmaxf(w, 0.0f) * fmaxf(w, 0.0f);
     keyA[j] = (w > 0.0f) ? __float_as_uint(w) : 0u;
   }
   for (int q = threadIdx.x; q < len; q += blockDim.x) {
@@ -791,7 +839,7 @@ __global__ void __launch_bounds__(kTopPThreads) topp_kernel(int* out, const floa
   __syncthreads();
 
   // 2. sort descending, stable: the head of the order alone where that is enough
-  const bool head = topp_select<1>(keyA, idxA, keyB, idxB, 0, V, topP, sm, 0);
+  const bool head = topp_select<1>(keyA, idxA, keyB, idxB, 0, V, V, topP, sq, sm, 0);
   if (!head) {
     radix_pass(keyA, nullptr, keyB, idxB, V, 0, true, sm);
     radix_pass(keyB, idxB, keyA, idxA, V, 8, false, sm);
@@ -989,8 +1037,10 @@ __global__ void __launch_bounds__(kTopPThreads) topp_cluster_kernel(int* out, co
   const int s_beg = min(V, crank * n_per), s_end = min(V, s_beg + n_per);
 
   // 1. keys of this CTA's slice (+ repeat penalty on the last occurrence of each id of the slice in the history)
+  float sq = 0.0f;
   for (int j = s_beg + threadIdx.x; j < s_end; j += blockDim.x) {
     const float w = p[j];
+    sq += fmaxf(w, 0.0f) * fmaxf(w, 0.0f);
     keyA[j] = (w > 0.0f) ? __float_as_uint(w) : 0u;
   }
   for (int q = threadIdx.x; q < len; q += blockDim.x) {
@@ -1018,7 +1068,7 @@ __global__ void __launch_bounds__(kTopPThreads) topp_cluster_kernel(int* out, co
   __syncthreads();
 
   // 2. sort descending, stable, over the cluster: the head of the order alone where that is enough
-  const bool head = topp_select<kToppCluster>(keyA, idxA, keyB, idxB, s_beg, s_end, topP, sm, crank);
+  const bool head = topp_select<kToppCluster>(keyA, idxA, keyB, idxB, s_beg, s_end, V, topP, sq, sm, crank);
   if (!head) {
     radix_pass_cluster(keyA, nullptr, keyB, idxB, V, 0, true, sm, crank);
     radix_pass_cluster(keyB, idxB, keyA, idxA, V, 8, false, sm, crank);

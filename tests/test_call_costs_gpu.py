@@ -108,3 +108,15 @@ def test_linear_of_64_short_rows(cuda):
 def test_linear_of_one_row_tile_against_two(cuda, K, n):
     one, two = times(linear(100, K, n, torch.float16), linear(160, K, n, torch.float16))
     assert one < 1.3 * two, (one, two)          # with K slices for the single row tile 1.7 to 2.3
+
+
+@pytest.mark.parametrize("B", [8, 32])
+def test_top_p_of_flat_rows_against_the_full_sort(cuda, B):
+    """topP = 2.6 leaves no choice but the sort; on a flat row the look at the largest weights must cost next to nothing beside it."""
+    V = 50257
+    p = torch.full((B, V), 1.0 / V, device="cuda")
+    u, ids = torch.rand(B, device="cuda"), torch.empty(B, dtype=torch.int32, device="cuda")
+    ws = torch.empty(N.lib().TSB200_TopPWorkspaceBytes(B, V), dtype=torch.uint8, device="cuda")
+    call = lambda top: lambda st: N.call("TSB200_TopPSample", 0, ids.data_ptr(), p.data_ptr(), B, V, top, 0.0, None, None, 0, u.data_ptr(), ws.data_ptr(), ws.numel(), st)  # noqa: E731
+    look, sort = times(call(0.95), call(2.6))
+    assert look < 1.06 * sort, (look, sort)     # one shared-memory add per key: 1.08 to 1.15
