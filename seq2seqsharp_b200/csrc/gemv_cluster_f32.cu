@@ -2,8 +2,8 @@
 //
 // The fp32 counterpart of gemm_cluster_tc.cu (no tensor-core type keeps fp32): a CTA streams its 16 KB tiles ([32 k][128 columns]) through a
 // ring of bulk copies, eight warps take four k of a tile each (a lane four columns of every row), the warps' sums meet in shared memory, the
-// cluster's through distributed shared memory in rank order.  Two CTAs fit an SM; the weights are asked for before the launch in front
-// has ended.  What bounds a small model's step is the chain of its launches (512-wide, six layers, one sequence, a
+// cluster's through distributed shared memory in rank order.  Two CTAs fit an SM while the rows over a CTA's K range take up to 28 KB; the
+// weights are asked for before the launch in front has ended.  What bounds a small model's step is the chain of its launches (512-wide, six layers, one sequence, a
 // 128-token request: 42.7 ms with the persistent stream-K kernel, 24.7 with this one).
 #include "cluster_sums.cuh"
 #include "stream_common.cuh"
@@ -185,10 +185,12 @@ int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const v
     a.rope = *rope;
   }
   const int groups = (N + 127) / 128, RM = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));
-  // K ranges while all CTAs are resident at once (two per SM), of at least two tiles of 32 k
+  auto smem_of = [&](int ks) { return fc_smem(RM, (a.KB + ks - 1) / ks); };
+  // K ranges while all CTAs are resident at once, of at least two tiles of 32 k.  An SM holds two CTAs, or one where the rows of a range are
+  // long (5 to 8 rows of more than 896 k)
   a.ks = 1;
-  while (a.ks < 8 && (int64_t)groups * a.ks * 2 <= 2 * st->sm_count && a.KB / (a.ks * 2) >= 2) a.ks *= 2;
-  const size_t smem = fc_smem(RM, (a.KB + a.ks - 1) / a.ks);
+  while (a.ks < 8 && (int64_t)groups * a.ks * 2 <= (int64_t)(smem_of(a.ks * 2) <= 112 * 1024 ? 2 : 1) * st->sm_count && a.KB / (a.ks * 2) >= 2) a.ks *= 2;
+  const size_t smem = smem_of(a.ks);
   if (smem > 220 * 1024) return 2;   // rows too long for the shared memory
   a.error = tc_error_word(device);
   switch (RM) {

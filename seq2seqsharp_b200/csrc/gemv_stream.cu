@@ -585,14 +585,20 @@ int TSB200_LinearPacked(int device, int dtype, void* y, float* y_f32, const void
   const int64_t z = workspace_bytes < kWsCounterBytes ? workspace_bytes : kWsCounterBytes;
   TSB_CUDA(cudaMemsetAsync(workspace, 0, (size_t)z, s));
   int* err = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsCounterBytes - 256);
-  static int gemv_rows = -1;
-  if (gemv_rows < 0) {
-    const char* e = getenv("TSB200_GEMV_MAXROWS");  // rows served by the FMA streaming GEMV here (default 4; the engine has its own default)
-    gemv_rows = e ? atoi(e) : 4;
+  static int gemv_rows = -2;   // rows served by the FMA streaming GEMV here; the engine has its own default
+  if (gemv_rows < -1) {
+    const char* e = getenv("TSB200_GEMV_MAXROWS");
+    gemv_rows = e && atoi(e) >= 0 ? atoi(e) : -1;
   }
-  if (M <= 4 && M <= gemv_rows) {
+  // not set: four, and fp32 rows that are not normed run on clusters (one row of 4096 -> 4096 10.4 us against 14.3, of 64 -> 64 4.4 against 5.7)
+  const int stream_rows = gemv_rows >= 0 ? gemv_rows : (dtype == TSB200_F32 && norm_type < 0 ? 0 : 4);
+  if (M <= 4 && M <= stream_rows) {
     const int r = launch_gemv_stream(device, st, dtype, Wp, norm_type < 0 ? x : (const void*)x_f32, norm_type < 0 ? 0 : (norm_type == 0 ? 2 : 1),
                                      gamma, norm_type == 0 ? beta : nullptr, eps, M, K, N, ep, err, false, workspace, workspace_bytes - 256, s);
+    if (r != 2) return r;
+  }
+  if (norm_type < 0 && dtype == TSB200_F32 && M <= 8) {
+    const int r = launch_gemv_cluster_f32(device, st, (const float*)x, Wp, M, K, N, ep, false, s);
     if (r != 2) return r;
   }
   if (norm_type >= 0 && dtype == TSB200_F16 && M <= 8) {

@@ -59,6 +59,13 @@ def test_fp16_rows(cuda, M, K, n):
     check(M, K, n, torch.float16, (0, 1))
 
 
+# 8 rows of 11008: one CTA per SM; 33, 100, 4097: K ends inside a tile; 4096 -> 130: eight ranks, the ring of five tiles wraps
+@pytest.mark.parametrize("M", [5, 6, 7, 8])
+@pytest.mark.parametrize("K,n", [(4, 5), (33, 127), (100, 130), (4097, 128), (4096, 130), (512, 2000), (96, 20000), (11008, 260)])
+def test_fp32_rows(cuda, M, K, n):
+    check(M, K, n, torch.float32, (0, 1))
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
 @pytest.mark.parametrize("M", [1, 3, 8, 20, 70])
 def test_weights_off_a_16_byte_boundary(cuda, dtype, M):
