@@ -66,6 +66,8 @@ TSB200_API int TSB200_MemcpyD2H(int device, void* dst, const void* src, int64_t 
 TSB200_API int TSB200_MemcpyD2D(int device, void* dst, const void* src, int64_t bytes, void* stream);
 /* cross-device copy; replaces cuMemcpyPeer in TensorSharp.CUDA/KernelOps/CopyOps.cs:47-97 */
 TSB200_API int TSB200_MemcpyPeer(int dst_device, void* dst, int src_device, const void* src, int64_t bytes);
+/* Waits for the stream.  Fails with "a kernel gave up waiting" when a bounded wait inside a stand-alone linear or prompt attention
+ * ran out since the last such report (so does TSB200_MemcpyD2H); those calls themselves return before their kernels have run. */
 TSB200_API int TSB200_Synchronize(int device, void* stream);
 /* IAllocator.GetAllocatedMemoryRatio (TensorSharp/IAllocator.cs:19) */
 TSB200_API int TSB200_MemoryInfo(int device, int64_t* free_bytes, int64_t* total_bytes);

@@ -1,7 +1,7 @@
 // Lifecycle, error reporting and memory entry points of libtsb200.
 #include <mutex>
 
-#include "common.cuh"
+#include "kernels.cuh"
 
 namespace tsb {
 
@@ -68,6 +68,14 @@ int check_tensor(const TSB200Tensor* t, const char* name) {
   TSB_CHECK(t->data != nullptr, "%s: null data pointer", name);
   TSB_CHECK(t->ndim >= 1 && t->ndim <= 4, "%s: ndim %d not in 1..4", name, t->ndim);
   for (int i = 0; i < t->ndim; ++i) TSB_CHECK(t->sizes[i] >= 0, "%s: negative size", name);
+  return 1;
+}
+
+// A stand-alone call returns before its kernels have run; a wait that ran out in one of them is reported where the host waits for it.
+static int check_waits(DeviceState* st) {
+  if (!st->waits) return 1;
+  const int e = tc_take_error() | gs_take_error();
+  TSB_CHECK(e == 0, "a kernel gave up waiting: outputs of calls since the last synchronisation are incomplete");
   return 1;
 }
 
@@ -158,7 +166,7 @@ int TSB200_MemcpyD2H(int device, void* dst, const void* src, int64_t bytes, void
   cudaStream_t s = pick_stream(st, stream);
   TSB_CUDA(cudaMemcpyAsync(dst, src, (size_t)bytes, cudaMemcpyDeviceToHost, s));
   TSB_CUDA(cudaStreamSynchronize(s));
-  return 1;
+  return check_waits(st);
 }
 
 int TSB200_MemcpyD2D(int device, void* dst, const void* src, int64_t bytes, void* stream) {
@@ -181,7 +189,7 @@ int TSB200_Synchronize(int device, void* stream) {
   DeviceState* st;
   TSB_TRY(use_device(device, &st));
   TSB_CUDA(cudaStreamSynchronize(pick_stream(st, stream)));
-  return 1;
+  return check_waits(st);
 }
 
 int TSB200_MemoryInfo(int device, int64_t* free_bytes, int64_t* total_bytes) {

@@ -39,13 +39,14 @@ struct PaArgs {
   int z_seq, z_head;                         // outermost coordinate of mapK / mapV: b * z_seq + head * z_head
   const int* starts;                         // packed rows: first row of every sequence (B + 1), or NULL: S rows each
   int vec_out;                               // out is 16-byte aligned
+  unsigned wait_limit;                       // polls of a wait before the CTA gives up
   int* error;
 };
 
-__device__ __forceinline__ bool pa_wait(uint64_t* bar, unsigned parity, volatile int* err) {
+__device__ __forceinline__ bool pa_wait(uint64_t* bar, unsigned parity, volatile int* err, unsigned limit) {
   const uint32_t a = s_u32(bar);
 #pragma unroll 1
-  for (unsigned i = 0; i < kTcSpin; ++i) {
+  for (unsigned i = 0; i < limit; ++i) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -219,7 +220,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
       int ks = 0, vs = 0;   // tiles asked for so far
       auto load_k = [&](int j) {
         const int st = j % NKS;
-        if (j >= NKS && !pa_wait(&k_empty[st], (unsigned)((j / NKS - 1) & 1), err)) return false;
+        if (j >= NKS && !pa_wait(&k_empty[st], (unsigned)((j / NKS - 1) & 1), err, a.wait_limit)) return false;
         tc_mbar_expect_tx(&k_full[st], QB * kPaBox);
 #pragma unroll
         for (int i = 0; i < QB; ++i) {
@@ -233,7 +234,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (j + 1 < n_tiles && !load_k(j + 1)) break;
         const int st = j % NVS;
-        if (j >= NVS && !pa_wait(&v_empty[st], (unsigned)((j / NVS - 1) & 1), err)) break;
+        if (j >= NVS && !pa_wait(&v_empty[st], (unsigned)((j / NVS - 1) & 1), err, a.wait_limit)) break;
         tc_mbar_expect_tx(&v_full[st], VB * kPaBox);
 #pragma unroll
         for (int i = 0; i < VB; ++i) pa_load_3d(sV + (st * VB + i) * kPaBox, &mapV, a.vx0 + kvh * a.vx + 64 * i, j * kPaKeys, z, &v_full[st]);
@@ -258,22 +259,22 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
         }
         umma_commit(&s_full[t]);
       };
-      bool ok = pa_wait(&k_full[0], 0, err);
+      bool ok = pa_wait(&k_full[0], 0, err, a.wait_limit);
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         if (!ok || n_of[t] == 0) continue;
-        ok = pa_wait(&q_full[t], 0, err);
+        ok = pa_wait(&q_full[t], 0, err, a.wait_limit);
         if (ok) qk(t, 0);
       }
       umma_commit(&k_empty[0]);
       for (int j = 0; j < n_tiles && ok; ++j) {
         const bool more = j + 1 < n_tiles;
-        ok = pa_wait(&v_full[j % NVS], (unsigned)((j / NVS) & 1), err);
-        if (ok && more) ok = pa_wait(&k_full[(j + 1) % NKS], (unsigned)(((j + 1) / NKS) & 1), err);
+        ok = pa_wait(&v_full[j % NVS], (unsigned)((j / NVS) & 1), err, a.wait_limit);
+        if (ok && more) ok = pa_wait(&k_full[(j + 1) % NKS], (unsigned)(((j + 1) / NKS) & 1), err, a.wait_limit);
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           if (!ok || j >= n_of[t]) continue;
-          if (!(ok = pa_wait(&p_full[t], (unsigned)(j & 1), err))) continue;
+          if (!(ok = pa_wait(&p_full[t], (unsigned)(j & 1), err, a.wait_limit))) continue;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           // V stage = [box][128 keys][128 B]: 8-key groups 1024 B apart (SBO), boxes kPaBox apart (LBO); 16 keys = 2048 B
           const uint32_t v = sV + (j % NVS) * VB * kPaBox;
@@ -285,10 +286,6 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
         }
         umma_commit(&v_empty[j % NVS]);
         if (more) umma_commit(&k_empty[(j + 1) % NKS]);
-      }
-      if (!ok) {   // products in flight end before TMEM is given back
-        umma_commit(drain);
-        tc_mbar_wait(drain, 0);
       }
     }
   } else {
@@ -305,7 +302,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
     float m = -INFINITY, l = 0.0f;
     bool ok = true;
     for (int j = 0; j < n; ++j) {
-      ok = __all_sync(0xffffffffu, pa_wait(&s_full[t], (unsigned)(j & 1), err));
+      ok = __all_sync(0xffffffffu, pa_wait(&s_full[t], (unsigned)(j & 1), err, a.wait_limit));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       uint32_t s[4][32];
@@ -367,7 +364,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       pa_arrive(&p_full[t]);
     }
-    if (n > 0 && ok && __all_sync(0xffffffffu, pa_wait(&o_full[t], 0, err))) {
+    if (n > 0 && ok && __all_sync(0xffffffffu, pa_wait(&o_full[t], 0, err, a.wait_limit))) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inv = l > 0.0f ? 1.0f / l : 0.0f;
       H* out = reinterpret_cast<H*>(a.out) + (((int64_t)row0 + pos) * a.H + head) * (VB * 64);
@@ -393,6 +390,11 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (w == 9) {
+    if (lane == 0 && s_err) {   // some warp gave up: products in flight end before TMEM is given back
+      umma_commit(drain);
+      tc_mbar_wait(drain, 0);
+    }
+    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
@@ -437,6 +439,7 @@ static int pa_launch(int device, const CUtensorMap& q, const CUtensorMap& k, con
   a.tiles = (a.S + 2 * a.QT - 1) / (2 * a.QT);
   a.vec_out = ((uintptr_t)a.out % 16) == 0 ? 1 : 0;
   a.error = tc_error_word(device);
+  a.wait_limit = tc_wait_limit();
   const int64_t grid = (int64_t)a.tiles * a.heads * a.B;
   TSB_CHECK(grid <= 0x7fffffff, "prompt attention: %lld blocks", (long long)grid);
   attn_prefill_tc_kernel<H, QB, VB, NKS, NVS><<<(int)grid, kPaThreads, smem, s>>>(q, k, r, v, a);

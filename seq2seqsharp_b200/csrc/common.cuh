@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <string>
@@ -50,6 +51,7 @@ struct DeviceState {
   int sm_count = 0;
   cudaStream_t stream = nullptr;  // library-owned non-blocking stream
   long long launches = 0;
+  std::atomic<bool> waits{false};  // a stand-alone call has launched a kernel whose bounded waits raise the device's error words
 };
 // Makes `device` current, lazily creates its state.  Fails when the device is absent or not sm_100.
 int use_device(int device, DeviceState** st);

@@ -205,6 +205,8 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   }
   __syncthreads();
   if (w == 1) {
+    if (lane == 0 && s_err) tc_mbar_wait(acc, 0);   // some warp gave up: products in flight end before TMEM is given back
+    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }

@@ -570,6 +570,16 @@ int tc_take_error() {
   return e;
 }
 
+unsigned tc_wait_limit() {
+  static unsigned limit = 0;
+  if (!limit) {
+    const char* e = getenv("TSB200_WAIT_LIMIT");
+    const int n = e ? atoi(e) : 0;
+    limit = n > 0 ? (unsigned)n : kTcSpin;
+  }
+  return limit;
+}
+
 int* tc_error_word(int device) {
   static int* word[kMaxDevices] = {};
   if (!word[device]) {

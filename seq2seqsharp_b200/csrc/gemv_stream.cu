@@ -581,10 +581,11 @@ int TSB200_LinearPacked(int device, int dtype, void* y, float* y_f32, const void
   TSB_CHECK(!ep.glu || N % 2 == 0, "linear_packed: gated activations need an even (interleaved) column count");
   cudaStream_t s = pick_stream(st, stream);
   TSB_TRY(init_stream_attrs(device));
-  // counters at the head of the workspace must start at zero; the last word of the workspace is the error flag
+  // counters at the head of the workspace must start at zero
   const int64_t z = workspace_bytes < kWsCounterBytes ? workspace_bytes : kWsCounterBytes;
   TSB_CUDA(cudaMemsetAsync(workspace, 0, (size_t)z, s));
-  int* err = reinterpret_cast<int*>(reinterpret_cast<char*>(workspace) + kWsCounterBytes - 256);
+  int* err = tc_error_word(device);
+  st->waits = true;
   static int gemv_rows = -2;   // rows served by the FMA streaming GEMV here; the engine has its own default
   if (gemv_rows < -1) {
     const char* e = getenv("TSB200_GEMV_MAXROWS");

@@ -1176,6 +1176,7 @@ int TSB200_PrefillAttention(int device, int dtype, void* out, const void* q, int
   DeviceState* st;
   TSB_TRY(use_device(device, &st));
   TSB_CHECK(out && q && cacheK && cacheV, "prefill_attention: null pointer");
+  st->waits = true;
   return launch_attention(device, st, dtype, out, q, q_row_stride, cacheK, cacheV, B, S, H, Hkv, hd, T0, nullptr, Tmax, 0,
                           nullptr, 0, pick_stream(st, stream));
 }

@@ -45,3 +45,31 @@ def test_a_wait_that_runs_out_fails_the_call_and_leaves_the_engine_usable(cuda, 
     np.testing.assert_array_equal(gpt.Prefill(prompt, opts), first)
     np.testing.assert_array_equal(gpt.Decode(6, opts), good)
     gpt.close()
+
+
+def test_a_wait_that_runs_out_in_a_stand_alone_call_is_reported_where_the_host_waits(cuda):
+    """One poll per wait (an environment variable, hence a process of its own): the prompt attention gives up before its first tile has
+    arrived, waits for its copies and products in flight, and returns; the synchronisation fails, and only the first one."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from seq2seqsharp_b200 import _native as N
+q = torch.randn(2, 300, 3 * 64, device="cuda", dtype=torch.float16)
+k, v = (torch.randn(2, 1, 300, 64, device="cuda", dtype=torch.float16) for _ in range(2))
+o = torch.empty(2, 300, 64, device="cuda", dtype=torch.float16)
+torch.cuda.synchronize()
+N.call("TSB200_PrefillAttention", 0, N.F16, o.data_ptr(), q.data_ptr(), 192, k.data_ptr(), v.data_ptr(), 2, 300, 1, 1, 64, 0, 300, None)
+try:
+    N.call("TSB200_Synchronize", 0, None)
+    print("silent")
+except N.TSB200Error as e:
+    print(e)
+N.call("TSB200_Synchronize", 0, None)
+print("usable", float(torch.ones(4, device="cuda").sum()))
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120, env=dict(os.environ, TSB200_WAIT_LIMIT="1"),
+                       cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+    assert r.returncode == 0, r.stderr
+    assert "gave up waiting" in r.stdout and "usable 4.0" in r.stdout, r.stdout
