@@ -263,7 +263,7 @@ struct RopeFuse {
 };
 int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, const void* gamma, const void* beta, int norm_type, float eps,
                                 const void* Wp, int M, int K, int N, const Epilogue& ep, int* error_flag, bool pdl, void* ws, int64_t ws_bytes,
-                                cudaStream_t s, const RopeFuse* rope = nullptr);
+                                cudaStream_t s);
 // 1..64 rows of a 16-bit type, the K ranges of 128 columns on the CTAs of a cluster (gemm_cluster_tc.cu); 1 ok, 0 error, 2 not handled
 int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
                            const RopeFuse* rope = nullptr);
