@@ -1,5 +1,5 @@
 """Linears at the edges of the rules that choose their kernels: fp32 rows beyond 16 (clusters over K), deep and shallow rings of the tensor-core
-kernel, narrow widths with the norm inside."""
+kernel, and the engine's step with rotation and append in the q | k | v epilogue at widths of all kinds."""
 import numpy as np
 import pytest
 import torch
@@ -48,22 +48,29 @@ def test_tensor_core_epilogues(cuda, oracle, M, K, Nn):
 
 @pytest.mark.parametrize("d,H,B,norm", [(64, 1, 8, "LayerNorm"), (320, 5, 3, "RMSNorm"), (768, 12, 8, "LayerNorm"), (992, 31, 7, "RMSNorm"), (1056, 33, 8, "LayerNorm"),
                                         (2080, 65, 4, "RMSNorm")])
-def test_norm_inside_the_step_at_any_width(cuda, monkeypatch, d, H, B, norm):
-    """The captured step with the norm inside its linears against the same step with a launch for every norm."""
+def test_rotation_and_append_in_the_epilogue_at_any_width(cuda, oracle, monkeypatch, d, H, B, norm):
+    """The captured step with rotation and append in the epilogue of q | k | v against the same step with a launch for them; norms, which are
+    launches in both, and all else against the oracle."""
     from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, GPT, GPTConfig, MultiHeadAttentionTypeEnums, NormEnums, PositionEmbeddingEnums, synthetic_weights)
     cfg = GPTConfig(L=2, d=d, H=H, hd=d // H, F=256, V=515, norm=getattr(NormEnums, norm), act=ActivateFuncEnums.GELU, pe=PositionEmbeddingEnums.RoPE,
                     attn=MultiHeadAttentionTypeEnums.MHA, dtype="float16")
     w = synthetic_weights(cfg, 7, std=0.05, bias_std=0.02)
     prompt = np.random.default_rng(d).integers(1, cfg.V, size=(B, 9)).astype(np.int32)
     opts = DecodingOptions(MaxTgtSentLength=20)
-    logits = []
+    logits, fed = [], [np.arange(B, dtype=np.int32) + 3 + i for i in range(3)]
     for fused in ("1", "0"):
         monkeypatch.setenv("TSB200_FUSED_STEP", fused)
         gpt = GPT(cfg, max_batch=B, max_tokens=24)
         gpt.LoadWeights(w)
         gpt.Prefill(prompt, opts)
-        for i in range(3):
-            gpt.StepHost(np.arange(B, dtype=np.int32) + 3 + i, opts)
+        for ids in fed:
+            gpt.StepHost(ids, opts)
         logits.append(gpt.Logits()[0].copy())
-    # the linears' sums are the same up to their order; a normed value next to a rounding boundary moves by 2^-11
+    # the same kernels sum in the same order, and the value is rounded to fp16 before it is rotated in both
     assert np.abs(logits[0] - logits[1]).max() <= 4 * 2.0 ** -11 * np.abs(logits[1]).max()
+    orc = oracle.OracleGPT(cfg, w, max_pos=24, threads=4)
+    ref = orc.step(prompt)[0]
+    for ids in fed:
+        ref = orc.step(ids[:, None])[0]
+    for got in logits:      # fp16 weights and activations through two layers: the bound of the token loop's tests
+        assert np.abs(got - ref).max() <= 2e-2 * np.abs(ref).max()

@@ -47,7 +47,7 @@ def test_at_the_limits_of_short_prompts(cuda, hd, H, Hkv, S, T0):
     test_against_float64(cuda, hd, H, Hkv, S, T0)
 
 
-@pytest.mark.parametrize("B", [37, 75])      # 16 rows on top of 60 keys, 8 KV heads: within and beyond two waves of whole SMs
+@pytest.mark.parametrize("B", [37, 75])      # 16 rows on top of 130 keys, 8 KV heads: within and beyond two waves of whole SMs
 def test_many_short_prompts_on_a_cache(cuda, B):
     H, Hkv, hd, S, T0 = 8, 8, 64, 16, 130
     q = torch.randn(B, S, H * hd, device="cuda").half()
