@@ -244,8 +244,9 @@ def make_options(strat, topP, max_tokens, seed, seq_base):
 
 def per_operation_engine(cfg, device, max_batch, max_tokens, seed):
     """An independent engine on ONE GPU that decodes with one launch per operation and none of the fusions of the
-    benchmarked path (no persistent decode-step kernel, no tensor parallelism; separate norm and RoPE-append launches; up to
-    four rows on the FMA streaming GEMV instead of the tensor-core kernel): the checker of the benchmarked engine."""
+    benchmarked path (no persistent decode-step kernel, no tensor parallelism; RoPE and append as a launch of their own; up to
+    four rows on the FMA streaming GEMV, which norms its rows itself, instead of a norm launch and the tensor-core kernel; more
+    rows share the norm launch with the benchmarked engine): the checker of the benchmarked engine."""
     from seq2seqsharp_b200.gpt import GPT
     knobs = {"TSB200_STACK": "0", "TSB200_FUSED_STEP": "0", "TSB200_GEMV_MAXROWS": "4"}    # read when the engine is created
     old = {k: os.environ.get(k) for k in knobs}

@@ -17,7 +17,7 @@
 //
 // What bounds it: the exponentials (16 per clock and SM: at head size 64 a tile's 16384 take twice as long as its products).  Measured, one
 // sequence of 16384 tokens, 32 heads, 8 KV heads: head size 64 6.55 ms -> 1.70 ms (645 TFLOP/s), 128 11.6 -> 1.97 ms (1117 TFLOP/s) against the
-// kernel on mma.sync with 64 rows per CTA that this one replaces; 1024 tokens of head size 64: 48 -> 23 us; 4 x 509 of 128: 71 -> 25 us.
+// kernel on mma.sync with 64 rows per CTA, which short prompts still take (ops_attention.cu); 1024 tokens of head size 64: 48 -> 23 us; 4 x 509 of 128: 71 -> 25 us.
 // Three sequences of 1537 tokens, 12 layers of 16 latent heads of 192 | 128: the whole prompt pass 18.9 -> 15.6 ms.
 #include "tc_common.cuh"
 

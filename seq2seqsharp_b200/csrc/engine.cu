@@ -271,8 +271,8 @@ struct Gpt {
   bool pdl = true;         // programmatic dependent launch between the kernels of a decode step
   // persistent decode-step kernel (decode_stack.cu): the program of operations and its scratch
   bool use_stack = true;
-  bool fuse_step = true;       // per-operation path, up to eight rows: norm (and RoPE + cache append) inside the linear's launch
-                               // (TSB200_FUSED_STEP=0: separate norm / RoPE-append launches, e.g. for a checker engine)
+  bool fuse_step = true;       // per-operation path, up to 64 rows (fp32: 8): RoPE + cache append in the epilogue of the q | k | v projection
+                               // (TSB200_FUSED_STEP=0: a launch of its own, e.g. for a checker engine); the norms are launches either way
   // One GPU: one launch per operation at every batch (linears on clusters; 7B-class fp16, one sequence: 2.69 ms per step against 3.20 with the
   // stream-K persistent kernel and 3.10 with the owner-partitioned one; tiny fp32 model: 0.18 ms against 0.30).
   // Tensor-parallel engines keep the persistent kernels (the exchange lives there).

@@ -4,6 +4,7 @@
     python -m seq2seqsharp_b200.kernel_cases decode [--workload c3_b1] [--steps 2]      (whole decode steps, small model)
     python -m seq2seqsharp_b200.kernel_cases topp   [--rows 8] [--V 32000]
     python -m seq2seqsharp_b200.kernel_cases attention [--B 4] [--H 32] [--Hkv 8] [--hd 64] [--T 16384]
+    python -m seq2seqsharp_b200.kernel_cases prompt [--B 1] [--H 32] [--Hkv 8] [--hd 64] [--T 4096]    (causal attention of a prompt)
     python -m seq2seqsharp_b200.kernel_cases beam   [--workload c3_b1] [--B 1] [--beams 4] [--prompt 1024] [--steps 32]
 
 Each case prints its own CUDA-event timing and the algorithmic bytes it moves, so a capture and a plain run can be
@@ -190,9 +191,19 @@ def case_attention(a):
     print("flash-decode B=%d H=%d Hkv=%d hd=%d T=%d: %.3f ms/launch, %.1f GB/s algorithmic" % (a.B, a.H, a.Hkv, a.hd, a.T, ms, nbytes / ms / 1e6))
 
 
+def case_prompt(a):
+    q = torch.randn(a.B, a.T, a.H * a.hd, device="cuda").half()
+    cK, cV = (torch.randn(a.B, a.Hkv, a.T, a.hd, device="cuda").half() for _ in range(2))
+    out = torch.empty_like(q)
+    ms = _time(lambda: N.call("TSB200_PrefillAttention", 0, N.F16, out.data_ptr(), q.data_ptr(), a.H * a.hd, cK.data_ptr(), cV.data_ptr(), a.B, a.T, a.H, a.Hkv,
+                              a.hd, 0, a.T, _stream()), a.iters)
+    flops = 2.0 * a.B * a.H * a.hd * a.T * (a.T + 1)     # Q K^T and P V over the visible keys
+    print("prompt attention B=%d H=%d Hkv=%d hd=%d T=%d: %.3f ms/launch, %.0f TFLOP/s" % (a.B, a.H, a.Hkv, a.hd, a.T, ms, flops / ms / 1e9))
+
+
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["gemv", "gemv_packed", "decode", "topp", "attention", "beam"])
+    ap.add_argument("case", choices=["gemv", "gemv_packed", "decode", "topp", "attention", "prompt", "beam"])
     ap.add_argument("--norm", type=int, default=0)
     ap.add_argument("--M", type=int, default=1)
     ap.add_argument("--K", type=int, default=4096)
@@ -217,7 +228,7 @@ def main():
     if not torch.cuda.is_available():
         raise SystemExit("kernel_cases needs a GPU (no CPU fallback)")
     torch.cuda.set_device(0)
-    {"gemv": case_gemv, "gemv_packed": case_gemv_packed, "decode": case_decode, "topp": case_topp, "attention": case_attention, "beam": case_beam}[a.case](a)
+    {"gemv": case_gemv, "gemv_packed": case_gemv_packed, "decode": case_decode, "topp": case_topp, "attention": case_attention, "prompt": case_prompt, "beam": case_beam}[a.case](a)
 
 
 if __name__ == "__main__":
