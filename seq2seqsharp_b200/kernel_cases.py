@@ -4,7 +4,7 @@
     python -m seq2seqsharp_b200.kernel_cases decode [--workload c3_b1] [--steps 2]      (whole decode steps, small model)
     python -m seq2seqsharp_b200.kernel_cases topp   [--rows 8] [--V 32000]
     python -m seq2seqsharp_b200.kernel_cases attention [--B 4] [--H 32] [--Hkv 8] [--hd 64] [--T 16384]
-    python -m seq2seqsharp_b200.kernel_cases prompt [--B 1] [--H 32] [--Hkv 8] [--hd 64] [--T 4096]    (causal attention of a prompt)
+    python -m seq2seqsharp_b200.kernel_cases prompt [--B 4] [--H 32] [--Hkv 8] [--hd 64] [--T 16384]    (causal attention of a prompt)
     python -m seq2seqsharp_b200.kernel_cases beam   [--workload c3_b1] [--B 1] [--beams 4] [--prompt 1024] [--steps 32]
 
 Each case prints its own CUDA-event timing and the algorithmic bytes it moves, so a capture and a plain run can be

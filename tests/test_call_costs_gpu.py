@@ -101,7 +101,7 @@ def linear(M, K, n, dtype):
 
 def test_linear_of_64_short_rows(cuda):
     many, few = times(linear(64, 64, 64, torch.float16), linear(5, 64, 64, torch.float16))
-    assert many < 2.0 * few, (many, few)        # one group of four columns after the other, each with its own loads: 3.1
+    assert many < 2.5 * few, (many, few)        # 10.6 against 5.5 us; with a division per pushed sum 19.5 against 6.2
 
 
 @pytest.mark.parametrize("K,n", [(4096, 4096), (2048, 3072)])
@@ -110,13 +110,12 @@ def test_linear_of_one_row_tile_against_two(cuda, K, n):
     assert one < 1.3 * two, (one, two)          # with K slices for the single row tile 1.7 to 2.3
 
 
-@pytest.mark.parametrize("B", [8, 32])
-def test_top_p_of_flat_rows_against_the_full_sort(cuda, B):
+def test_top_p_of_flat_rows_against_the_full_sort(cuda):
     """topP = 2.6 leaves no choice but the sort; on a flat row the look at the largest weights must cost next to nothing beside it."""
-    V = 50257
+    B, V = 32, 50257
     p = torch.full((B, V), 1.0 / V, device="cuda")
     u, ids = torch.rand(B, device="cuda"), torch.empty(B, dtype=torch.int32, device="cuda")
     ws = torch.empty(N.lib().TSB200_TopPWorkspaceBytes(B, V), dtype=torch.uint8, device="cuda")
     call = lambda top: lambda st: N.call("TSB200_TopPSample", 0, ids.data_ptr(), p.data_ptr(), B, V, top, 0.0, None, None, 0, u.data_ptr(), ws.data_ptr(), ws.numel(), st)  # noqa: E731
     look, sort = times(call(0.95), call(2.6))
-    assert look < 1.06 * sort, (look, sort)     # one shared-memory add per key: 1.08 to 1.15
+    assert look < 1.07 * sort, (look, sort)     # 1.00; with one shared counter for all keys of a bin 1.11
