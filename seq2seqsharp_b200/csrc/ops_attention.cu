@@ -57,12 +57,12 @@ __global__ void rope_table_kernel(float2* __restrict__ tab, int Tmax, int hd, do
 }
 
 // q [rows,H,hd] rotated in place; k rotated and stored with v into the cache at positions T0 + s.  A thread takes V elements
-// (16 bytes, or one pair where a pointer or a size is not a multiple of that, or without a table); a CTA takes a part of a row
-// (blockIdx.y) or several short rows.  `where`: packed rows (kernels.cuh); from row `rows` on, up to `listed`, the position's value is cleared.
+// (16 bytes, or one pair where a pointer or a size is not a multiple of that, or without a table) at a time; a CTA takes a row (WHOLE), a
+// part of one (blockIdx.y; a thread one piece) or several short rows.  `where`: packed rows (kernels.cuh); from row `rows` on, up to `listed`, the position's value is cleared.
 // tab may be NULL: cos/sin are evaluated here, in double, one pair per thread - that chain is what bounds such a call (one row of 48 heads
 // of 128: 3.2 us; 13.7 with four pairs per thread and a CTA per row).
 // What bounds it with a table: bytes (16384 rows of 48 heads of 64: 200 MB; 154 us with one pair per thread and 64-bit index arithmetic).
-template <typename T, int V>
+template <typename T, int V, bool WHOLE>
 __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
                                    int64_t kv_rs, T* cK, T* cV, int rows, int listed, const int2* where, int S, int H, int Hkv, int hd,
                                    int T0_arg, const int* dT0, int Tmax, int use_rope, double base,
@@ -74,47 +74,54 @@ __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
   const int sub = rows_here > 1 ? (int)threadIdx.x / per_row : 0;
   if (rows_here > 1 && sub >= rows_here) return;
   const int row = (rows_here > 1 ? (int)blockIdx.x * rows_here : (int)blockIdx.x) + sub;
-  const int it = rows_here > 1 ? (int)threadIdx.x - sub * per_row : (int)(blockIdx.y * blockDim.x + threadIdx.x);
-  if (row >= listed || it >= per_row) return;
+  if (row >= listed) return;
   const int b = where ? where[row].x : row / S, s = where ? where[row].y : row % S;
   const int T0 = state_len(dT0, b, T0_arg);  // the engine keeps the cache lengths on the device so one CUDA graph serves every step
   const int pos = T0 + s;
   TSB_DEV_CHECK(attention, pos >= 0 && pos < Tmax, 0x201, (void)0)   // append position outside the cache (row skipped)
   if (pos >= Tmax) return;  // capacity is checked on the host; never write past the cache
   const bool clear = row >= rows;
-  const int head = it / pieces, i = (it % pieces) * V;
-  if (clear && head < H + Hkv) return;
-  Piece x;
-  if (clear) {
+  auto piece = [&](int it) {
+    const int head = it / pieces, i = (it % pieces) * V;
+    if (clear && head < H + Hkv) return;
+    Piece x;
+    if (clear) {
 #pragma unroll
-    for (int e = 0; e < V; ++e) x.e[e] = from_f<T>(0.0f);
-  } else {
-    const T* src = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
-                            : (head < H + Hkv ? k + (int64_t)row * kv_rs + (int64_t)(head - H) * hd : v + (int64_t)row * kv_rs + (int64_t)(head - H - Hkv) * hd);
-    if constexpr (V > 2) x = *reinterpret_cast<const Piece*>(src + i);
-    else x.e[0] = src[i], x.e[1] = src[i + 1];
-  }
-  if (use_rope && head < H + Hkv) {
-#pragma unroll
-    for (int e = 0; e < V; e += 2) {
-      float c, sn;
-      if (tab) {
-        const float2 cs = tab[(int64_t)pos * (hd / 2) + (i + e) / 2];
-        c = cs.x;
-        sn = cs.y;
-      } else {
-        rope_cs((i + e) / 2, hd, pos, base, c, sn);
-      }
-      const float x0 = to_f<T>(x.e[e]), x1 = to_f<T>(x.e[e + 1]);
-      x.e[e] = from_f<T>(x0 * c - x1 * sn);
-      x.e[e + 1] = from_f<T>(x1 * c + x0 * sn);
+      for (int e = 0; e < V; ++e) x.e[e] = from_f<T>(0.0f);
+    } else {
+      const T* src = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
+                              : (head < H + Hkv ? k + (int64_t)row * kv_rs + (int64_t)(head - H) * hd : v + (int64_t)row * kv_rs + (int64_t)(head - H - Hkv) * hd);
+      if constexpr (V > 2) x = *reinterpret_cast<const Piece*>(src + i);
+      else x.e[0] = src[i], x.e[1] = src[i + 1];
     }
+    if (use_rope && head < H + Hkv) {
+#pragma unroll
+      for (int e = 0; e < V; e += 2) {
+        float c, sn;
+        if (tab) {
+          const float2 cs = tab[(int64_t)pos * (hd / 2) + (i + e) / 2];
+          c = cs.x;
+          sn = cs.y;
+        } else {
+          rope_cs((i + e) / 2, hd, pos, base, c, sn);
+        }
+        const float x0 = to_f<T>(x.e[e]), x1 = to_f<T>(x.e[e + 1]);
+        x.e[e] = from_f<T>(x0 * c - x1 * sn);
+        x.e[e + 1] = from_f<T>(x1 * c + x0 * sn);
+      }
+    }
+    if (head < H && !use_rope) return;
+    T* dst = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
+                      : (head < H + Hkv ? cK : cV) + (((int64_t)b * Hkv + (head < H + Hkv ? head - H : head - H - Hkv)) * Tmax + pos) * hd;
+    if constexpr (V > 2) *reinterpret_cast<Piece*>(dst + i) = x;
+    else dst[i] = x.e[0], dst[i + 1] = x.e[1];
+  };
+  if constexpr (WHOLE) {
+    for (int it = threadIdx.x; it < per_row; it += blockDim.x) piece(it);
+  } else {
+    const int it = rows_here > 1 ? (int)threadIdx.x - sub * per_row : (int)(blockIdx.y * blockDim.x + threadIdx.x);
+    if (it < per_row) piece(it);
   }
-  if (head < H && !use_rope) return;
-  T* dst = head < H ? q + (int64_t)row * q_rs + (int64_t)head * hd
-                    : (head < H + Hkv ? cK : cV) + (((int64_t)b * Hkv + (head < H + Hkv ? head - H : head - H - Hkv)) * Tmax + pos) * hd;
-  if constexpr (V > 2) *reinterpret_cast<Piece*>(dst + i) = x;
-  else dst[i] = x.e[0], dst[i + 1] = x.e[1];
 }
 
 // ------------------------------------------------------------------------------------------------ attention
@@ -1081,11 +1088,15 @@ static int launch_rope_append_t(int device, DeviceState* st, T* q, const T* k, c
                                 cudaStream_t s) {
   const int rows = pack ? pack->rows : B * S, listed = pack ? pack->listed : rows;
   const int64_t per_row = (int64_t)(H + 2 * Hkv) * (hd / V);
-  const int64_t parts = (per_row + 383) / 384;   // equal parts of up to 384 pieces; several rows of up to 128
-  const int threads = per_row <= 128 ? 256 : (int)((per_row + parts - 1) / parts + 31) / 32 * 32;
+  // Equal parts of up to 384 pieces, several rows of up to 128 - or, with a table and more rows than SMs, a CTA of 256 for a long row (2036 rows of
+  // 768 pieces, cold: 18.9 us against 21.7 in two parts; one piece per thread is faster where a row fits a CTA: 8192 rows of 384 pieces 39 us, 45
+  // in a loop)
+  const bool whole = V > 2 && tab && per_row > 512 && listed > 2 * st->sm_count;
+  const int64_t parts = whole ? 1 : (per_row + 383) / 384;
+  const int threads = per_row <= 128 || whole ? 256 : (int)((per_row + parts - 1) / parts + 31) / 32 * 32;
   const int64_t rows_here = threads / per_row > 1 ? threads / per_row : 1;
   TSB_CHECK(parts <= 65535, "rope_append: rows of %lld elements", (long long)per_row * V);
-  TSB_CUDA(launch_k(rope_append_kernel<T, V>, dim3((unsigned)((listed + rows_here - 1) / rows_here), (unsigned)parts), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, listed, pack ? pack->where : (const int2*)nullptr,
+  TSB_CUDA(launch_k(whole ? rope_append_kernel<T, V, (V > 2)> : rope_append_kernel<T, V, false>, dim3((unsigned)((listed + rows_here - 1) / rows_here), (unsigned)parts), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, listed, pack ? pack->where : (const int2*)nullptr,
                     S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
   return 1;
 }

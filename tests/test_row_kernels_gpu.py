@@ -106,3 +106,23 @@ def test_nuclei_around_the_selection_limit(cuda, oracle, rows, n):
 def test_softmax_at_the_limits_of_the_clusters(cuda, oracle, B, V):
     """Rows and widths at both sides of the rule that gives a row eight CTAs or one."""
     test_softmax_and_first_maximum(cuda, oracle, B, V)
+
+
+def test_rotation_of_many_long_rows_with_a_table(cuda):
+    """400 rows of 768 pieces, a CTA each, against 200 at a time, where a row is shared out: the engine's prompt pass, where the table is."""
+    from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, GPT, GPTConfig, MultiHeadAttentionTypeEnums, NormEnums, PositionEmbeddingEnums, synthetic_weights)
+    cfg = GPTConfig(L=1, d=2048, H=32, hd=64, F=256, V=515, norm=NormEnums.RMSNorm, act=ActivateFuncEnums.SwiGLU, pe=PositionEmbeddingEnums.RoPE,
+                    attn=MultiHeadAttentionTypeEnums.MHA, dtype="float16")
+    w = synthetic_weights(cfg, 9, std=0.05)
+    prompt = np.random.default_rng(2).integers(1, cfg.V, size=(2, 200)).astype(np.int32)
+    opts = DecodingOptions(MaxTgtSentLength=204)
+    gpt = GPT(cfg, max_batch=2, max_tokens=206)
+    gpt.LoadWeights(w)
+
+    def run(p):
+        gpt.Reset()
+        gpt.Prefill(p, opts)
+        gpt.StepHost(np.full(len(p), 7, np.int32), opts)     # attends over every appended row
+        return gpt.Logits(want_probs=False)[0].copy()
+    both, each = run(prompt), np.concatenate([run(prompt[i:i + 1]) for i in range(2)])
+    assert np.abs(both - each).max() <= 8 * 2.0 ** -11 * np.abs(each).max()      # the linears' sums in another order, rounded to fp16 through one layer
