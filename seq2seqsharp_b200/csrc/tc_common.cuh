@@ -78,6 +78,88 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
+// ---- the same for a whole warp -------------------------------------------------------------------------------------------
+// One elected lane issues; the loop around it is the warp's.  In a branch of one lane every operand of these instructions, which live in
+// uniform registers, is moved there one by one, and rebuilding 64-bit descriptors for each product made a step of four products 630 cycles
+// of one thread's dependent instructions whatever their width (256 x 256: 512 of tensor time, 256 x 128: 256).  Descriptors are therefore a
+// constant upper word and a lower word that only ever has offsets added (the address field cannot carry: shared memory ends below 2^18).
+__device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr >> 4) & 0x3FFF) | ((lbo_bytes >> 4) << 16); }
+__device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
+#define TSB_ELECTED_MMA(NAME, GROUP)                                                                                                        \
+  __device__ __forceinline__ void NAME(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t idesc,       \
+                                       uint32_t accumulate) {                                                                               \
+    asm volatile(                                                                                                                           \
+        "{\n\t.reg .pred p, q;\n\t.reg .b64 da, db;\n\t"                                                                                    \
+        "elect.sync _|q, 0xffffffff;\n\t"                                                                                                  \
+        "setp.ne.b32 p, %6, 0;\n\t"                                                                                                        \
+        "mov.b64 da, {%1, %2};\n\tmov.b64 db, {%3, %4};\n\t"                                                                              \
+        "@q tcgen05.mma.cta_group::" GROUP ".kind::f16 [%0], da, db, %5, p;\n\t}" ::"r"(tmem_d),                                           \
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate)                                                             \
+        : "memory");                                                                                                                        \
+  }
+TSB_ELECTED_MMA(umma_el, "1")
+TSB_ELECTED_MMA(umma_pair_el, "2")
+#undef TSB_ELECTED_MMA
+__device__ __forceinline__ void umma_commit_el(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar)
+      : "memory");
+}
+// arrives at this barrier of both CTAs of a pair when the products issued so far are done
+__device__ __forceinline__ void umma_commit_pair_el(uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}" ::"r"(bar), "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void tc_mbar_expect_el(uint32_t bar, unsigned bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_el(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}" ::"r"(dst),
+      "l"(map), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tc_bulk_g2s_el(uint32_t dst, const void* src, unsigned bytes, uint32_t bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n\t}" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+      : "memory");
+}
+__device__ __forceinline__ bool tc_try_wait(uint32_t bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded; gives up early when another wait of the CTA has (*err), raises *err when it runs out itself
+__device__ __forceinline__ bool tc_wait_or(uint32_t bar, unsigned parity, volatile int* err) {
+  if (tc_try_wait(bar, parity)) return true;
+#pragma unroll 1
+  for (unsigned i = 1; i < kTcSpin; ++i) {
+    if (tc_try_wait(bar, parity)) return true;
+    if ((i & 63) == 63 && *err) return false;
+  }
+  *err = 1;
+  return false;
+}
+__device__ __forceinline__ bool tc_wait_short(uint32_t bar, unsigned parity) {   // after an error: bounded, raises nothing
+#pragma unroll 1
+  for (unsigned i = 0; i < kTcSpin; ++i)
+    if (tc_try_wait(bar, parity)) return true;
+  return false;
+}
+// what a warp's index is to the compiler: the same in all lanes
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
