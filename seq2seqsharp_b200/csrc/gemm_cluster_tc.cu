@@ -4,27 +4,33 @@
 // The WEIGHTS are the 128-row operand of tcgen05.mma (A, read in place from the packed tiles, MN-major, 128-byte swizzle), the activation
 // rows its N dimension (B: [16 / 32 / 64 rows][64 k], K-major, one TMA tensor copy per stage, rows beyond M zero-filled).  A CTA owns
 // 128 columns over a range of K; the 1, 2, 4 or 8 CTAs of a cluster share the columns.  When its products are done a CTA pushes every
-// sum into the shared memory of the CTA that finishes it (each finishes 1 / ks of the columns), one cluster barrier, and the sums
-// are added in rank order (bitwise reproducible): no scratch in global memory, no counters, no last arriver that reads the others' slots.
+// sum, four rows at a time, into the shared memory of the CTA that finishes it (each finishes 1 / ks of the columns); the stores report to
+// that CTA's mbarrier, and the sums are added in rank order (bitwise reproducible): no scratch in global memory, no counters, no last arriver
+// that reads the others' slots, and nobody waits for more than its own sums.
 //
 // What bounds a decode step's linears is the chain from one launch to the next, not their bytes: a CTA takes at most half of an SM's
 // shared memory, so that the next launch's CTAs are resident, have their barriers, TMEM and first weight tiles (at these sizes often
 // their whole share) before the current launch ends.  Only the activation tiles wait for it.
 // warp 0: copies; warp 1: TMEM and products; warps 2-5: accumulators out of TMEM; all warps: sums and epilogue.
+// Parts of a launch in clocks after the one before it has ended (8 rows of 768 -> 768, three steps of 64 k a CTA): first operands 1100, products
+// 700, push 270, the cluster's sums 350, epilogue 1000, leaving 400.  Before the products were issued by a whole warp, the sums pushed four
+// rows at a time with a barrier of their own and the epilogue's kinds had loops of their own: 1350, 1900, 650, 1400, 1450, 400.  Launches of
+// a captured step, before -> now (us): 8 rows of the 768-wide model 4.80 -> 3.58, 32 rows of the 2048-wide one 10.1 -> 8.4, one row of the
+// 4096-wide one 16.5 -> 14.7, 64 rows 23.2 -> 20.2.  Four CTAs' registers fit an SM (64 a thread): the kernels behind need room beside two of these.
 #include "cluster_sums.cuh"
 #include "stream_common.cuh"
 #include "tc_common.cuh"
 
 namespace tsb {
 
-constexpr int kLcThreads = 192;
+constexpr int kLcThreads = 256;
 constexpr int kLcMaxSections = 4;
 
 struct LcSection {
   int ct_end;   // first column tile (256 columns) after the section
   int N;
   int x_block;  // stacked row block it reads
-  int pieces;   // four columns at a time in the epilogue
+  int kind;     // ClKind: which loop finishes it
   Epilogue ep;
 };
 struct LcArgs {
@@ -33,7 +39,7 @@ struct LcArgs {
   int* error;
   int n_sec;
   LcSection sec[kLcMaxSections];
-  int rope_on;  // one section only
+  // one section only, of kind kClRope
   RopeFuse rope;
 };
 
@@ -55,20 +61,19 @@ __device__ __forceinline__ void lc_tmem_ld(uint32_t taddr, uint32_t* r) {
 }
 
 template <typename H, int NR>
-__global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __grid_constant__ CUtensorMap mapX, LcArgs a) {
+__global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __grid_constant__ CUtensorMap mapX, LcArgs a) {
   constexpr int kX = NR * 128, kStage = 16384 + kX;
   constexpr uint32_t kCols = NR < 32 ? 32 : NR;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int S = a.stages, ks = a.ks, M = a.M, KB = a.KB;
-  float* red = reinterpret_cast<float*>(smem + S * kStage);   // [source rank][items of this CTA][4 columns]
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * kStage + NR * 512);
-  uint64_t* empty = full + 8;
-  uint64_t* acc = empty + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc + 1);
+  float* red = reinterpret_cast<float*>(smem + S * kStage);   // [source rank][row quad][column of a group][group][4 rows]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * kStage + NR * 512);
+  const uint32_t full = s_u32(bars), empty = full + 64, acc = empty + 64, sums = acc + 8;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   __shared__ int s_err;
 
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31, w = warp_index();
   const int rank = (int)(blockIdx.x % ks), group = (int)(blockIdx.x / ks);
   int si = 0;
   while (si < a.n_sec - 1 && (group >> 1) >= a.sec[si].ct_end) ++si;
@@ -76,15 +81,18 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   const int N = a.sec[si].N, xrow = a.sec[si].x_block * M;
   const int col0 = (group - (si ? a.sec[si - 1].ct_end * 2 : 0)) * 128;   // of the section
   const int KP = (KB + 1) / 2, p0 = KP * rank / ks, n_it = KP * (rank + 1) / ks - p0;   // pairs of k tiles
+  const int quads = (M + 3) >> 2;
 
   if (tid == 0) {
     for (int i = 0; i < S; ++i) {
-      tc_mbar_init(&full[i], 1);
-      tc_mbar_init(&empty[i], 1);
+      tc_mbar_init(bars + i, 1);
+      tc_mbar_init(bars + 8 + i, 1);
     }
-    tc_mbar_init(acc, 1);
+    tc_mbar_init(bars + 16, 1);
+    tc_mbar_init(bars + 17, 1);
     s_err = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (ks > 1) tc_mbar_expect_tx(bars + 17, quads * 2048);   // 128 / ks columns from each of ks CTAs
   }
   if (w == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(kCols) : "memory");
@@ -95,122 +103,138 @@ __global__ void __launch_bounds__(kLcThreads) gemm_cluster_tc_kernel(const __gri
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
   pdl_trigger();
+  volatile int* err = &s_err;
+  const uint32_t ring = s_u32(smem);
   // weights do not depend on the previous kernel
-  const unsigned char* wsrc = a.Wp + ((size_t)(group >> 1) * KB) * kTileBytes + (size_t)(group & 1) * 8192;
-  auto weights = [&](int i) {
-    const int s = i % S, kb = (p0 + i) * 2;
-    const bool two = kb + 1 < KB;
-    tc_mbar_expect_tx(&full[s], (two ? 16384 : 8192) + kX);
-    tc_bulk_g2s(smem + s * kStage, wsrc + (size_t)kb * kTileBytes, 8192, &full[s]);
-    if (two) tc_bulk_g2s(smem + s * kStage + 8192, wsrc + (size_t)(kb + 1) * kTileBytes, 8192, &full[s]);
+  const unsigned char* wsrc = a.Wp + ((size_t)(group >> 1) * KB + (size_t)p0 * 2) * kTileBytes + (size_t)(group & 1) * 8192;
+  auto weights = [&](int i, int s) {
+    const bool two = (p0 + i) * 2 + 1 < KB;
+    const unsigned char* src = wsrc + (size_t)i * (2 * kTileBytes);
+    const uint32_t dst = ring + s * kStage, bar = full + s * 8;
+    tc_mbar_expect_el(bar, (two ? 16384 : 8192) + kX);
+    tc_bulk_g2s_el(dst, src, 8192, bar);
+    if (two) tc_bulk_g2s_el(dst + 8192, src + kTileBytes, 8192, bar);
   };
   const int n_pre = min(S, n_it);
-  if (tid == 0)
-    for (int i = 0; i < n_pre; ++i) weights(i);
-  __syncwarp();
-  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if (w == 0) {
+    if (elect_one()) asm volatile("prefetch.tensormap [%0];" ::"l"(&mapX) : "memory");
+    __syncwarp();
+    for (int i = 0; i < n_pre; ++i) weights(i, i);
+  }
+  if (ks > 1) cl_sync();   // the other CTAs' barriers exist before anything is pushed to them
   pdl_wait();
 
-  if (tid == 0) {
+  if (w == 0) {
     // ---------------- copies
-    int i = 0;
-    for (; i < n_it; ++i) {
-      const int s = i % S;
+    int s = 0;
+    unsigned phase = 1;   // parity of the ring's previous round
+    for (int i = 0; i < n_it; ++i) {
       if (i >= S) {
-        if (!tc_mbar_wait(&empty[s], (unsigned)((i / S - 1) & 1))) {
-          s_err = 1;
-          break;
-        }
-        weights(i);
+        if (!tc_wait_or(empty + s * 8, phase, err)) break;
+        weights(i, s);
       }
-      tma_load_2d(smem + s * kStage + 16384, &mapX, (p0 + i) * 64, xrow, &full[s]);   // rows behind the block's are columns nobody reads
+      tma_load_2d_el(ring + s * kStage + 16384, &mapX, (p0 + i) * 64, xrow, full + s * 8);   // rows behind the block's are columns nobody reads
+      if (++s == S) s = 0, phase ^= 1;
     }
-    if (s_err)   // copies in flight land first
-      for (int j = max(0, i - S); j < i; ++j) tc_mbar_wait(&full[j % S], (unsigned)((j / S) & 1));
-  } else if (tid == 32) {
+    if (*err)   // copies in flight land first: the last S that were asked for
+      for (int j = 0; j < n_pre; ++j) {
+        if (--s < 0) s = S - 1, phase ^= 1;
+        tc_wait_short(full + s * 8, phase ^ 1);
+      }
+  } else if (w == 1) {
     // ---------------- products.  Instruction descriptor: fp32 accumulator, A MN-major, B K-major, N = NR, M = 128
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (1u << 15) | ((uint32_t)(NR >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    // A: [k tile][64-column box 2][32 k][128 B]: boxes 4096 B apart (LBO), 8-k groups 1024 B apart (SBO); B: rows of 128 B, atoms of 8 rows
+    const uint32_t hi = desc_hi(1024), a0 = desc_lo(ring, 4096), b0 = desc_lo(ring + 16384, 16);
+    int s = 0;
+    unsigned phase = 0;
     for (int i = 0; i < n_it; ++i) {
-      const int s = i % S;
-      if (!tc_mbar_wait(&full[s], (unsigned)((i / S) & 1))) {
-        s_err = 1;
-        break;
-      }
+      if (!tc_wait_or(full + s * 8, phase, err)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t wb = s_u32(smem + s * kStage), xb = wb + 16384;
-      const int kk_end = (p0 + i) * 2 + 1 < KB ? 4 : 2;
-#pragma unroll
-      for (int kk = 0; kk < 4; ++kk) {
-        if (kk >= kk_end) break;
-        // A: [k tile][64-column box 2][32 k][128 B]: boxes 4096 B apart (LBO), 8-k groups 1024 B apart (SBO); B: rows of 128 B, atoms of 8 rows
-        umma_f16(tmem, make_desc(wb + (kk >> 1) * 8192 + (kk & 1) * 2048, 4096, 1024), make_desc(xb + kk * 32, 16, 1024), idesc, (i > 0 || kk > 0) ? 1u : 0u);
+      const uint32_t ad = a0 + s * (kStage >> 4), bd = b0 + s * (kStage >> 4);
+      umma_el(tmem, ad, hi, bd, hi, idesc, i > 0);
+      umma_el(tmem, ad + 128, hi, bd + 2, hi, idesc, 1);
+      if ((p0 + i) * 2 + 1 < KB) {
+        umma_el(tmem, ad + 512, hi, bd + 4, hi, idesc, 1);
+        umma_el(tmem, ad + 640, hi, bd + 6, hi, idesc, 1);
       }
-      umma_commit(&empty[s]);
+      umma_commit_el(empty + s * 8);
+      if (++s == S) s = 0, phase ^= 1;
     }
-    umma_commit(acc);
+    umma_commit_el(acc);
   }
   __syncwarp();
 
-  // This CTA finishes 128 / ks of the columns, in groups of four, of every row.  The CTA that finishes a column is the same for all rows, and a
-  // thread's groups, kLcThreads apart, have the same columns: no index arithmetic per row.  (Rows x columns shared out as one range cost a
-  // division per pushed sum; as straight-line code of 40 KB that was the launch's longest part, 0.15 us per row: 64 rows of 64 -> 64 19.5 us,
-  // now 10.7; of 4096 -> 22016 53.0, now 42.0.)  Bias and the first group's residual are on their way while the products run.
-  const int gsh = 5 - (31 - __clz(ks)), per = M << gsh;   // log2 of a row's groups here; groups of this CTA
-  const int c = col0 + ((rank << gsh) + (tid & ((1 << gsh) - 1))) * 4;
-  const bool pieces = a.sec[si].pieces != 0;
-  float bias[4], res[4];
-  cl_bias<H>(ep, N, c, bias);
-  if (tid < per) cl_residual(ep, N, tid >> gsh, c, pieces, res);
-  if (w >= 2) {
+  // This CTA finishes 128 / ks of the columns, in groups of four, of every row.  A warp takes eight groups of the four rows of a quad at a time
+  // (quad-major, so that its reads of a slot are 32 different banks); a thread's columns are the same in all of its quads: no index
+  // arithmetic per row.  Bias and the first quad's residual are on their way while the products run.
+  const int gsh = 5 - (31 - __clz(ks)), G = 1 << gsh;          // groups here
+  const int g = (tid >> 2) & (G - 1);
+  const int c = col0 + ((rank << gsh) + g) * 4, row0 = (tid >> (gsh + 2)) * 4 + (tid & 3), step = (kLcThreads >> (gsh + 2)) * 4;
+  ClAhead<H> ahead;
+  ahead.start(ep, a.sec[si].kind, N, c, row0, M, a.rope);
+  if (w >= 2 && w < 6) {
     // ---------------- sums out of TMEM: warp w reads lanes 32 (w % 4) .. = columns of the group
-    const bool ok = __all_sync(0xffffffffu, tc_mbar_wait(acc, 0));
-    if (!ok) s_err = 1;
+    tc_wait_or(acc, 0, err);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int col = (w & 3) * 32 + lane, owner = col >> (gsh + 2);
-    float* at = red + ((size_t)rank * per + ((col >> 2) & ((1 << gsh) - 1))) * 4 + (col & 3);   // [source rank][row][group][4]
-    const uint32_t local = s_u32(at), step = 16u << gsh;
-    uint32_t remote = local;
-    if (ks > 1) asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(owner));
+    const int col = (w & 3) * 32 + lane, owner = col >> (gsh + 2), e = col & 3, here = ((col >> 2) + 2 * e) & (G - 1);
+    const uint32_t local = s_u32(red) + ((uint32_t)rank * quads * (G * 4) + e * G + here) * 16, hop = G * 64;
+    uint32_t remote = local, bar = sums;
+    if (ks > 1) {
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local), "r"(owner));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(sums), "r"(owner));
+    }
 #pragma unroll
     for (int h = 0; h < (NR + 31) / 32; ++h) {
       uint32_t v[NR < 32 ? NR : 32];
       lc_tmem_ld<NR>(tmem + ((uint32_t)((w & 3) * 32) << 16) + h * 32, v);
 #pragma unroll
-      for (int r = 0; r < (NR < 32 ? NR : 32); ++r) {
-        const int row = h * 32 + r;
-        if (row < M) {
-          if (ks > 1) asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(remote + row * step), "r"(v[r]) : "memory");
-          else asm volatile("st.shared.b32 [%0], %1;" ::"r"(local + row * step), "r"(v[r]) : "memory");
+      for (int r = 0; r < (NR < 32 ? NR : 32); r += 4) {
+        const int qd = (h * 32 + r) >> 2;
+        if (qd < quads) {
+          if (ks > 1)
+            asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(remote + qd * hop), "r"(v[r]), "r"(v[r + 1]),
+                         "r"(v[r + 2]), "r"(v[r + 3]), "r"(bar)
+                         : "memory");
+          else
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(local + qd * hop), "r"(v[r]), "r"(v[r + 1]), "r"(v[r + 2]), "r"(v[r + 3]) : "memory");
         }
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.arrive 1, 160;" ::: "memory");   // TMEM has been read
   }
-  if (ks > 1) cl_sync();
-  else __syncthreads();
+  if (ks > 1) {
+    // arrived when everything is pushed (a CTA that gave up has pushed too); waited for before the CTA leaves, so that nobody pushes to one that has
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    tc_wait_or(sums, 0, err);
+  } else {
+    __syncthreads();
+  }
 
-  // ---------------- epilogue
-#pragma unroll 1
-  for (int i = tid; i < per; i += kLcThreads) {
-    float next[4];
-    if (i + kLcThreads < per) cl_residual(ep, N, (i + kLcThreads) >> gsh, c, pieces, next);
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int r = 0; r < ks; ++r) {
-      const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + i) * 4);
-      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+  // ---------------- epilogue: rank order; a group's column e lies 2 e groups further on, so that neither the pushes nor these reads meet in a bank
+  const float* from = red + ((size_t)(row0 >> 2) * (G * 4)) * 4 + (row0 & 3);
+  const int at0 = g * 4, at1 = (G + ((g + 2) & (G - 1))) * 4, at2 = (2 * G + ((g + 4) & (G - 1))) * 4, at3 = (3 * G + ((g + 6) & (G - 1))) * 4;
+  const int hop = quads * (G * 16), skip = (step >> 2) * (G * 16);
+  auto sum4 = [&](const float* f, float* v) {
+    v[0] = f[at0]; v[1] = f[at1]; v[2] = f[at2]; v[3] = f[at3];
+    for (int r = 1; r < ks; ++r) {
+      f += hop;
+      v[0] += f[at0]; v[1] += f[at1]; v[2] += f[at2]; v[3] += f[at3];
     }
-    cl_finish4<H>(ep, N, i >> gsh, c, pieces, v, bias, res, a.rope_on, a.rope);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) res[e] = next[e];
+  };
+  cl_finish_rows<H>(ep, a.sec[si].kind, N, c, row0, M, step, from, skip, ahead, a.rope, sum4);
+  if (ks > 1) {
+    if (*err) tc_wait_short(sums, 0);   // what is on its way here lands first
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  __syncthreads();
   if (w == 1) {
-    if (lane == 0 && s_err) tc_mbar_wait(acc, 0);   // some warp gave up: products in flight end before TMEM is given back
-    __syncwarp();
+    if (*err) tc_wait_short(acc, 0);   // some warp gave up: products in flight end before TMEM is given back
+    asm volatile("bar.sync 1, 160;" ::: "memory");
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }
-  if (tid == 0 && s_err && a.error) *a.error = 1;
+  if (*err && lane == 0 && a.error) *a.error = 1;   // the warp that gave up, at least, sees it
 }
 
 template <typename H, int NR>
@@ -284,10 +308,9 @@ int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x
   LcArgs a{};
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
   a.M = M; a.n_sec = 1;
-  a.sec[0].ct_end = (N + 255) / 256; a.sec[0].N = N; a.sec[0].ep = ep; a.sec[0].pieces = cl_whole_pieces(ep, N, 2);
+  a.sec[0].ct_end = (N + 255) / 256; a.sec[0].N = N; a.sec[0].ep = ep; a.sec[0].kind = rope ? kClRope : cl_kind(ep, N, 2);
   if (rope) {
     if (!cl_rope_fits(*rope, ep, N, 2)) return 2;
-    a.rope_on = 1;
     a.rope = *rope;
   }
   return lc_run(device, st, dtype, x, M, K, a, (N + 127) / 128, pdl, s);
@@ -304,7 +327,7 @@ int launch_gemm_cluster_sections(int device, DeviceState* st, int dtype, const v
   for (int i = 0; i < n_sec; ++i) {
     ct += (sec[i].N + 255) / 256;
     a.sec[i].ct_end = ct; a.sec[i].N = sec[i].N; a.sec[i].ep = sec[i].ep; a.sec[i].x_block = sec[i].x_block;
-    a.sec[i].pieces = cl_whole_pieces(sec[i].ep, sec[i].N, 2);
+    a.sec[i].kind = cl_kind(sec[i].ep, sec[i].N, 2);
     if (sec[i].x_block + 1 > blocks) blocks = sec[i].x_block + 1;
   }
   const int last = sec[n_sec - 1].N;   // an odd half of the last column tile is left out

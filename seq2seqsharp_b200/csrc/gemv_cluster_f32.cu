@@ -4,7 +4,7 @@
 // ring of bulk copies, eight warps take four k of a tile each (a lane four columns of every row), the warps' sums meet in shared memory, the
 // cluster's through distributed shared memory in rank order.  Two CTAs fit an SM while the rows over a CTA's K range take up to 28 KB; the
 // weights are asked for before the launch in front has ended.  What bounds a small model's step is the chain of its launches (512-wide, six layers, one sequence, a
-// 128-token request: 42.7 ms with the persistent stream-K kernel, 24.7 with this one).
+// 128-token request: 42.7 ms with the persistent stream-K kernel, 22.9 with this one).
 #include "cluster_sums.cuh"
 #include "stream_common.cuh"
 
@@ -18,8 +18,7 @@ struct FcArgs {
   int M, N, K, KB, ks;
   int* error;
   Epilogue ep;
-  int pieces;  // four columns at a time in the epilogue
-  int rope_on;
+  int kind;    // ClKind
   RopeFuse rope;
 };
 // dynamic shared memory: ring | sums of the cluster [M * 32 groups][4] | rows of x over the CTA's range
@@ -28,7 +27,7 @@ static size_t fc_smem(int RM, int tiles) { return (size_t)kFcStages * kTileBytes
 template <int RM>
 __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) {
   extern __shared__ __align__(1024) unsigned char fc_raw[];
-  __shared__ uint64_t full[kFcStages], empty[kFcStages];
+  __shared__ uint64_t full[kFcStages], empty[kFcStages], sums;
   __shared__ int s_err;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int ks = a.ks, M = a.M, rank = (int)(blockIdx.x % ks), group = (int)(blockIdx.x / ks);
@@ -40,8 +39,10 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       mbar_init(&full[i], 1);
       mbar_init(&empty[i], 8);
     }
+    mbar_init(&sums, 1);
     s_err = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (ks > 1) mbar_expect_tx(&sums, M * 512);   // four columns of M * 32 / ks groups from each of ks CTAs
   }
   __syncthreads();
   pdl_trigger();
@@ -55,9 +56,9 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   __syncwarp();
   if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
-  float bias[4], res[4];
+  ClAhead<float> ahead;
   const int per = M * 32 / ks;   // groups of four columns this CTA finishes: at most 256, one per thread
-  const int c = group * 128 + ((rank * per + tid) & 31) * 4;
+  const int c = group * 128 + ((rank * per + tid) & 31) * 4, row = (rank * per + tid) >> 5;
   if (w == 8) {
     if (lane == 0) {
       for (int i = n_pre; i < n_it; ++i) {
@@ -73,10 +74,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     }
     __syncwarp();
   } else {
-    if (tid < per) {
-      cl_bias<float>(a.ep, a.N, c, bias);
-      cl_residual(a.ep, a.N, (rank * per + tid) >> 5, c, a.pieces != 0, res);
-    }
+    if (tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
     const int kc = n_it * 32;
     for (int i = tid; i < RM * kc; i += 256) {
       const int m = i / kc, k = t0 * 32 + i % kc;
@@ -123,27 +121,37 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       const int owner = i / per;
       float* at = red + (size_t)(rank * per + i - owner * per) * 4;
       if (ks > 1) {
-        cl_push(at, (uint32_t)owner, v.x);
-        cl_push(at + 1, (uint32_t)owner, v.y);
-        cl_push(at + 2, (uint32_t)owner, v.z);
-        cl_push(at + 3, (uint32_t)owner, v.w);
+        cl_push4(at, &sums, (uint32_t)owner, v);
       } else {
         *reinterpret_cast<float4*>(at) = v;
       }
     }
     __syncwarp();
   }
-  if (ks > 1) cl_sync();
-  else __syncthreads();
-  if (tid < per) {
-    float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int r = 0; r < ks; ++r) {
-      const float4 t = *reinterpret_cast<const float4*>(red + (size_t)(r * per + tid) * 4);
-      v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
-    }
-    cl_finish4<float>(a.ep, a.N, (rank * per + tid) >> 5, c, a.pieces != 0, v, bias, res, a.rope_on, a.rope);
+  if (ks > 1) {
+    // arrived when everything is pushed; waited for before the CTA leaves, so that nobody pushes to one that has
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (tid < per && !cl_wait(&sums)) s_err = 1;
+  } else {
+    __syncthreads();
   }
-  if (tid == 0 && s_err && a.error) *a.error = 1;
+  if (tid < per) {
+    const int hop = per * 4;
+    cl_finish_rows<float>(a.ep, a.kind, a.N, c, row, row + 1, 1, red + tid * 4, 0, ahead, a.rope, [&](const float* f, float* v) {
+      v[0] = v[1] = v[2] = v[3] = 0.0f;
+      for (int r = 0; r < ks; ++r, f += hop) {
+        const float4 t = *reinterpret_cast<const float4*>(f);
+        v[0] += t.x; v[1] += t.y; v[2] += t.z; v[3] += t.w;
+      }
+    });
+  }
+  __syncwarp();
+  if (ks > 1) {
+    if (*(volatile int*)&s_err) cl_wait(&sums);   // what is on its way here lands first
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  }
+  if (lane == 0 && *(volatile int*)&s_err && a.error) *a.error = 1;   // the warp that gave up, at least, sees it
 }
 
 template <int RM>
@@ -178,10 +186,9 @@ int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const v
   if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
   FcArgs a{};
   a.x = x; a.Wp = reinterpret_cast<const unsigned char*>(Wp);
-  a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.pieces = cl_whole_pieces(ep, N, 4);
+  a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.kind = rope ? kClRope : cl_kind(ep, N, 4);
   if (rope) {
     if (!cl_rope_fits(*rope, ep, N, 4)) return 2;
-    a.rope_on = 1;
     a.rope = *rope;
   }
   const int groups = (N + 127) / 128, RM = M <= 1 ? 1 : (M <= 2 ? 2 : (M <= 4 ? 4 : 8));

@@ -83,6 +83,11 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
 // uniform registers, is moved there one by one, and rebuilding 64-bit descriptors for each product made a step of four products 630 cycles
 // of one thread's dependent instructions whatever their width (256 x 256: 512 of tensor time, 256 x 128: 256).  Descriptors are therefore a
 // constant upper word and a lower word that only ever has offsets added (the address field cannot carry: shared memory ends below 2^18).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t e;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(e));
+  return e != 0;
+}
 __device__ __forceinline__ uint32_t desc_lo(uint32_t smem_addr, uint32_t lbo_bytes) { return ((smem_addr >> 4) & 0x3FFF) | ((lbo_bytes >> 4) << 16); }
 __device__ __forceinline__ uint32_t desc_hi(uint32_t sbo_bytes) { return (sbo_bytes >> 4) | (1u << 14) | (2u << 29); }
 #define TSB_ELECTED_MMA(NAME, GROUP)                                                                                                        \

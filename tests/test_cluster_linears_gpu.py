@@ -71,3 +71,9 @@ def test_fp32_rows(cuda, M, K, n):
 def test_weights_off_a_16_byte_boundary(cuda, dtype, M):
     """No kernel that copies whole pieces may take them."""
     check(M, 64, 130, dtype, ((1, 0),))
+
+
+# sums travel four rows at a time: quads with one to four rows that exist, groups of four columns that share a bank, eight ranks and one
+@pytest.mark.parametrize("M,K,n", [(1, 8, 4), (1, 4096, 512), (2, 2048, 132), (3, 520, 2052), (4, 264, 1024), (7, 1024, 40000), (9, 4096, 128), (61, 136, 256)])
+def test_row_quads(cuda, M, K, n):
+    check(M, K, n, torch.float16, (0, 1))
