@@ -45,8 +45,10 @@ template <typename T>
 __global__ void embed_kernel(float* x, const T* E, const T* PE, const int* ids,
                              int rows, int S, int d, int V, float sf, int pe_mode, int pe_rows, int T0_arg,
                              const int* dT0, const int2* where) {
-  pdl_trigger();
+  // In this order: nothing of the step starts before everything in front of it has ended, so that its kernels may read the step state and
+  // cached rows of earlier steps before their own pdl_wait().
   pdl_wait();
+  pdl_trigger();
   for (int r = blockIdx.x; r < rows; r += gridDim.x) {
     int id = ids[r];
     TSB_DEV_CHECK(engine, id >= 0 && id < V, 0x101, (void)0)          // token id outside the vocabulary (the row is embedded as id 0)

@@ -130,6 +130,11 @@ __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
 // the K row and the V row, so every load is a 128-bit coalesced read and K/V are read exactly once for all G
 // heads.  Each lane group runs an online softmax over its own token subsequence; the partial (max, sum, acc)
 // states are merged through shared memory, and across splits by attn_combine_kernel.
+// Decode attention reads the step state and the rows of earlier steps BEFORE pdl_wait(): all kernels of a step start after everything that
+// ran before the step's first kernel has ended (embed_kernel waits before it lets its successors start), and rows below T0 and the state
+// are not written during the step before its last kernel.  Only the row at T0, appended by the launch in front, and the queries wait.
+// Launches of a captured step, us: 8 sequences of 160 tokens, 12 heads of 64 4.7 -> 3.1; one of 530, 32 / 8 heads of 128 6.8 -> 4.9; 32 of 1040,
+// 32 / 8 of 64 15.7 -> 14.3; 64 of 520 of 128 27.8 -> 25.3; fp32, one of 100, 8 heads 5.1 -> 4.0.
 // Scores: (q . k) * (1/sqrt(hd)) in fp32; softmax in fp32; P.V accumulated in fp32
 // (the reference promotes Q and K to fp32 for the scores as well: MultiHeadAttention.cs:203-221).
 template <typename T> struct Vec16;
@@ -227,8 +232,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
   extern __shared__ float sm[];  // [nstates][G][hd + 2]
   float* box = BOX ? sm + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
-  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
-  pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z / S, T0_arg);
   const int lpt = hd / EPL;              // lanes per token (power of two, <= 32)
   const int tpw = 32 / lpt;              // tokens per warp iteration
@@ -244,6 +247,24 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
   const int Tk = min(T0 + s + 1, Tmax);  // causal: keys 0 .. T0+s
   const int per_split = (Tk + splits - 1) / splits;
   const int t_beg = split * per_split, t_end = min(Tk, t_beg + per_split);
+  const T* Kb = cK + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
+  const T* Vb = cV + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
+  const int stride = nwarps * tpw, tb0 = t_beg + w * tpw;
+  // kAhead tokens of a lane group are on their way at any time, the first of them before the kernel in front has ended (tokens below T0)
+  constexpr int kAhead = 4;
+  Vec16<T> kv[kAhead], vv[kAhead];
+  auto fetch = [&](int u, int t) {
+    kv[u].load(Kb + (int64_t)t * hd);
+    vv[u].load(Vb + (int64_t)t * hd);
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (const int t = tb0 + u * stride + sub; t < min(t_end, T0)) fetch(u, t);
+  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
+  pdl_wait();
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u)
+    if (const int t = tb0 + u * stride + sub; t >= T0 && t < t_end) fetch(u, t);
 
   float qf[G][EPL];
 #pragma unroll
@@ -262,38 +283,37 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.0f;
   }
-  const T* Kb = cK + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
-  const T* Vb = cV + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
-  const int stride = nwarps * tpw;
-  for (int tb = t_beg + w * tpw; tb < t_end; tb += stride) {
-    // all lanes of the warp iterate together (shuffles below need full participation); `live` masks the tail
-    const int t = tb + sub;
-    const bool live = t < t_end;
-    float kf[EPL], vf[EPL];
-    if (live) {
-      Vec16<T> kv, vv;
-      kv.load(Kb + (int64_t)t * hd);
-      vv.load(Vb + (int64_t)t * hd);
-      kv.get(kf);
-      vv.get(vf);
-    } else {
+  for (int tb = tb0; tb < t_end; tb += kAhead * stride) {
 #pragma unroll
-      for (int e = 0; e < EPL; ++e) kf[e] = vf[e] = 0.0f;
-    }
-#pragma unroll
-    for (int g = 0; g < G; ++g) {
-      float d = 0.0f;
-#pragma unroll
-      for (int e = 0; e < EPL; ++e) d += qf[g][e] * kf[e];
-      for (int o = lpt >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+    for (int u = 0; u < kAhead; ++u) {
+      // all lanes of the warp iterate together (shuffles below need full participation); `live` masks the tail
+      const int t = tb + u * stride + sub;
+      if (tb + u * stride >= t_end) break;
+      const bool live = t < t_end;
+      float kf[EPL], vf[EPL];
       if (live) {
-        const float mn = fmaxf(m[g], d);
-        const float corr = __expf(m[g] - mn);  // exp(-inf) = 0 on the first token
-        const float p = __expf(d - mn);
-        l[g] = l[g] * corr + p;
+        kv[u].get(kf);
+        vv[u].get(vf);
+      } else {
 #pragma unroll
-        for (int e = 0; e < EPL; ++e) acc[g][e] = acc[g][e] * corr + p * vf[e];
-        m[g] = mn;
+        for (int e = 0; e < EPL; ++e) kf[e] = vf[e] = 0.0f;
+      }
+      if (t + kAhead * stride < t_end) fetch(u, t + kAhead * stride);
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float d = 0.0f;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) d += qf[g][e] * kf[e];
+        for (int o = lpt >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (live) {
+          const float mn = fmaxf(m[g], d);
+          const float corr = __expf(m[g] - mn);  // exp(-inf) = 0 on the first token
+          const float p = __expf(d - mn);
+          l[g] = l[g] * corr + p;
+#pragma unroll
+          for (int e = 0; e < EPL; ++e) acc[g][e] = acc[g][e] * corr + p * vf[e];
+          m[g] = mn;
+        }
       }
     }
   }
@@ -504,8 +524,6 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
   extern __shared__ __align__(128) unsigned char attn_smem[];
   float* box = BOX ? reinterpret_cast<float*>(attn_smem) + box_at : nullptr;   // splits as a cluster
   pdl_trigger();
-  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
-  pdl_wait();
   const int T0 = state_len(dT0, (int)blockIdx.z, T0_arg);
   TSB_DEV_CHECK(attention, T0 >= 0 && T0 < Tmax, 0x202, (void)0)   // cache length beyond the capacity (keys are clamped to Tmax below)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -535,7 +553,12 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
     }
     cp_async_commit();
   };
-  for (int i = 0; i < kMmaStages - 1; ++i) issue(i);
+  // stages of tokens below T0 only are asked for before the kernel in front has ended
+  int asked = 0;
+  while (asked < kMmaStages - 1 && t_beg + (asked + 1) * kMmaStageTokens <= min(t_end, T0)) issue(asked++);
+  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
+  pdl_wait();
+  for (; asked < kMmaStages - 1; ++asked) issue(asked);
 
   // Q fragments: row g8 = head h0 + g8 (zero rows beyond the group), a0 = k 2*t4.., a2 = k 8 + 2*t4..
   uint32_t qa[KS][2];
