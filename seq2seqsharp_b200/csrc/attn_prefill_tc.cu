@@ -204,6 +204,8 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  pdl_trigger();   // after the allocation: a successor's CTA on this SM cannot take the columns first
+  pdl_wait();      // (a.starts was there before the pass began)
   volatile int* err = &s_err;
 
   if (w >= 8) {
@@ -442,7 +444,7 @@ static int pa_launch(int device, const CUtensorMap& q, const CUtensorMap& k, con
   a.wait_limit = tc_wait_limit();
   const int64_t grid = (int64_t)a.tiles * a.heads * a.B;
   TSB_CHECK(grid <= 0x7fffffff, "prompt attention: %lld blocks", (long long)grid);
-  attn_prefill_tc_kernel<H, QB, VB, NKS, NVS><<<(int)grid, kPaThreads, smem, s>>>(q, k, r, v, a);
+  TSB_CUDA(launch_k(attn_prefill_tc_kernel<H, QB, VB, NKS, NVS>, dim3((unsigned)grid), dim3(kPaThreads), smem, s, q, k, r, v, a));
   count_launch(device);
   return check_launch("attn_prefill_tc");
 }

@@ -955,7 +955,8 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
     return enqueue_layered(g, B, S, T0, use_state, use_state ? splits : T0 + S);
   }
   NvtxRange nvtx_(S == 1 ? "tsb200.forward.step" : "tsb200.forward.prompt");
-  PdlScope pdl_scope(g->pdl && S == 1);
+  // prompts too: a launch's barriers, TMEM and descriptors are ready when the one in front ends
+  PdlScope pdl_scope(g->pdl && (S == 1 || g->tp == 1));
   const TSB200GptConfig& c = g->c;
   const int dev = c.device, dt = c.dtype, d = c.d;
   const PackedRows* pack = g->pack.rows > 0 ? &g->pack : nullptr;

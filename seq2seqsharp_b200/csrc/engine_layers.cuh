@@ -723,7 +723,7 @@ static int sandwich_layers(Gpt* g, LayerPass& ps) {
 static int enqueue_layered(Gpt* g, int B, int S, int T0, bool use_state, int T_plan) {
   NvtxRange nvtx_(S == 1 ? "tsb200.forward.step" : "tsb200.forward.prompt");
   // sandwich blocks, ms per step with / without chained launches: 8 sequences 1.07 / 1.10 (4k), 16: 1.29 / 1.30, 32: 1.06 / 1.03 (2k), 64: 1.56 / 1.43
-  PdlScope pdl_scope(g->pdl && S == 1 && (B <= 16 || g->ly->c.block != TSB200_BLOCK_SANDWICH));
+  PdlScope pdl_scope(g->pdl && (S > 1 || B <= 16 || g->ly->c.block != TSB200_BLOCK_SANDWICH));
   Layered* ly = g->ly;
   const int dev = g->c.device, dt = g->c.dtype, d = ly->c.d, rows = B * S;
   const int* dT = use_state ? g->state : nullptr;

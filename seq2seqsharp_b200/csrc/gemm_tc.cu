@@ -278,6 +278,8 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_acc = *tmem_slot;
+  pdl_trigger();   // after the allocation: a successor's CTA on this SM cannot take the columns first
+  pdl_wait();
 
   volatile int* err = &s_err;
   if (w == 0) {
@@ -957,7 +959,7 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
   const bool deep = (int64_t)grid.x * grid.y * grid.z <= st->sm_count;
   auto k = dtype == TSB200_BF16 ? (deep ? gemm_tc_kernel<__nv_bfloat16, kTcDeepStages> : gemm_tc_kernel<__nv_bfloat16, kTcStages>)
                                 : (deep ? gemm_tc_kernel<__half, kTcDeepStages> : gemm_tc_kernel<__half, kTcStages>);
-  k<<<grid, kTcThreads, tc_smem(deep ? kTcDeepStages : kTcStages), s>>>(mapA, a);
+  TSB_CUDA(launch_k(k, grid, dim3(kTcThreads), tc_smem(deep ? kTcDeepStages : kTcStages), s, mapA, a));
   count_launch(device);
   return check_launch("gemm_tc");
 }
