@@ -163,6 +163,7 @@ struct ClAhead {
       }
     }
   }
+  // before the wait: weights, and the step state, which was there before the step's first kernel ran (embed_kernel)
   __device__ __forceinline__ void start(const Epilogue& ep, int kind, int N, int c, int row0, int M, const RopeFuse& rf) {
     cl_bias<H>(ep, N, c, bias);
     if (kind == kClRope) {
@@ -171,7 +172,11 @@ struct ClAhead {
       head = cc / rf.hd;
       e0 = cc - head * rf.hd;
     }
-    if (row0 < M) row(ep, kind, N, c, row0, rf);
+    if (kind == kClRope && row0 < M) row(ep, kind, N, c, row0, rf);
+  }
+  // what the launch in front may have written
+  __device__ __forceinline__ void first(const Epilogue& ep, int kind, int N, int c, int row0, int M, const RopeFuse& rf) {
+    if (kind != kClRope && row0 < M) row(ep, kind, N, c, row0, rf);
   }
 };
 template <typename H, int ACT, typename Sum>

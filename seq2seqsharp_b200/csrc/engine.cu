@@ -780,6 +780,16 @@ static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid
       return r;
     }
   }
+  const RowNorm rn{ng, c.norm_type == 0 ? nb : nullptr, c.norm_type, c.eps};
+  if (ng && dt == TSB200_F32 && rows <= 8 && g->fuse_step) {
+    prof_begin(g, KC_LINEAR);
+    const int r = launch_gemv_cluster_f32(dev, g->st, x_resid, Wp, rows, K, N, ep, g->pdl, g->s, nullptr, &rn);
+    if (r != 2) {
+      g->lin_syms_used = true;
+      if (r == 1) prof_end(g, KC_LINEAR);
+      return r == 1;
+    }
+  }
   if (ng) {
     PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, h_tmp, const_cast<float*>(x_resid), nullptr, ng, c.norm_type == 0 ? nb : nullptr,
                                        c.norm_type, c.eps, rows, K, g->s));
@@ -1019,12 +1029,21 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
       RopeFuse rf{};
       rf.cK = L.cK; rf.cV = L.cV; rf.Hd = Hd; rf.KVd = KVd; rf.hd = c.hd; rf.Tmax = c.max_tokens;
       rf.use_rope = c.pe_type == 2 ? 1 : 0; rf.T0 = T0; rf.state = dT; rf.tab = g->rope_tab;
-      PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, g->h, g->x, nullptr, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, rows, d, g->s));
-      prof_begin(g, KC_LINEAR);
       const Epilogue ep = make_ep(L.bqkv, nullptr, g->qkv, nullptr, TSB200_ACT_NONE, 0);
-      const int r = dt == TSB200_F16 ? launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf)
-                                     : launch_gemv_cluster_f32(dev, g->st, (const float*)g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
-      if (r == 0) return 0;
+      const RowNorm rn{L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps};
+      int r = 2;
+      if (dt == TSB200_F32) {   // the norm inside the linear where it takes it
+        prof_begin(g, KC_LINEAR);
+        r = launch_gemv_cluster_f32(dev, g->st, g->x, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf, &rn);
+        if (r == 0) return 0;
+      }
+      if (r == 2) {
+        PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, g->h, g->x, nullptr, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, rows, d, g->s));
+        prof_begin(g, KC_LINEAR);
+        r = dt == TSB200_F16 ? launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf)
+                                       : launch_gemv_cluster_f32(dev, g->st, (const float*)g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
+        if (r == 0) return 0;
+      }
       g->lin_syms_used = true;
       if (r == 2) {
         TSB_TRY(launch_linear(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->lin_ws, g->lin_ws_bytes, g->s, true));

@@ -121,6 +121,14 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     __syncwarp();
     for (int i = 0; i < n_pre; ++i) weights(i, i);
   }
+  // This CTA finishes 128 / ks of the columns, in groups of four, of every row.  A warp takes eight groups of the four rows of a quad at a time
+  // (quad-major, so that its reads of a slot are 32 different banks); a thread's columns are the same in all of its quads: no index
+  // arithmetic per row.  Bias, position and rotation are asked for before the wait, the first row's residual while the products run.
+  const int gsh = 5 - (31 - __clz(ks)), G = 1 << gsh;          // groups here
+  const int g = (tid >> 2) & (G - 1);
+  const int c = col0 + ((rank << gsh) + g) * 4, row0 = (tid >> (gsh + 2)) * 4 + (tid & 3), step = (kLcThreads >> (gsh + 2)) * 4;
+  ClAhead<H> ahead;
+  ahead.start(ep, a.sec[si].kind, N, c, row0, M, a.rope);
   if (ks > 1) cl_sync();   // the other CTAs' barriers exist before anything is pushed to them
   pdl_wait();
 
@@ -165,14 +173,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   }
   __syncwarp();
 
-  // This CTA finishes 128 / ks of the columns, in groups of four, of every row.  A warp takes eight groups of the four rows of a quad at a time
-  // (quad-major, so that its reads of a slot are 32 different banks); a thread's columns are the same in all of its quads: no index
-  // arithmetic per row.  Bias and the first quad's residual are on their way while the products run.
-  const int gsh = 5 - (31 - __clz(ks)), G = 1 << gsh;          // groups here
-  const int g = (tid >> 2) & (G - 1);
-  const int c = col0 + ((rank << gsh) + g) * 4, row0 = (tid >> (gsh + 2)) * 4 + (tid & 3), step = (kLcThreads >> (gsh + 2)) * 4;
-  ClAhead<H> ahead;
-  ahead.start(ep, a.sec[si].kind, N, c, row0, M, a.rope);
+  ahead.first(ep, a.sec[si].kind, N, c, row0, M, a.rope);
   if (w >= 2 && w < 6) {
     // ---------------- sums out of TMEM: warp w reads lanes 32 (w % 4) .. = columns of the group
     tc_wait_or(acc, 0, err);

@@ -4,13 +4,16 @@
 // ring of bulk copies, eight warps take four k of a tile each (a lane four columns of every row), the warps' sums meet in shared memory, the
 // cluster's through distributed shared memory in rank order.  Two CTAs fit an SM while the rows over a CTA's K range take up to 28 KB; the
 // weights are asked for before the launch in front has ended.  What bounds a small model's step is the chain of its launches (512-wide, six layers, one sequence, a
-// 128-token request: 42.7 ms with the persistent stream-K kernel, 22.9 with this one).
+// 128-token request: 42.7 ms with the persistent stream-K kernel, 19.6 with this one).
 #include "cluster_sums.cuh"
 #include "stream_common.cuh"
 
 namespace tsb {
 
 constexpr int kFcThreads = 288, kFcStages = 5;
+// Rows of up to 1024 are normed here instead of by a launch in front, which takes 2.1 us of a step's chain of launches; reading the whole rows
+// and their two sums costs this launch about 0.9 us (512 wide, one row: a 128-token request 22.4 -> 20.4 ms).  Longer rows would be read by every CTA for more than that.
+constexpr int kFcNormRegs = 8;   // float4 of a row per lane
 
 struct FcArgs {
   const float* x;
@@ -19,6 +22,10 @@ struct FcArgs {
   int* error;
   Epilogue ep;
   int kind;    // ClKind
+  int norm;    // 0: rows as they are, 1: RMSNorm, 2: LayerNorm of them (gamma, beta, eps) first
+  const float* gamma;
+  const float* beta;
+  float eps;
   RopeFuse rope;
 };
 // dynamic shared memory: ring | sums of the cluster [M * 32 groups][4] | rows of x over the CTA's range
@@ -28,6 +35,7 @@ template <int RM>
 __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) {
   extern __shared__ __align__(1024) unsigned char fc_raw[];
   __shared__ uint64_t full[kFcStages], empty[kFcStages], sums;
+  __shared__ float2 stat[8];   // mean and divisor of a row
   __shared__ int s_err;
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int ks = a.ks, M = a.M, rank = (int)(blockIdx.x % ks), group = (int)(blockIdx.x / ks);
@@ -54,11 +62,20 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       bulk_g2s(fc_raw + i * kTileBytes, src + (size_t)i * kTileBytes, kTileBytes, &full[i]);
     }
   __syncwarp();
-  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
-  pdl_wait();
+  float g0 = 0.0f, b0 = 0.0f;   // gain and shift of the first element this thread norms
+  if (a.norm) {
+    const int k = t0 * 32 + tid % (n_it * 32);
+    if (k < a.K) {
+      g0 = a.gamma[k];
+      if (a.beta) b0 = a.beta[k];
+    }
+  }
   ClAhead<float> ahead;
   const int per = M * 32 / ks;   // groups of four columns this CTA finishes: at most 256, one per thread
   const int c = group * 128 + ((rank * per + tid) & 31) * 4, row = (rank * per + tid) >> 5;
+  if (tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
+  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
+  pdl_wait();
   if (w == 8) {
     if (lane == 0) {
       for (int i = n_pre; i < n_it; ++i) {
@@ -74,11 +91,44 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     }
     __syncwarp();
   } else {
-    if (tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
+    if (tid < per) ahead.first(a.ep, a.kind, a.N, c, row, M, a.rope);
     const int kc = n_it * 32;
+    if (a.norm) {
+      // A warp takes the statistics of a row (one row: every warp, so that nobody waits), the arithmetic of the norm kernels
+      if (RM == 1 || w < M) {
+        const float4* xr = reinterpret_cast<const float4*>(a.x + (size_t)(RM == 1 ? 0 : w) * a.K);
+        const int n4 = a.K >> 2;
+        float4 v[kFcNormRegs];
+        float s = 0.0f, mean = 0.0f;
+#pragma unroll
+        for (int j = 0; j < kFcNormRegs; ++j) v[j] = lane + j * 32 < n4 ? xr[lane + j * 32] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int j = 0; j < kFcNormRegs; ++j)
+          s += a.norm == 2 ? (v[j].x + v[j].y) + (v[j].z + v[j].w) : (v[j].x * v[j].x + v[j].y * v[j].y) + (v[j].z * v[j].z + v[j].w * v[j].w);
+        s = warp_sum(s);
+        if (a.norm == 2) {
+          mean = s / a.K;
+          s = 0.0f;
+#pragma unroll
+          for (int j = 0; j < kFcNormRegs; ++j) {
+            const float p = v[j].x - mean, q = v[j].y - mean, r = v[j].z - mean, t = v[j].w - mean;
+            if (lane + j * 32 < n4) s += (p * p + q * q) + (r * r + t * t);
+          }
+          s = warp_sum(s);
+        }
+        stat[RM == 1 ? 0 : w] = make_float2(mean, sqrtf(s / (float)a.K + a.eps));   // every warp of one row writes the same
+      }
+      if (RM == 1) __syncwarp();
+      else asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
     for (int i = tid; i < RM * kc; i += 256) {
       const int m = i / kc, k = t0 * 32 + i % kc;
-      xs[i] = m < M && k < a.K ? a.x[(size_t)m * a.K + k] : 0.0f;
+      float v = m < M && k < a.K ? a.x[(size_t)m * a.K + k] : 0.0f;
+      if (a.norm && m < M && k < a.K) {
+        v = (i == tid ? g0 : a.gamma[k]) * ((v - stat[m].x) / stat[m].y);
+        if (a.beta) v += i == tid ? b0 : a.beta[k];
+      }
+      xs[i] = v;
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
     float4 acc[RM];
@@ -182,9 +232,14 @@ static int fc_launch(int device, const FcArgs& a, int groups, size_t smem, bool 
 
 // 1 ok, 0 error, 2 shape not handled (the caller takes another kernel)
 int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
-                            const RopeFuse* rope) {
+                            const RopeFuse* rope, const RowNorm* norm) {
   if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
+  if (norm && (K % 4 != 0 || K > kFcNormRegs * 128 || ((uintptr_t)x % 16) != 0)) return 2;
   FcArgs a{};
+  if (norm) {
+    a.norm = norm->type == 0 ? 2 : 1;
+    a.gamma = reinterpret_cast<const float*>(norm->gamma); a.beta = reinterpret_cast<const float*>(norm->beta); a.eps = norm->eps;
+  }
   a.x = x; a.Wp = reinterpret_cast<const unsigned char*>(Wp);
   a.M = M; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.kind = rope ? kClRope : cl_kind(ep, N, 4);
   if (rope) {

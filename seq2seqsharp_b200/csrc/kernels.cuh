@@ -261,6 +261,13 @@ struct RopeFuse {
   const int* state;    // device step state (per-sequence lengths), may be null
   const float2* tab;   // [Tmax, hd / 2] cos / sin
 };
+// rows that a linear norms itself (type 0: LayerNorm, 1: RMSNorm; beta may be null)
+struct RowNorm {
+  const void* gamma;
+  const void* beta;
+  int type;
+  float eps;
+};
 int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, const void* gamma, const void* beta, int norm_type, float eps,
                                 const void* Wp, int M, int K, int N, const Epilogue& ep, int* error_flag, bool pdl, void* ws, int64_t ws_bytes,
                                 cudaStream_t s);
@@ -269,7 +276,7 @@ int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x
                            const RopeFuse* rope = nullptr);
 // 1..8 fp32 rows in the same manner on the CUDA cores (gemv_cluster_f32.cu)
 int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
-                            const RopeFuse* rope = nullptr);
+                            const RopeFuse* rope = nullptr, const RowNorm* norm = nullptr);
 int64_t gemm_stream_mma_workspace_bytes(int M, int K, int N, int sm_count);
 int gs_take_error();
 // ---- blocks of layered engines (ops_blocks.cu) ---------------------------------------------------------------------------

@@ -1,4 +1,5 @@
-"""What a captured step reads before the launch in front of it has ended: cached rows of earlier positions and the step state."""
+"""What a captured step reads before the launch in front of it has ended (cached rows of earlier positions, the step state) and what a linear does
+before its products (the norm of fp32 rows): against engines that do neither."""
 import numpy as np
 import pytest
 
@@ -29,3 +30,29 @@ def test_cached_rows_around_the_new_position(cuda, hd, dtype, lens):
         whole = gpt.Logits(want_probs=False)[0]
         # the same sums in another order, through two layers of 16-bit (32-bit) activations
         assert np.abs(stepped - whole).max() <= (8 * 2.0 ** -11 if dtype == "float16" else 1e-5) * np.abs(whole).max()
+
+
+# 64 to 1024: normed by the linears (a lane's registers full at 1024); 1056: by a launch
+@pytest.mark.parametrize("d,H,B,norm", [(64, 1, 1, "LayerNorm"), (64, 1, 8, "RMSNorm"), (416, 13, 2, "LayerNorm"), (512, 8, 1, "LayerNorm"), (512, 8, 5, "RMSNorm"),
+                                        (1024, 16, 8, "LayerNorm"), (1056, 33, 3, "LayerNorm")])
+def test_fp32_rows_normed_by_the_linear(cuda, oracle, monkeypatch, d, H, B, norm):
+    cfg = GPTConfig(L=2, d=d, H=H, hd=d // H, F=192, V=515, norm=getattr(NormEnums, norm), act=ActivateFuncEnums.ReLU, pe=PositionEmbeddingEnums.RoPE,
+                    attn=MultiHeadAttentionTypeEnums.MHA, dtype="float32")
+    w = synthetic_weights(cfg, 7, std=0.05, bias_std=0.02)
+    prompt = np.random.default_rng(d).integers(1, cfg.V, size=(B, 9)).astype(np.int32)
+    opts, logits = DecodingOptions(MaxTgtSentLength=20), []
+    fed = [np.arange(B, dtype=np.int32) + 3 + i for i in range(3)]
+    for fused in ("1", "0"):
+        monkeypatch.setenv("TSB200_FUSED_STEP", fused)
+        gpt = GPT(cfg, max_batch=B, max_tokens=24)
+        gpt.LoadWeights(w)
+        gpt.Prefill(prompt, opts)
+        for ids in fed:
+            gpt.StepHost(ids, opts)
+        logits.append(gpt.Logits()[0].copy())
+    assert np.abs(logits[0] - logits[1]).max() <= 1e-5 * np.abs(logits[1]).max()      # fp32 sums of the rows in another order
+    orc = oracle.OracleGPT(cfg, w, max_pos=24, threads=4)
+    ref = orc.step(prompt)[0]
+    for ids in fed:
+        ref = orc.step(ids[:, None])[0]
+    assert np.abs(logits[0] - ref).max() <= 1e-3 * np.abs(ref).max()                  # the bound of the token loop's tests
