@@ -57,12 +57,12 @@ __global__ void rope_table_kernel(float2* __restrict__ tab, int Tmax, int hd, do
 }
 
 // q [rows,H,hd] rotated in place; k rotated and stored with v into the cache at positions T0 + s.  A thread takes V elements
-// (16 bytes, or one pair where a pointer or a size is not a multiple of that, or without a table) at a time; a CTA takes a row (WHOLE), a
-// part of one (blockIdx.y; a thread one piece) or several short rows.  `where`: packed rows (kernels.cuh); from row `rows` on, up to `listed`, the position's value is cleared.
+// (16 bytes, or one pair where a pointer or a size is not a multiple of that, or without a table) at a time; a CTA takes a row, a
+// part of one (blockIdx.y; a thread one piece) or several short rows (many rows of 16-byte pieces: rope_append_rows_kernel).  `where`: packed rows (kernels.cuh); from row `rows` on, up to `listed`, the position's value is cleared.
 // tab may be NULL: cos/sin are evaluated here, in double, one pair per thread - that chain is what bounds such a call (one row of 48 heads
 // of 128: 3.2 us; 13.7 with four pairs per thread and a CTA per row).
 // What bounds it with a table: bytes (16384 rows of 48 heads of 64: 200 MB; 154 us with one pair per thread and 64-bit index arithmetic).
-template <typename T, int V, bool WHOLE>
+template <typename T, int V>
 __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
                                    int64_t kv_rs, T* cK, T* cV, int rows, int listed, const int2* where, int S, int H, int Hkv, int hd,
                                    int T0_arg, const int* dT0, int Tmax, int use_rope, double base,
@@ -116,11 +116,53 @@ __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
     if constexpr (V > 2) *reinterpret_cast<Piece*>(dst + i) = x;
     else dst[i] = x.e[0], dst[i + 1] = x.e[1];
   };
-  if constexpr (WHOLE) {
-    for (int it = threadIdx.x; it < per_row; it += blockDim.x) piece(it);
-  } else {
-    const int it = rows_here > 1 ? (int)threadIdx.x - sub * per_row : (int)(blockIdx.y * blockDim.x + threadIdx.x);
-    if (it < per_row) piece(it);
+  const int it = rows_here > 1 ? (int)threadIdx.x - sub * per_row : (int)(blockIdx.y * blockDim.x + threadIdx.x);
+  if (it < per_row) piece(it);
+}
+
+// The same for many rows of 16-byte pieces with a table (or without rotation): a CTA per row, a thread one piece (or every 256th of a long row), the
+// table by 16 bytes and what a piece is decided before its loads.  What bounds it: bytes and the warps that ask for them.  us, one element of
+// the table at a time -> here: 16384 rows of 48 heads of 64 (200 MB) 82 -> 61, 1024 rows 6.6 -> 5.5, 1273 packed rows of 48 heads of 128 11.2 ->
+// 9.2, 4096 of those 38 -> 28, 400 rows of 48 heads of 64 3.8 -> 3.4.  Two and four rows per thread at a time are slower (97 and 148 us: fewer warps).
+template <typename T, int V>
+__global__ void __launch_bounds__(384) rope_append_rows_kernel(T* q, const T* k, const T* v, int64_t q_rs, int64_t kv_rs, T* cK, T* cV, int rows,
+                                                               const int2* where, int S, int H, int Hkv, int hd, int T0_arg, const int* dT0, int Tmax,
+                                                               int use_rope, const float2* tab) {
+  pdl_trigger();
+  pdl_wait();
+  struct __align__(16) Piece { T e[V]; };
+  const int pieces = hd / V, per_row = (H + 2 * Hkv) * pieces, row = (int)blockIdx.x;
+  const int b = where ? where[row].x : row / S, pos = (where ? where[row].y : row % S) + state_len(dT0, b, T0_arg);
+  TSB_DEV_CHECK(attention, pos >= 0 && pos < Tmax, 0x201, (void)0)   // append position outside the cache (row skipped)
+  if (pos >= Tmax) return;  // capacity is checked on the host; never write past the cache
+  const bool clear = row >= rows;   // a listed position behind the rows: its value is cleared
+  for (int it = threadIdx.x; it < per_row; it += blockDim.x) {
+    const int head = it / pieces, i = (it - head * pieces) * V;
+    const bool is_q = head < H, is_v = head >= H + Hkv;
+    if ((is_q && !use_rope) || (clear && !is_v)) continue;
+    Piece x;
+    if (clear) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) x.e[e] = from_f<T>(0.0f);
+    } else {
+      x = *reinterpret_cast<const Piece*>(is_q ? q + (int64_t)row * q_rs + (int64_t)head * hd + i
+                                               : (is_v ? v + (int64_t)row * kv_rs + (int64_t)(head - H - Hkv) * hd + i : k + (int64_t)row * kv_rs + (int64_t)(head - H) * hd + i));
+      if (use_rope && !is_v) {
+        const float4* t = reinterpret_cast<const float4*>(tab + (int64_t)pos * (hd / 2) + i / 2);   // (cos, sin) of two pairs
+        float4 cs[V / 4];
+#pragma unroll
+        for (int e = 0; e < V / 4; ++e) cs[e] = t[e];
+#pragma unroll
+        for (int e = 0; e < V; e += 2) {
+          const float c = e & 2 ? cs[e / 4].z : cs[e / 4].x, sn = e & 2 ? cs[e / 4].w : cs[e / 4].y;
+          const float x0 = to_f<T>(x.e[e]), x1 = to_f<T>(x.e[e + 1]);
+          x.e[e] = from_f<T>(x0 * c - x1 * sn);
+          x.e[e + 1] = from_f<T>(x1 * c + x0 * sn);
+        }
+      }
+    }
+    T* dst = is_q ? q + (int64_t)row * q_rs + (int64_t)head * hd : (is_v ? cV : cK) + (((int64_t)b * Hkv + (is_v ? head - H - Hkv : head - H)) * Tmax + pos) * hd;
+    *reinterpret_cast<Piece*>(dst + i) = x;
   }
 }
 
@@ -1111,16 +1153,23 @@ static int launch_rope_append_t(int device, DeviceState* st, T* q, const T* k, c
                                 cudaStream_t s) {
   const int rows = pack ? pack->rows : B * S, listed = pack ? pack->listed : rows;
   const int64_t per_row = (int64_t)(H + 2 * Hkv) * (hd / V);
-  // Equal parts of up to 384 pieces, several rows of up to 128 - or, with a table and more rows than SMs, a CTA of 256 for a long row (2036 rows of
-  // 768 pieces, cold: 18.9 us against 21.7 in two parts; one piece per thread is faster where a row fits a CTA: 8192 rows of 384 pieces 39 us, 45
-  // in a loop)
-  const bool whole = V > 2 && tab && per_row > 512 && listed > 2 * st->sm_count;
-  const int64_t parts = whole ? 1 : (per_row + 383) / 384;
-  const int threads = per_row <= 128 || whole ? 256 : (int)((per_row + parts - 1) / parts + 31) / 32 * 32;
+  if constexpr (V > 2) {
+    // from a few rows per SM on; fewer rows (a decode step's) are shared out below, and short rows several to a CTA
+    if (listed > 2 * st->sm_count && per_row > 128 && (!use_rope || ((uintptr_t)tab % 16 == 0 && hd % 4 == 0))) {
+      const int threads = per_row > 384 ? (per_row % 384 == 0 ? 384 : 256) : (int)(per_row + 31) / 32 * 32;
+      TSB_CUDA(launch_k(rope_append_rows_kernel<T, V>, dim3((unsigned)listed), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, pack ? pack->where : (const int2*)nullptr, S, H, Hkv,
+                        hd, T0, dT0, Tmax, use_rope, tab));
+      return 1;
+    }
+  }
+  // Equal parts of up to 384 pieces, several rows of up to 128 (one piece per thread is faster where few rows fit a CTA: in a loop 2036 rows of 768
+  // pieces took 18.9 us, in two parts 21.7, but 8192 rows of 384 pieces 45 in a loop and 39 at one each)
+  const int64_t parts = (per_row + 383) / 384;
+  const int threads = per_row <= 128 ? 256 : (int)((per_row + parts - 1) / parts + 31) / 32 * 32;
   const int64_t rows_here = threads / per_row > 1 ? threads / per_row : 1;
   TSB_CHECK(parts <= 65535, "rope_append: rows of %lld elements", (long long)per_row * V);
-  TSB_CUDA(launch_k(whole ? rope_append_kernel<T, V, (V > 2)> : rope_append_kernel<T, V, false>, dim3((unsigned)((listed + rows_here - 1) / rows_here), (unsigned)parts), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, listed, pack ? pack->where : (const int2*)nullptr,
-                    S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
+  TSB_CUDA(launch_k(rope_append_kernel<T, V>, dim3((unsigned)((listed + rows_here - 1) / rows_here), (unsigned)parts), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, listed,
+                    pack ? pack->where : (const int2*)nullptr, S, H, Hkv, hd, T0, dT0, Tmax, use_rope, base, tab));
   return 1;
 }
 
