@@ -92,6 +92,7 @@ __device__ __forceinline__ void pa_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uin
       "+r"(r[31])
 // 32 lanes x 32 columns; the registers are valid after pa_ld_wait on them
 __device__ __forceinline__ void pa_ld32(uint32_t taddr, uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -103,8 +104,12 @@ __device__ __forceinline__ void pa_ld32(uint32_t taddr, uint32_t* r) {
       : "r"(taddr)
       : "memory");
 }
-__device__ __forceinline__ void pa_ld_wait(uint32_t* r) { asm volatile("tcgen05.wait::ld.sync.aligned;" : PA_R32(r)::"memory"); }
+__device__ __forceinline__ void pa_ld_wait(uint32_t* r) {
+  __syncwarp();
+  asm volatile("tcgen05.wait::ld.sync.aligned;" : PA_R32(r)::"memory");
+}
 __device__ __forceinline__ void pa_st32(uint32_t taddr, const uint32_t* r) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -115,7 +120,10 @@ __device__ __forceinline__ void pa_st32(uint32_t taddr, const uint32_t* r) {
       "r"(r[31])
       : "memory");
 }
-__device__ __forceinline__ void pa_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void pa_st_wait() {
+  __syncwarp();
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 __device__ __forceinline__ float pa_ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -141,9 +149,15 @@ __device__ __forceinline__ void pa_add_pair(float& s, uint32_t v) {
     asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %1;\n\tadd.rn.f32.f16 %0, lo, %0;\n\tadd.rn.f32.f16 %0, hi, %0;\n\t}" : "+f"(s) : "r"(v));
 }
 template <int N>
-__device__ __forceinline__ void pa_more_registers() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+__device__ __forceinline__ void pa_more_registers() {
+  __syncwarp();
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
 template <int N>
-__device__ __forceinline__ void pa_fewer_registers() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+__device__ __forceinline__ void pa_fewer_registers() {
+  __syncwarp();
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
 
 template <int QB, int VB>
 constexpr int pa_smem(int nks, int nvs) { return (2 * QB + nks * QB + nvs * VB) * kPaBox + 1024 + 256; }
@@ -197,6 +211,7 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (w == 9) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -396,8 +411,8 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
       umma_commit(drain);
       tc_mbar_wait(drain, 0);
     }
-    __syncwarp();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
   }
   if (tid == 0 && s_err && a.error) *a.error = 1;

@@ -34,10 +34,6 @@ __device__ __forceinline__ bool cl_wait(uint64_t* bar) {
   }
   return false;
 }
-__device__ __forceinline__ void cl_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 template <typename H>
 __device__ __forceinline__ void cl_store4(H* dst, const float* t) {
   if constexpr (sizeof(H) == 4) *reinterpret_cast<float4*>(dst) = make_float4(t[0], t[1], t[2], t[3]);

@@ -59,6 +59,36 @@ inline cudaStream_t pick_stream(DeviceState* st, void* stream) { return stream ?
 void count_launch(int device, long long n = 1);
 int check_launch(const char* what);
 
+// ---- instructions that a warp has to reach as one ---------------------------------------------------
+// What a PTX instruction with .aligned (and bar.sync, bar.arrive: the aligned forms of barrier.*) does while the lanes of a warp are apart is
+// undefined, and any branch or loop of the lanes in front may have left them so.  Each is therefore issued behind a __syncwarp(), here and
+// wherever else one stands.
+#ifdef __CUDACC__
+template <int ID, int THREADS>
+__device__ __forceinline__ void named_sync() {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+template <int ID, int THREADS>
+__device__ __forceinline__ void named_arrive() {
+  __syncwarp();
+  asm volatile("bar.arrive %0, %1;" ::"n"(ID), "n"(THREADS) : "memory");
+}
+__device__ __forceinline__ void cluster_arrive_relaxed() {   // orders no memory
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+#endif
+
 // ---- programmatic dependent launch ------------------------------------------------------------------
 // Kernels of a decode step are chained with programmatic stream serialization: a kernel may become resident while its
 // predecessor is still running.  It calls pdl_wait() before it touches anything an earlier kernel wrote (a no-op when

@@ -80,7 +80,7 @@ __device__ __forceinline__ bool poll_count(const unsigned* p, unsigned target, u
   return false;
 }
 // the eight worker (consumer) warps are threads 0..255 in both kernels
-__device__ __forceinline__ void consumers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void consumers_sync() { named_sync<1, 256>(); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Geometry of one linear for a grid of G CTAs: CTAs 0..Gop-1 each own a contiguous, evenly sized range of the

@@ -46,6 +46,7 @@ struct LcArgs {
 template <int NR>
 __device__ __forceinline__ void lc_tmem_ld(uint32_t taddr, uint32_t* r) {
   if constexpr (NR == 16) {
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
@@ -95,6 +96,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     if (ks > 1) tc_mbar_expect_tx(bars + 17, quads * 2048);   // 128 / ks columns from each of ks CTAs
   }
   if (w == 1) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(kCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -129,7 +131,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   const int c = col0 + ((rank << gsh) + g) * 4, row0 = (tid >> (gsh + 2)) * 4 + (tid & 3), step = (kLcThreads >> (gsh + 2)) * 4;
   ClAhead<H> ahead;
   ahead.start(ep, a.sec[si].kind, N, c, row0, M, a.rope);
-  if (ks > 1) cl_sync();   // the other CTAs' barriers exist before anything is pushed to them
+  if (ks > 1) cluster_sync();   // the other CTAs' barriers exist before anything is pushed to them
   pdl_wait();
 
   if (w == 0) {
@@ -203,11 +205,11 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    asm volatile("bar.arrive 1, 160;" ::: "memory");   // TMEM has been read
+    named_arrive<1, 160>();   // TMEM has been read
   }
   if (ks > 1) {
     // arrived when everything is pushed (a CTA that gave up has pushed too); waited for before the CTA leaves, so that nobody pushes to one that has
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_arrive_relaxed();
     tc_wait_or(sums, 0, err);
   } else {
     __syncthreads();
@@ -227,12 +229,13 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   cl_finish_rows<H>(ep, a.sec[si].kind, N, c, row0, M, step, from, skip, ahead, a.rope, sum4);
   if (ks > 1) {
     if (*err) tc_wait_short(sums, 0);   // what is on its way here lands first
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_wait();
   }
   if (w == 1) {
     if (*err) tc_wait_short(acc, 0);   // some warp gave up: products in flight end before TMEM is given back
-    asm volatile("bar.sync 1, 160;" ::: "memory");
+    named_sync<1, 160>();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
   }
   if (*err && lane == 0 && a.error) *a.error = 1;   // the warp that gave up, at least, sees it

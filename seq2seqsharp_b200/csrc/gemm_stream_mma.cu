@@ -68,7 +68,7 @@ __device__ __forceinline__ unsigned gs_atom_add_acq_rel(unsigned* p, unsigned v)
   asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
   return old;
 }
-__device__ __forceinline__ void gs_consumers_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void gs_consumers_sync() { named_sync<1, 256>(); }
 // KQ == 0: activation rows arrive as TMA tiles beside every weight tile.  KQ > 0 (NB == 1, K == KQ * 1024, M * KQ <= 16): the
 // rows are read from the fp32 residual stream, normed by the consumer warps (LayerNorm / RMSNorm, the arithmetic of
 // norm_kernel) and kept in shared memory as fp16 for the whole kernel - the norm launch in front of the linear disappears and

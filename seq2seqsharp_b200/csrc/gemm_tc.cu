@@ -271,6 +271,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (w == 2) {  // TMEM allocation: 128 columns of fp32 accumulator (one warp, whole-warp instruction)
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(kBN) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -360,14 +361,14 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
     }
     if (a.ksplit > 1) {
       __threadfence();
-      asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
+      named_sync<1, 128>();  // the four epilogue warps
       if (w == 4 && lane == 0) {
         const unsigned int tile = blockIdx.y * gridDim.x + blockIdx.x;
         const unsigned int prev = atomicAdd(&a.counters[tile], 1u);
         s_last = (prev == (unsigned int)(a.ksplit - 1));
         if (s_last) a.counters[tile] = 0u;
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      named_sync<1, 128>();
       if (s_last) {
         __threadfence();
         tc_ahead<H>(a, at, n_live, n0, ahead);
@@ -407,6 +408,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
   __syncthreads();
   if (w == 2) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(kBN) : "memory");
   }
   if (tid == 0 && s_err) {
@@ -465,6 +467,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (w == 1) {  // all 512 TMEM columns: two accumulators of 256
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -561,6 +564,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
   __syncthreads();
   if (w == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
   }
   if (tid == 0 && s_err) {
@@ -595,10 +599,6 @@ __device__ __forceinline__ uint32_t tc_leader_addr(uint32_t addr) {   // the sam
   uint32_t r;
   asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
   return r;
-}
-__device__ __forceinline__ void tc_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tc_pair_load_2d(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
@@ -642,12 +642,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (w == 1) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_u32(tmem_slot)), "r"(kTmem) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  tc_cluster_sync();   // both CTAs' barriers exist
+  cluster_sync();   // both CTAs' barriers exist
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();   // after the allocation: a successor's CTA on this SM cannot take the columns first
@@ -735,9 +736,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  tc_cluster_sync();   // nobody reports to a CTA that has left
+  cluster_sync();   // nobody reports to a CTA that has left
   if (w == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmem) : "memory");
   }
   if (tid == 0 && s_err) {

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   const int per = M * 32 / ks;   // groups of four columns this CTA finishes: at most 256, one per thread
   const int c = group * 128 + ((rank * per + tid) & 31) * 4, row = (rank * per + tid) >> 5;
   if (tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
-  if (ks > 1) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if (ks > 1) cluster_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   if (w == 8) {
     if (lane == 0) {
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
         stat[RM == 1 ? 0 : w] = make_float2(mean, sqrtf(s / (float)a.K + a.eps));   // every warp of one row writes the same
       }
       if (RM == 1) __syncwarp();
-      else asm volatile("bar.sync 1, 256;" ::: "memory");
+      else named_sync<1, 256>();
     }
     for (int i = tid; i < RM * kc; i += 256) {
       const int m = i / kc, k = t0 * 32 + i % kc;
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       }
       xs[i] = v;
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+    named_sync<1, 256>();
     float4 acc[RM];
 #pragma unroll
     for (int m = 0; m < RM; ++m) acc[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -156,11 +156,11 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
     }
-    asm volatile("bar.sync 1, 256;" ::: "memory");   // every tile is read: the ring holds the warps' sums now
+    named_sync<1, 256>();   // every tile is read: the ring holds the warps' sums now
     float4* part = reinterpret_cast<float4*>(fc_raw);   // [warp][row][32 groups]
 #pragma unroll
     for (int m = 0; m < RM; ++m) part[(w * RM + m) * 32 + lane] = acc[m];
-    asm volatile("bar.sync 1, 256;" ::: "memory");
+    named_sync<1, 256>();
     for (int i = tid; i < M * 32; i += 256) {
       float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   }
   if (ks > 1) {
     // arrived when everything is pushed; waited for before the CTA leaves, so that nobody pushes to one that has
-    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    cluster_arrive_relaxed();
     if (tid < per && !cl_wait(&sums)) s_err = 1;
   } else {
     __syncthreads();
@@ -195,11 +195,9 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       }
     });
   }
-  __syncwarp();
   if (ks > 1) {
     if (*(volatile int*)&s_err) cl_wait(&sums);   // what is on its way here lands first
-    __syncwarp();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_wait();
   }
   if (lane == 0 && *(volatile int*)&s_err && a.error) *a.error = 1;   // the warp that gave up, at least, sees it
 }

@@ -245,8 +245,7 @@ __device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm
     }
   }
   if constexpr (BOX) {
-    __syncwarp();
-    cl_sync();
+    cluster_sync();
     for (int i = threadIdx.x; i < per; i += kAttnThreads) {
       const int idx = ((i >> 5) * splits + split) * 32 + (i & 31);
       if (idx >= items) continue;
@@ -302,7 +301,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
 #pragma unroll
   for (int u = 0; u < kAhead; ++u)
     if (const int t = tb0 + u * stride + sub; t < min(t_end, T0)) fetch(u, t);
-  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if constexpr (BOX) cluster_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
 #pragma unroll
   for (int u = 0; u < kAhead; ++u)
@@ -598,7 +597,7 @@ __global__ void __launch_bounds__(kAttnThreads) attn_mma_kernel(__half* out, flo
   // stages of tokens below T0 only are asked for before the kernel in front has ended
   int asked = 0;
   while (asked < kMmaStages - 1 && t_beg + (asked + 1) * kMmaStageTokens <= min(t_end, T0)) issue(asked++);
-  if constexpr (BOX) cl_sync();   // the other CTAs exist before anything is pushed to them
+  if constexpr (BOX) cluster_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   for (; asked < kMmaStages - 1; ++asked) issue(asked);
 

@@ -339,8 +339,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* x, const flo
 #pragma unroll
   for (int i = 0; i < TM; ++i) mine[(ty * TM + i) * 16 + tx] = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
   if (ks > 1) {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
   } else {
     __syncthreads();
   }
@@ -376,8 +375,7 @@ __global__ void __launch_bounds__(256) gemm_f32_kernel(const float* x, const flo
     }
   }
   if (ks > 1) {   // the others have read this CTA's sums
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_sync();
   }
 }
 

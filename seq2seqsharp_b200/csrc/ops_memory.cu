@@ -32,10 +32,6 @@ int chk_take_memory() { return 0; }
 __device__ __forceinline__ float log_sigmoid(float z) { return z >= 0.0f ? -log1pf(expf(-z)) : z - log1pf(expf(z)); }
 __device__ __forceinline__ float soft_cap(float z, float cap) { return cap * tanhf(z / cap); }
 
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float cluster_read(const float* p, unsigned rank) {
   uint32_t a;
   float v;

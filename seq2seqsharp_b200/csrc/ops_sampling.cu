@@ -151,10 +151,6 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ uint32_t ld_dsmem_u32(const uint32_t* local_ptr, uint32_t cta) {
   uint32_t a = (uint32_t)__cvta_generic_to_shared(local_ptr), ra, v;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(cta));
@@ -185,7 +181,7 @@ __global__ void __launch_bounds__(kSmThreads) softmax_argmax_cluster_kernel(int*
   }
   mx = block_max(mx, red);
   if (threadIdx.x == 0) part[0] = __float_as_uint(mx);
-  cluster_sync_all();
+  cluster_sync();
   mx = __uint_as_float(ld_dsmem_u32(&part[0], (uint32_t)(lane % kSmCluster)));
   mx = warp_max(mx);
   float s = 0.0f;
@@ -199,7 +195,7 @@ __global__ void __launch_bounds__(kSmThreads) softmax_argmax_cluster_kernel(int*
   }
   s = block_sum(s, red);
   if (threadIdx.x == 0) part[1] = __float_as_uint(s);
-  cluster_sync_all();
+  cluster_sync();
   s = __uint_as_float(ld_dsmem_u32(&part[1], (uint32_t)(lane % kSmCluster)));
 #pragma unroll
   for (int o = 1; o < kSmCluster; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
@@ -225,7 +221,7 @@ __global__ void __launch_bounds__(kSmThreads) softmax_argmax_cluster_kernel(int*
     part[2] = __float_as_uint(best.v);
     part[3] = (uint32_t)best.i;
   }
-  cluster_sync_all();
+  cluster_sync();
   if (crank == 0 && threadIdx.x == 0 && out_ids) {
     for (int c = 1; c < kSmCluster; ++c) {
       ValIdx o;
@@ -235,7 +231,7 @@ __global__ void __launch_bounds__(kSmThreads) softmax_argmax_cluster_kernel(int*
     }
     out_ids[r] = best.i == 0x7fffffff ? 0 : best.i;
   }
-  cluster_sync_all();   // CTA 0 has read the others' results
+  cluster_sync();   // CTA 0 has read the others' results
 }
 
 // ------------------------------------------------------------------------------------------------ Philox4x32-10
@@ -644,7 +640,7 @@ __device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_
   const float least = topP * topP * (0.999f / kSelMax);
   if (CL == 1 || V >= 65536) {
     if constexpr (CL > 1) {
-      cluster_sync_all();
+      cluster_sync();
       sq = 0.0f;
 #pragma unroll
       for (int c = 0; c < CL; ++c) sq += __uint_as_float(ld_dsmem_u32(&sm.share[1], (uint32_t)c));
@@ -683,7 +679,7 @@ __device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_
   }
   if (tid == 0) sm.share[0] = __float_as_uint(sum);
   if constexpr (CL > 1) {
-    cluster_sync_all();
+    cluster_sync();
     sum = sq = 0.0f;
 #pragma unroll
     for (int c = 0; c < CL; ++c) {
@@ -727,7 +723,7 @@ __device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_
     fits = block_sum(n, reinterpret_cast<float*>(sm.warp_tot)) <= (float)kSelMax;
   }
   if (!fits) {
-    if constexpr (CL > 1) cluster_sync_all();   // the others have read this CTA's bins
+    if constexpr (CL > 1) cluster_sync();   // the others have read this CTA's bins
     return false;
   }
   cut += kSelLow;
@@ -750,9 +746,9 @@ __device__ bool topp_select(uint32_t* keys, uint32_t* idx, uint32_t* tk, uint32_
   }
   uint32_t n;
   if constexpr (CL > 1) {
-    cluster_sync_all();
+    cluster_sync();
     n = ld_dsmem_u32(&sm.n_sel, 0u);
-    cluster_sync_all();   // everybody has the count: CTA 0 may go on and the others may leave
+    cluster_sync();   // everybody has the count: CTA 0 may go on and the others may leave
   } else {
     __syncthreads();
     n = sm.n_sel;
@@ -961,7 +957,7 @@ __device__ __forceinline__ void radix_pass_cluster(const uint32_t* kin, const ui
     const int d = threadIdx.x;
     sm.tot[d] = (d == 255 ? (uint32_t)n_loc : sm.hist[0][d + 1]) - sm.hist[0][d];
   }
-  cluster_sync_all();  // every CTA's totals are in place (and all reads of the previous pass are done)
+  cluster_sync();  // every CTA's totals are in place (and all reads of the previous pass are done)
   // C: global base of (digit, this CTA): keys of smaller digits anywhere + keys of this digit in earlier CTAs
   if (threadIdx.x < 256) {
     const int d = threadIdx.x;
@@ -979,7 +975,7 @@ __device__ __forceinline__ void radix_pass_cluster(const uint32_t* kin, const ui
       if (lane >= o) incl += t;
     }
     if (lane == 31) sm.warp_tot[w] = incl;  // 8 warps take part
-    asm volatile("bar.sync 2, 256;" ::: "memory");
+    named_sync<2, 256>();
     uint32_t wbase = 0;
     for (int i = 0; i < w; ++i) wbase += sm.warp_tot[i];
     sm.base[d] = wbase + incl - all + before - sm.hist[0][d];
@@ -1013,7 +1009,7 @@ __device__ __forceinline__ void radix_pass_cluster(const uint32_t* kin, const ui
       __syncwarp();
     }
   }
-  cluster_sync_all();  // the scattered keys are visible to the whole cluster; sm.tot may be rewritten
+  cluster_sync();  // the scattered keys are visible to the whole cluster; sm.tot may be rewritten
 }
 
 __global__ void __launch_bounds__(kTopPThreads) topp_cluster_kernel(int* out, const float* probs, int V, float topP, float repeatPenalty,

@@ -51,7 +51,7 @@ __device__ __forceinline__ long long gtimer() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-__device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void consumer_sync() { named_sync<1, 256>(); }
 
 template <typename T> struct TileVec;
 template <> struct TileVec<__half> {
