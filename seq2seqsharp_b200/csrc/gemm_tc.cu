@@ -336,7 +336,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
     const int row = m_tile * kBM + q * 32 + lane;
     const int n0 = n_tile * kBN;
     const bool live = ok && row < a.M;
-    const int n_live = __all_sync(0xffffffffu, ok) ? min(32, a.M - (m_tile * kBM + q * 32)) : 0;
+    const int n_live = ok ? min(32, a.M - (m_tile * kBM + q * 32)) : 0;
     float* stage = reinterpret_cast<float*>(smem) + q * kStageFloats;   // every product has read its operands
     const size_t Npad = (size_t)gridDim.x * kBN;
     const TcLane at = tc_lane(a, row - lane, n0);
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
       const int n_live = min(32, min(rb.rows - q * 32, a.M - row0));
       const TcLane at = tc_lane(a, row0, n0);
       tc_ahead<H>(a, at, n_live, n0, ahead);
-      if (!__all_sync(0xffffffffu, tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err))) break;  // warp-uniform outcome
+      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tc_drain<H, 128>(a, at, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kP_BN + half * 128), row0, n_live, n0, stage, ahead, [](int, float*) {});
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -726,7 +726,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
       const int n_live = min(32, a.M - row0);
       const TcLane at = tc_lane(a, row0, n0);
       tc_ahead<H>(a, at, n_live, n0, ahead);
-      if (!__all_sync(0xffffffffu, tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err))) break;
+      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tc_drain<H, P::kCols>(a, at, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * P::kCols), row0, n_live, n0, stage, ahead, [](int, float*) {});
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");

@@ -146,16 +146,19 @@ __device__ __forceinline__ bool tc_try_wait(uint32_t bar, unsigned parity) {
       : "memory");
   return ok != 0;
 }
-// bounded; gives up early when another wait of the CTA has (*err), raises *err when it runs out itself
-__device__ __forceinline__ bool tc_wait_or(uint32_t bar, unsigned parity, volatile int* err) {
-  if (tc_try_wait(bar, parity)) return true;
+// Bounded; gives up early when another wait of the CTA has (*err), raises *err when it runs out itself.  For whole warps: their lanes poll for
+// themselves and may see a phase end, or the limit, at different polls, so the warp votes, and one answer sends all of it on or out of its loop
+// (the elected issue behind it needs all lanes).
+__device__ __forceinline__ bool tc_wait_or(uint32_t bar, unsigned parity, volatile int* err, unsigned limit = kTcSpin) {
+  bool ok = tc_try_wait(bar, parity);
 #pragma unroll 1
-  for (unsigned i = 1; i < kTcSpin; ++i) {
-    if (tc_try_wait(bar, parity)) return true;
-    if ((i & 63) == 63 && *err) return false;
+  for (unsigned i = 1; !ok && i < limit; ++i) {
+    ok = tc_try_wait(bar, parity);
+    if (!ok && (i & 63) == 63 && *err) break;
   }
-  *err = 1;
-  return false;
+  ok = __all_sync(0xffffffffu, ok);
+  if (!ok) *err = 1;
+  return ok;
 }
 __device__ __forceinline__ bool tc_wait_short(uint32_t bar, unsigned parity) {   // after an error: bounded, raises nothing
 #pragma unroll 1
