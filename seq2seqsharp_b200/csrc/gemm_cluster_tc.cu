@@ -36,6 +36,7 @@ struct LcSection {
 struct LcArgs {
   const unsigned char* Wp;
   int M, KB, ks, stages;
+  unsigned wait_limit;  // polls of a wait before the CTA gives up
   int* error;
   int n_sec;
   LcSection sec[kLcMaxSections];
@@ -72,7 +73,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S * kStage + NR * 512);
   const uint32_t full = s_u32(bars), empty = full + 64, acc = empty + 64, sums = acc + 8;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
-  __shared__ int s_err;
+  __shared__ int s_err, s_asked;   // s_asked: steps whose copies are under way or done (warp 0)
 
   const int tid = threadIdx.x, lane = tid & 31, w = warp_index();
   const int rank = (int)(blockIdx.x % ks), group = (int)(blockIdx.x / ks);
@@ -138,19 +139,16 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     // ---------------- copies
     int s = 0;
     unsigned phase = 1;   // parity of the ring's previous round
-    for (int i = 0; i < n_it; ++i) {
+    int i = 0;
+    for (; i < n_it; ++i) {
       if (i >= S) {
-        if (!tc_wait_or(empty + s * 8, phase, err)) break;
+        if (!tc_wait_or(empty + s * 8, phase, err, a.wait_limit)) break;
         weights(i, s);
       }
       tma_load_2d_el(ring + s * kStage + 16384, &mapX, (p0 + i) * 64, xrow, full + s * 8);   // rows behind the block's are columns nobody reads
       if (++s == S) s = 0, phase ^= 1;
     }
-    if (*err)   // copies in flight land first: the last S that were asked for
-      for (int j = 0; j < n_pre; ++j) {
-        if (--s < 0) s = S - 1, phase ^= 1;
-        tc_wait_short(full + s * 8, phase ^ 1);
-      }
+    if (lane == 0) s_asked = i;
   } else if (w == 1) {
     // ---------------- products.  Instruction descriptor: fp32 accumulator, A MN-major, B K-major, N = NR, M = 128
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (1u << 15) | ((uint32_t)(NR >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -159,7 +157,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     int s = 0;
     unsigned phase = 0;
     for (int i = 0; i < n_it; ++i) {
-      if (!tc_wait_or(full + s * 8, phase, err)) break;
+      if (!tc_wait_or(full + s * 8, phase, err, a.wait_limit)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ad = a0 + s * (kStage >> 4), bd = b0 + s * (kStage >> 4);
       umma_el(tmem, ad, hi, bd, hi, idesc, i > 0);
@@ -178,7 +176,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   ahead.first(ep, a.sec[si].kind, N, c, row0, M, a.rope);
   if (w >= 2 && w < 6) {
     // ---------------- sums out of TMEM: warp w reads lanes 32 (w % 4) .. = columns of the group
-    tc_wait_or(acc, 0, err);
+    tc_wait_or(acc, 0, err, a.wait_limit);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int col = (w & 3) * 32 + lane, owner = col >> (gsh + 2), e = col & 3, here = ((col >> 2) + 2 * e) & (G - 1);
     const uint32_t local = s_u32(red) + ((uint32_t)rank * quads * (G * 4) + e * G + here) * 16, hop = G * 64;
@@ -210,7 +208,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
   if (ks > 1) {
     // arrived when everything is pushed (a CTA that gave up has pushed too); waited for before the CTA leaves, so that nobody pushes to one that has
     cluster_arrive_relaxed();
-    tc_wait_or(sums, 0, err);
+    tc_wait_or(sums, 0, err, a.wait_limit);
   } else {
     __syncthreads();
   }
@@ -231,8 +229,9 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     if (*err) tc_wait_short(sums, 0);   // what is on its way here lands first
     cluster_wait();
   }
+  if (w == 0) tc_land(full, S, s_asked);
   if (w == 1) {
-    if (*err) tc_wait_short(acc, 0);   // some warp gave up: products in flight end before TMEM is given back
+    tc_wait_short(acc, 0);   // where a warp has given up, products may still be running
     named_sync<1, 160>();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncwarp();
@@ -285,6 +284,7 @@ static int lc_run(int device, DeviceState* st, int dtype, const void* x, int row
   a.ks = 1;
   while (a.ks < 8 && (int64_t)groups * a.ks * 2 <= 2 * st->sm_count && KP / (a.ks * 2) >= 2) a.ks *= 2;
   a.error = tc_error_word(device);
+  a.wait_limit = tc_wait_limit();
   const int NR = a.M <= 16 ? 16 : (a.M <= 32 ? 32 : 64);
   CUtensorMap map;
   const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};

@@ -45,6 +45,7 @@ struct TcArgs {
   unsigned int* counters;  // one per output tile, zero on entry, self-resetting
   int* error_flag;
   const unsigned char* Wp;  // packed weight tiles
+  unsigned wait_limit;      // polls of a wait before the CTA gives up
   int kind;                 // TcKind: what the 16-byte epilogue has to read and write; kTcAny: element by element
   Epilogue ep;
 };
@@ -286,24 +287,19 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
   if (w == 0) {
     // ---------------- copies.  B: this CTA's 128 columns are boxes (2p, 2p+1) of column tile ct: 8 KB contiguous in every packed k tile
     const unsigned char* wsrc = a.Wp + ((size_t)(n_tile >> 1) * a.KB + k_begin * 2) * 16384 + (size_t)(n_tile & 1) * 8192;
-    int s = 0, used = 0;
+    int s = 0, asked = 0;
     unsigned phase = 1;
-    for (int it = 0; it < k_iters; ++it, wsrc += 32768) {
-      if (used == kTcStages && !tc_wait_or(empty + s * 8, phase, err)) break;
-      const bool two = (k_begin + it) * 2 + 1 < a.KB;  // the last 64-k block of an odd tile count has one packed tile only
+    for (; asked < k_iters; ++asked, wsrc += 32768) {
+      if (asked >= kTcStages && !tc_wait_or(empty + s * 8, phase, err, a.wait_limit)) break;
+      const bool two = (k_begin + asked) * 2 + 1 < a.KB;  // the last 64-k block of an odd tile count has one packed tile only
       const uint32_t bar = full + s * 8, dB = sB + s * kBBytes;
       tc_mbar_expect_el(bar, kABytes + (two ? 16384 : 8192));
-      tma_load_2d_el(sA + s * kABytes, &mapA, (k_begin + it) * kBK, m_tile * kBM, bar);
+      tma_load_2d_el(sA + s * kABytes, &mapA, (k_begin + asked) * kBK, m_tile * kBM, bar);
       tc_bulk_g2s_el(dB, wsrc, 8192, bar);
       if (two) tc_bulk_g2s_el(dB + 8192, wsrc + 16384, 8192, bar);
-      if (used < kTcStages) ++used;
       if (++s == kTcStages) s = 0, phase ^= 1;
     }
-    if (*err)   // copies in flight land first
-      for (int j = 0; j < used; ++j) {
-        if (--s < 0) s = kTcStages - 1, phase ^= 1;
-        tc_wait_short(full + s * 8, phase ^ 1);
-      }
+    tc_land(full, kTcStages, asked);
   } else if (w == 1) {
     // ---------------- products.  Instruction descriptor: D fp32, A/B fp16 or bf16, A K-major, B MN-major, N = 128, M = 128
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (0u << 15) | (1u << 16) | ((uint32_t)(kBN >> 3) << 17) |
@@ -315,7 +311,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
     int s = 0;
     unsigned phase = 0;
     for (int it = 0; it < k_iters; ++it) {
-      if (!tc_wait_or(full + s * 8, phase, err)) break;
+      if (!tc_wait_or(full + s * 8, phase, err, a.wait_limit)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t ad = a0 + s * (kABytes >> 4), bd = b0 + s * (kBBytes >> 4);
       umma_el(tmem_acc, ad, hi, bd, hi, idesc, it > 0);
@@ -328,10 +324,11 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
       if (++s == kTcStages) s = 0, phase ^= 1;
     }
     umma_commit_el(acc_ready);    // accumulator complete
+    tc_wait_short(acc_ready, 0);
   } else if (w >= 4) {
     // ---------------- epilogue: warp (w - 4) owns TMEM lanes 32*(w-4) .. +31 = rows of the tile
     const int q = w - 4;
-    const bool ok = tc_wait_or(acc_ready, 0, err);
+    const bool ok = tc_wait_or(acc_ready, 0, err, a.wait_limit);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const int row = m_tile * kBM + q * 32 + lane;
     const int n0 = n_tile * kBN;
@@ -482,7 +479,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
 
   if (w == 0) {
     // ---------------- copies
-    int s = 0, used = 0;
+    int s = 0, asked = 0;
     unsigned phase = 1;   // parity of the ring's previous round
     bool ok = true;
     for (int t = blockIdx.x; t < n_total && ok; t += gridDim.x) {
@@ -490,22 +487,18 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
       const RowBlock rb = g.table[tl.m_tile];
       const unsigned char* wsrc = a.Wp + (size_t)rb.matrix * g.matrix_bytes + ((size_t)tl.n_tile * a.KB) * 16384;
       for (int it = 0; it < k_total; ++it, wsrc += 32768) {
-        if (used == kGStages && !(ok = tc_wait_or(empty + s * 8, phase, err))) break;
+        if (asked >= kGStages && !(ok = tc_wait_or(empty + s * 8, phase, err, a.wait_limit))) break;
         const bool two = it * 2 + 1 < a.KB;
         const uint32_t bar = full + s * 8, dB = sB + s * 32768;
         tc_mbar_expect_el(bar, kABytes + (two ? 32768 : 16384));
         tma_load_2d_el(sA + s * kABytes, &mapA, it * kBK, rb.row0, bar);
         tc_bulk_g2s_el(dB, wsrc, 16384, bar);
         if (two) tc_bulk_g2s_el(dB + 16384, wsrc + 16384, 16384, bar);
-        if (used < kGStages) ++used;
+        ++asked;
         if (++s == kGStages) s = 0, phase ^= 1;
       }
     }
-    if (*err)   // copies in flight land first
-      for (int j = 0; j < used; ++j) {
-        if (--s < 0) s = kGStages - 1, phase ^= 1;
-        tc_wait_short(full + s * 8, phase ^ 1);
-      }
+    tc_land(full, kGStages, asked);
   } else if (w == 1) {
     // ---------------- products.  Instruction descriptor: fp32 accumulator, A K-major, B MN-major, N = 256, M = 128
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (1u << 16) | ((uint32_t)(kP_BN >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
@@ -517,11 +510,11 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
     bool ok = true;
     for (int t = blockIdx.x; t < n_total && ok; t += gridDim.x, ++n_done) {
       const int buf = n_done & 1;
-      if (n_done >= 2 && !(ok = tc_wait_or(acc_empty + buf * 8, (unsigned)(((n_done >> 1) - 1) & 1), err))) break;
+      if (n_done >= 2 && !(ok = tc_wait_or(acc_empty + buf * 8, (unsigned)(((n_done >> 1) - 1) & 1), err, a.wait_limit))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + buf * kP_BN;
       for (int it = 0; it < k_total; ++it) {
-        if (!(ok = tc_wait_or(full + s * 8, phase, err))) break;
+        if (!(ok = tc_wait_or(full + s * 8, phase, err, a.wait_limit))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ad = a0 + s * (kABytes >> 4), bd = b0 + s * (32768 >> 4);
         umma_el(acc, ad, hi, bd, hi, idesc, it > 0);
@@ -535,10 +528,8 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
       }
       if (ok) umma_commit_el(acc_full + buf * 8);
     }
-    if (!ok) {   // products in flight end before TMEM is given back
-      umma_commit_el(drain);
-      tc_wait_short(drain, 0);
-    }
+    umma_commit_el(drain);
+    tc_wait_short(drain, 0);
   } else if (w >= 2) {
     // ---------------- epilogue: TMEM lanes 32 (w % 4) .. = rows of the tile, columns 128 ((w - 2) / 4) ..
     const int q = w & 3, half = (w - 2) >> 2;
@@ -552,7 +543,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
       const int n_live = min(32, min(rb.rows - q * 32, a.M - row0));
       const TcLane at = tc_lane(a, row0, n0);
       tc_ahead<H>(a, at, n_live, n0, ahead);
-      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err)) break;
+      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err, a.wait_limit)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tc_drain<H, 128>(a, at, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * kP_BN + half * 128), row0, n_live, n0, stage, ahead, [](int, float*) {});
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -633,6 +624,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
   const int rank = (int)(blockIdx.x & 1), pair = (int)(blockIdx.x >> 1), n_pairs = (int)(gridDim.x >> 1);
   const int k_total = (a.K + kBK - 1) / kBK, n_total = m_tiles * n_tiles;
   constexpr uint32_t kTmem = 2 * BN;
+  __shared__ int2 s_peer;   // from the other CTA: whether it has given up, and the stages it has asked for
+  int asked = 0;            // (warp 0)
 
   if (tid == 0) {
     for (int i = 0; i < 2 * P::kStages + 2; ++i) tc_mbar_init(bars + i, 1);
@@ -658,7 +651,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
   if (w == 0) {
     // ---------------- copies of this CTA
     const uint32_t full0 = tc_leader_addr(full);
-    int s = 0, used = 0;
+    int s = 0;
     unsigned phase = 1;   // parity of the ring's previous round
     bool ok = true;
     for (int t = pair; t < n_total && ok; t += n_pairs) {
@@ -667,19 +660,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
       const int kb0 = (BN == 256 ? tl.n_tile : tl.n_tile >> 1) * a.KB;
       const int box_row = (BN == 256 ? rank * 2 : (tl.n_tile & 1) * 2 + rank) * 32, row = (tl.m_tile * 2 + rank) * kBM;
       for (int it = 0; it < k_total; ++it) {
-        if (used == P::kStages && !(ok = tc_wait_or(empty + s * 8, phase, err))) break;
+        if (asked >= P::kStages && !(ok = tc_wait_or(empty + s * 8, phase, err, a.wait_limit))) break;
         if (rank == 0) tc_mbar_expect_el(full + s * 8, 2 * P::kStage);
         tc_pair_load_2d(sA + s * kABytes, &mapA, it * kBK, row, full0 + s * 8);
         tc_pair_load_3d(sB + s * P::kB, &mapB, 0, box_row, kb0 + it * 2, full0 + s * 8);   // the second k tile of an odd count is not multiplied
-        if (used < P::kStages) ++used;
+        ++asked;
         if (++s == P::kStages) s = 0, phase ^= 1;
       }
     }
-    if (*err && rank == 0)   // copies in flight land first (the last ones may have been asked for by one CTA only: bounded)
-      for (int j = 0; j < used; ++j) {
-        if (--s < 0) s = P::kStages - 1, phase ^= 1;
-        tc_wait_short(full + s * 8, phase ^ 1);
-      }
   } else if (w == 1 && rank == 0) {
     // ---------------- products.  Instruction descriptor: fp32 accumulator, A K-major, B MN-major, N = BN, M = 256
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (1u << 16) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(2 * kBM >> 4) << 24);
@@ -691,11 +679,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
     bool ok = true;
     for (int t = pair; t < n_total && ok; t += n_pairs, ++n_done) {
       const int buf = n_done & 1;
-      if (n_done >= 2 && !(ok = tc_wait_or(acc_empty + buf * 8, (unsigned)(((n_done >> 1) - 1) & 1), err))) break;
+      if (n_done >= 2 && !(ok = tc_wait_or(acc_empty + buf * 8, (unsigned)(((n_done >> 1) - 1) & 1), err, a.wait_limit))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t acc = tmem_base + buf * BN;
       for (int it = 0; it < k_total; ++it) {
-        if (!(ok = tc_wait_or(full + s * 8, phase, err))) break;
+        if (!(ok = tc_wait_or(full + s * 8, phase, err, a.wait_limit))) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ad = a0 + s * (kABytes >> 4), bd = b0 + s * (P::kB >> 4);
         umma_pair_el(acc, ad, hi, bd, hi, idesc, it > 0);
@@ -709,10 +697,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
       }
       if (ok) umma_commit_pair_el(acc_full + buf * 8);
     }
-    if (!ok) {   // products in flight end before TMEM is given back
-      umma_commit_pair_el(drain);
-      tc_wait_short(drain, 0);
-    }
+    umma_commit_pair_el(drain);
+    tc_wait_short(drain, 0);
   } else if (w >= 2) {
     // ---------------- epilogue: TMEM lanes 32 (w % 4) .. = rows of this CTA's half, columns kCols ((w - 2) / 4) ..
     const int q = w & 3, half = (w - 2) >> 2;
@@ -726,7 +712,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
       const int n_live = min(32, a.M - row0);
       const TcLane at = tc_lane(a, row0, n0);
       tc_ahead<H>(a, at, n_live, n0, ahead);
-      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err)) break;
+      if (!tc_wait_or(acc_full + buf * 8, (unsigned)((n_done >> 1) & 1), err, a.wait_limit)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       tc_drain<H, P::kCols>(a, at, tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN + half * P::kCols), row0, n_live, n0, stage, ahead, [](int, float*) {});
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -736,8 +722,27 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPThreads, 1)
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (tid == 0) {
+    uint32_t to;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(s_u32(&s_peer)), "r"(rank ^ 1));
+    asm volatile("st.shared::cluster.v2.s32 [%0], {%1, %2};" ::"r"(to), "r"(s_err), "r"(asked) : "memory");
+  }
   cluster_sync();   // nobody reports to a CTA that has left
+  if (s_err | s_peer.x) {
+    // Copies in flight land in both CTAs.  One CTA may have asked for up to kStages stages more than the other, whose part the leader's barrier
+    // then waits for in vain, or does not know of: the difference is put right, in the phases that are open, before they are waited for.
+    if (w == 0 && rank == 0) {
+      for (int j = min(asked, s_peer.y); j < max(asked, s_peer.y); ++j) {
+        const uint32_t bar = full + (j % P::kStages) * 8;
+        if (asked > s_peer.y) tc_mbar_complete_el(bar, P::kStage);
+        else tc_mbar_expect_el(bar, P::kStage);
+      }
+      tc_land(full, P::kStages, max(asked, s_peer.y));
+    }
+    cluster_sync();
+  }
   if (w == 1) {
+    if (rank == 1) tc_wait_short(drain, 0);   // the leader has seen its own arrive
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmem) : "memory");
@@ -872,6 +877,7 @@ int launch_gemm_tc_grouped(int device, DeviceState* st, int dtype, const void* x
   TcArgs a{};
   a.M = rows; a.N = N; a.K = K; a.KB = (K + 31) / 32; a.ep = ep; a.ksplit = 1;
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
+  a.wait_limit = tc_wait_limit();
   a.kind = tc_kind(N, ep);
   TSB_CUDA(launch_k(gemm_tc_grouped_kernel<__nv_bfloat16>, dim3(st->sm_count), dim3(kPThreads), kGSmem, s, mapA, a, (N + kP_BN - 1) / kP_BN, groups));
   count_launch(device);
@@ -921,6 +927,7 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
   TcArgs a{};
   a.M = M; a.N = N; a.K = K; a.KB = KB; a.error_flag = error_flag; a.ep = ep;
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
+  a.wait_limit = tc_wait_limit();
   a.kind = tc_kind(N, ep);
   {
     static int pers = -1;

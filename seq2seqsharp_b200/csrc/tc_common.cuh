@@ -122,6 +122,10 @@ __device__ __forceinline__ void umma_commit_pair_el(uint32_t bar) {
 __device__ __forceinline__ void tc_mbar_expect_el(uint32_t bar, unsigned bytes) {
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
 }
+// takes `bytes` off what a phase waits for, as a copy that lands does
+__device__ __forceinline__ void tc_mbar_complete_el(uint32_t bar, unsigned bytes) {
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t@q mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d_el(uint32_t dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
@@ -160,11 +164,18 @@ __device__ __forceinline__ bool tc_wait_or(uint32_t bar, unsigned parity, volati
   if (!ok) *err = 1;
   return ok;
 }
-__device__ __forceinline__ bool tc_wait_short(uint32_t bar, unsigned parity) {   // after an error: bounded, raises nothing
+__device__ __forceinline__ bool tc_wait_short(uint32_t bar, unsigned parity) {   // bounded, raises nothing
 #pragma unroll 1
   for (unsigned i = 0; i < kTcSpin; ++i)
     if (tc_try_wait(bar, parity)) return true;
   return false;
+}
+// How a CTA may end, whichever of its waits has run out: its copies have landed (the copying warp sees to the last `asked` of a ring) and its
+// products are done (the issuing warp waits for a commit behind them) before its shared memory and TMEM go to another CTA.  Both are waited
+// for in every case and not upon an error flag, which another warp may raise after it was looked at; those warps have nothing else to do.
+__device__ __forceinline__ void tc_land(uint32_t full, int stages, int asked) {
+#pragma unroll 1
+  for (int j = max(0, asked - stages); j < asked; ++j) tc_wait_short(full + (j % stages) * 8, (unsigned)((j / stages) & 1));
 }
 // what a warp's index is to the compiler: the same in all lanes
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
