@@ -257,12 +257,11 @@ __global__ void __launch_bounds__(kPaThreads, 1) attn_prefill_tc_kernel(const __
         for (int i = 0; i < VB; ++i) pa_load_3d(sV + (st * VB + i) * kPaBox, &mapV, a.vx0 + kvh * a.vx + 64 * i, j * kPaKeys, z, &v_full[st]);
         vs = j + 1;
       }
-      if (*err) {   // copies in flight land before the CTA ends (they need nobody's help)
-        for (int t = 0; t < 2; ++t)
-          if (n_of[t]) tc_mbar_wait(&q_full[t], 0);
-        for (int j = max(0, ks - NKS); j < ks; ++j) tc_mbar_wait(&k_full[j % NKS], (unsigned)((j / NKS) & 1));
-        for (int j = max(0, vs - NVS); j < vs; ++j) tc_mbar_wait(&v_full[j % NVS], (unsigned)((j / NVS) & 1));
-      }
+      // copies in flight land before the CTA ends (tc_land): they need nobody's help, and a wait may run out after this thread has asked for its last
+      for (int t = 0; t < 2; ++t)
+        if (n_of[t]) tc_mbar_wait(&q_full[t], 0);
+      tc_land(s_u32(k_full), NKS, ks);
+      tc_land(s_u32(v_full), NVS, vs);
     } else if (w == 9 && lane == 0) {
       // ---------------- MMA issuer.  Instruction descriptors: fp32 accumulator, A K-major, 128 rows; K: N = 128 K-major; V: N = 64 VB MN-major
       const uint32_t fmt = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | ((uint32_t)(kPaRows >> 4) << 24);
