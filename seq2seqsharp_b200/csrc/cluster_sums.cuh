@@ -18,10 +18,10 @@ __device__ __forceinline__ void cl_push4(float* local, uint64_t* bar, uint32_t c
   asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(ra), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "r"(rb) : "memory");
 }
 // first phase of an mbarrier that other CTAs' pushes complete; bounded
-__device__ __forceinline__ bool cl_wait(uint64_t* bar) {
+__device__ __forceinline__ bool cl_wait(uint64_t* bar, unsigned limit = 1u << 22) {
   const uint32_t at = (uint32_t)__cvta_generic_to_shared(bar);
 #pragma unroll 1
-  for (unsigned i = 0; i < (1u << 22); ++i) {
+  for (unsigned i = 0; i < limit; ++i) {
     unsigned ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"

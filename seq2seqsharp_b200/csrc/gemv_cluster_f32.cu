@@ -19,6 +19,7 @@ struct FcArgs {
   const float* x;
   const unsigned char* Wp;
   int M, N, K, KB, ks;
+  unsigned wait_limit;  // polls of a wait before a warp gives up
   int* error;
   Epilogue ep;
   int kind;    // ClKind
@@ -78,18 +79,19 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   pdl_wait();
   if (w == 8) {
     if (lane == 0) {
-      for (int i = n_pre; i < n_it; ++i) {
+      int i = n_pre;
+      for (; i < n_it; ++i) {
         const int s = i % kFcStages;
-        if (!mbar_wait(&empty[s], (unsigned)((i / kFcStages - 1) & 1))) {
+        if (!mbar_wait(&empty[s], (unsigned)((i / kFcStages - 1) & 1), a.wait_limit)) {
           s_err = 1;
-          for (int j = i - kFcStages; j < i; ++j) mbar_wait(&full[j % kFcStages], (unsigned)((j / kFcStages) & 1));   // copies in flight land first
           break;
         }
         mbar_expect_tx(&full[s], kTileBytes);
         bulk_g2s(fc_raw + s * kTileBytes, src + (size_t)i * kTileBytes, kTileBytes, &full[s]);
       }
+      // copies in flight land before the CTA ends, whichever warp has given up
+      for (int j = max(0, i - kFcStages); j < i; ++j) mbar_wait(&full[j % kFcStages], (unsigned)((j / kFcStages) & 1));
     }
-    __syncwarp();
   } else {
     if (tid < per) ahead.first(a.ep, a.kind, a.N, c, row, M, a.rope);
     const int kc = n_it * 32;
@@ -136,7 +138,10 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     for (int m = 0; m < RM; ++m) acc[m] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (int i = 0; i < n_it; ++i) {
       const int s = i % kFcStages;
-      if (!mbar_wait(&full[s], (unsigned)((i / kFcStages) & 1))) s_err = 1;
+      if (!__all_sync(0xffffffffu, mbar_wait(&full[s], (unsigned)((i / kFcStages) & 1), a.wait_limit))) {
+        s_err = 1;
+        break;   // the stage is not handed back: its copy may still be on its way
+      }
       const float4* t = reinterpret_cast<const float4*>(fc_raw + s * kTileBytes) + w * 4 * 32 + lane;
       float4 wv[4];
 #pragma unroll
@@ -181,7 +186,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   if (ks > 1) {
     // arrived when everything is pushed; waited for before the CTA leaves, so that nobody pushes to one that has
     cluster_arrive_relaxed();
-    if (tid < per && !cl_wait(&sums)) s_err = 1;
+    if (tid < per && !cl_wait(&sums, a.wait_limit)) s_err = 1;
   } else {
     __syncthreads();
   }
@@ -253,6 +258,7 @@ int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const v
   const size_t smem = smem_of(a.ks);
   if (smem > 220 * 1024) return 2;   // rows too long for the shared memory
   a.error = tc_error_word(device);
+  a.wait_limit = tc_wait_limit();
   switch (RM) {
     case 1: return fc_launch<1>(device, a, groups, smem, pdl, s);
     case 2: return fc_launch<2>(device, a, groups, smem, pdl, s);

@@ -451,6 +451,7 @@ int launch_matrix_memory(int device, DeviceState* st, int dtype, const MemoryArg
 int init_tc_attrs(int device);
 int tc_take_error();
 int* tc_error_word(int device);   // device address of the word that tc_take_error() reads
+unsigned tc_wait_limit();         // polls of a bounded wait: 2^22, or TSB200_WAIT_LIMIT (tests that make a wait run out)
 int64_t linear_workspace_bytes(int M, int K, int N);
 // Prompts of different lengths one after the other (no pad rows): `rows` of them; where[r] = (sequence, position) of row r, for
 // `listed` rows: those from `rows` on are positions whose values the append clears; starts[b]: first row of sequence b, starts[B] = rows.

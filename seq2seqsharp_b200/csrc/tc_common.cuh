@@ -184,7 +184,5 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn get_encode();       // cuTensorMapEncodeTiled, or null where the driver has none
-int* tc_error_word(int device);   // device address of the word that tc_take_error() reads
-unsigned tc_wait_limit();         // kTcSpin, or TSB200_WAIT_LIMIT polls (tests that make a wait run out)
 
 }  // namespace tsb

@@ -75,9 +75,9 @@ print("usable", float(torch.ones(4, device="cuda").sum()))
     assert "gave up waiting" in r.stdout and "usable 4.0" in r.stdout, r.stdout
 
 
-@pytest.mark.parametrize("rows", [1, 64, 100, 300])
-def test_linears_end_in_order_when_a_wait_runs_out(cuda, rows):
-    """The same for the tensor-core linears: one row and 64 on clusters, 100 on tiles of one CTA with K slices, 300 on pairs of CTAs.  Every warp gives up in its
+@pytest.mark.parametrize("rows,dtype", [(1, "16"), (64, "16"), (100, "16"), (300, "16"), (3, "32")])
+def test_linears_end_in_order_when_a_wait_runs_out(cuda, rows, dtype):
+    """The same for the linears: one fp16 row and 64 on clusters, 100 on tiles of one CTA with K slices, 300 on pairs of CTAs, fp32 rows on clusters.  Every warp gives up in its
     own place; copies and products in flight end before a CTA leaves its shared memory and TMEM, so the calls behind it are sound."""
     import os
     import subprocess
@@ -85,24 +85,25 @@ def test_linears_end_in_order_when_a_wait_runs_out(cuda, rows):
     code = """
 import torch
 from seq2seqsharp_b200 import _native as N
-M, K, n = %d, 11008, 8192
-W = torch.randn(K, n, device="cuda", dtype=torch.float16)
-Wp = torch.empty(N.lib().TSB200_PackedWeightBytes(N.F16, K, n), device="cuda", dtype=torch.uint8)
-x, y = torch.randn(M, K, device="cuda", dtype=torch.float16), torch.empty(M, n, device="cuda", dtype=torch.float16)
-ws = torch.empty(N.lib().TSB200_LinearPackedWorkspaceBytes(N.F16, M, K, n), device="cuda", dtype=torch.uint8)
+M, K, n, code = %d, 11008, 8192, N.F%s
+t = torch.float16 if code == N.F16 else torch.float32
+W = torch.randn(K, n, device="cuda", dtype=t)
+Wp = torch.empty(N.lib().TSB200_PackedWeightBytes(code, K, n), device="cuda", dtype=torch.uint8)
+x, y = torch.randn(M, K, device="cuda", dtype=t), torch.empty(M, n, device="cuda", dtype=t)
+ws = torch.empty(N.lib().TSB200_LinearPackedWorkspaceBytes(code, M, K, n), device="cuda", dtype=torch.uint8)
 torch.cuda.synchronize()
-N.call("TSB200_PackWeight", 0, N.F16, Wp.data_ptr(), W.data_ptr(), N.F16, K, n, None)
+N.call("TSB200_PackWeight", 0, code, Wp.data_ptr(), W.data_ptr(), code, K, n, None)
 N.call("TSB200_Synchronize", 0, None)
 for i in range(8):
-    N.call("TSB200_LinearPacked", 0, N.F16, y.data_ptr(), None, x.data_ptr(), None, None, None, -1, 0.0, Wp.data_ptr(), None, None, M, K, n, N.ACT_NONE, ws.data_ptr(), ws.numel(), None)
+    N.call("TSB200_LinearPacked", 0, code, y.data_ptr(), None, x.data_ptr(), None, None, None, -1, 0.0, Wp.data_ptr(), None, None, M, K, n, N.ACT_NONE, ws.data_ptr(), ws.numel(), None)
 try:
     N.call("TSB200_Synchronize", 0, None)
     print("silent")
 except N.TSB200Error as e:
     print(e)
 N.call("TSB200_Synchronize", 0, None)
-print("usable", torch.equal(W[:, :64] @ torch.eye(64, device="cuda", dtype=torch.float16), W[:, :64]), float(torch.ones(4, device="cuda").sum()))
-""" % rows
+print("usable", torch.equal(W.flip(1).flip(1), W), float(torch.ones(4, device="cuda").sum()))
+""" % (rows, dtype)
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=120, cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
                        env=dict(os.environ, TSB200_WAIT_LIMIT="1", TSB200_GEMV_MAXROWS="0"))
     assert r.returncode == 0, r.stderr
