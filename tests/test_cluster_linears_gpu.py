@@ -77,3 +77,9 @@ def test_weights_off_a_16_byte_boundary(cuda, dtype, M):
 @pytest.mark.parametrize("M,K,n", [(1, 8, 4), (1, 4096, 512), (2, 2048, 132), (3, 520, 2052), (4, 264, 1024), (7, 1024, 40000), (9, 4096, 128), (61, 136, 256)])
 def test_row_quads(cuda, M, K, n):
     check(M, K, n, torch.float16, (0, 1))
+
+
+# 65 to 128 rows and 6144 k or more: K slices, whose sums the last CTA of a tile adds; a slice that ends in half a step, ragged rows, both epilogues
+@pytest.mark.parametrize("M,K,n", [(65, 6144, 300), (100, 11008, 4096), (127, 6152, 130), (128, 8200, 2048)])
+def test_k_slices(cuda, M, K, n):
+    check(M, K, n, torch.float16, (0, 1))

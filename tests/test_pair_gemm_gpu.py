@@ -33,3 +33,17 @@ def test_outputs_with_other_companions(cuda, M, n):
     got = host(linear(x, W, b, N.ACT_GLU_NOACT, f32_out=True))
     big = max(1.0, float(np.abs(ref).max()))
     np.testing.assert_allclose(got, ref[:, 0::2] * ref[:, 1::2], atol=2 * tol * big + 1e-6)
+
+
+# chunks of 32 columns with the gate's activation (a loop of its own), and the element-wise form
+@pytest.mark.parametrize("M,K,n", [(130, 72, 320), (515, 264, 4096), (129, 40, 50)])
+def test_gated_products(cuda, M, K, n):
+    rng = np.random.default_rng(M)
+    x, W = dev(rng.standard_normal((M, K)).astype(np.float32), torch.float16), dev((rng.standard_normal((K, n)) * 0.05).astype(np.float32), torch.float16)
+    b = dev((rng.standard_normal(n) * 0.1).astype(np.float32), torch.float16)
+    ref = host(x).astype(np.float64) @ host(W).astype(np.float64) + host(b)
+    a, g = ref[:, 0::2], ref[:, 1::2]
+    want = a / (1.0 + np.exp(-a)) * g
+    tol = K * 2.0 ** -23 * float(np.abs(host(x)).max() * np.abs(host(W)).max()) + 1e-6      # of a sum; silu's slope is below 1.1, expf and the divide add 2^-21
+    big = max(1.0, float(np.abs(ref).max()))
+    np.testing.assert_allclose(host(linear(x, W, b, N.ACT_SWIGLU)), want, atol=(2.2 * tol + 2.0 ** -11 * big + 2.0 ** -21 * big) * big)
