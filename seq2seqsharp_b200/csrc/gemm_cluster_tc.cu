@@ -149,6 +149,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
       if (++s == S) s = 0, phase ^= 1;
     }
     if (lane == 0) s_asked = i;
+    named_arrive<1, 192>();
   } else if (w == 1) {
     // ---------------- products.  Instruction descriptor: fp32 accumulator, A MN-major, B K-major, N = NR, M = 128
     const uint32_t idesc = (1u << 4) | (Pair16<H>::kUmmaFormat << 7) | (Pair16<H>::kUmmaFormat << 10) | (1u << 15) | ((uint32_t)(NR >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    named_arrive<1, 160>();   // TMEM has been read
+    named_arrive<1, 192>();   // TMEM has been read
   }
   if (ks > 1) {
     // arrived when everything is pushed (a CTA that gave up has pushed too); waited for before the CTA leaves, so that nobody pushes to one that has
@@ -229,10 +230,12 @@ __global__ void __launch_bounds__(kLcThreads, 4) gemm_cluster_tc_kernel(const __
     if (*err) tc_wait_short(sums, 0);   // what is on its way here lands first
     cluster_wait();
   }
-  if (w == 0) tc_land(full, S, s_asked);
   if (w == 1) {
-    tc_wait_short(acc, 0);   // where a warp has given up, products may still be running
-    named_sync<1, 160>();
+    named_sync<1, 192>();
+    if (*err) {   // warp 0, 1 or one of those that read TMEM has given up: copies and products in flight end first (otherwise the products have waited for every
+      tc_land(full, S, s_asked);   // copy, and TMEM was read behind the last product)
+      tc_wait_short(acc, 0);
+    }
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");

@@ -151,18 +151,17 @@ __device__ __forceinline__ bool tc_try_wait(uint32_t bar, unsigned parity) {
   return ok != 0;
 }
 // Bounded; gives up early when another wait of the CTA has (*err), raises *err when it runs out itself.  For whole warps: their lanes poll for
-// themselves and may see a phase end, or the limit, at different polls, so the warp votes, and one answer sends all of it on or out of its loop
-// (the elected issue behind it needs all lanes).
+// themselves and may see a phase end, or the error, at different polls, so the warp votes on each, and one answer sends all of it on or out of
+// its loop (the elected issue behind it needs all lanes).
 __device__ __forceinline__ bool tc_wait_or(uint32_t bar, unsigned parity, volatile int* err, unsigned limit = kTcSpin) {
-  bool ok = tc_try_wait(bar, parity);
+  if (__all_sync(0xffffffffu, tc_try_wait(bar, parity))) return true;
 #pragma unroll 1
-  for (unsigned i = 1; !ok && i < limit; ++i) {
-    ok = tc_try_wait(bar, parity);
-    if (!ok && (i & 63) == 63 && *err) break;
+  for (unsigned i = 1; i < limit; ++i) {
+    if (__all_sync(0xffffffffu, tc_try_wait(bar, parity))) return true;
+    if ((i & 63) == 63 && __any_sync(0xffffffffu, *err != 0)) return false;
   }
-  ok = __all_sync(0xffffffffu, ok);
-  if (!ok) *err = 1;
-  return ok;
+  *err = 1;
+  return false;
 }
 __device__ __forceinline__ bool tc_wait_short(uint32_t bar, unsigned parity) {   // bounded, raises nothing
 #pragma unroll 1

@@ -19,15 +19,18 @@ HARNESS = r"""
 #define __forceinline__
 constexpr unsigned kTcSpin = 1u << 22;
 static int g_ready[32];                     // poll at which a lane sees the phase end; -1: never
-static thread_local int t_lane, t_poll;
+static thread_local int t_lane, t_poll, t_vote;
 static std::barrier<> g_meet(32);
-static std::atomic<unsigned> g_votes[2];
+static std::atomic<unsigned> g_votes[4096];
 static bool tc_try_wait(uint32_t, unsigned) { const int i = t_poll++; return g_ready[t_lane] >= 0 && i >= g_ready[t_lane]; }
-static bool __all_sync(unsigned, bool p) {
-  g_votes[0] += p ? 1u : 0u;
+static unsigned ballot(bool p) {
+  std::atomic<unsigned>& votes = g_votes[t_vote++];
+  votes += p ? 1u : 0u;
   g_meet.arrive_and_wait();
-  return g_votes[0] == 32u;
+  return votes;
 }
+static bool __all_sync(unsigned, bool p) { return ballot(p) == 32u; }
+static bool __any_sync(unsigned, bool p) { return ballot(p) != 0u; }
 %s
 int main(int argc, char** argv) {
   for (int i = 0; i < 32; ++i) g_ready[i] = atoi(argv[2 + i]);
