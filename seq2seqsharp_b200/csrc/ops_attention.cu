@@ -263,7 +263,13 @@ __device__ __forceinline__ void attn_finish(T* out, float* part, const float* sm
   }
 }
 
-template <typename T, int G, bool BOX>
+// Tokens of a lane group on their way at a time.  Decode: four, its few CTAs wait for memory (one fp32 sequence of 1000 tokens, 8 heads of 64,
+// 14.5 -> 12.0 us).  Prompts are a CTA per row and many waves, where CTAs per SM hide the loads: four cost 40 registers and up to 29 %, one gains
+// except for 16-bit rows of single heads.  us with none / one / four: fp32, 8 heads of 64, 8 x 200 88 / 85 / 98; 4 x 1000 753 / 772 / 847; 16 / 4 heads,
+// 2 x 500 188 / 186 / 243; one of 32 4.0 / 3.5 / 3.8; fp16, 2 x 500, 16 / 4 heads of 32 81 / 76 / 92; 8 single heads of 32 49 / 50 / 60, of 16 39 / 42 / 50.
+template <typename T, int G>
+constexpr int attn_ahead(bool prompt) { return !prompt ? 4 : (sizeof(T) == 2 && G == 1 ? 0 : 1); }
+template <typename T, int G, bool BOX, int AHEAD>
 __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
                                                             const T* q, int64_t q_rs,
                                                             const T* cK, const T* cV, int S, int H,
@@ -291,20 +297,21 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
   const T* Kb = cK + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
   const T* Vb = cV + ((int64_t)b * Hkv + kvh) * Tmax * hd + li * EPL;
   const int stride = nwarps * tpw, tb0 = t_beg + w * tpw;
-  // kAhead tokens of a lane group are on their way at any time, the first of them before the kernel in front has ended (tokens below T0)
-  constexpr int kAhead = 4;
-  Vec16<T> kv[kAhead], vv[kAhead];
+  // AHEAD tokens of a lane group are on their way at any time, the first of them before the kernel in front has ended (tokens below T0);
+  // 0: a token is asked for when it is its turn (attn_ahead)
+  constexpr int kSlots = AHEAD > 0 ? AHEAD : 1;
+  Vec16<T> kv[kSlots], vv[kSlots];
   auto fetch = [&](int u, int t) {
     kv[u].load(Kb + (int64_t)t * hd);
     vv[u].load(Vb + (int64_t)t * hd);
   };
 #pragma unroll
-  for (int u = 0; u < kAhead; ++u)
+  for (int u = 0; u < AHEAD; ++u)
     if (const int t = tb0 + u * stride + sub; t < min(t_end, T0)) fetch(u, t);
   if constexpr (BOX) cluster_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
 #pragma unroll
-  for (int u = 0; u < kAhead; ++u)
+  for (int u = 0; u < AHEAD; ++u)
     if (const int t = tb0 + u * stride + sub; t >= T0 && t < t_end) fetch(u, t);
 
   float qf[G][EPL];
@@ -324,22 +331,23 @@ __global__ void __launch_bounds__(kAttnThreads) attn_kernel(T* out, float* part,
 #pragma unroll
     for (int e = 0; e < EPL; ++e) acc[g][e] = 0.0f;
   }
-  for (int tb = tb0; tb < t_end; tb += kAhead * stride) {
+  for (int tb = tb0; tb < t_end; tb += kSlots * stride) {
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
+    for (int u = 0; u < kSlots; ++u) {
       // all lanes of the warp iterate together (shuffles below need full participation); `live` masks the tail
       const int t = tb + u * stride + sub;
       if (tb + u * stride >= t_end) break;
       const bool live = t < t_end;
       float kf[EPL], vf[EPL];
       if (live) {
+        if (AHEAD == 0) fetch(u, t);
         kv[u].get(kf);
         vv[u].get(vf);
       } else {
 #pragma unroll
         for (int e = 0; e < EPL; ++e) kf[e] = vf[e] = 0.0f;
       }
-      if (t + kAhead * stride < t_end) fetch(u, t + kAhead * stride);
+      if (AHEAD > 0 && t + AHEAD * stride < t_end) fetch(u, t + AHEAD * stride);
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         float d = 0.0f;
@@ -1093,10 +1101,11 @@ static int launch_attn_t(int device, DeviceState* st, T* out, const T* q, int64_
 #define TSB_ATTN(GG)                                                                                                                                        \
   do {                                                                                                                                                      \
     if (in_cluster)                                                                                                                                         \
-      TSB_CUDA(launch_clusters(attn_kernel<T, GG, true>, grid, dim3(kAttnThreads), smem + box_bytes, splits, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
+      TSB_CUDA(launch_clusters(attn_kernel<T, GG, true, attn_ahead<T, GG>(false)>, grid, dim3(kAttnThreads), smem + box_bytes, splits, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
                                Tmax, splits, scale, (int)(smem / 4)));                                                                                      \
     else                                                                                                                                                    \
-      TSB_CUDA(launch_k(attn_kernel<T, GG, false>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, Tmax, splits, scale, 0));  \
+      TSB_CUDA(launch_k(S == 1 ? attn_kernel<T, GG, false, attn_ahead<T, GG>(false)> : attn_kernel<T, GG, false, attn_ahead<T, GG>(true)>, grid, dim3(kAttnThreads), smem, s, out, ws, q, q_rs, cK, cV, S, H, Hkv, hd, T0, dT0, \
+                        Tmax, splits, scale, 0));                                                                                                           \
   } while (0)
   switch (G) {
     case 8: TSB_ATTN(8); break;
