@@ -120,7 +120,7 @@ __global__ void rope_append_kernel(T* q, const T* k, const T* v, int64_t q_rs,
   if (it < per_row) piece(it);
 }
 
-// The same for many rows of 16-byte pieces with a table (or without rotation): a CTA per row, a thread one piece, or one of every pass over a long row, the
+// The same for many rows of 16-byte pieces with a table (or without rotation): a CTA per row, a thread one piece, or every 256th of a long row, the
 // table by 16 bytes and what a piece is decided before its loads.  What bounds it: bytes and the warps that ask for them.  us, one element of
 // the table at a time -> here: 16384 rows of 48 heads of 64 (200 MB) 82 -> 61, 1024 rows 6.6 -> 5.5, 1273 packed rows of 48 heads of 128 11.2 ->
 // 9.2, 4096 of those 38 -> 28, 400 rows of 48 heads of 64 3.8 -> 3.4.  Two and four rows per thread at a time are slower (97 and 148 us: fewer warps).
@@ -1164,9 +1164,9 @@ static int launch_rope_append_t(int device, DeviceState* st, T* q, const T* k, c
   if constexpr (V > 2) {
     // from a few rows per SM on; fewer rows (a decode step's) are shared out below, and short rows several to a CTA
     if (listed > 2 * st->sm_count && per_row > 128 && (!use_rope || ((uintptr_t)tab % 16 == 0 && hd % 4 == 0))) {
-      // equal passes of up to 384 pieces
-      const int64_t passes = (per_row + 383) / 384;
-      const int threads = (int)((per_row + passes - 1) / passes + 31) / 32 * 32;
+      // Passes of 256 over a row of more than 384 pieces: eight such CTAs fill an SM whatever the row.  Without rotation, us: 4000 rows of 768 pieces
+      // 11.3, with 384 threads 12.8; 8000 of 640 16.7, in equal passes of 320 18.5; 4000 of 1056 12.9, in passes of 352 14.2.
+      const int threads = per_row > 384 ? 256 : (int)(per_row + 31) / 32 * 32;
       TSB_CUDA(launch_k(rope_append_rows_kernel<T, V>, dim3((unsigned)listed), dim3(threads), 0, s, q, k, v, q_rs, kv_rs, cK, cV, rows, pack ? pack->where : (const int2*)nullptr, S, H, Hkv,
                         hd, T0, dT0, Tmax, use_rope, tab));
       return 1;

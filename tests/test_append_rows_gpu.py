@@ -10,7 +10,7 @@ from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, GPT, GPTC
 pytestmark = pytest.mark.gpu
 
 
-# rows of 144, 384, 512, 544 (a second pass that is not full), 768 and 960 (three passes) pieces; lengths that differ lie one after the other with cleared positions behind each
+# rows of 144, 384, 512, 544 (a third pass that is not full), 768 and 960 (four passes) pieces; lengths that differ lie one after the other with cleared positions behind each
 @pytest.mark.parametrize("H,Hkv,hd,dtype", [(14, 2, 64, "float16"), (32, 8, 64, "float16"), (24, 4, 128, "float16"), (30, 2, 128, "float16"), (48, 6, 128, "float16"), (32, 8, 128, "float16"), (8, 4, 64, "float32")])
 @pytest.mark.parametrize("lens", [(140, 140, 140), (190, 33, 171)])
 def test_many_rows_against_few(cuda, H, Hkv, hd, dtype, lens):
