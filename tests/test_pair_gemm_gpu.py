@@ -6,6 +6,7 @@ import torch
 
 from seq2seqsharp_b200 import _native as N
 from tests.test_cluster_linears_gpu import check, linear
+from tests import layered_models as LM, test_layered_gpu as LG
 from tests.test_fused_gpu import dev, host
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +48,24 @@ def test_gated_products(cuda, M, K, n):
     tol = K * 2.0 ** -23 * float(np.abs(host(x)).max() * np.abs(host(W)).max()) + 1e-6      # of a sum; silu's slope is below 1.1, expf and the divide add 2^-21
     big = max(1.0, float(np.abs(ref).max()))
     np.testing.assert_allclose(host(linear(x, W, b, N.ACT_SWIGLU)), want, atol=(2.2 * tol + 2.0 ** -11 * big + 2.0 ** -21 * big) * big)
+
+
+@pytest.mark.parametrize("keep", ["attention", "gate", "experts"])
+def test_bf16_rows_of_one_layer(cuda, keep):
+    """One bf16 layer whose weights leave one mechanism: its projections, the gate times output plus residual, the experts' clamped gated products; 300 rows at once
+    and in portions that other kernels take."""
+    cfg = LM.config([LM.layer(3, 16, 8, 16, 24, scale=1.5, experts=5 if keep == "experts" else None, top=2, ff=96, limit=0.5)], 256, 67, groups=4, taps=4)
+    w = LM.weights(cfg, 5)
+    w["l0.canon1"][:] = 0.0
+    if keep != "gate":
+        w["l0.rg1"][:] = 0.0
+        w["l0.rg1.b"][:] = 8.0
+    if keep == "experts":
+        w["l0.mix.o"][:] = 0.0
+    ids = LM.tokens(cfg, 300)
+    want = LM.oracle(cfg, w).forward(ids)
+    g = LG.engine(cfg, w, "bfloat16")
+    for cuts in (None, [129, 171], [64] * 5, [100] * 3):
+        assert LM.rel(LG.score(g, ids, cuts=cuts), want) < LM.TOL["bfloat16"], cuts
+    g.CheckGuards()
+    g.close()

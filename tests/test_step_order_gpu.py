@@ -3,8 +3,9 @@ before its products (the norm of fp32 rows): against engines that do neither."""
 import numpy as np
 import pytest
 
-from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, GPT, GPTConfig, MultiHeadAttentionTypeEnums, NormEnums, PositionEmbeddingEnums,
+from seq2seqsharp_b200.gpt import (ActivateFuncEnums, DecodingOptions, DecodingStrategyEnums, GPT, GPTConfig, MultiHeadAttentionTypeEnums, NormEnums, PositionEmbeddingEnums,
                                    synthetic_weights)
+from tests import gunuvik_models as GM, layered_models as LM, test_gunuvik_gpu as GG, test_layered_gpu as LG
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,37 @@ def test_fp32_rows_normed_by_the_linear(cuda, oracle, monkeypatch, d, H, B, norm
     for ids in fed:
         ref = orc.step(ids[:, None])[0]
     assert np.abs(logits[0] - ref).max() <= 1e-3 * np.abs(ref).max()                  # the bound of the token loop's tests
+
+
+def steps_from(g, ids, at, n):
+    """Logits of positions at .. at + n - 1: a prompt of `at` tokens, then n steps."""
+    opts, rows = DecodingOptions(DecodingStrategy=DecodingStrategyEnums.GreedySearch), []
+    g.Reset()
+    g.SlotLogits(0, ids[:at], [])
+    for t in ids[at:at + n]:
+        g.StepHost([t], opts)
+        rows.append(g.Logits(want_probs=False)[0][0])
+    return rows
+
+
+# stages of 32 cached rows: the new position opens one, closes one, or lies in its middle
+@pytest.mark.parametrize("at", [1, 31, 32, 33, 63, 64, 65, 95, 96, 127, 128, 129, 191, 192])
+def test_the_newest_row_of_the_latent_cache(cuda, at):
+    """The token on which the answer hangs is the first that is decoded: its own step reads the row that the launch in front has appended, the next ones read it early."""
+    cfg, w, ids = LG._needle(at=at)
+    want = LM.oracle(cfg, w).forward(ids)[at:at + 4]
+    g = LG.engine(cfg, w, "bfloat16")
+    assert LM.rel(steps_from(g, ids, at, 4), want) < LM.TOL["bfloat16"]
+    g.close()
+
+
+# stages of 64; windows that have not begun to leave rows out, do so at this step, and did before; first rows that are kept in front of them
+@pytest.mark.parametrize("window,keep", [(16, 4), (64, 0), (65, 17), (130, 1), (5, 70)])
+def test_the_newest_row_of_grouped_attention(cuda, window, keep):
+    n = 210
+    for at in sorted({1, 15, 16, 63, 64, 65, 127, 128, 129, window - 1, window, window + 1, keep, keep + 1, 192} - {0}):
+        cfg, w, ids = GM.needle(at, n, window, keep, layers=2)
+        want = GM.Expected(cfg, w, ids, "bfloat16")
+        g = GG.engine(cfg, w, "bfloat16")
+        assert want.worst(steps_from(g, ids, at, 4), slice(at, at + 4)) < 1, at
+        g.close()
