@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
   __shared__ int s_err;
 
   const int tid = threadIdx.x, lane = tid & 31, w = warp_index();
-  const int n_tile = blockIdx.x, m_tile = blockIdx.y;
+  const int n_tile = blockIdx.x;   // one tile of rows
   const int k_total = (a.K + kBK - 1) / kBK;
   const int k_per = (k_total + a.ksplit - 1) / a.ksplit;
   const int k_begin = blockIdx.z * k_per;
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
       const bool two = (k_begin + asked) * 2 + 1 < a.KB;  // the last 64-k block of an odd tile count has one packed tile only
       const uint32_t bar = full + s * 8, dB = sB + s * kBBytes;
       tc_mbar_expect_el(bar, kABytes + (two ? 16384 : 8192));
-      tma_load_2d_el(sA + s * kABytes, &mapA, (k_begin + asked) * kBK, m_tile * kBM, bar);
+      tma_load_2d_el(sA + s * kABytes, &mapA, (k_begin + asked) * kBK, 0, bar);
       tc_bulk_g2s_el(dB, wsrc, 8192, bar);
       if (two) tc_bulk_g2s_el(dB + 8192, wsrc + 16384, 8192, bar);
       if (++s == kTcStages) s = 0, phase ^= 1;
@@ -330,10 +330,10 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
     const int q = w - 4;
     const bool ok = tc_wait_or(acc_ready, 0, err, a.wait_limit);
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const int row = m_tile * kBM + q * 32 + lane;
+    const int row = q * 32 + lane;
     const int n0 = n_tile * kBN;
     const bool live = ok && row < a.M;
-    const int n_live = ok ? min(32, a.M - (m_tile * kBM + q * 32)) : 0;
+    const int n_live = ok ? min(32, a.M - q * 32) : 0;
     float* stage = reinterpret_cast<float*>(smem) + q * kStageFloats;   // every product has read its operands
     const size_t Npad = (size_t)gridDim.x * kBN;
     const TcLane at = tc_lane(a, row - lane, n0);
@@ -360,10 +360,9 @@ __global__ void __launch_bounds__(kTcThreads, kTcStages == 3 ? 2 : 1) gemm_tc_ke
       __threadfence();
       named_sync<1, 128>();  // the four epilogue warps
       if (w == 4 && lane == 0) {
-        const unsigned int tile = blockIdx.y * gridDim.x + blockIdx.x;
-        const unsigned int prev = atomicAdd(&a.counters[tile], 1u);
+        const unsigned int prev = atomicAdd(&a.counters[n_tile], 1u);
         s_last = (prev == (unsigned int)(a.ksplit - 1));
-        if (s_last) a.counters[tile] = 0u;
+        if (s_last) a.counters[n_tile] = 0u;
       }
       named_sync<1, 128>();
       if (s_last) {
@@ -929,26 +928,17 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
   a.Wp = reinterpret_cast<const unsigned char*>(Wp);
   a.wait_limit = tc_wait_limit();
   a.kind = tc_kind(N, ep);
-  {
-    static int pers = -1;
-    if (pers < 0) {
-      const char* e = getenv("TSB200_TC_PERSISTENT");  // "0": one 128 x 128 tile per CTA for every M (A/B measurements)
-      pers = (e && e[0] == '0') ? 0 : 1;
-    }
-    if (pers && M > kBM) return launch_pair(device, st, dtype, mapA, a, s);
-  }
-  dim3 grid((N + kBN - 1) / kBN, (M + kBM - 1) / kBM, 1);
-  TSB_CHECK(grid.y <= 65535, "gemm_tc: too many row tiles");
+  if (M > kBM) return launch_pair(device, st, dtype, mapA, a, s);
+  dim3 grid((N + kBN - 1) / kBN, 1, 1);
   // few output tiles (decode-sized M): share each tile's K range among several CTAs so that all SMs stream weights
   a.ksplit = 1;
   {
-    const int64_t tiles = (int64_t)grid.x * grid.y;
+    const int64_t tiles = grid.x;
     const int k_total = (K + kBK - 1) / kBK;
-    // Only with a single row tile (more rows come here only for an A/B measurement).
-    // And only for long K: a slice saves its part of 0.37 us per 64 k of a tile alone, and costs the last arriver 2 to 4 us to add.  100 rows
+    // Only for long K: a slice saves its part of 0.37 us per 64 k of a tile alone, and costs the last arriver 2 to 4 us to add.  100 rows
     // with slices / without: 4096 x 4096 67.0 / 27.1 us, 2048 x 3072 32.1 / 17.4, 8192 x 2048 33.4 / 47.  No more slices than SMs, which
     // keeps the deep rings (100 x 11008 x 4096: six slices of three stages 76.9, four of six stages 36.6).
-    if (grid.y == 1 && k_total >= 96 && ws) {
+    if (k_total >= 96 && ws) {
       int ks = (int)(st->sm_count / tiles);
       if (ks > 6) ks = 6;
       if (ks > 1) {
@@ -965,7 +955,7 @@ int launch_gemm_tc(int device, DeviceState* st, int dtype, const void* x, const 
       }
     }
   }
-  const bool deep = (int64_t)grid.x * grid.y * grid.z <= st->sm_count;
+  const bool deep = (int64_t)grid.x * grid.z <= st->sm_count;
   auto k = dtype == TSB200_BF16 ? (deep ? gemm_tc_kernel<__nv_bfloat16, kTcDeepStages> : gemm_tc_kernel<__nv_bfloat16, kTcStages>)
                                 : (deep ? gemm_tc_kernel<__half, kTcDeepStages> : gemm_tc_kernel<__half, kTcStages>);
   TSB_CUDA(launch_k(k, grid, dim3(kTcThreads), tc_smem(deep ? kTcDeepStages : kTcStages), s, mapA, a));

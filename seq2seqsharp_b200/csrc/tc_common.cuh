@@ -31,17 +31,6 @@ __device__ __forceinline__ bool tc_mbar_wait(uint64_t* bar, unsigned parity) {
   }
   return false;
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(s_u32(dst)),
-      "l"(map), "r"(s_u32(bar)), "r"(c0), "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tc_bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(s_u32(dst)),
-               "l"(src), "r"(bytes), "r"(s_u32(bar))
-               : "memory");
-}
 // Shared-memory matrix descriptor (sm_100 format): start address, leading / stride byte offsets in 16-byte units,
 // version 1, 128-byte swizzle.
 __device__ __forceinline__ uint64_t make_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
