@@ -90,10 +90,19 @@ __device__ __forceinline__ void cluster_sync() {
 #endif
 
 // ---- programmatic dependent launch ------------------------------------------------------------------
-// Kernels of a decode step are chained with programmatic stream serialization: a kernel may become resident while its
-// predecessor is still running.  It calls pdl_wait() before it touches anything an earlier kernel wrote (a no-op when
-// the launch carried no such attribute) and pdl_trigger() as early as possible so that its own successor can be
-// scheduled.  The engine switches the attribute on for the launches it issues (PdlScope); stand-alone ops never use it.
+// Kernels of a decode step, and of a prompt pass on one GPU, are chained with programmatic stream serialization: a kernel may become
+// resident while its predecessor is still running.  The engine switches the attribute on for the launches it issues (PdlScope); stand-alone
+// ops never use it, and without it both calls are no-ops.
+//  * Every kernel launched with the attribute calls pdl_wait() in every CTA that does not leave at once, before it touches what a kernel
+//    of the step or pass in front of it may have written; it then knows that all of them have ended.
+//  * pdl_trigger() as early as possible, so that the successor can be scheduled; a kernel with TMEM first allocates it, or its successor's
+//    CTA on the same SM might take the columns it is about to ask for and keep them until this kernel has ended.
+//  * The FIRST kernel of a step or pass (embed_kernel, in every engine) waits BEFORE it triggers.  So nothing behind it starts before all that
+//    was enqueued in front of the step or pass has ended, and every later kernel may read before its pdl_wait() what no kernel of the step or
+//    pass writes: weights, biases, the rotation table, row tables copied by the host, cached rows of earlier positions, and the step state
+//    (which commit_kernel, the last one, writes).  That is relied on in ops_attention.cu, ops_grouped.cu, ops_latent.cu (cached rows, state),
+//    cluster_sums.cuh (ClAhead::start: biases, state, rotation) and attn_prefill_tc.cu (starts).  A kernel put in front of embed_kernel has to
+//    keep that order, and one that changes cached rows or the state has to stay outside of the step.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

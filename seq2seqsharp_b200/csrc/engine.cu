@@ -270,11 +270,12 @@ struct Gpt {
   int step_ev_n = 0;
   int* pin_ids = nullptr;  // pinned host staging for TSB200_GptStepHost
   int* err_flag = nullptr; // device word raised by a kernel whose bounded wait ran out
-  bool pdl = true;         // programmatic dependent launch between the kernels of a decode step
+  bool pdl = true;         // programmatic dependent launch between the kernels of a decode step or prompt pass
   // persistent decode-step kernel (decode_stack.cu): the program of operations and its scratch
   bool use_stack = true;
   bool fuse_step = true;       // per-operation path, up to 64 rows (fp32: 8): RoPE + cache append in the epilogue of the q | k | v projection
-                               // (TSB200_FUSED_STEP=0: a launch of its own, e.g. for a checker engine); the norms are launches either way
+                               // (TSB200_FUSED_STEP=0: a launch of its own, e.g. for a checker engine).  Norms are launches, but for fp32 rows that the
+                               // linear behind them norms itself (launch_gemv_cluster_f32)
   // One GPU: one launch per operation at every batch (linears on clusters; 7B-class fp16, one sequence: 2.69 ms per step against 3.20 with the
   // stream-K persistent kernel and 3.10 with the owner-partitioned one; tiny fp32 model: 0.18 ms against 0.30).
   // Tensor-parallel engines keep the persistent kernels (the exchange lives there).
@@ -764,8 +765,8 @@ static std::vector<size_t> parts_layout(Gpt* g) {   // two engines with the same
 }
 
 // One linear layer of the engine on packed weights.  With `ng` the input is the fp32 residual stream and the layer's
-// LayerNorm / RMSNorm comes first, as a launch of its own into g->h (inside the FMA streaming GEMV where
-// TSB200_GEMV_MAXROWS asks for that kernel).
+// LayerNorm / RMSNorm comes first: inside the linear for the fp32 rows that launch_gemv_cluster_f32 norms (and in the FMA streaming GEMV where
+// TSB200_GEMV_MAXROWS asks for that kernel), otherwise as a launch of its own into g->h.
 static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid, const void* ng, const void* nb, void* h_tmp,
                          const void* Wp, int K, int N, const Epilogue& ep) {
   const TSB200GptConfig& c = g->c;
