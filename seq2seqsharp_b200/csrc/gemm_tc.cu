@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(kPThreads, 1) gemm_tc_grouped_kernel(const __g
 // of B into its shared memory, the leader's one thread issues the products for both, each CTA's TMEM receives its own 128 rows.
 // What bounds it: the tensor pipe, from about 4 waves on the power limit (16384 x 2048 x 16384 751 us = 1464 TFLOP/s, cuBLAS 749); an SM takes
 // in about 64 bytes per clock from L2, a tile of one CTA needs 94 at full tensor rate (128 x 256) or 128 (128 x 128), a pair 64.  A step of
-// 64 k takes 0.25 us (470 clocks) for 256 columns and 0.16 for 128.  With one 128 x 128 tile per CTA, or 128 x 256 on a CTA of its own,
+// 64 k whose operands are there takes 470 clocks for 256 columns and 296 for 128; in whole launches, operands from memory, 0.34 and 0.19 us (launch_pair).  With one 128 x 128 tile per CTA, or 128 x 256 on a CTA of its own,
 // products issued by a thread and the epilogue's loads where they are needed, us before -> now: 1024 x 8192 x 2048 with residual 68 -> 30,
 // 1024 x 2048 x 16384 gated 62 -> 51, 1273 x 4096 x 4096 with residual 111 -> 42, 1273 x 11008 x 4096 166 -> 100, 16384 x 2048 x 2048 with
 // residual 333 -> 112, 256 x 11008 x 4096 80 -> 36.
@@ -883,8 +883,8 @@ int launch_gemm_tc_grouped(int device, DeviceState* st, int dtype, const void* x
   return check_launch("gemm_tc_grouped");
 }
 
-// Pairs of CTAs.  Tiles of 256 columns or of 128, whichever is done first: whole waves of pairs times 64-k steps (0.33 and 0.19 us, measured over
-// launches of one to four waves) and the last tile's epilogue (3.3 and 1.6 us).  The estimate names the faster one at 31 of 36 sizes of 160 to
+// Pairs of CTAs.  Tiles of 256 columns or of 128, whichever is done first: whole waves of pairs times 64-k steps (0.33 and 0.19 us; four waves of
+// 1024 x 1024 .. 4096 x 18944 0.34, of x 9472 0.19) and the last tile's epilogue (3.3 and 1.6 us).  The estimate names the faster one at 31 of 36 sizes of 160 to
 // 16384 rows and costs 3 % at most at the others.
 static int launch_pair(int device, DeviceState* st, int dtype, const CUtensorMap& mapA, const TcArgs& a, cudaStream_t s) {
   const int pairs = st->sm_count / 2, m_tiles = (a.M + 2 * kBM - 1) / (2 * kBM), k_total = (a.K + kBK - 1) / kBK;

@@ -12,8 +12,11 @@ namespace tsb {
 
 constexpr int kFcThreads = 288, kFcStages = 5;
 // Rows of up to 1024 are normed here instead of by a launch in front, which takes 2.1 us of a step's chain of launches; reading the whole rows
-// and their two sums costs this launch about 0.9 us (512 wide, one row: a 128-token request 22.4 -> 20.4 ms).  Longer rows would be read by every CTA for more than that.
+// and their two sums costs this launch about 0.9 us for one row (512 wide: a 128-token request 22.4 -> 20.4 ms).  Longer rows would be read by every
+// CTA for more than that, and so are 5 to 8 rows of 512 and more.  us per step of six layers, normed here / by a launch: 512 wide, 1 row 119 / 132,
+// 4 143 / 157, 5 221 / 218, 8 227 / 225; 1024 wide, 1 row 170 / 187, 4 241 / 254, 8 390 / 367; 448 wide, 5 rows 179 / 185, 8 209 / 217; 256 wide, 8 146 / 152.
 constexpr int kFcNormRegs = 8;   // float4 of a row per lane
+static bool fc_norms(int M, int K) { return K % 4 == 0 && K <= kFcNormRegs * 128 && (M <= 4 || K < 512); }
 
 struct FcArgs {
   const float* x;
@@ -237,7 +240,7 @@ static int fc_launch(int device, const FcArgs& a, int groups, size_t smem, bool 
 int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
                             const RopeFuse* rope, const RowNorm* norm) {
   if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
-  if (norm && (K % 4 != 0 || K > kFcNormRegs * 128 || ((uintptr_t)x % 16) != 0)) return 2;
+  if (norm && (!fc_norms(M, K) || ((uintptr_t)x % 16) != 0)) return 2;
   FcArgs a{};
   if (norm) {
     a.norm = norm->type == 0 ? 2 : 1;

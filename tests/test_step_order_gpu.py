@@ -33,8 +33,8 @@ def test_cached_rows_around_the_new_position(cuda, hd, dtype, lens):
         assert np.abs(stepped - whole).max() <= (8 * 2.0 ** -11 if dtype == "float16" else 1e-5) * np.abs(whole).max()
 
 
-# 64 to 1024: normed by the linears (a lane's registers full at 1024); 1056: by a launch
-@pytest.mark.parametrize("d,H,B,norm", [(64, 1, 1, "LayerNorm"), (64, 1, 8, "RMSNorm"), (416, 13, 2, "LayerNorm"), (512, 8, 1, "LayerNorm"), (512, 8, 5, "RMSNorm"),
+# 64 to 1024: normed by the linears (a lane's registers full at 1024), 5 rows and more only below 512; 1056: by a launch
+@pytest.mark.parametrize("d,H,B,norm", [(64, 1, 1, "LayerNorm"), (64, 1, 8, "RMSNorm"), (416, 13, 2, "LayerNorm"), (512, 8, 1, "LayerNorm"), (448, 7, 8, "LayerNorm"), (512, 8, 5, "RMSNorm"), (1024, 16, 4, "RMSNorm"),
                                         (1024, 16, 8, "LayerNorm"), (1056, 33, 3, "LayerNorm")])
 def test_fp32_rows_normed_by_the_linear(cuda, oracle, monkeypatch, d, H, B, norm):
     cfg = GPTConfig(L=2, d=d, H=H, hd=d // H, F=192, V=515, norm=getattr(NormEnums, norm), act=ActivateFuncEnums.ReLU, pe=PositionEmbeddingEnums.RoPE,
