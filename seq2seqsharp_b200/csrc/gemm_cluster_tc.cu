@@ -281,8 +281,9 @@ static int lc_run(int device, DeviceState* st, int dtype, const void* x, int row
   if (!enc) return 2;
   a.KB = (K + 31) / 32;
   // K ranges while all CTAs are resident at once (two per SM), of at least two steps of 64 k each: more copies in flight and a shorter chain
-  // per CTA.  Against one CTA per SM (more room for the next launch): 16384-token decode of the 1B-class model 22.3 / 23.2 ms, 7B-class
-  // step 2.68 / 2.98 ms, 64 sequences 5.33 / 5.57 ms.
+  // per CTA.  Against one CTA per SM (fewer ranks, fewer pushes, more room for the next launch), ms of whole calls: 32 steps of one row of the 7B-class
+  // model 71.5 / 76.6, 16 of its 64 rows 60.1 / 63.0, 16 of four rows of the 1B-class one after 16384 tokens 17.2 / 17.4; 8 rows of 768 and 32 of
+  // 2048 the same (21.6, 28.6): the rule does not look at the rows.
   const int KP = (a.KB + 1) / 2;
   a.ks = 1;
   while (a.ks < 8 && (int64_t)groups * a.ks * 2 <= 2 * st->sm_count && KP / (a.ks * 2) >= 2) a.ks *= 2;
