@@ -799,7 +799,7 @@ static int engine_linear(Gpt* g, int rows, const void* x_T, const float* x_resid
   g->lin_syms_used = true;   // these kernels report a wait that ran out through their own error symbols
   prof_begin(g, KC_LINEAR);
   int r = 2;
-  if (dt == TSB200_F32 && rows <= 8) r = launch_gemv_cluster_f32(dev, g->st, (const float*)x_T, Wp, rows, K, N, ep, g->pdl, g->s);
+  if (dt == TSB200_F32 && rows <= 8) r = launch_gemv_cluster_f32(dev, g->st, (const float*)x_T, Wp, rows, K, N, ep, g->pdl, g->s, nullptr, nullptr, c.d);
   if (r == 2) r = launch_linear(dev, g->st, dt, x_T, Wp, rows, K, N, ep, g->lin_ws, g->lin_ws_bytes, g->s, true);
   if (r == 1) prof_end(g, KC_LINEAR);
   return r == 1;
@@ -1042,7 +1042,7 @@ static int enqueue_forward(Gpt* g, int B, int S, int T0, bool use_state, int spl
         PROF(KC_NORM, launch_norm_residual(dev, g->st, dt, g->h, g->x, nullptr, L.n1_g, c.norm_type == 0 ? L.n1_b : nullptr, c.norm_type, c.eps, rows, d, g->s));
         prof_begin(g, KC_LINEAR);
         r = dt == TSB200_F16 ? launch_gemm_cluster_tc(dev, g->st, dt, g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf)
-                                       : launch_gemv_cluster_f32(dev, g->st, (const float*)g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf);
+                                       : launch_gemv_cluster_f32(dev, g->st, (const float*)g->h, L.wqkv, rows, d, g->Nqkv, ep, g->pdl, g->s, &rf, nullptr, d);
         if (r == 0) return 0;
       }
       g->lin_syms_used = true;

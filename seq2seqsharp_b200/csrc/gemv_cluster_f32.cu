@@ -14,9 +14,9 @@ constexpr int kFcThreads = 288, kFcStages = 5;
 // Rows of up to 1024 are normed here instead of by a launch in front, which takes 2.1 us of a step's chain of launches; reading the whole rows
 // and their two sums costs this launch about 0.9 us for one row (512 wide: a 128-token request 22.4 -> 20.4 ms).  Longer rows would be read by every
 // CTA for more than that, and so are 5 to 8 rows of 512 and more.  us per step of six layers, normed here / by a launch: 512 wide, 1 row 119 / 132,
-// 4 143 / 157, 5 221 / 218, 8 227 / 225; 1024 wide, 1 row 170 / 187, 4 241 / 254, 8 390 / 367; 448 wide, 5 rows 179 / 185, 8 209 / 217; 256 wide, 8 146 / 152.
+// 4 143 / 157, 5 221 / 195, 8 227 / 198; 1024 wide, 1 row 170 / 187, 4 241 / 254, 8 390 / 283; 448 wide, 5 rows 179 / 185, 8 209 / 217; 256 wide, 8 146 / 152.
 constexpr int kFcNormRegs = 8;   // float4 of a row per lane
-static bool fc_norms(int M, int K) { return K % 4 == 0 && K <= kFcNormRegs * 128 && (M <= 4 || K < 512); }
+static bool fc_norms(int M, int K) { return K > 0 && K % 4 == 0 && K <= kFcNormRegs * 128 && (M <= 4 || K < 512); }
 
 struct FcArgs {
   const float* x;
@@ -35,8 +35,13 @@ struct FcArgs {
 // dynamic shared memory: ring | sums of the cluster [M * 32 groups][4] | rows of x over the CTA's range
 static size_t fc_smem(int RM, int tiles) { return (size_t)kFcStages * kTileBytes + (size_t)RM * 512 + (size_t)RM * tiles * 128; }
 
-template <int RM>
-__global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) {
+// 5 to 8 rows: nine warps of more than 96 registers are one CTA per SM (a quarter of the register file holds four of 112).  That suits models of less
+// than 512, which norm their rows here and whose launches have CTAs for a part of the SMs; of wider models half the launches would take two waves (8 x
+// 1024 x 4096 19.7 us, now 10.7; a step of six layers, 8 rows of 1024, 363 and 281).  Those have no norm in their kernel and ask for what the epilogue
+// reads behind the products instead of in front of the wait (kLate): 93 registers.
+template <int RM, bool NORM>
+__global__ void __launch_bounds__(kFcThreads, RM == 8 && !NORM ? 2 : 0) gemv_cluster_f32_kernel(FcArgs a) {
+  constexpr bool kLate = RM == 8 && !NORM;
   extern __shared__ __align__(1024) unsigned char fc_raw[];
   __shared__ uint64_t full[kFcStages], empty[kFcStages], sums;
   __shared__ float2 stat[8];   // mean and divisor of a row
@@ -67,7 +72,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     }
   __syncwarp();
   float g0 = 0.0f, b0 = 0.0f;   // gain and shift of the first element this thread norms
-  if (a.norm) {
+  if (NORM && a.norm) {
     const int k = t0 * 32 + tid % (n_it * 32);
     if (k < a.K) {
       g0 = a.gamma[k];
@@ -77,7 +82,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   ClAhead<float> ahead;
   const int per = M * 32 / ks;   // groups of four columns this CTA finishes: at most 256, one per thread
   const int c = group * 128 + ((rank * per + tid) & 31) * 4, row = (rank * per + tid) >> 5;
-  if (tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
+  if (!kLate && tid < per) ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
   if (ks > 1) cluster_sync();   // the other CTAs exist before anything is pushed to them
   pdl_wait();
   if (w == 8) {
@@ -96,9 +101,9 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       for (int j = max(0, i - kFcStages); j < i; ++j) mbar_wait(&full[j % kFcStages], (unsigned)((j / kFcStages) & 1));
     }
   } else {
-    if (tid < per) ahead.first(a.ep, a.kind, a.N, c, row, M, a.rope);
+    if (!kLate && tid < per) ahead.first(a.ep, a.kind, a.N, c, row, M, a.rope);
     const int kc = n_it * 32;
-    if (a.norm) {
+    if (NORM && a.norm) {
       // A warp takes the statistics of a row (one row: every warp, so that nobody waits), the arithmetic of the norm kernels
       if (RM == 1 || w < M) {
         const float4* xr = reinterpret_cast<const float4*>(a.x + (size_t)(RM == 1 ? 0 : w) * a.K);
@@ -129,7 +134,7 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
     for (int i = tid; i < RM * kc; i += 256) {
       const int m = i / kc, k = t0 * 32 + i % kc;
       float v = m < M && k < a.K ? a.x[(size_t)m * a.K + k] : 0.0f;
-      if (a.norm && m < M && k < a.K) {
+      if (NORM && a.norm && m < M && k < a.K) {
         v = (i == tid ? g0 : a.gamma[k]) * ((v - stat[m].x) / stat[m].y);
         if (a.beta) v += i == tid ? b0 : a.beta[k];
       }
@@ -163,6 +168,10 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[s]);
+    }
+    if (kLate && tid < per) {
+      ahead.start(a.ep, a.kind, a.N, c, row, M, a.rope);
+      ahead.first(a.ep, a.kind, a.N, c, row, M, a.rope);
     }
     named_sync<1, 256>();   // every tile is read: the ring holds the warps' sums now
     float4* part = reinterpret_cast<float4*>(fc_raw);   // [warp][row][32 groups]
@@ -210,11 +219,12 @@ __global__ void __launch_bounds__(kFcThreads) gemv_cluster_f32_kernel(FcArgs a) 
   if (lane == 0 && *(volatile int*)&s_err && a.error) *a.error = 1;   // the warp that gave up, at least, sees it
 }
 
-template <int RM>
+constexpr size_t kFcAlone = 116 * 1024;   // more than half of an SM's shared memory
+template <int RM, bool NORM>
 static int fc_launch(int device, const FcArgs& a, int groups, size_t smem, bool pdl, cudaStream_t s) {
   static bool done[kMaxDevices] = {};
   if (!done[device]) {
-    TSB_CUDA(cudaFuncSetAttribute(gemv_cluster_f32_kernel<RM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
+    TSB_CUDA(cudaFuncSetAttribute(gemv_cluster_f32_kernel<RM, NORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 224 * 1024));
     done[device] = true;
   }
   cudaLaunchConfig_t cfg{};
@@ -230,15 +240,28 @@ static int fc_launch(int device, const FcArgs& a, int groups, size_t smem, bool 
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
+  if constexpr (RM == 8 && !NORM) {
+    // Where two CTAs fit an SM, a small launch's clusters lie two CTAs to an SM and leave others idle: here they get an SM each while all clusters are
+    // resident that way (a step of six layers, 8 rows of 512 217 us, so 198; of 768 268 / 234).
+    static int fit[kMaxDevices][9] = {};   // clusters of so many CTAs, plus one; 0: not asked yet
+    if (!fit[device][a.ks]) {
+      int n = 0;
+      cfg.dynamicSmemBytes = kFcAlone;
+      cfg.numAttrs = 1;
+      TSB_CUDA(cudaOccupancyMaxActiveClusters(&n, gemv_cluster_f32_kernel<RM, NORM>, &cfg));
+      fit[device][a.ks] = n + 1;
+    }
+    cfg.dynamicSmemBytes = smem < kFcAlone && groups < fit[device][a.ks] ? kFcAlone : smem;
+  }
   cfg.numAttrs = (pdl && pdl_enabled()) ? 2 : 1;
-  TSB_CUDA(cudaLaunchKernelEx(&cfg, gemv_cluster_f32_kernel<RM>, a));
+  TSB_CUDA(cudaLaunchKernelEx(&cfg, gemv_cluster_f32_kernel<RM, NORM>, a));
   count_launch(device);
   return check_launch("gemv_cluster_f32");
 }
 
 // 1 ok, 0 error, 2 shape not handled (the caller takes another kernel)
 int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
-                            const RopeFuse* rope, const RowNorm* norm) {
+                            const RopeFuse* rope, const RowNorm* norm, int norm_width) {
   if (M < 1 || M > 8 || ((uintptr_t)Wp % 16) != 0) return 2;
   if (norm && (!fc_norms(M, K) || ((uintptr_t)x % 16) != 0)) return 2;
   FcArgs a{};
@@ -263,10 +286,11 @@ int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const v
   a.error = tc_error_word(device);
   a.wait_limit = tc_wait_limit();
   switch (RM) {
-    case 1: return fc_launch<1>(device, a, groups, smem, pdl, s);
-    case 2: return fc_launch<2>(device, a, groups, smem, pdl, s);
-    case 4: return fc_launch<4>(device, a, groups, smem, pdl, s);
-    default: return fc_launch<8>(device, a, groups, smem, pdl, s);
+    case 1: return fc_launch<1, true>(device, a, groups, smem, pdl, s);
+    case 2: return fc_launch<2, true>(device, a, groups, smem, pdl, s);
+    case 4: return fc_launch<4, true>(device, a, groups, smem, pdl, s);
+    default:   // one kernel for all launches of a step: two in turn would each fetch their code anew (8 rows of 448: 223 us a step against 209)
+      return norm || fc_norms(M, norm_width) ? fc_launch<8, true>(device, a, groups, smem, pdl, s) : fc_launch<8, false>(device, a, groups, smem, pdl, s);
   }
 }
 

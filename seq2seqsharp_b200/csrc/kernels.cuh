@@ -274,9 +274,9 @@ int launch_gemm_stream_mma_norm(int device, DeviceState* st, const float* x32, c
 // 1..64 rows of a 16-bit type, the K ranges of 128 columns on the CTAs of a cluster (gemm_cluster_tc.cu); 1 ok, 0 error, 2 not handled
 int launch_gemm_cluster_tc(int device, DeviceState* st, int dtype, const void* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
                            const RopeFuse* rope = nullptr);
-// 1..8 fp32 rows in the same manner on the CUDA cores (gemv_cluster_f32.cu)
+// 1..8 fp32 rows in the same manner on the CUDA cores (gemv_cluster_f32.cu); norm_width: of the rows that other launches of the step give a norm for
 int launch_gemv_cluster_f32(int device, DeviceState* st, const float* x, const void* Wp, int M, int K, int N, const Epilogue& ep, bool pdl, cudaStream_t s,
-                            const RopeFuse* rope = nullptr, const RowNorm* norm = nullptr);
+                            const RopeFuse* rope = nullptr, const RowNorm* norm = nullptr, int norm_width = 0);
 int64_t gemm_stream_mma_workspace_bytes(int M, int K, int N, int sm_count);
 int gs_take_error();
 // ---- blocks of layered engines (ops_blocks.cu) ---------------------------------------------------------------------------
